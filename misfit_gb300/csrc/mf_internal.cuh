@@ -506,7 +506,7 @@ struct Scratch {
   DBuf<int64_t> hist_scan;
   DBuf<uint64_t> keys_alt;
   DBuf<uint32_t> vals_alt;
-  DBuf<unsigned long long> scan_status;   // look-back scan: 3 words per tile, tagged with scan_seq
+  DBuf<unsigned long long> scan_status;   // look-back scan: {value, tag} per tile, tagged with scan_seq
   unsigned long long scan_seq = 0;
   void release() {
     scan_status.release();

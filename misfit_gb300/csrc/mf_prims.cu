@@ -1,9 +1,7 @@
 // mf_prims.cu -- device scans and a stable LSD radix sort.
 //
 // Scans: one launch.  Small inputs in one block; larger ones with the
-// single-pass decoupled look-back scan (k_scan_lookback).  Tiles are 256
-// threads x 8 items, loaded striped for coalescing and scanned per thread out
-// of shared memory.
+// single-pass decoupled look-back scan (k_scan_lookback, mf_scan.cuh).
 // Radix sort: 8-bit digits, per-tile digit histograms, a scan over the
 // digit-major histogram and a stable scatter that ranks items inside a tile
 // with __match_any_sync.  Stability is what the callers rely on: equal keys
