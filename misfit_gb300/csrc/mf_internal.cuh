@@ -493,27 +493,46 @@ struct Scratch;  // workspace for primitives
 void scan_exclusive_i64(const int64_t* in, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s);
 void scan_exclusive_i32(const int32_t* in, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s);
 void scan_exclusive_u8(const uint8_t* in, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s);
-// Packed scan of the hop-1 marks: high 32 bits count marked vertices, low 32
-// bits marked vertices that are not seed rows (v2i < 0).
 
-// Stable LSD radix sort of (key, value) on key bits [0, bits); result in keys/vals.
-void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, Scratch& ws, cudaStream_t s);
+// Stable LSD radix sort of (key, value) on key bits [first_bit, end_bit) (the
+// bits from end_bit on must be zero).  The result is in the returned arrays: keys/vals themselves, or the workspace's (valid
+// until its next sort).
+struct SortedPairs {
+  uint64_t* keys;
+  uint32_t* vals;
+};
+SortedPairs radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
+                             cudaStream_t s);
+// The same with the result always in keys/vals.
+void radix_sort_pairs_in_place(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
+                               cudaStream_t s);
+// Stable sort on the top `bits` bits (a multiple of 8) of mix_key(key): equal
+// keys end up in one run of equal mixed bits, in input order, with possibly
+// some others between them.
+SortedPairs radix_group_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, Scratch& ws, cudaStream_t s);
+
+// 64-bit finaliser of MurmurHash3 (Appleby, public domain).
+__host__ __device__ __forceinline__ uint64_t mix_key(uint64_t x) {
+  x ^= x >> 33;
+  x *= 0xff51afd7ed558ccdull;
+  x ^= x >> 33;
+  x *= 0xc4ceb9fe1a85ec53ull;
+  x ^= x >> 33;
+  return x;
+}
 
 struct Scratch {
-  DBuf<int64_t> block_sums;
-  DBuf<int64_t> block_sums2;
-  DBuf<int32_t> hist;
-  DBuf<int64_t> hist_scan;
+  DBuf<uint32_t> hist;                    // digit counts of every pass of a sort
+  DBuf<unsigned long long> sort_status;   // sort look-back: 256 words per tile, tagged with sort_seq
+  unsigned long long sort_seq = 0;
   DBuf<uint64_t> keys_alt;
   DBuf<uint32_t> vals_alt;
   DBuf<unsigned long long> scan_status;   // look-back scan: {value, tag} per tile, tagged with scan_seq
   unsigned long long scan_seq = 0;
   void release() {
     scan_status.release();
-    block_sums.release();
-    block_sums2.release();
     hist.release();
-    hist_scan.release();
+    sort_status.release();
     keys_alt.release();
     vals_alt.release();
   }
@@ -726,11 +745,11 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->big_best); f(c->fpos); f(c->work);
   f(c->p2_mask); f(c->p2_filt); f(c->p2_racc); f(c->p2_vol); f(c->p2_tasks); f(c->p2_grp); f(c->p2_huge);
   f(c->p2_cnt);
-  f(c->ws.block_sums); f(c->ws.block_sums2); f(c->ws.hist); f(c->ws.hist_scan); f(c->ws.keys_alt);
+  f(c->ws.hist); f(c->ws.sort_status); f(c->ws.keys_alt);
   f(c->ws.vals_alt); f(c->ws.scan_status);
   for (auto& fr : c->front) {
     f(fr.bits); f(fr.bits_sums); f(fr.uacc); f(fr.hlist); f(fr.cands); f(fr.lb_offs); f(fr.cnt);
-    f(fr.ws.block_sums); f(fr.ws.block_sums2); f(fr.ws.hist); f(fr.ws.hist_scan); f(fr.ws.keys_alt);
+    f(fr.ws.hist); f(fr.ws.sort_status); f(fr.ws.keys_alt);
     f(fr.ws.vals_alt); f(fr.ws.scan_status);
   }
 }

@@ -144,17 +144,29 @@ __global__ void k_init_acnt(const int64_t* aoff, int32_t n, int32_t* acnt) {
 
 enum : int { kStN = 0, kStA = 1, kStR = 2 };
 
-// One thread per run of equal pair keys (the updates of one unordered pair
-// in batch order).  counters[0] = appended entries, counters[1] = killed.
+// The updates of one unordered pair lie in one run of equal mixed key bits, in
+// batch order, seldom with another pair's between them; the thread of the
+// pair's first update walks them.  Two updates are in one run when the top
+// `gbits` of their mixed keys agree.
+__device__ __forceinline__ bool same_run(uint64_t a, uint64_t b, int gbits) {
+  return a == b || ((mix_key(a) ^ mix_key(b)) >> (64 - gbits)) == 0;
+}
+
+// One thread per unordered pair.  counters[0] = appended entries,
+// counters[1] = killed.  app_keys = owner << seq_bits | batch index.
 __global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_t* rcnt, bool sorted,
-                              const uint64_t* keys, const uint32_t* vals, int64_t m, int nbits,
-                              const int32_t* u, const int32_t* v, const uint8_t* ins,
+                              const uint64_t* keys, const uint32_t* vals, int64_t m, int nbits, int gbits,
+                              int seq_bits, const int32_t* u, const int32_t* v, const uint8_t* ins,
                               int32_t* acnt, uint8_t* akill, uint64_t* app_keys, uint32_t* app_vals,
                               int64_t* counters) {
   int64_t j0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j0 >= m) return;
-  if (j0 > 0 && keys[j0 - 1] == keys[j0]) return;  // not the head of a run
   const uint64_t key = keys[j0];
+  for (int64_t j = j0 - 1; j >= 0; --j) {
+    const uint64_t k = keys[j];
+    if (k == key) return;   // not the pair's first update
+    if (!same_run(k, key, gbits)) break;
+  }
   const int32_t a = (int32_t)(key >> nbits);
   const int32_t b = (int32_t)(key & ((1ull << nbits) - 1));
   const int64_t pos_ab = added_find(g, a, b);
@@ -167,7 +179,12 @@ __global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_
   int st = st0;
   bool appended = false, old_killed = false;
   uint32_t last_seq = 0;
-  for (int64_t j = j0; j < m && keys[j] == key; ++j) {
+  for (int64_t j = j0; j < m; ++j) {
+    const uint64_t k = keys[j];
+    if (k != key) {
+      if (!same_run(k, key, gbits)) break;
+      continue;
+    }
     const uint32_t i = vals[j];
     const int32_t x = u[i];
     const bool base_xy = (x == a) ? in_base_ab : in_base_ba;
@@ -202,9 +219,9 @@ __global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_
   }
   if (appended) {
     const unsigned long long slot = atomicAdd((unsigned long long*)counters, 2ull);
-    app_keys[slot] = ((uint64_t)a << 32) | last_seq;
+    app_keys[slot] = ((uint64_t)a << seq_bits) | last_seq;
     app_vals[slot] = (uint32_t)b;
-    app_keys[slot + 1] = ((uint64_t)b << 32) | last_seq;
+    app_keys[slot + 1] = ((uint64_t)b << seq_bits) | last_seq;
     app_vals[slot + 1] = (uint32_t)a;
     atomicAdd(acnt + a, 1);
     atomicAdd(acnt + b, 1);
@@ -224,20 +241,20 @@ __global__ void k_move_survivors(const int64_t* aoff, const int32_t* aadj, const
   nown[pos] = x;
 }
 
-__global__ void k_place_appends(const uint64_t* keys, const uint32_t* vals, int64_t cnt,
+__global__ void k_place_appends(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int seq_bits,
                                 const int64_t* noff, int32_t* nadj, int32_t* nown) {
   int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
-  const uint64_t owner = keys[k] >> 32;
+  const uint64_t owner = keys[k] >> seq_bits;
   int64_t lo = 0, hi = k;  // first index with this owner
   while (lo < hi) {
     int64_t mid = (lo + hi) >> 1;
-    if ((keys[mid] >> 32) < owner) lo = mid + 1; else hi = mid;
+    if ((keys[mid] >> seq_bits) < owner) lo = mid + 1; else hi = mid;
   }
   int64_t lo2 = k + 1, hi2 = cnt;  // one past the last index with this owner
   while (lo2 < hi2) {
     int64_t mid = (lo2 + hi2) >> 1;
-    if ((keys[mid] >> 32) <= owner) lo2 = mid + 1; else hi2 = mid;
+    if ((keys[mid] >> seq_bits) <= owner) lo2 = mid + 1; else hi2 = mid;
   }
   const int32_t x = (int32_t)owner;
   const int64_t pos = noff[x + 1] - (lo2 - lo) + (k - lo);
@@ -523,7 +540,12 @@ void apply_overlay(mf_ctx* c, int64_t m) {
   c->keys.reserve(2 * m);
   c->vals.reserve(2 * m);
   MF_K(k_pair_keys<<<grid_for(m), kTB, 0, s>>>(c->bu.p, c->bv.p, m, nbits, c->keys.p, c->vals.p));
-  radix_sort_pairs(c->keys.p, c->vals.p, m, 2 * nbits, c->ws, s);
+  // grouped on mixed bits, three to eleven more than the line count needs: two
+  // 8-bit digits up to 2^13 lines and three up to 2^21, where the pair itself
+  // has 2 * nbits bits (six digits at 2^22 vertices)
+  const int gbits = std::min(64, (bits_for(m) + 3 + 7) / 8 * 8);
+  const int seq_bits = bits_for(std::max<int64_t>(m - 1, 1));
+  const SortedPairs pairs = radix_group_pairs(c->keys.p, c->vals.p, m, gbits, c->ws, s);
 
   const int64_t cap_new = c->a_total + 2 * m;
   c->akill.reserve(std::max<int64_t>(c->a_total, 1));
@@ -538,7 +560,7 @@ void apply_overlay(mf_ctx* c, int64_t m) {
   MF_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(int64_t) * 2, s));
   MF_K(k_init_acnt<<<grid_for(c->n), kTB, 0, s>>>(c->aoff.p, c->n, c->acnt_new.p));
   MF_K(k_apply_pairs<<<grid_for(m), kTB, 0, s>>>(c->view(), c->live.p, c->dead.p, c->rcnt.p, c->rows_sorted,
-                                            c->keys.p, c->vals.p, m, nbits, c->bu.p, c->bv.p, c->bins.p,
+                                            pairs.keys, pairs.vals, m, nbits, gbits, seq_bits, c->bu.p, c->bv.p, c->bins.p,
                                             c->acnt_new.p, c->akill.p, c->app_keys.p, c->app_vals.p,
                                             c->counters.p));
   MF_CUDA(cudaGetLastError());
@@ -558,8 +580,8 @@ void apply_overlay(mf_ctx* c, int64_t m) {
                                                           c->a_total, c->aoff_alt.p, c->aadj_alt.p, c->aown_alt.p));
   }
   if (appended > 0) {
-    radix_sort_pairs(c->app_keys.p, c->app_vals.p, appended, 32 + nbits, c->ws, s);
-    MF_K(k_place_appends<<<grid_for(appended), kTB, 0, s>>>(c->app_keys.p, c->app_vals.p, appended, c->aoff_alt.p,
+    const SortedPairs app = radix_sort_pairs(c->app_keys.p, c->app_vals.p, appended, 0, seq_bits + nbits, c->ws, s);
+    MF_K(k_place_appends<<<grid_for(appended), kTB, 0, s>>>(app.keys, app.vals, appended, seq_bits, c->aoff_alt.p,
                                                        c->aadj_alt.p, c->aown_alt.p));
   }
   MF_CUDA(cudaGetLastError());

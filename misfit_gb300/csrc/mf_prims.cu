@@ -2,10 +2,14 @@
 //
 // Scans: one launch.  Small inputs in one block; larger ones with the
 // single-pass decoupled look-back scan (k_scan_lookback, mf_scan.cuh).
-// Radix sort: 8-bit digits, per-tile digit histograms, a scan over the
-// digit-major histogram and a stable scatter that ranks items inside a tile
-// with __match_any_sync.  Stability is what the callers rely on: equal keys
-// keep their input (value) order.
+// Radix sort: 8-bit digits, stable (equal keys keep their input order, which
+// is what the callers rely on).  Up to kBlockSortMax pairs the whole sort is one
+// block's work in shared memory (block_sort); longer inputs take one launch
+// per digit, each tile finding its place by a decoupled look-back per digit
+// (Adinets and Merrill, "Onesweep", 2022).
+#include <algorithm>
+#include <atomic>
+
 #include "mf_scan.cuh"
 
 namespace mf {
@@ -16,133 +20,316 @@ using namespace scan_detail;
 
 // ---- radix sort --------------------------------------------------------------
 
-__global__ void k_radix_hist(const uint64_t* keys, int64_t n, int shift, int32_t* hist, int nblocks) {
-  __shared__ int32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-  for (int k = 0; k < kItems; ++k) {
-    const int64_t i = base + (int64_t)k * kThreads + threadIdx.x;
-    if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255u], 1);
-  }
-  __syncthreads();
-  hist[(int64_t)threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+// Sort digits come from the key itself, or from a mixed copy of it when the
+// caller only needs equal keys to end up in one run of equal mixed bits.
+template <bool Mixed>
+__device__ __forceinline__ uint32_t sort_digit(uint64_t key, int shift) {
+  return (uint32_t)((Mixed ? mix_key(key) : key) >> shift) & 255u;
 }
 
-__global__ void k_radix_scatter(const uint64_t* keys, const uint32_t* vals, int64_t n, int shift,
-                                const int64_t* offs, int nblocks, uint64_t* okeys, uint32_t* ovals) {
-  __shared__ int32_t wcnt[kThreads / 32][256];
-  __shared__ int32_t running[256];
-  __shared__ int32_t itotal[256];
-  __shared__ int64_t base_off[256];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  base_off[threadIdx.x] = offs[(int64_t)threadIdx.x * nblocks + blockIdx.x];
-  running[threadIdx.x] = 0;
+constexpr int kDigits = 256;
+
+// Rank of each of the warp's items among the warp's items of the same digit
+// (in item order), and the digit counts of the warp (cnt[256], zeroed here).
+// A thread's items are at warp base + r * 32 + lane.
+template <int Items>
+__device__ __forceinline__ void warp_rank(const uint32_t (&d)[Items], int (&rank)[Items], uint32_t* cnt) {
+  const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  const int64_t base = (int64_t)blockIdx.x * kTile;
-  for (int k = 0; k < kItems; ++k) {
-    for (int j = 0; j < kThreads / 32; ++j) wcnt[j][threadIdx.x] = 0;
-    __syncthreads();
-    const int64_t i = base + (int64_t)k * kThreads + threadIdx.x;
-    const bool valid = i < n;
-    uint64_t key = 0;
-    uint32_t val = 0;
-    int d = 256;
-    if (valid) {
-      key = keys[i];
-      val = vals[i];
-      d = (int)((key >> shift) & 255u);
+#pragma unroll
+  for (int j = 0; j < kDigits / 32; ++j) cnt[lane + 32 * j] = 0;
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    const unsigned peers = __match_any_sync(0xffffffffu, d[r]);
+    const int lead = __ffs(peers) - 1;
+    int old = 0;
+    if (lane == lead) {
+      old = (int)cnt[d[r]];
+      cnt[d[r]] = (uint32_t)(old + __popc(peers));
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int rank = __popc(peers & lt);
-    if (valid && rank == 0) wcnt[w][d] = __popc(peers);
-    __syncthreads();
-    {
-      int acc = 0;
-      for (int j = 0; j < kThreads / 32; ++j) {
-        const int t = wcnt[j][threadIdx.x];
-        wcnt[j][threadIdx.x] = acc;
-        acc += t;
-      }
-      itotal[threadIdx.x] = acc;
-    }
-    __syncthreads();
-    if (valid) {
-      const int64_t pos = base_off[d] + running[d] + wcnt[w][d] + rank;
-      okeys[pos] = key;
-      ovals[pos] = val;
-    }
-    __syncthreads();
-    running[threadIdx.x] += itotal[threadIdx.x];
-    __syncthreads();
+    rank[r] = __shfl_sync(0xffffffffu, old, lead) + __popc(peers & lt);
+    __syncwarp();
   }
 }
 
-// Whole stable LSD sort of up to kSmallSort pairs in one block: every 8-bit
-// pass ranks the items with per-warp match_any counts, in shared memory.
-constexpr int kSmallSort = 1024;
+// Thread d < 256: the warps' counts of digit d become exclusive prefixes over
+// the warps; returns the digit's total.
+__device__ __forceinline__ uint32_t digit_columns(uint32_t* cnt, int warps) {
+  uint32_t acc = 0;
+#pragma unroll 8
+  for (int j = 0; j < warps; ++j) {
+    const uint32_t t = cnt[j * kDigits + threadIdx.x];
+    cnt[j * kDigits + threadIdx.x] = acc;
+    acc += t;
+  }
+  return acc;
+}
 
-__global__ void __launch_bounds__(kThreads) k_radix_small(uint64_t* keys, uint32_t* vals, int n, int bits) {
-  __shared__ uint64_t sk[2][kSmallSort];
-  __shared__ uint32_t sv[2][kSmallSort];
-  __shared__ int32_t wcnt[kThreads / 32][256];
-  __shared__ int32_t dbase[256];
-  __shared__ int32_t itotal[256];
+// Exclusive scan over the 256 digits, by the first eight warps (every thread
+// of the block calls it; the others pass anything).
+__device__ __forceinline__ uint32_t digit_scan(uint32_t total, uint32_t* sw) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    sk[0][i] = keys[i];
-    sv[0][i] = vals[i];
+  uint32_t inc = total;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31 && w < kDigits / 32) sw[w] = inc;
+  __syncthreads();
+  uint32_t before = 0;
+  for (int j = 0; j < w && j < kDigits / 32; ++j) before += sw[j];
+  return before + inc - total;
+}
+
+// One block sorts up to Items * blockDim.x pairs held in registers: one pass
+// per digit ranks them (warp_rank) and moves them through shared memory.
+// Positions from n on are padding: their digit counts as 255 and they come
+// last in item order, so they stay behind every pair.
+template <int Items, bool Mixed>
+__device__ void block_sort(uint64_t (&key)[Items], uint32_t (&val)[Items], int n, int first_bit, int end_bit,
+                           uint64_t* sk, uint32_t* sv, uint32_t* cnt, uint32_t* dbase, uint32_t* sw) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int at = w * 32 * Items + lane;
+  for (int shift = first_bit; shift < end_bit; shift += 8) {
+    uint32_t d[Items];
+    int rank[Items];
+#pragma unroll
+    for (int r = 0; r < Items; ++r) d[r] = at + r * 32 < n ? sort_digit<Mixed>(key[r], shift) : 255u;
+    warp_rank<Items>(d, rank, cnt + w * kDigits);
+    __syncthreads();
+    uint32_t total = 0;
+    if (threadIdx.x < kDigits) total = digit_columns(cnt, warps);
+    const uint32_t base = digit_scan(total, sw);
+    if (threadIdx.x < kDigits) dbase[threadIdx.x] = base;
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      const uint32_t pos = dbase[d[r]] + cnt[w * kDigits + d[r]] + (uint32_t)rank[r];
+      sk[pos] = key[r];
+      sv[pos] = val[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      key[r] = sk[at + r * 32];
+      val[r] = sv[at + r * 32];
+    }
+    __syncthreads();
+  }
+}
+
+template <int Items, bool Mixed>
+__global__ void __launch_bounds__(1024) k_sort_block(uint64_t* keys, uint32_t* vals, int n, int first_bit,
+                                                     int end_bit) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  __shared__ uint32_t dbase[kDigits];
+  __shared__ uint32_t sw[kDigits / 32];
+  const int cap = Items * (int)blockDim.x;
+  uint64_t* sk = reinterpret_cast<uint64_t*>(sort_smem);
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + cap);
+  uint32_t* cnt = sv + cap;
+  const int at = (threadIdx.x >> 5) * 32 * Items + (threadIdx.x & 31);
+  uint64_t key[Items];
+  uint32_t val[Items];
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    key[r] = at + r * 32 < n ? keys[at + r * 32] : 0;
+    val[r] = at + r * 32 < n ? vals[at + r * 32] : 0;
+  }
+  block_sort<Items, Mixed>(key, val, n, first_bit, end_bit, sk, sv, cnt, dbase, sw);
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    if (at + r * 32 < n) {
+      keys[at + r * 32] = key[r];
+      vals[at + r * 32] = val[r];
+    }
+  }
+}
+
+// Registers bound one block: eight 12-byte pairs, their digits and ranks in the
+// 64 registers a thread of a 1,024-thread block has.
+constexpr int kBlockSortMax = 8192;
+
+template <int Items, bool Mixed>
+void sort_block(uint64_t* keys, uint32_t* vals, int n, int threads, int first_bit, int end_bit, cudaStream_t s) {
+  const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * kDigits * 4;
+  if (smem > 48 * 1024) {
+    // raised once per device for this kernel
+    static std::atomic<unsigned long long> raised{0};
+    int dev = 0;
+    MF_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (dev > 63 || !(raised.load(std::memory_order_acquire) & bit)) {
+      MF_CUDA(cudaFuncSetAttribute(k_sort_block<Items, Mixed>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   Items * 1024 * 12 + 32 * kDigits * 4));
+      raised.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  MF_K(launch_pdl(k_sort_block<Items, Mixed>, 1, (unsigned)threads, smem, s, keys, vals, n, first_bit, end_bit));
+}
+
+// Digit counts of every pass over the whole input (hist zeroed before).
+constexpr int kMaxPasses = 8;
+
+template <bool Mixed>
+__global__ void __launch_bounds__(kThreads) k_sort_hist(const uint64_t* keys, int64_t n, int first_bit, int passes,
+                                                        uint32_t* hist) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ uint32_t h[kMaxPasses * kDigits];
+  for (int i = threadIdx.x; i < passes * kDigits; i += blockDim.x) h[i] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = Mixed ? mix_key(keys[i]) : keys[i];
+    for (int p = 0; p < passes; ++p) atomicAdd(&h[p * kDigits + ((k >> (first_bit + 8 * p)) & 255u)], 1u);
   }
   __syncthreads();
-  int cur = 0;
-  for (int shift = 0; shift < bits; shift += 8) {
-    // digit histogram -> exclusive digit bases
-    dbase[threadIdx.x] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kThreads) atomicAdd(&dbase[(sk[cur][i] >> shift) & 255u], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int acc = 0;
-      for (int d = 0; d < 256; ++d) { const int t = dbase[d]; dbase[d] = acc; acc += t; }
-    }
-    __syncthreads();
-    for (int base = 0; base < n; base += kThreads) {
-      for (int j = 0; j < kThreads / 32; ++j) wcnt[j][threadIdx.x] = 0;
-      __syncthreads();
-      const int i = base + threadIdx.x;
-      const bool valid = i < n;
-      int d = 256;
-      if (valid) d = (int)((sk[cur][i] >> shift) & 255u);
-      const unsigned peers = __match_any_sync(0xffffffffu, d);
-      const int rank = __popc(peers & lt);
-      if (valid && rank == 0) wcnt[w][d] = __popc(peers);
-      __syncthreads();
-      {
-        int acc = 0;
-        for (int j = 0; j < kThreads / 32; ++j) {
-          const int t = wcnt[j][threadIdx.x];
-          wcnt[j][threadIdx.x] = acc;
-          acc += t;
-        }
-        itotal[threadIdx.x] = acc;
-      }
-      __syncthreads();
-      if (valid) {
-        const int pos = dbase[d] + wcnt[w][d] + rank;
-        sk[cur ^ 1][pos] = sk[cur][i];
-        sv[cur ^ 1][pos] = sv[cur][i];
-      }
-      __syncthreads();
-      dbase[threadIdx.x] += itotal[threadIdx.x];
-      __syncthreads();
-    }
-    cur ^= 1;
+  for (int i = threadIdx.x; i < passes * kDigits; i += blockDim.x)
+    if (h[i]) atomicAdd(hist + i, h[i]);
+}
+
+// One digit of the sort: tiles of 256 threads x 8 items.  A tile ranks its
+// items, publishes its digit counts and sums its predecessors' (thread d looks
+// back for digit d, eight tiles' words in flight), then writes its pairs out in
+// digit runs.  Status word: seq << 34 | flag << 32 | count (flag 1: the tile's
+// count, 2: the count up to and including the tile); `seq` is new for every
+// pass, so the words are never reset.  A wait gives up after kLookbackSpin
+// reads, and the thread then counts its digit over all earlier items itself.
+//
+// A pass over 200,000 pairs moves 4.8 MB; what bounds it is latency (two loads,
+// the ranking, the look-back, the store).  It replaces three launches (digit
+// histogram, scan, scatter) of 19 us together at 2,000-4,000 pairs.
+template <bool Mixed>
+__global__ void __launch_bounds__(kThreads) k_sort_pass(const uint64_t* keys, const uint32_t* vals, int64_t n, int shift,
+                                                        const uint32_t* hist, unsigned long long* status,
+                                                        unsigned long long seq, uint64_t* okeys, uint32_t* ovals) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ uint64_t sk[kTile];
+  __shared__ uint32_t sv[kTile];
+  __shared__ uint32_t cnt[(kThreads / 32) * kDigits];
+  __shared__ uint32_t dbase[kDigits];
+  __shared__ int64_t gofs[kDigits];
+  __shared__ uint32_t sw[kDigits / 32];
+  __shared__ uint32_t sw2[kDigits / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t t = blockIdx.x;
+  const int64_t base = t * kTile;
+  const int cap = (int)min((int64_t)kTile, n - base);
+  const int at = w * 32 * kItems + lane;
+  uint64_t key[kItems];
+  uint32_t val[kItems];
+  uint32_t d[kItems];
+  int rank[kItems];
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const bool ok = at + r * 32 < cap;
+    key[r] = ok ? keys[base + at + r * 32] : 0;
+    val[r] = ok ? vals[base + at + r * 32] : 0;
   }
-  for (int i = threadIdx.x; i < n; i += kThreads) {
-    keys[i] = sk[cur][i];
-    vals[i] = sv[cur][i];
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) d[r] = at + r * 32 < cap ? sort_digit<Mixed>(key[r], shift) : 255u;
+  warp_rank<kItems>(d, rank, cnt + w * kDigits);
+  __syncthreads();
+  const uint32_t padded = digit_columns(cnt, kThreads / 32);
+  // the padding sits in digit 255
+  const uint32_t mine = threadIdx.x == 255 ? padded - (uint32_t)(kTile - cap) : padded;
+  unsigned long long* my = status + t * kDigits + threadIdx.x;
+  *(volatile unsigned long long*)my = (seq << 34) | (t == 0 ? 2ull << 32 : 1ull << 32) | mine;
+  const uint32_t local = digit_scan(padded, sw);
+  dbase[threadIdx.x] = local;
+  const uint32_t global = digit_scan(hist[threadIdx.x], sw2);
+  int64_t excl = 0;
+  bool found = t == 0, lost = false;
+  for (int64_t q = t - 1; q >= 0 && !found && !lost; q -= 8) {
+    unsigned long long x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      x[j] = q - j >= 0 ? *(volatile const unsigned long long*)(status + (q - j) * kDigits + threadIdx.x) : 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (found || lost || q - j < 0) continue;
+      int64_t spins = 0;
+      while ((x[j] >> 34) != seq && ++spins < kLookbackSpin)
+        x[j] = *(volatile const unsigned long long*)(status + (q - j) * kDigits + threadIdx.x);
+      if ((x[j] >> 34) != seq) {
+        lost = true;
+        continue;
+      }
+      excl += (int64_t)(x[j] & 0xffffffffull);
+      found = ((x[j] >> 32) & 3ull) == 2ull;
+    }
   }
+  if (lost) {
+    excl = 0;
+    for (int64_t i = 0; i < base; ++i) excl += sort_digit<Mixed>(keys[i], shift) == threadIdx.x;
+  }
+  if (t > 0) *(volatile unsigned long long*)my = (seq << 34) | (2ull << 32) | (unsigned long long)(excl + mine);
+  gofs[threadIdx.x] = (int64_t)global + excl - (int64_t)local;
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    if (r == 0) __syncthreads();
+    const uint32_t pos = dbase[d[r]] + cnt[w * kDigits + d[r]] + (uint32_t)rank[r];
+    sk[pos] = key[r];
+    sv[pos] = val[r];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < kItems; ++r) {
+    const int i = r * kThreads + threadIdx.x;
+    if (i < cap) {
+      const uint64_t k = sk[i];
+      const int64_t pos = gofs[sort_digit<Mixed>(k, shift)] + i;
+      okeys[pos] = k;
+      ovals[pos] = sv[i];
+    }
+  }
+}
+
+template <bool Mixed>
+SortedPairs sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
+                       cudaStream_t s) {
+  if (n <= 1) return {keys, vals};
+  if (n <= kBlockSortMax) {
+    // one to eight items a thread; 256 threads at least, one per digit
+    if (n <= 256) sort_block<1, Mixed>(keys, vals, (int)n, 256, first_bit, end_bit, s);
+    else if (n <= 1024) sort_block<1, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
+    else if (n <= 2048) sort_block<2, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
+    else if (n <= 4096) sort_block<4, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
+    else sort_block<8, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
+    MF_CUDA(cudaGetLastError());
+    return {keys, vals};
+  }
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  const int passes = (end_bit - first_bit + 7) / 8;
+  ws.keys_alt.reserve(n);
+  ws.vals_alt.reserve(n);
+  ws.hist.reserve(kMaxPasses * kDigits);
+  if (ws.sort_status.cap < tiles * kDigits) {
+    ws.sort_status.reserve(tiles * kDigits);
+    // fresh memory may hold anything: no tag may match a later sequence number
+    MF_CUDA(cudaMemsetAsync(ws.sort_status.p, 0, sizeof(unsigned long long) * (size_t)ws.sort_status.cap, s));
+    ws.sort_seq = 0;
+  }
+  if (ws.sort_seq + kMaxPasses >= (1ull << 30)) {   // the tag's 30 bits are used up
+    MF_CUDA(cudaMemsetAsync(ws.sort_status.p, 0, sizeof(unsigned long long) * (size_t)ws.sort_status.cap, s));
+    ws.sort_seq = 0;
+  }
+  MF_CUDA(cudaMemsetAsync(ws.hist.p, 0, sizeof(uint32_t) * (size_t)passes * kDigits, s));
+  MF_K(launch_pdl(k_sort_hist<Mixed>, (unsigned)std::min<int64_t>(tiles, 304), kThreads, 0, s, keys, n, first_bit, passes,
+                  ws.hist.p));
+  SortedPairs a{keys, vals}, b{ws.keys_alt.p, ws.vals_alt.p};
+  for (int pass = 0; pass < passes; ++pass) {
+    const unsigned long long seq = ++ws.sort_seq;
+    MF_K(launch_pdl(k_sort_pass<Mixed>, (unsigned)tiles, kThreads, 0, s, a.keys, a.vals, n, first_bit + 8 * pass,
+                    ws.hist.p + pass * kDigits, ws.sort_status.p, seq, b.keys, b.vals));
+    std::swap(a, b);
+  }
+  MF_CUDA(cudaGetLastError());
+  return a;
 }
 
 }  // namespace
@@ -163,36 +350,22 @@ void scan_exclusive_u8(const uint8_t* in, int64_t* out, int64_t n, Scratch& ws, 
   scan_exclusive(Loader<uint8_t>{in}, out, n, ws, s);
 }
 
-void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, Scratch& ws, cudaStream_t s) {
-  if (n <= 1) return;
-  if (n <= kSmallSort) {
-    MF_K(k_radix_small<<<1, kThreads, 0, s>>>(keys, vals, (int)n, bits));
-    MF_CUDA(cudaGetLastError());
-    return;
+SortedPairs radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
+                             cudaStream_t s) {
+  return sort_pairs<false>(keys, vals, n, first_bit, end_bit, ws, s);
+}
+
+void radix_sort_pairs_in_place(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
+                               cudaStream_t s) {
+  const SortedPairs r = radix_sort_pairs(keys, vals, n, first_bit, end_bit, ws, s);
+  if (r.keys != keys) {
+    MF_CUDA(cudaMemcpyAsync(keys, r.keys, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
+    MF_CUDA(cudaMemcpyAsync(vals, r.vals, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
   }
-  const int nblocks = (int)((n + kTile - 1) / kTile);
-  ws.keys_alt.reserve(n);
-  ws.vals_alt.reserve(n);
-  ws.hist.reserve((int64_t)256 * nblocks);
-  ws.hist_scan.reserve((int64_t)256 * nblocks + 1);
-  uint64_t* ka = keys;
-  uint32_t* va = vals;
-  uint64_t* kb = ws.keys_alt.p;
-  uint32_t* vb = ws.vals_alt.p;
-  const int passes = (bits + 7) / 8;
-  for (int pass = 0; pass < passes; ++pass) {
-    const int shift = pass * 8;
-    MF_K(k_radix_hist<<<nblocks, kThreads, 0, s>>>(ka, n, shift, ws.hist.p, nblocks));
-    scan_exclusive_i32(ws.hist.p, ws.hist_scan.p, (int64_t)256 * nblocks, ws, s);
-    MF_K(k_radix_scatter<<<nblocks, kThreads, 0, s>>>(ka, va, n, shift, ws.hist_scan.p, nblocks, kb, vb));
-    MF_CUDA(cudaGetLastError());
-    uint64_t* tk = ka; ka = kb; kb = tk;
-    uint32_t* tv = va; va = vb; vb = tv;
-  }
-  if (ka != keys) {
-    MF_CUDA(cudaMemcpyAsync(keys, ka, sizeof(uint64_t) * n, cudaMemcpyDeviceToDevice, s));
-    MF_CUDA(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-  }
+}
+
+SortedPairs radix_group_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, Scratch& ws, cudaStream_t s) {
+  return sort_pairs<true>(keys, vals, n, 64 - bits, 64, ws, s);
 }
 
 }  // namespace mf

@@ -63,20 +63,22 @@ __device__ __forceinline__ int64_t warp_id() {
 
 // ---- split ------------------------------------------------------------------
 
-__global__ void k_slot_keys(const int32_t* u, const int32_t* v, int64_t m, int sbits, uint64_t* keys, uint32_t* vals) {
+// Endpoint slots (2j: source, 2j + 1: destination of line j) keyed by their
+// vertex; the sort is stable, so each vertex's slots stay in slot order.
+__global__ void k_slot_keys(const int32_t* u, const int32_t* v, int64_t m, uint64_t* keys, uint32_t* vals) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * m) return;
   const int32_t x = (i & 1) ? v[i >> 1] : u[i >> 1];
-  keys[i] = ((uint64_t)x << sbits) | (uint64_t)i;
+  keys[i] = (uint64_t)(uint32_t)x;
   vals[i] = (uint32_t)i;
 }
 
-__global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int sbits, int32_t* prev) {
+__global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int32_t* prev) {
   int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= cnt) return;
   const uint32_t slot = vals[j];
   int32_t pe = -1;
-  if (j > 0 && (keys[j - 1] >> sbits) == (keys[j] >> sbits)) pe = (int32_t)(vals[j - 1] >> 1);
+  if (j > 0 && keys[j - 1] == keys[j]) pe = (int32_t)(vals[j - 1] >> 1);
   prev[slot] = pe;
 }
 
@@ -1854,7 +1856,7 @@ __global__ void k_finalize_all(const uint32_t* wval, int32_t n, uint32_t epoch, 
 // The cluster count (*ccp, the new-id scan total) comes from the device; ids
 // at or beyond min(cluster_count, MAX_BATCH_SIZE) are dropped.
 __global__ void k_assign(const int32_t* u, const int32_t* v, int64_t p, int64_t len, const int32_t* cid,
-                         const int64_t* ccp, uint64_t* keys, uint32_t* vals, unsigned long long* count) {
+                         const int64_t* ccp, int tbits, uint64_t* keys, uint32_t* vals, unsigned long long* count) {
   pdl_wait();
   pdl_trigger();
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1865,7 +1867,7 @@ __global__ void k_assign(const int32_t* u, const int32_t* v, int64_t p, int64_t 
   if (c == -1) c = cid[v[j]];
   if (c < 0 || (int64_t)c >= limit) return;
   const unsigned long long k = atomicAdd(count, 1ull);
-  keys[k] = ((uint64_t)c << kRowBits) | (uint64_t)(kRowMask - (uint32_t)t);
+  keys[k] = ((uint64_t)c << tbits) | (uint64_t)(((1u << tbits) - 1u) - (uint32_t)t);
   vals[k] = (uint32_t)t;
 }
 
@@ -3508,7 +3510,8 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
       dbg_chunks += tot;
       dbg_scanned += (int64_t)q[3];
     }
-    radix_sort_pairs(c->rp_keys2.p, c->rp_vals2.p, nk, 32 + nbits, c->ws, s);
+    // the writes are in position order already: a stable sort on the vertex
+    radix_sort_pairs_in_place(c->rp_keys2.p, c->rp_vals2.p, nk, 32, 32 + nbits, c->ws, s);
     if (nview > 0) MF_K(k_spec_clear_flags<<<grid_for(nview), kTB, 0, s>>>(c->rp_keys.p, nview, c->mis.p));
     const uint64_t last = (uint64_t)std::min<int64_t>(f, nproc - 1);
     if (nk > 0) MF_K(k_spec_commit<<<grid_for(nk), kTB, 0, s>>>(c->rp_keys2.p, c->rp_vals2.p, nk, last, c->mis.p));
@@ -3547,16 +3550,15 @@ void process_batch(mf_ctx* c, int64_t m) {
 
   if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
   // previous occurrence of every endpoint slot (for "not seen in this sub-batch")
-  const int sbits = bits_for(std::max<int64_t>(2 * m - 1, 1));
   const int nbits = bits_for(std::max<int32_t>(n - 1, 1));
   c->keys.reserve(2 * m);
   c->vals.reserve(2 * m);
   c->prev.reserve(2 * m);
   std::optional<StageScope> sc;
   sc.emplace(c, kStSplit);
-  MF_K(k_slot_keys<<<grid_for(2 * m), kTB, 0, s>>>(c->bu.p, c->bv.p, m, sbits, c->keys.p, c->vals.p));
-  radix_sort_pairs(c->keys.p, c->vals.p, 2 * m, sbits + nbits, c->ws, s);
-  MF_K(k_prev<<<grid_for(2 * m), kTB, 0, s>>>(c->keys.p, c->vals.p, 2 * m, sbits, c->prev.p));
+  MF_K(k_slot_keys<<<grid_for(2 * m), kTB, 0, s>>>(c->bu.p, c->bv.p, m, c->keys.p, c->vals.p));
+  const SortedPairs slots = radix_sort_pairs(c->keys.p, c->vals.p, 2 * m, 0, nbits, c->ws, s);
+  MF_K(k_prev<<<grid_for(2 * m), kTB, 0, s>>>(slots.keys, slots.vals, 2 * m, c->prev.p));
   MF_CUDA(cudaGetLastError());
   sc.reset();
 
@@ -3872,15 +3874,17 @@ void process_batch(mf_ctx* c, int64_t m) {
 
     // ---- assignment + order (cluster ascending, index descending)
     sc.emplace(c, kStAssign);
-    MF_K(launch_pdl(k_assign, grid_for(q - p), kTB, 0, s, c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows, c->keys.p,
-                                                  c->vals.p, ucnt + 55));
+    const int tbits = bits_for(std::max<int64_t>(q - p - 1, 1));   // the sub-batch index of an edge
+    MF_K(launch_pdl(k_assign, grid_for(q - p), kTB, 0, s, c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows, tbits,
+                    c->keys.p, c->vals.p, ucnt + 55));
     MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
     const int64_t cc = h[7];
     const int64_t limit = std::min<int64_t>(cc, kMaxBatchEdges);
     const int64_t nproc = h[9];
     if (tr) tr->hdr[6] = cc;
-    radix_sort_pairs(c->keys.p, c->vals.p, nproc, kRowBits + bits_for(std::max<int64_t>(limit, 1)), c->ws, s);
+    radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, tbits + bits_for(std::max<int64_t>(limit, 1)), c->ws,
+                              s);
 
     // ---- repair (times itself: rounds vs grid-wide searches)
     sc.reset();

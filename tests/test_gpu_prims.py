@@ -36,3 +36,35 @@ def test_line_scan_at_tile_edges(gb, lines, tmp_path):
         gu, gv, ins = g.parse_batch_file(path)
         assert np.array_equal(ins, g.flag_updates(gu, gv))
     assert np.array_equal(gu, u[keep] - 1) and np.array_equal(gv, v[keep] - 1)
+
+
+# one block sorts 256 / 1,024 / 2,048 / 4,096 / 8,192 pairs, longer inputs take 2,048-pair tiles; a batch of m lines
+# sorts m pairs, its 2m endpoint slots and its appended entries
+@pytest.mark.parametrize("m", [1, 2, 128, 129, 256, 257, 512, 513, 1024, 1025, 2048, 2049, 4096, 4097, 8192, 8193, 16385])
+def test_batch_sorts_at_block_edges(gb, m):
+    """Pairs repeated within the batch (grouping in batch order), vertices repeated (previous occurrence, order of
+    appended entries), free flags: rows, degrees, membership and cluster ids equal the oracle's."""
+    import oracle as O
+    n = 3000
+    nindex, nlist = W.er_graph(n, 6, 2)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    rng = np.random.default_rng(m)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        g.set_mis(mis)
+        orc.set_mis(mis)
+        for _ in range(2):
+            u = rng.integers(0, n, m)
+            hot = rng.random(m) < 0.3
+            u[hot] = rng.integers(0, 3, hot.sum())
+            v = (u + 1 + rng.integers(0, np.where(hot, 40, n - 1))) % n
+            flip = rng.random(m) < 0.5
+            u, v = np.where(flip, v, u).astype(np.int32), np.where(flip, u, v).astype(np.int32)
+            ins = rng.integers(0, 2, m).astype(np.uint8)
+            orc.apply_batch(u, v, ins)
+            g.apply_batch(u, v, ins)
+            assert np.array_equal(g.degrees(), orc.degrees())
+            for x in np.unique(np.concatenate([u, v]))[:300]:
+                assert np.array_equal(g.row(int(x)), orc.row(int(x))), x
+            assert np.array_equal(g.get_mis(), orc.get_mis())
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
