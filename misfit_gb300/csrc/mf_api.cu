@@ -144,7 +144,8 @@ void need(bool cond, int status, const char* msg) {
 void release_all(mf_ctx* c) {
   mf::release_device_state(c);
   if (c->h_counters) cudaFreeHost(c->h_counters);
-  c->h_counters = nullptr;
+  c->h_counters = c->h_plan = nullptr;
+  c->h_stage = nullptr;
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   c->ev_pool.clear();
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -191,7 +192,10 @@ mf_ctx* new_ctx(int gpu) {
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_a, cudaEventDisableTiming));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_b, cudaEventDisableTiming));
     mf::note_alloc();
-    MF_CUDA(cudaMallocHost(&c->h_counters, sizeof(int64_t) * 64));
+    // one pinned block: 64 counter words, the batch plan, a small batch's lines
+    MF_CUDA(cudaMallocHost(&c->h_counters, sizeof(int64_t) * (64 + mf::kPlanWords) + 9 * (size_t)mf::kSmallBatch));
+    c->h_plan = c->h_counters + 64;
+    c->h_stage = reinterpret_cast<uint8_t*>(c->h_plan + mf::kPlanWords);
     c->counters.reserve(64);
   } catch (...) {
     release_all(c);
@@ -212,26 +216,22 @@ void bind(const mf_ctx* c) {
   mf::g_alloc_stream = c->stream;
 }
 
-// Inputs of a batch are already in c->bu / c->bv / c->bins.
-void run_batch(mf_ctx* c, int64_t m) {
+// One batch of m lines.  Invalid lines fail it before anything changes.
+void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
-  c->stats = mf_batch_stats{};
-  c->stats.updates = m;
-  c->stats.packed_total = -1;
-  c->stats.row_degree_total = -1;
-  c->traces.clear();
-  c->work.reserve(2 * mf::kStCount + 8);
+  c->work.reserve(mf::kWorkWords);
   c->touched_total = 0;
   c->pull_runs = 0;
-  MF_CUDA(cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long) * (2 * mf::kStCount + 8), s));
+  MF_CUDA(cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long) * mf::kWorkWords, s));
   MF_CUDA(cudaEventRecord(c->ev0, s));
   if (m > 0) {
-    {
-      mf::StageScope sc(c, mf::kStOverlay);
-      mf::apply_overlay(c, m);
-    }
-    mf::process_batch(c, m);
+    mf::process_batch(c, in, m);
     if (c->exact) mf::exact_fixup(c);
+  } else {
+    c->stats = mf_batch_stats{};
+    c->stats.packed_total = -1;
+    c->stats.row_degree_total = -1;
+    c->traces.clear();
   }
   MF_CUDA(cudaEventRecord(c->ev1, s));
   MF_CUDA(cudaEventSynchronize(c->ev1));
@@ -295,16 +295,40 @@ __global__ void k_validate(const int32_t* u, const int32_t* v, int64_t m, int32_
   if (a < 0 || a >= n || b < 0 || b >= n || a == b) atomicAdd(bad, 1ull);
 }
 
-void stage_inputs(mf_ctx* c, const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t m,
-                  cudaMemcpyKind kind) {
+// Host lines of a batch where the device can read them: a small batch in the
+// context's pinned block (no copy is queued; the caller's call runs to the
+// end of the batch before the block is used again), a larger one copied.
+mf::BatchIn host_input(mf_ctx* c, const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t m) {
+  cudaStream_t s = c->stream;
+  if (m <= mf::kSmallBatch) {
+    int32_t* hu = reinterpret_cast<int32_t*>(c->h_stage);
+    int32_t* hv = hu + mf::kSmallBatch;
+    uint8_t* hi = reinterpret_cast<uint8_t*>(hv + mf::kSmallBatch);
+    if (m > 0) {
+      std::memcpy(hu, u, sizeof(int32_t) * (size_t)m);
+      std::memcpy(hv, v, sizeof(int32_t) * (size_t)m);
+      std::memcpy(hi, ins, (size_t)m);
+    }
+    return {hu, hv, hi};
+  }
+  c->bu.reserve(m);
+  c->bv.reserve(m);
+  c->bins.reserve(m);
+  MF_CUDA(cudaMemcpyAsync(c->bu.p, u, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
+  MF_CUDA(cudaMemcpyAsync(c->bv.p, v, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
+  MF_CUDA(cudaMemcpyAsync(c->bins.p, ins, (size_t)m, cudaMemcpyHostToDevice, s));
+  return {c->bu.p, c->bv.p, c->bins.p};
+}
+
+// The pairs of a flag query into c->bu / c->bv, checked.
+void stage_pairs(mf_ctx* c, const int32_t* u, const int32_t* v, int64_t m) {
   cudaStream_t s = c->stream;
   c->bu.reserve(m);
   c->bv.reserve(m);
   c->bins.reserve(m);
   if (m == 0) return;
-  MF_CUDA(cudaMemcpyAsync(c->bu.p, u, sizeof(int32_t) * (size_t)m, kind, s));
-  MF_CUDA(cudaMemcpyAsync(c->bv.p, v, sizeof(int32_t) * (size_t)m, kind, s));
-  if (ins) MF_CUDA(cudaMemcpyAsync(c->bins.p, ins, (size_t)m, kind, s));
+  MF_CUDA(cudaMemcpyAsync(c->bu.p, u, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
+  MF_CUDA(cudaMemcpyAsync(c->bv.p, v, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
   MF_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(int64_t), s));
   MF_K(k_validate<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(c->bu.p, c->bv.p, m, c->n,
                                                           reinterpret_cast<unsigned long long*>(c->counters.p)));
@@ -367,8 +391,7 @@ void async_worker(mf_ctx* c) {
     }
     const int st = guarded([&] {
       mf::bind_device(c);
-      stage_inputs(c, j->u, j->v, j->ins, j->m, cudaMemcpyHostToDevice);
-      run_batch(c, j->m);
+      run_batch(c, host_input(c, j->u, j->v, j->ins, j->m), j->m);
     });
     {
       std::lock_guard<std::mutex> lk(q.mu);
@@ -704,7 +727,7 @@ int mf_flag_updates(mf_ctx* c, const int32_t* u, const int32_t* v, int64_t m, ui
   return guarded([&] {
     need(c && m >= 0 && (m == 0 || (u && v && ins_out)), MF_EINVAL, "bad arguments");
     bind(c);
-    stage_inputs(c, u, v, nullptr, m, cudaMemcpyHostToDevice);
+    stage_pairs(c, u, v, m);
     mf::flag_updates(c, m);
     if (m > 0) MF_CUDA(cudaMemcpyAsync(ins_out, c->bins.p, (size_t)m, cudaMemcpyDeviceToHost, c->stream));
     MF_CUDA(cudaStreamSynchronize(c->stream));
@@ -724,8 +747,7 @@ int mf_apply_batch(mf_ctx* c, const int32_t* u, const int32_t* v, const uint8_t*
     need(c && m >= 0 && (m == 0 || (u && v && ins)), MF_EINVAL, "bad arguments");
     need(!c->pending, MF_EINVAL, "asynchronous batches are pending; collect them (mf_collect / mf_sync) first");
     bind(c);
-    stage_inputs(c, u, v, ins, m, cudaMemcpyHostToDevice);
-    run_batch(c, m);
+    run_batch(c, host_input(c, u, v, ins, m), m);
   });
 }
 
@@ -734,8 +756,7 @@ int mf_apply_batch_device(mf_ctx* c, const int32_t* d_u, const int32_t* d_v, con
     need(c && m >= 0 && (m == 0 || (d_u && d_v && d_ins)), MF_EINVAL, "bad arguments");
     need(!c->pending, MF_EINVAL, "asynchronous batches are pending; collect them (mf_collect / mf_sync) first");
     bind(c);
-    stage_inputs(c, d_u, d_v, d_ins, m, cudaMemcpyDeviceToDevice);
-    run_batch(c, m);
+    run_batch(c, mf::BatchIn{d_u, d_v, d_ins}, m);
   });
 }
 
@@ -865,7 +886,7 @@ int mf_is_adjacent(mf_ctx* c, int32_t u, int32_t v, int* adjacent) {
     need(c && adjacent && u >= 0 && v >= 0 && u < c->n && v < c->n, MF_EINVAL, "bad arguments");
     bind(c);
     uint8_t ins = 0;
-    stage_inputs(c, &u, &v, nullptr, 1, cudaMemcpyHostToDevice);
+    stage_pairs(c, &u, &v, 1);
     mf::flag_updates(c, 1);
     MF_CUDA(cudaMemcpyAsync(&ins, c->bins.p, 1, cudaMemcpyDeviceToHost, c->stream));
     MF_CUDA(cudaStreamSynchronize(c->stream));

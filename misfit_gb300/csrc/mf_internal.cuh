@@ -162,6 +162,13 @@ struct DBuf {
     }
     cap = c;
   }
+  // reserve with half as much again when it grows, for buffers whose need
+  // creeps up from batch to batch; true when it grew
+  bool grow(int64_t count) {
+    if (count <= cap) return false;
+    reserve(count + count / 2);
+    return true;
+  }
   void release() {
     if (p) {
       if (s) cudaFreeAsync(p, s);
@@ -601,10 +608,12 @@ struct mf_ctx {
   mf::DBuf<int32_t> i32a, i32b, i32c;
   mf::DBuf<uint8_t> u8a;
   // overlay rebuild
-  mf::DBuf<int32_t> acnt_new;
-  mf::DBuf<uint8_t> akill;
-  mf::DBuf<uint64_t> app_keys;
-  mf::DBuf<uint32_t> app_vals;
+  mf::DBuf<int32_t> adelta;     // change of each vertex's added count; zero between batches
+  mf::DBuf<uint8_t> akill;      // added entries that go; zero between batches
+  mf::DBuf<uint8_t> app_line;   // lines of the batch that append their pair
+  mf::DBuf<uint64_t> slot_keys; // endpoint slots sorted by vertex
+  mf::DBuf<uint32_t> slot_vals;
+  mf::DBuf<int64_t> atail;      // prefix over akill and the appending slots
   // sub-batch buffers
   mf::DBuf<int32_t> seeds, cands, hlist, touched;
   mf::DBuf<int32_t> rowcid;
@@ -702,9 +711,10 @@ struct mf_ctx {
   int64_t touched_total = 0;
   int64_t dbg_first[5] = {};           // debug: first-hit calls, rows, warp-level rows, chunk rows, chunks
 
-  // pinned staging for host-input batches
+  // parts of the pinned block that starts at h_counters: the batch plan's first
+  // records, and the staged input of a small batch
+  int64_t* h_plan = nullptr;
   uint8_t* h_stage = nullptr;
-  int64_t h_stage_cap = 0;
   // the pipelined engine: batches enqueued by mf_apply_batch_async run in
   // order on this context's worker thread (made on first use); `pending`
   // counts the ones not yet collected
@@ -727,21 +737,21 @@ template <class F>
 void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->nindex); f(c->aoff); f(c->aoff_alt); f(c->i64a); f(c->i64b); f(c->rowlens); f(c->rp_pos);
   f(c->big_pos); f(c->big_off); f(c->big_nr); f(c->big_chunks); f(c->big_pre); f(c->dense_light);
-  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base);
+  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base); f(c->atail);
   f(c->n2cache); f(c->n2bound); f(c->un_cnt); f(c->counters); f(c->lb_offs);
   f(c->nlist); f(c->dead); f(c->rcnt); f(c->deg); f(c->aadj); f(c->aown); f(c->aadj_alt); f(c->aown_alt);
   f(c->cid); f(c->v2i); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
-  f(c->acnt_new); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
+  f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
   f(c->pull_long); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
-  f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->app_vals); f(c->rp_vals); f(c->rp_vals2);
+  f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
   f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->ncbits); f(c->n2stamp);
   f(c->n2bstamp); f(c->nmark); f(c->cidbits);
-  f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->creates); f(c->rp_u8); f(c->plan_flags);
+  f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
   f(c->xst); f(c->xleave); f(c->cta_vert); f(c->cta_ws);
-  f(c->keys); f(c->app_keys); f(c->rp_keys); f(c->rp_keys2);
+  f(c->keys); f(c->slot_keys); f(c->rp_keys); f(c->rp_keys2);
   f(c->big_best); f(c->fpos); f(c->work);
   f(c->p2_mask); f(c->p2_filt); f(c->p2_racc); f(c->p2_vol); f(c->p2_tasks); f(c->p2_grp); f(c->p2_huge);
   f(c->p2_cnt);
@@ -778,7 +788,7 @@ inline void release_device_state(mf_ctx* c) {
 inline void release_batch_scratch(mf_ctx* c) {
   const void* keep[] = {&c->nindex, &c->nlist, &c->live, &c->dead, &c->rcnt, &c->deg, &c->aoff, &c->aadj,
                         &c->aown, &c->mis, &c->cid, &c->v2i, &c->bval, &c->wval, &c->f1, &c->nmark,
-                        &c->nlist_need, &c->touched, &c->hlist, &c->acnt_new, &c->aoff_alt, &c->counters,
+                        &c->nlist_need, &c->touched, &c->hlist, &c->adelta, &c->aoff_alt, &c->counters,
                         &c->cta_vert};
   for_each_buffer(c, [&](auto& b) {
     for (const void* k : keep)
@@ -835,7 +845,32 @@ struct StageScope {
 
 // mf_overlay.cu
 void upload_base(mf_ctx* c, int32_t n, const int64_t* nindex, const int32_t* nlist, int64_t nnz);
-void apply_overlay(mf_ctx* c, int64_t m);          // uses c->bu/bv/bins
+// A batch's lines, readable by the device (device memory or pinned host memory).
+struct BatchIn {
+  const int32_t* u;
+  const int32_t* v;
+  const uint8_t* ins;
+};
+// Batches of up to this many lines are sorted by one block each for the pairs
+// and the endpoint slots, planned by one block, and staged in pinned memory.
+constexpr int64_t kSmallBatch = 4096;
+// Batch counters, after the work counters in c->work (zeroed with them).
+constexpr int kCntBad = 2 * kStCount + 8;        // lines with invalid endpoints
+constexpr int kCntAppended = kCntBad + 1;        // entries added to the overlay
+constexpr int kCntKilled = kCntBad + 2;          // added entries that go
+constexpr int kWorkWords = kCntBad + 8;
+// The batch plan in pinned memory: [0] sub-batches, [1] invalid lines, [2, 3]
+// appended and killed entries, from [8] the first kPlanHost {cut, estimate,
+// seed end} records.
+constexpr int64_t kPlanHost = 160;
+constexpr int64_t kPlanWords = 8 + 3 * kPlanHost;
+// lines -> c->bu/bv/bins, endpoint slots by vertex, previous occurrences, and
+// the pairs' state changes (nothing changes when a line is invalid)
+void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m);
+// the added entries' new arrays, in the alternate buffers; swap_overlay makes
+// them current once the host knows that the batch is valid
+void rebuild_added(mf_ctx* c, int64_t m);
+void swap_overlay(mf_ctx* c, int64_t appended, int64_t killed);
 void flag_updates(mf_ctx* c, int64_t m);           // c->bu/bv -> c->bins
 // host u/v -> host ins_out through a fixed device array; m <= MF_NOALLOC_MAX_UPDATES
 void flag_updates_noalloc(mf_ctx* c, const int32_t* u, const int32_t* v, int64_t m, uint8_t* ins_out);
@@ -848,6 +883,6 @@ void exact_fixup(mf_ctx* c);                       // exact-MIS mode after a bat
 // mf_parse.cu: batch file -> c->bu / c->bv (valid lines, file order); returns the count
 int64_t parse_batch_file_device(mf_ctx* c, const char* path);
 // mf_repair.cu
-void process_batch(mf_ctx* c, int64_t m);          // everything after the overlay apply
+void process_batch(mf_ctx* c, const BatchIn& in, int64_t m);
 int64_t initial_max_csr(int32_t n, uint64_t edges);
 }  // namespace mf

@@ -14,11 +14,16 @@
 // three-state machine none / added / tombstoned that insertEdge, removeEdge,
 // un_tombstone and forget_delta_edge implement, core/FlashGraph.h:196-275).
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "mf_internal.cuh"
+#include "mf_scan.cuh"
+#include "mf_sort.cuh"
 
 namespace mf {
+
+using scan_detail::scan_exclusive_to;
 
 namespace {
 
@@ -129,17 +134,131 @@ __device__ int64_t added_find(const GraphView& g, int32_t x, int32_t y) {
   return -1;
 }
 
-__global__ void k_pair_keys(const int32_t* u, const int32_t* v, int64_t m, int nbits, uint64_t* keys, uint32_t* vals) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const uint64_t a = (uint64_t)min(u[i], v[i]), b = (uint64_t)max(u[i], v[i]);
-  keys[i] = (a << nbits) | b;
-  vals[i] = (uint32_t)i;
+// ---- batch input -----------------------------------------------------------------
+
+__device__ __forceinline__ uint64_t pair_key(int32_t x, int32_t y, int nbits) {
+  return ((uint64_t)(uint32_t)min(x, y) << nbits) | (uint64_t)(uint32_t)max(x, y);
 }
 
-__global__ void k_init_acnt(const int64_t* aoff, int32_t n, int32_t* acnt) {
-  int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < n) acnt[x] = (int32_t)(aoff[x + 1] - aoff[x]);
+__device__ __forceinline__ bool bad_line(int32_t x, int32_t y, int32_t n) {
+  return x < 0 || x >= n || y < 0 || y >= n || x == y;
+}
+
+// The lines into the context's arrays (unless they are there), checked; the
+// pair keys and the endpoint slots' vertices for the sorts.
+__global__ void k_stage(BatchIn in, int64_t m, int32_t n, int nbits, int32_t* u, int32_t* v, uint8_t* ins,
+                        uint8_t* app_line, uint64_t* pair_keys, uint32_t* pair_vals, uint64_t* slot_keys,
+                        uint32_t* slot_vals, unsigned long long* bad) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m) return;
+  const int32_t x = in.u[i], y = in.v[i];
+  if (in.u != u) {
+    u[i] = x;
+    v[i] = y;
+    ins[i] = in.ins[i];
+  }
+  app_line[i] = 0;
+  if (bad_line(x, y, n)) atomicAdd(bad, 1ull);
+  pair_keys[i] = pair_key(x, y, nbits);
+  pair_vals[i] = (uint32_t)i;
+  reinterpret_cast<ulonglong2*>(slot_keys)[i] = make_ulonglong2((uint32_t)x, (uint32_t)y);
+  reinterpret_cast<uint2*>(slot_vals)[i] = make_uint2((uint32_t)(2 * i), (uint32_t)(2 * i + 1));
+}
+
+// Previous edge index of every endpoint slot's vertex (sorted slots: each
+// vertex's in slot order).
+__global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int32_t* prev) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= cnt) return;
+  prev[vals[j]] = j > 0 && keys[j - 1] == keys[j] ? (int32_t)(vals[j - 1] >> 1) : -1;
+}
+
+// A small batch's input in one launch: block 0 stages and checks the lines and
+// groups the pairs, block 1 sorts the endpoint slots and finds the previous
+// occurrences.  Both read the lines where the caller's copy is (pinned host
+// memory or the device).  Latency of one block's sort bounds it; as separate
+// launches (three copies, a check, key kernels, three sorts, k_prev) the same
+// work took 16 launches and two round trips to the host.
+template <int Items>
+__global__ void __launch_bounds__(1024) k_small_input(BatchIn in, int m, int32_t n, int nbits, int gbits, int32_t* u,
+                                                      int32_t* v, uint8_t* ins, uint8_t* app_line, uint64_t* pair_keys,
+                                                      uint32_t* pair_vals, uint64_t* slot_keys, uint32_t* slot_vals,
+                                                      int32_t* prev, unsigned long long* bad) {
+  extern __shared__ __align__(16) unsigned char in_smem[];
+  __shared__ uint32_t dbase[sort_detail::kDigits];
+  __shared__ uint32_t sw[sort_detail::kDigits / 32];
+  const int cap = Items * (int)blockDim.x;
+  uint64_t* sk = reinterpret_cast<uint64_t*>(in_smem);
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + cap);
+  uint32_t* cnt = sv + cap;
+  const int at = (threadIdx.x >> 5) * 32 * Items + (threadIdx.x & 31);
+  uint64_t key[Items];
+  uint32_t val[Items];
+  if (blockIdx.x == 0) {
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      const int i = at + r * 32;
+      key[r] = 0;
+      val[r] = (uint32_t)i;
+      if (i < m) {
+        const int32_t x = in.u[i], y = in.v[i];
+        if (in.u != u) {
+          u[i] = x;
+          v[i] = y;
+          ins[i] = in.ins[i];
+        }
+        app_line[i] = 0;
+        if (bad_line(x, y, n)) atomicAdd(bad, 1ull);
+        key[r] = pair_key(x, y, nbits);
+      }
+    }
+    sort_detail::block_sort<Items>(true, key, val, m, 64 - gbits, 64, sk, sv, cnt, dbase, sw);
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      const int i = at + r * 32;
+      if (i < m) {
+        pair_keys[i] = key[r];
+        pair_vals[i] = val[r];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      const int i = at + r * 32;
+      val[r] = (uint32_t)i;
+      key[r] = i < 2 * m ? (uint32_t)((i & 1) ? in.v[i >> 1] : in.u[i >> 1]) : 0;
+    }
+    sort_detail::block_sort<Items>(false, key, val, 2 * m, 0, nbits, sk, sv, cnt, dbase, sw);
+#pragma unroll
+    for (int r = 0; r < Items; ++r) {
+      const int i = at + r * 32;
+      if (i < 2 * m) {
+        slot_keys[i] = key[r];
+        slot_vals[i] = val[r];
+        prev[val[r]] = i > 0 && sk[i - 1] == key[r] ? (int32_t)(sv[i - 1] >> 1) : -1;
+      }
+    }
+  }
+}
+
+template <int Items>
+void small_input(mf_ctx* c, const BatchIn& in, int m, int threads, int nbits, int gbits) {
+  const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * sort_detail::kDigits * 4;
+  if (smem > 48 * 1024) {
+    // raised once per device for this kernel
+    static std::atomic<unsigned long long> raised{0};
+    const unsigned long long bit = 1ull << (c->device & 63);
+    if (c->device > 63 || !(raised.load(std::memory_order_acquire) & bit)) {
+      MF_CUDA(cudaFuncSetAttribute(k_small_input<Items>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   Items * 1024 * 12 + 32 * sort_detail::kDigits * 4));
+      raised.fetch_or(bit, std::memory_order_release);
+    }
+  }
+  MF_K(k_small_input<Items><<<2, threads, smem, c->stream>>>(
+      in, m, c->n, nbits, gbits, c->bu.p, c->bv.p, c->bins.p, c->app_line.p, c->keys.p, c->vals.p, c->slot_keys.p,
+      c->slot_vals.p, c->prev.p, c->work.p + kCntBad));
 }
 
 enum : int { kStN = 0, kStA = 1, kStR = 2 };
@@ -152,13 +271,18 @@ __device__ __forceinline__ bool same_run(uint64_t a, uint64_t b, int gbits) {
   return a == b || ((mix_key(a) ^ mix_key(b)) >> (64 - gbits)) == 0;
 }
 
-// One thread per unordered pair.  counters[0] = appended entries,
-// counters[1] = killed.  app_keys = owner << seq_bits | batch index.
-__global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_t* rcnt, bool sorted,
+// One thread per unordered pair.  Besides the base tombstones it records what
+// the added arrays' rebuild needs: the change of the added counts (adelta),
+// the entries that go (akill) and the line whose pair is appended
+// (app_line).  cnt = the batch counters from kCntBad; with invalid lines
+// nothing is touched.
+__global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_t* rcnt, int32_t* deg, bool sorted,
                               const uint64_t* keys, const uint32_t* vals, int64_t m, int nbits, int gbits,
-                              int seq_bits, const int32_t* u, const int32_t* v, const uint8_t* ins,
-                              int32_t* acnt, uint8_t* akill, uint64_t* app_keys, uint32_t* app_vals,
-                              int64_t* counters) {
+                              const int32_t* u, const int32_t* v, const uint8_t* ins, int32_t* adelta, uint8_t* akill,
+                              uint8_t* app_line, unsigned long long* cnt) {
+  pdl_wait();
+  pdl_trigger();
+  if (*cnt != 0) return;
   int64_t j0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j0 >= m) return;
   const uint64_t key = keys[j0];
@@ -212,59 +336,103 @@ __global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_
     atomicAdd(dead + a, sgn * (live_ab + dead_ab));
     atomicAdd(dead + b, sgn * (live_ba + dead_ba));
   }
+  // degree = base - tombstones + added (DeltaOverlay::degree)
+  int da = 0, db = 0;
+  if ((st0 == kStR) != (st == kStR)) da = db = st0 == kStR ? 1 : -1;
   if (old_killed) {
-    if (pos_ab >= 0) { akill[pos_ab] = 1; atomicSub(acnt + a, 1); }
-    if (pos_ba >= 0) { akill[pos_ba] = 1; atomicSub(acnt + b, 1); }
-    atomicAdd((unsigned long long*)(counters + 1), 2ull);
+    if (pos_ab >= 0) { akill[pos_ab] = 1; atomicSub(adelta + a, 1); --da; }
+    if (pos_ba >= 0) { akill[pos_ba] = 1; atomicSub(adelta + b, 1); --db; }
+    atomicAdd(cnt + (kCntKilled - kCntBad), 2ull);
   }
   if (appended) {
-    const unsigned long long slot = atomicAdd((unsigned long long*)counters, 2ull);
-    app_keys[slot] = ((uint64_t)a << seq_bits) | last_seq;
-    app_vals[slot] = (uint32_t)b;
-    app_keys[slot + 1] = ((uint64_t)b << seq_bits) | last_seq;
-    app_vals[slot + 1] = (uint32_t)a;
-    atomicAdd(acnt + a, 1);
-    atomicAdd(acnt + b, 1);
+    app_line[last_seq] = 1;
+    atomicAdd(adelta + a, 1);
+    atomicAdd(adelta + b, 1);
+    ++da;
+    ++db;
+    atomicAdd(cnt + (kCntAppended - kCntBad), 2ull);
   }
+  if (da) atomicAdd(deg + a, da);
+  if (db) atomicAdd(deg + b, db);
 }
 
-__global__ void k_move_survivors(const int64_t* aoff, const int32_t* aadj, const int32_t* aown,
-                                 const uint8_t* akill, const int64_t* kp, int64_t a_total,
-                                 const int64_t* noff, int32_t* nadj, int32_t* nown) {
-  int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= a_total || akill[j]) return;
-  const int32_t x = aown[j];
-  const int64_t s = aoff[x];
-  const int64_t r = (j - s) - (kp[j] - kp[s]);
-  const int64_t pos = noff[x] + r;
-  nadj[pos] = aadj[j];
+// ---- rebuild of the added arrays -----------------------------------------------------
+// One scan over three segments: the n new added counts (prefix = the new
+// offsets), the a_total kill marks, and the 2m endpoint slots (by vertex, in
+// slot order) whose line appends its pair.  The last two give every survivor
+// and every new entry its rank, so one more launch places them all.
+
+struct RebuildCounts {
+  int64_t n, a_total;
+  const int64_t* aoff;
+  const int32_t* adelta;
+  const uint8_t* akill;
+  const uint32_t* slot_vals;
+  const uint8_t* app_line;
+  __device__ __forceinline__ int64_t operator()(int64_t i) const {
+    if (i < n) return aoff[i + 1] - aoff[i] + adelta[i];
+    if (i < n + a_total) return akill[i - n];
+    return app_line[slot_vals[i - n - a_total] >> 1];
+  }
+};
+
+struct RebuildOut {   // tail[j]: prefix at item n + j
+  int64_t n;
+  int64_t* noff;
+  int64_t* tail;
+  __device__ __forceinline__ void operator()(int64_t i, int64_t v) const {
+    if (i <= n) noff[i] = v;
+    if (i >= n) tail[i - n] = v;
+  }
+};
+
+__global__ void k_rebuild_added(const int64_t* aoff, const int32_t* aadj, const int32_t* aown, int64_t a_total,
+                                const int64_t* noff, const int64_t* tail, const uint64_t* slot_keys,
+                                const uint32_t* slot_vals, int64_t slots, const int32_t* u, const int32_t* v,
+                                const uint8_t* app_line, const unsigned long long* bad, uint8_t* akill,
+                                int32_t* adelta, int32_t* nadj, int32_t* nown) {
+  pdl_wait();
+  pdl_trigger();
+  if (*bad != 0) return;
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < a_total) {
+    // a surviving entry: behind the row's earlier survivors
+    if (akill[j]) {
+      akill[j] = 0;
+      return;
+    }
+    const int32_t x = aown[j];
+    const int64_t s = aoff[x];
+    const int64_t pos = noff[x] + (j - s) - (tail[j] - tail[s]);
+    nadj[pos] = aadj[j];
+    nown[pos] = x;
+    return;
+  }
+  const int64_t k = j - a_total;
+  if (k >= slots) return;
+  const int32_t x = (int32_t)slot_keys[k];
+  adelta[x] = 0;
+  const uint32_t slot = slot_vals[k];
+  if (!app_line[slot >> 1]) return;
+  // a new entry: behind the row's survivors and the vertex's earlier new ones;
+  // the vertex's first slot is found by doubling steps back, then bisection
+  int64_t lo = k, step = 1;
+  while (lo > 0 && slot_keys[max(lo - step, (int64_t)0)] == (uint64_t)(uint32_t)x) {
+    lo = max(lo - step, (int64_t)0);
+    step *= 2;
+  }
+  if (lo > 0) {
+    int64_t out = max(lo - step, (int64_t)0);   // another vertex's
+    while (lo - out > 1) {
+      const int64_t mid = (lo + out) >> 1;
+      if (slot_keys[mid] == (uint64_t)(uint32_t)x) lo = mid; else out = mid;
+    }
+  }
+  const int64_t b = aoff[x], e = aoff[x + 1];
+  const int64_t survivors = (e - b) - (tail[e] - tail[b]);
+  const int64_t pos = noff[x] + survivors + (tail[a_total + k] - tail[a_total + lo]);
+  nadj[pos] = (slot & 1) ? u[slot >> 1] : v[slot >> 1];
   nown[pos] = x;
-}
-
-__global__ void k_place_appends(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int seq_bits,
-                                const int64_t* noff, int32_t* nadj, int32_t* nown) {
-  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= cnt) return;
-  const uint64_t owner = keys[k] >> seq_bits;
-  int64_t lo = 0, hi = k;  // first index with this owner
-  while (lo < hi) {
-    int64_t mid = (lo + hi) >> 1;
-    if ((keys[mid] >> seq_bits) < owner) lo = mid + 1; else hi = mid;
-  }
-  int64_t lo2 = k + 1, hi2 = cnt;  // one past the last index with this owner
-  while (lo2 < hi2) {
-    int64_t mid = (lo2 + hi2) >> 1;
-    if ((keys[mid] >> seq_bits) <= owner) lo2 = mid + 1; else hi2 = mid;
-  }
-  const int32_t x = (int32_t)owner;
-  const int64_t pos = noff[x + 1] - (lo2 - lo) + (k - lo);
-  nadj[pos] = (int32_t)vals[k];
-  nown[pos] = x;
-}
-
-__global__ void k_degrees(const int64_t* nindex, const int32_t* rcnt, const int64_t* aoff, int32_t n, int32_t* deg) {
-  int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (x < n) deg[x] = (int32_t)((nindex[x + 1] - nindex[x]) - rcnt[x] + (aoff[x + 1] - aoff[x]));
 }
 
 // isAdjacent (core/FlashGraph.h:291-301) for every update.
@@ -516,12 +684,13 @@ void alloc_vertex_scratch(mf_ctx* c) {
   c->nlist_need.reserve(n);
   c->touched.reserve(n);
   c->hlist.reserve(n);
-  c->acnt_new.reserve(n);
+  c->adelta.reserve(n);
   if (n > 0) {
     MF_CUDA(cudaMemsetAsync(c->v2i.p, 0xFF, sizeof(int32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->bval.p, 0, sizeof(uint32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->wval.p, 0, sizeof(uint32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->nmark.p, 0, sizeof(uint32_t) * (size_t)n, s));
+    MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
   }
   c->epoch = 0;
   c->counters.reserve(64);
@@ -533,64 +702,69 @@ void flag_updates(mf_ctx* c, int64_t m) {
   MF_CUDA(cudaGetLastError());
 }
 
-void apply_overlay(mf_ctx* c, int64_t m) {
-  if (m <= 0) return;
+void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
   const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
+  // pairs are grouped on mixed bits, three to ten more than the line count
+  // needs: two 8-bit digits up to 2^13 lines and three up to 2^21, where the
+  // pair itself has 2 * nbits bits (six digits at 2^22 vertices)
+  const int gbits = std::min(64, (bits_for(m) + 3 + 7) / 8 * 8);
+  c->bu.reserve(m);
+  c->bv.reserve(m);
+  c->bins.reserve(m);
+  c->app_line.reserve(m);
   c->keys.reserve(2 * m);
   c->vals.reserve(2 * m);
-  MF_K(k_pair_keys<<<grid_for(m), kTB, 0, s>>>(c->bu.p, c->bv.p, m, nbits, c->keys.p, c->vals.p));
-  // grouped on mixed bits, three to eleven more than the line count needs: two
-  // 8-bit digits up to 2^13 lines and three up to 2^21, where the pair itself
-  // has 2 * nbits bits (six digits at 2^22 vertices)
-  const int gbits = std::min(64, (bits_for(m) + 3 + 7) / 8 * 8);
-  const int seq_bits = bits_for(std::max<int64_t>(m - 1, 1));
-  const SortedPairs pairs = radix_group_pairs(c->keys.p, c->vals.p, m, gbits, c->ws, s);
+  c->slot_keys.reserve(2 * m);
+  c->slot_vals.reserve(2 * m);
+  c->prev.reserve(2 * m);
+  // grown with every mark cleared: the rebuild clears the ones it used
+  if (c->akill.grow(std::max<int64_t>(c->a_total, 1)))
+    MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
+  SortedPairs pairs{c->keys.p, c->vals.p};
+  if (m <= kSmallBatch) {
+    const int slots = (int)(2 * m);
+    if (slots <= 256) small_input<1>(c, in, (int)m, 256, nbits, gbits);
+    else if (slots <= 1024) small_input<1>(c, in, (int)m, 1024, nbits, gbits);
+    else if (slots <= 2048) small_input<2>(c, in, (int)m, 1024, nbits, gbits);
+    else if (slots <= 4096) small_input<4>(c, in, (int)m, 1024, nbits, gbits);
+    else small_input<8>(c, in, (int)m, 1024, nbits, gbits);
+  } else {
+    MF_K(k_stage<<<grid_for(m), kTB, 0, s>>>(in, m, c->n, nbits, c->bu.p, c->bv.p, c->bins.p, c->app_line.p, c->keys.p,
+                                             c->vals.p, c->slot_keys.p, c->slot_vals.p, c->work.p + kCntBad));
+    pairs = radix_group_pairs(c->keys.p, c->vals.p, m, gbits, c->ws, s);
+  }
+  MF_K(launch_pdl(k_apply_pairs, grid_for(m), kTB, 0, s, c->view(), c->live.p, c->dead.p, c->rcnt.p, c->deg.p,
+                  c->rows_sorted, pairs.keys, pairs.vals, m, nbits, gbits, c->bu.p, c->bv.p, c->bins.p, c->adelta.p,
+                  c->akill.p, c->app_line.p, c->work.p + kCntBad));
+  if (m > kSmallBatch) {
+    radix_sort_pairs_in_place(c->slot_keys.p, c->slot_vals.p, 2 * m, 0, nbits, c->ws, s);
+    MF_K(launch_pdl(k_prev, grid_for(2 * m), kTB, 0, s, c->slot_keys.p, c->slot_vals.p, 2 * m, c->prev.p));
+  }
+  MF_CUDA(cudaGetLastError());
+}
 
-  const int64_t cap_new = c->a_total + 2 * m;
-  c->akill.reserve(std::max<int64_t>(c->a_total, 1));
-  c->app_keys.reserve(2 * m);
-  c->app_vals.reserve(2 * m);
-  c->aadj_alt.reserve(cap_new);
-  c->aown_alt.reserve(cap_new);
-  c->aadj.reserve(std::max<int64_t>(c->a_total, 1));
-  c->aown.reserve(std::max<int64_t>(c->a_total, 1));
-  c->i64a.reserve(std::max<int64_t>(c->a_total, 1) + 1);
-  if (c->a_total > 0) MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->a_total, s));
-  MF_CUDA(cudaMemsetAsync(c->counters.p, 0, sizeof(int64_t) * 2, s));
-  MF_K(k_init_acnt<<<grid_for(c->n), kTB, 0, s>>>(c->aoff.p, c->n, c->acnt_new.p));
-  MF_K(k_apply_pairs<<<grid_for(m), kTB, 0, s>>>(c->view(), c->live.p, c->dead.p, c->rcnt.p, c->rows_sorted,
-                                            pairs.keys, pairs.vals, m, nbits, gbits, seq_bits, c->bu.p, c->bv.p, c->bins.p,
-                                            c->acnt_new.p, c->akill.p, c->app_keys.p, c->app_vals.p,
-                                            c->counters.p));
+void rebuild_added(mf_ctx* c, int64_t m) {
+  cudaStream_t s = c->stream;
+  const int64_t n = c->n, a = c->a_total, slots = 2 * m;
+  c->aadj_alt.grow(a + slots);
+  c->aown_alt.grow(a + slots);
+  c->aadj.reserve(std::max<int64_t>(a, 1));
+  c->aown.reserve(std::max<int64_t>(a, 1));
+  c->atail.grow(a + slots + 1);
+  scan_exclusive_to(RebuildCounts{n, a, c->aoff.p, c->adelta.p, c->akill.p, c->slot_vals.p, c->app_line.p},
+                    RebuildOut{n, c->aoff_alt.p, c->atail.p}, n + a + slots, c->ws, s);
+  MF_K(launch_pdl(k_rebuild_added, grid_for(a + slots), kTB, 0, s, c->aoff.p, c->aadj.p, c->aown.p, a, c->aoff_alt.p,
+                  c->atail.p, c->slot_keys.p, c->slot_vals.p, slots, c->bu.p, c->bv.p, c->app_line.p,
+                  c->work.p + kCntBad, c->akill.p, c->adelta.p, c->aadj_alt.p, c->aown_alt.p));
   MF_CUDA(cudaGetLastError());
-  MF_CUDA(cudaMemcpyAsync(c->h_counters, c->counters.p, sizeof(int64_t) * 2, cudaMemcpyDeviceToHost, s));
-  MF_CUDA(cudaStreamSynchronize(s));
-  const int64_t appended = c->h_counters[0], killed = c->h_counters[1];
-  if (appended == 0 && killed == 0) {
-    MF_K(k_degrees<<<grid_for(c->n), kTB, 0, s>>>(c->nindex.p, c->rcnt.p, c->aoff.p, c->n, c->deg.p));
-    MF_CUDA(cudaGetLastError());
-    return;
-  }
-  // new offsets
-  scan_exclusive_i32(c->acnt_new.p, c->aoff_alt.p, c->n, c->ws, s);
-  if (c->a_total > 0) {
-    scan_exclusive_u8(c->akill.p, c->i64a.p, c->a_total, c->ws, s);
-    MF_K(k_move_survivors<<<grid_for(c->a_total), kTB, 0, s>>>(c->aoff.p, c->aadj.p, c->aown.p, c->akill.p, c->i64a.p,
-                                                          c->a_total, c->aoff_alt.p, c->aadj_alt.p, c->aown_alt.p));
-  }
-  if (appended > 0) {
-    const SortedPairs app = radix_sort_pairs(c->app_keys.p, c->app_vals.p, appended, 0, seq_bits + nbits, c->ws, s);
-    MF_K(k_place_appends<<<grid_for(appended), kTB, 0, s>>>(app.keys, app.vals, appended, seq_bits, c->aoff_alt.p,
-                                                       c->aadj_alt.p, c->aown_alt.p));
-  }
-  MF_CUDA(cudaGetLastError());
+}
+
+void swap_overlay(mf_ctx* c, int64_t appended, int64_t killed) {
   std::swap(c->aoff, c->aoff_alt);
   std::swap(c->aadj, c->aadj_alt);
   std::swap(c->aown, c->aown_alt);
-  c->a_total = c->a_total + appended - killed;
-  MF_K(k_degrees<<<grid_for(c->n), kTB, 0, s>>>(c->nindex.p, c->rcnt.p, c->aoff.p, c->n, c->deg.p));
-  MF_CUDA(cudaGetLastError());
+  c->a_total += appended - killed;
 }
 
 void compact_graph(mf_ctx* c, std::vector<int64_t>& nindex_out, std::vector<int32_t>& nlist_out) {

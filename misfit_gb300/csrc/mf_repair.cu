@@ -63,25 +63,6 @@ __device__ __forceinline__ int64_t warp_id() {
 
 // ---- split ------------------------------------------------------------------
 
-// Endpoint slots (2j: source, 2j + 1: destination of line j) keyed by their
-// vertex; the sort is stable, so each vertex's slots stay in slot order.
-__global__ void k_slot_keys(const int32_t* u, const int32_t* v, int64_t m, uint64_t* keys, uint32_t* vals) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * m) return;
-  const int32_t x = (i & 1) ? v[i >> 1] : u[i >> 1];
-  keys[i] = (uint64_t)(uint32_t)x;
-  vals[i] = (uint32_t)i;
-}
-
-__global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, int32_t* prev) {
-  int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= cnt) return;
-  const uint32_t slot = vals[j];
-  int32_t pe = -1;
-  if (j > 0 && keys[j - 1] == keys[j]) pe = (int32_t)(vals[j - 1] >> 1);
-  prev[slot] = pe;
-}
-
 // ---- sub-batch plan ---------------------------------------------------------------
 // The split and the seed lists depend only on the batch, the degrees and
 // MAX_CSR_ELEMENTS, not on the clustering or repair of earlier sub-batches,
@@ -90,71 +71,187 @@ __global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, 
 // Cuts of all sub-batches from p0 (src/misfit/misfit.cu:494-523): each edge
 // adds deg * 1000 for every endpoint not seen yet in its sub-batch
 // (:501-507), and the sub-batch ends before the first edge t >= 1 whose
-// running estimate reaches MAX_CSR_ELEMENTS (:509-511).  One CTA:
-// per sub-batch the estimates of a window of 1024 edges are scanned in shared
-// memory; the cut is the first t >= 1 whose running estimate reaches maxcsr,
+// running estimate reaches MAX_CSR_ELEMENTS (:509-511).  One CTA of
+// kCutThreads: per sub-batch the estimates of a window of 1024 edges are
+// scanned; the cut is the first t >= 1 whose running estimate reaches maxcsr,
 // else the length (min(m - p, MAX_BATCH_SIZE)).  cuts[k] = end of sub-batch
-// k, ests[k] = estimate of the edges before the cut.
+// k, ests[k] = estimate of the edges before the cut; returns the count.
+//
+// The windows form one serial chain, so their latency bounds it.  The edges'
+// degrees and previous occurrences are gathered into shared memory kCutChunk
+// edges at a time, so that a window (or the next sub-batch's, which starts
+// inside the last one) is a shared-memory read, two warp scans and two
+// barriers.
 constexpr int kCutThreads = 1024;
+constexpr int kCutChunk = 2 * kCutThreads;
 
-__global__ void __launch_bounds__(kCutThreads) k_cuts(const int32_t* u, const int32_t* v, const int32_t* prev,
-                                                      const int32_t* deg, int64_t m, int64_t p0, int64_t maxcsr,
-                                                      int64_t* cuts, int64_t* ests, unsigned long long* count) {
-  __shared__ int64_t s_warp[kCutThreads / 32];
-  __shared__ int64_t s_total;
-  __shared__ int64_t s_cut, s_est;
+__device__ int64_t plan_cuts(const int32_t* u, const int32_t* v, const int32_t* prev, const int32_t* deg, int64_t m,
+                             int64_t p0, int64_t maxcsr, int64_t* cuts, int64_t* ests) {
+  __shared__ int4 s_edge[kCutChunk];   // previous edge of u and of v, deg[u], deg[v]
+  __shared__ int64_t s_warp[2][kCutThreads / 32];
+  __shared__ unsigned long long s_cut[2];
+  __shared__ int64_t s_est;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  int64_t p = p0, k = 0;
+  constexpr unsigned long long kNone = ~0ull;
+  if (tid == 0) s_cut[0] = kNone;
+  int64_t p = p0, k = 0, c0 = p0, c1 = p0;   // edges [c0, c1) are in shared memory
+  int buf = 0;
   while (p < m) {
     const int64_t len = min(m - p, kMaxBatchEdges);
-    int64_t acc = 0;
-    if (tid == 0) { s_cut = len; s_est = -1; }
-    __syncthreads();
-    for (int64_t t0 = 0; t0 < len; t0 += kCutThreads) {
+    int64_t acc = 0, cut = len, est = -1;
+    for (int64_t t0 = 0; t0 < len; t0 += kCutThreads, buf ^= 1) {
+      const int64_t need = min(p + t0 + kCutThreads, m);
+      if (p + t0 < c0 || need > c1) {
+        c0 = p + t0;
+        c1 = min(c0 + kCutChunk, m);
+        __syncthreads();
+        for (int64_t j = c0 + tid; j < c1; j += kCutThreads) {
+          const int2 pe = *reinterpret_cast<const int2*>(prev + 2 * j);
+          s_edge[j - c0] = make_int4(pe.x, pe.y, deg[u[j]], deg[v[j]]);
+        }
+        __syncthreads();
+      }
       const int64_t t = t0 + tid;
       int64_t c = 0;
       if (t < len) {
-        const int64_t j = p + t;
-        if (prev[2 * j] < p) c += (int64_t)deg[u[j]] * kEstimateWeight;
-        if (prev[2 * j + 1] < p) c += (int64_t)deg[v[j]] * kEstimateWeight;
+        const int4 e = s_edge[p + t - c0];
+        if (e.x < p) c += (int64_t)e.z * kEstimateWeight;
+        if (e.y < p) c += (int64_t)e.w * kEstimateWeight;
       }
       int64_t inc = c;
       for (int o = 1; o < 32; o <<= 1) {
         const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
       }
-      if (lane == 31) s_warp[wid] = inc;
+      if (lane == 31) s_warp[buf][wid] = inc;
       __syncthreads();
-      if (tid == 0) {
-        int64_t run = 0;
-        for (int w = 0; w < kCutThreads / 32; ++w) { const int64_t y = s_warp[w]; s_warp[w] = run; run += y; }
-        s_total = run;
+      if (tid == 0) s_cut[buf ^ 1] = kNone;   // every thread is past the last window's reads
+      int64_t ws = s_warp[buf][lane];   // every warp scans the warp totals
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += y;
       }
+      const int64_t before = __shfl_sync(0xffffffffu, ws, max(wid - 1, 0));
+      const int64_t incl = acc + (wid > 0 ? before : 0) + inc;  // estimate of edges 0..t
+      const unsigned hit = __ballot_sync(0xffffffffu, t >= 1 && t < len && incl >= maxcsr);
+      if (hit && lane == __ffs(hit) - 1) atomicMin(&s_cut[buf], (unsigned long long)t);
       __syncthreads();
-      const int64_t incl = acc + s_warp[wid] + inc;  // estimate of edges 0..t
-      if (t >= 1 && t < len && incl >= maxcsr) atomicMin((unsigned long long*)&s_cut, (unsigned long long)t);
-      __syncthreads();
-      if (t == s_cut) s_est = incl - c;
-      acc += s_total;
-      __syncthreads();
-      if (s_cut < len) break;
+      acc += __shfl_sync(0xffffffffu, ws, 31);
+      if (s_cut[buf] != kNone) {
+        cut = (int64_t)s_cut[buf];
+        if (t == cut) s_est = incl - c;
+        __syncthreads();
+        est = s_est;
+        buf ^= 1;
+        break;
+      }
     }
-    const int64_t cut = s_cut;
     if (tid == 0) {
       cuts[k] = p + cut;
-      ests[k] = s_est >= 0 ? s_est : acc;
+      ests[k] = est >= 0 ? est : acc;
     }
-    __syncthreads();
     p += cut;
     ++k;
   }
-  if (tid == 0) *count = (unsigned long long)k;
+  return k;
+}
+
+// Header of the plan in pinned memory (see kPlanWords).
+__device__ __forceinline__ void plan_header(int64_t count, const unsigned long long* bc, int64_t* host) {
+  host[0] = count;
+  for (int k = 0; k < 3; ++k) host[1 + k] = (int64_t)bc[k];
+}
+
+__device__ __forceinline__ void plan_record(int64_t k, const int64_t* cuts, const int64_t* ests, int64_t seed_end,
+                                            int64_t* host) {
+  if (k >= kPlanHost) return;
+  host[8 + 3 * k] = cuts[k];
+  host[8 + 3 * k + 1] = ests[k];
+  host[8 + 3 * k + 2] = seed_end;
+}
+
+__global__ void __launch_bounds__(kCutThreads) k_cuts(const int32_t* u, const int32_t* v, const int32_t* prev,
+                                                      const int32_t* deg, int64_t m, int64_t p0, int64_t maxcsr,
+                                                      int64_t* cuts, int64_t* ests, unsigned long long* count,
+                                                      const unsigned long long* bc, int64_t* host) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t k = bc[0] != 0 ? 0 : plan_cuts(u, v, prev, deg, m, p0, maxcsr, cuts, ests);
+  if (threadIdx.x == 0) {
+    *count = (unsigned long long)k;
+    plan_header(k, bc, host);
+  }
+}
+
+// The whole plan of up to 2 * kSmallBatch endpoint slots in one block: the
+// cuts, then the seeds (each slot whose vertex first appears in its
+// sub-batch), 1024 slots at a time.  As six launches and two read-backs the
+// same took 24 us of kernels.
+__global__ void __launch_bounds__(kCutThreads) k_plan_small(const int32_t* u, const int32_t* v, const int32_t* prev,
+                                                            const int32_t* deg, int64_t m, int64_t p0, int64_t maxcsr,
+                                                            int64_t* cuts, int64_t* ests, int64_t* seed_end,
+                                                            int32_t* seeds_all, const unsigned long long* bc,
+                                                            int64_t* host) {
+  pdl_wait();
+  pdl_trigger();
+  if (bc[0] != 0) {
+    if (threadIdx.x == 0) plan_header(0, bc, host);
+    return;
+  }
+  __shared__ int s_warp[33];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t count = plan_cuts(u, v, prev, deg, m, p0, maxcsr, cuts, ests);
+  __syncthreads();
+  int64_t carry = 0;
+  const int64_t slots = 2 * (m - p0);
+  for (int64_t base = 0; base < slots; base += kCutThreads) {
+    const int64_t i = base + threadIdx.x;
+    bool seed = false;
+    int64_t lo = 0, start = p0;
+    int32_t x = 0;
+    if (i < slots) {
+      const int64_t slot = 2 * p0 + i, j = slot >> 1;
+      int64_t hi = count;   // first k with cuts[k] > j
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (cuts[mid] <= j) lo = mid + 1; else hi = mid;
+      }
+      start = lo == 0 ? p0 : cuts[lo - 1];
+      seed = prev[slot] < start;
+      x = (slot & 1) ? v[j] : u[j];
+    }
+    const unsigned mask = __ballot_sync(0xffffffffu, seed);
+    if (lane == 0) s_warp[wid] = __popc(mask);
+    __syncthreads();
+    int w = s_warp[lane];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
+    }
+    const int before = wid > 0 ? __shfl_sync(0xffffffffu, w, wid - 1) : 0;
+    const int64_t pos = carry + before + __popc(mask & ((1u << lane) - 1u));
+    if (seed) seeds_all[pos] = x;
+    // a sub-batch's first slot ends the one before it
+    if (i < slots && lo > 0 && 2 * p0 + i == 2 * start) {
+      seed_end[lo - 1] = pos;
+      plan_record(lo - 1, cuts, ests, pos, host);
+    }
+    carry += __shfl_sync(0xffffffffu, w, 31);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    seed_end[count - 1] = carry;
+    plan_record(count - 1, cuts, ests, carry, host);
+    plan_header(count, bc, host);
+  }
 }
 
 // Seed flag of every endpoint slot from 2*p0: first appearance within its own
 // sub-batch (the sub-batch of edge j starts at the last cut <= j).
 __global__ void k_plan_seed_flags(const int32_t* prev, const int64_t* cuts, const unsigned long long* count, int64_t m,
                                   int64_t p0, uint8_t* flags) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * (m - p0)) return;
   const int64_t slot = 2 * p0 + i;
@@ -170,6 +267,8 @@ __global__ void k_plan_seed_flags(const int32_t* prev, const int64_t* cuts, cons
 
 __global__ void k_plan_seed_compact(const int32_t* u, const int32_t* v, const uint8_t* flags, const int64_t* pos,
                                     int64_t m, int64_t p0, int32_t* seeds_all) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 2 * (m - p0) || !flags[i]) return;
   const int64_t slot = 2 * p0 + i;
@@ -177,10 +276,15 @@ __global__ void k_plan_seed_compact(const int32_t* u, const int32_t* v, const ui
 }
 
 // seed_end[k] = number of seeds of sub-batches 0..k.
-__global__ void k_plan_seed_ends(const int64_t* cuts, const unsigned long long* count, const int64_t* pos, int64_t p0,
-                                 int64_t* seed_end) {
+__global__ void k_plan_seed_ends(const int64_t* cuts, const int64_t* ests, const unsigned long long* count,
+                                 const int64_t* pos, int64_t p0, int64_t* seed_end, int64_t* host) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < (int64_t)*count) seed_end[k] = pos[2 * (cuts[k] - p0)];
+  if (k >= (int64_t)*count) return;
+  const int64_t e = pos[2 * (cuts[k] - p0)];
+  seed_end[k] = e;
+  plan_record(k, cuts, ests, e, host);
 }
 
 // Seeds of one sub-batch into their rows: seeds[i], v2i[seeds[i]] = i.
@@ -3540,27 +3644,18 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
 
 }  // namespace
 
-void process_batch(mf_ctx* c, int64_t m) {
+void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
   const int32_t n = c->n;
-  const GraphView g = c->view();
   int64_t* cnt = c->counters.p;
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(cnt);
   int64_t* h = c->h_counters;
 
-  if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
-  // previous occurrence of every endpoint slot (for "not seen in this sub-batch")
-  const int nbits = bits_for(std::max<int32_t>(n - 1, 1));
-  c->keys.reserve(2 * m);
-  c->vals.reserve(2 * m);
-  c->prev.reserve(2 * m);
   std::optional<StageScope> sc;
-  sc.emplace(c, kStSplit);
-  MF_K(k_slot_keys<<<grid_for(2 * m), kTB, 0, s>>>(c->bu.p, c->bv.p, m, c->keys.p, c->vals.p));
-  const SortedPairs slots = radix_sort_pairs(c->keys.p, c->vals.p, 2 * m, 0, nbits, c->ws, s);
-  MF_K(k_prev<<<grid_for(2 * m), kTB, 0, s>>>(slots.keys, slots.vals, 2 * m, c->prev.p));
-  MF_CUDA(cudaGetLastError());
+  sc.emplace(c, kStOverlay);
+  apply_overlay(c, in, m);
   sc.reset();
+  if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
 
   if (c->heavy_used > 0) {
     MF_K(k_heavy_reset<<<grid_for(c->heavy_used), kTB, 0, s>>>(c->heavy_list.p, c->heavy_used, c->heavy_slot.p));
@@ -3598,35 +3693,75 @@ void process_batch(mf_ctx* c, int64_t m) {
   std::vector<int64_t> cuts, ests, seed_end;
   size_t kidx = 0;
   int64_t seed_base = 0;
-  auto plan = [&](int64_t p0) {
-    sc.emplace(c, kStSplit);
+  const unsigned long long* bc = c->work.p + kCntBad;
+  auto plan_launch = [&](int64_t p0) {
     unsigned long long* kcount = ucnt + 37;
-    MF_K(k_cuts<<<1, kCutThreads, 0, s>>>(c->bu.p, c->bv.p, c->prev.p, c->deg.p, m, p0, c->max_csr,
-                                          c->plan_cuts.p, c->plan_ests.p, kcount));
     const int64_t nslots = 2 * (m - p0);
-    MF_K(k_plan_seed_flags<<<grid_for(nslots), kTB, 0, s>>>(c->prev.p, c->plan_cuts.p, kcount, m, p0,
-                                                              c->plan_flags.p));
+    if (m - p0 <= kSmallBatch) {
+      MF_K(launch_pdl(k_plan_small, 1, kCutThreads, 0, s, c->bu.p, c->bv.p, c->prev.p, c->deg.p, m, p0, c->max_csr,
+                      c->plan_cuts.p, c->plan_ests.p, c->plan_send.p, c->seeds_all.p, bc, c->h_plan));
+      return;
+    }
+    MF_K(launch_pdl(k_cuts, 1, kCutThreads, 0, s, c->bu.p, c->bv.p, c->prev.p, c->deg.p, m, p0, c->max_csr,
+                    c->plan_cuts.p, c->plan_ests.p, kcount, bc, c->h_plan));
+    MF_K(launch_pdl(k_plan_seed_flags, grid_for(nslots), kTB, 0, s, c->prev.p, c->plan_cuts.p, kcount, m, p0,
+                    c->plan_flags.p));
     scan_exclusive_u8(c->plan_flags.p, c->plan_pos.p, nslots, c->ws, s);
-    MF_K(k_plan_seed_compact<<<grid_for(nslots), kTB, 0, s>>>(c->bu.p, c->bv.p, c->plan_flags.p, c->plan_pos.p, m,
-                                                                p0, c->seeds_all.p));
-    MF_K(k_plan_seed_ends<<<grid_for(m - p0), kTB, 0, s>>>(c->plan_cuts.p, kcount, c->plan_pos.p, p0,
-                                                             c->plan_send.p));
-    MF_CUDA(cudaMemcpyAsync(h + 37, cnt + 37, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaStreamSynchronize(s));
-    const int64_t nk = h[37];
+    MF_K(launch_pdl(k_plan_seed_compact, grid_for(nslots), kTB, 0, s, c->bu.p, c->bv.p, c->plan_flags.p, c->plan_pos.p,
+                    m, p0, c->seeds_all.p));
+    MF_K(launch_pdl(k_plan_seed_ends, grid_for(m - p0), kTB, 0, s, c->plan_cuts.p, c->plan_ests.p, kcount, c->plan_pos.p,
+                    p0, c->plan_send.p, c->h_plan));
+  };
+  // the plan's records, once the stream has passed its launches
+  auto plan_read = [&] {
+    const int64_t nk = c->h_plan[0];
     cuts.resize((size_t)nk);
     ests.resize((size_t)nk);
     seed_end.resize((size_t)nk);
-    MF_CUDA(cudaMemcpyAsync(cuts.data(), c->plan_cuts.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaMemcpyAsync(ests.data(), c->plan_ests.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaMemcpyAsync(seed_end.data(), c->plan_send.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost,
-                            s));
-    MF_CUDA(cudaStreamSynchronize(s));
+    for (int64_t k = 0; k < std::min(nk, kPlanHost); ++k) {
+      cuts[(size_t)k] = c->h_plan[8 + 3 * k];
+      ests[(size_t)k] = c->h_plan[8 + 3 * k + 1];
+      seed_end[(size_t)k] = c->h_plan[8 + 3 * k + 2];
+    }
+    if (nk > kPlanHost) {
+      MF_CUDA(cudaMemcpyAsync(cuts.data(), c->plan_cuts.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost, s));
+      MF_CUDA(cudaMemcpyAsync(ests.data(), c->plan_ests.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost, s));
+      MF_CUDA(cudaMemcpyAsync(seed_end.data(), c->plan_send.p, sizeof(int64_t) * (size_t)nk, cudaMemcpyDeviceToHost,
+                              s));
+      MF_CUDA(cudaStreamSynchronize(s));
+    }
     kidx = 0;
     seed_base = 0;
+  };
+  auto plan = [&](int64_t p0) {
+    sc.emplace(c, kStSplit);
+    plan_launch(p0);
+    MF_CUDA(cudaStreamSynchronize(s));
+    plan_read();
     sc.reset();
   };
-  plan(0);
+  // The plan of the whole batch, then the added arrays' rebuild: the host
+  // waits for the plan alone, and the rebuild runs while it goes on.  The
+  // header says whether the lines were valid (nothing has changed if not).
+  sc.emplace(c, kStSplit);
+  plan_launch(0);
+  MF_CUDA(cudaEventRecord(c->ev_a, s));
+  sc.emplace(c, kStOverlay);
+  rebuild_added(c, m);
+  sc.reset();
+  MF_CUDA(cudaEventSynchronize(c->ev_a));
+  if (c->h_plan[1] != 0) {
+    MF_CUDA(cudaStreamSynchronize(s));
+    MF_FAIL(MF_EINVAL, "update endpoints must be distinct vertex ids in [0, n)");
+  }
+  swap_overlay(c, c->h_plan[2], c->h_plan[3]);
+  c->stats = mf_batch_stats{};
+  c->stats.updates = m;
+  c->stats.packed_total = -1;
+  c->stats.row_degree_total = -1;
+  c->traces.clear();
+  plan_read();
+  const GraphView g = c->view();
 
   // the first sub-batch's front, on this stream.  Later fronts overlap the
   // previous sub-batch on the second stream for large graphs; for small ones

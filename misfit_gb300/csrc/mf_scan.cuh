@@ -19,6 +19,12 @@ struct Loader {
   __device__ __forceinline__ int64_t operator()(int64_t i) const { return (int64_t)p[i]; }
 };
 
+// Where the prefix goes: out(i, prefix) for i in [0, n].
+struct Store {
+  int64_t* p;
+  __device__ __forceinline__ void operator()(int64_t i, int64_t v) const { p[i] = v; }
+};
+
 __device__ __forceinline__ int64_t block_sum(int64_t v, int64_t* smem_warp) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -65,8 +71,8 @@ __device__ __forceinline__ int64_t block_exclusive(int64_t v, int64_t* smem_warp
 // One block, one item per thread, for inputs of up to kSingleThreads items.
 constexpr int kSingleThreads = 1024;
 
-template <typename L>
-__global__ void __launch_bounds__(kSingleThreads) k_scan_single(L load, int64_t n, int64_t* out) {
+template <typename L, typename O>
+__global__ void __launch_bounds__(kSingleThreads) k_scan_single(L load, int64_t n, O out) {
   pdl_wait();
   pdl_trigger();
   __shared__ int64_t sw[33];
@@ -74,8 +80,8 @@ __global__ void __launch_bounds__(kSingleThreads) k_scan_single(L load, int64_t 
   const int64_t v = i < n ? load(i) : 0;
   int64_t tot;
   const int64_t pre = block_exclusive(v, sw, &tot);
-  if (i < n) out[i] = pre;
-  if (i == 0) out[n] = tot;
+  if (i < n) out(i, pre);
+  if (i == 0) out(n, tot);
 }
 
 // A tile's status: {value, tag}, tag = seq << 2 | flag (1: value is the
@@ -110,8 +116,8 @@ __device__ __forceinline__ void status_store(ulonglong2* p, unsigned long long v
 // split that replaced it.
 constexpr int64_t kLookbackSpin = (int64_t)1 << 22;
 
-template <int Threads, int Items, typename L>
-__global__ void __launch_bounds__(Threads) k_scan_lookback(L load, int64_t n, int64_t* out, ulonglong2* st,
+template <int Threads, int Items, typename L, typename O>
+__global__ void __launch_bounds__(Threads) k_scan_lookback(L load, int64_t n, O out, ulonglong2* st,
                                                            unsigned long long seq) {
   pdl_wait();
   pdl_trigger();
@@ -200,17 +206,17 @@ __global__ void __launch_bounds__(Threads) k_scan_lookback(L load, int64_t n, in
     for (int k = 0; k < Items; ++k) {
       const int idx = k * Threads + threadIdx.x;
       const int64_t i = base + idx;
-      if (i < n) out[i] = tile[idx];
+      if (i < n) out(i, tile[idx]);
     }
   } else {
     const int64_t i = base + threadIdx.x;
-    if (i < n) out[i] = pre;
+    if (i < n) out(i, pre);
   }
-  if (t == (int64_t)gridDim.x - 1 && threadIdx.x == 0) out[n] = excl + tot;
+  if (t == (int64_t)gridDim.x - 1 && threadIdx.x == 0) out(n, excl + tot);
 }
 
-template <int Threads, int Items, typename L>
-void scan_lookback(L load, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s) {
+template <int Threads, int Items, typename L, typename O>
+void scan_lookback(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
   const int64_t nb = (n + Threads * Items - 1) / (Threads * Items);
   if (ws.scan_status.cap < 2 * nb) {
     ws.scan_status.reserve(2 * nb);
@@ -218,7 +224,7 @@ void scan_lookback(L load, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s)
     MF_CUDA(cudaMemsetAsync(ws.scan_status.p, 0, sizeof(unsigned long long) * (size_t)ws.scan_status.cap, s));
   }
   const unsigned long long seq = ++ws.scan_seq;
-  MF_K(launch_pdl(k_scan_lookback<Threads, Items, L>, (unsigned)nb, Threads, 0, s, load, n, out,
+  MF_K(launch_pdl(k_scan_lookback<Threads, Items, L, O>, (unsigned)nb, Threads, 0, s, load, n, out,
                   reinterpret_cast<ulonglong2*>(ws.scan_status.p), seq));
 }
 
@@ -231,21 +237,23 @@ void scan_lookback(L load, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s)
 // k_scan_lookback.
 constexpr int64_t kSmallTiles = 192;
 
-template <typename L>
-void scan_exclusive(L load, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s) {
-  if (n <= 0) {
-    MF_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), s));
-    return;
-  }
+template <typename L, typename O>
+void scan_exclusive_to(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
   if (n <= kSingleThreads) {
     const unsigned threads = (unsigned)((n + 31) & ~(int64_t)31);
-    MF_K(launch_pdl(k_scan_single<L>, 1, threads, 0, s, load, n, out));
+    MF_K(launch_pdl(k_scan_single<L, O>, 1, threads, 0, s, load, n, out));
   } else if (n <= kSmallTiles * 256) {
     scan_lookback<256, 1>(load, out, n, ws, s);
   } else {
     scan_lookback<512, 4>(load, out, n, ws, s);
   }
   MF_CUDA(cudaGetLastError());
+}
+
+template <typename L>
+void scan_exclusive(L load, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s) {
+  if (n <= 0) MF_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), s));
+  else scan_exclusive_to(load, Store{out}, n, ws, s);
 }
 
 }  // namespace scan_detail

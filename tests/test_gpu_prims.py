@@ -68,3 +68,30 @@ def test_batch_sorts_at_block_edges(gb, m):
                 assert np.array_equal(g.row(int(x)), orc.row(int(x))), x
             assert np.array_equal(g.get_mis(), orc.get_mis())
             assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
+
+
+# one block plans up to 4,096 lines; the first 160 sub-batches come back with the plan, the rest by a copy
+@pytest.mark.parametrize("m,max_csr", [(700, 100000), (1500, 40000), (4096, 200000), (4097, 200000), (5000, 60000)])
+def test_plan_cuts(gb, m, max_csr):
+    """Many short sub-batches (and re-plans after the limit grows): cuts, limit, membership and ids equal the oracle's."""
+    import oracle as O
+    n = 2500
+    nindex, nlist = W.er_graph(n, 5, 7)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    u, v, ins = W.ToggleStream(n, nindex, nlist, m).next_batch(m, with_flags=True)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for x in (g, orc):
+            x.max_csr = max_csr
+            x.set_mis(mis)
+        g.trace(True)
+        orc.trace(True)
+        g.apply_batch(u, v, ins)
+        orc.apply_batch(u, v, ins)
+        a, b = g.trace_records(), orc.trace_records()
+        assert len(a) == len(b)
+        for x, y in zip(a, b):
+            assert np.array_equal(x[0][[0, 1, 2, 3, 5, 6, 7]], np.asarray(y[0])[[0, 1, 2, 3, 5, 6, 7]])
+        assert g.max_csr == orc.max_csr
+        assert np.array_equal(g.get_mis(), orc.get_mis())
+        assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
