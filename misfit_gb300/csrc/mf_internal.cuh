@@ -565,11 +565,10 @@ struct SubBatchTrace {
 namespace mf {
 struct Front {
   mf::DBuf<uint32_t> bits;                  // hop-1 bitmap, then the seed bitmap
-  mf::DBuf<int64_t> bits_sums;              // per-block counts of the bitmap scan
   mf::DBuf<unsigned long long> uacc;        // per-seed sums of the size bound
   mf::DBuf<int32_t> hlist, cands;           // swapped into the context when its sub-batch runs
   mf::DBuf<int64_t> lb_offs;                // row offsets of the seeds
-  mf::DBuf<int64_t> cnt;                    // [0] (hop-1 << 32 | candidates), [1] size bound
+  mf::DBuf<int64_t> cnt;                    // [0] (hop-1 << 32 | candidates), [1] size bound, [2] blocks done
   mf::Scratch ws;
 };
 }  // namespace mf
@@ -720,6 +719,7 @@ struct mf_ctx {
   // counts the ones not yet collected
   mf::AsyncQueue* aq = nullptr;
   bool pending = false;
+  bool mid_batch = false;   // a batch began and has not ended: zeroed scratch may not be zero
   // load-balancing settings (mf_set_tuning); they move work between kernels,
   // never a result
   mf_tuning tune = mf_tuning{2048, 2048, 64, 256, 0, 1};
@@ -758,7 +758,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->ws.hist); f(c->ws.sort_status); f(c->ws.keys_alt);
   f(c->ws.vals_alt); f(c->ws.scan_status);
   for (auto& fr : c->front) {
-    f(fr.bits); f(fr.bits_sums); f(fr.uacc); f(fr.hlist); f(fr.cands); f(fr.lb_offs); f(fr.cnt);
+    f(fr.bits); f(fr.uacc); f(fr.hlist); f(fr.cands); f(fr.lb_offs); f(fr.cnt);
     f(fr.ws.hist); f(fr.ws.sort_status); f(fr.ws.keys_alt);
     f(fr.ws.vals_alt); f(fr.ws.scan_status);
   }

@@ -30,6 +30,7 @@
 
 #include "mf_internal.cuh"
 #include "mf_scan.cuh"
+#include "mf_sort.cuh"
 
 namespace mf {
 
@@ -287,11 +288,15 @@ __global__ void k_plan_seed_ends(const int64_t* cuts, const int64_t* ests, const
   plan_record(k, cuts, ests, e, host);
 }
 
-// Seeds of one sub-batch into their rows: seeds[i], v2i[seeds[i]] = i.
-__global__ void k_seed_rows(const int32_t* seeds_all, int64_t ns, int32_t* seeds, int32_t* v2i) {
+// Seeds of one sub-batch into their rows: seeds[i], v2i[seeds[i]] = i; and the
+// sub-batch's device counters to zero.
+__global__ void k_seed_rows(const int32_t* seeds_all, int64_t ns, int32_t* seeds, int32_t* v2i,
+                            unsigned long long* cnt) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 4) cnt[33 + i] = 0;
+  if (i < 8) cnt[48 + i] = 0;
   if (i >= ns) return;
   const int32_t x = seeds_all[i];
   seeds[i] = x;
@@ -344,23 +349,22 @@ __device__ __forceinline__ void add_work(unsigned long long* work, int64_t visit
 
 // ---- hop-1 set as a bitmap ----------------------------------------------------------
 // The hop-1 marks of a sub-batch go into a bitmap (hbits) and the seeds into
-// another (sbits); a two-level popcount scan over the words gives, per word,
+// another (sbits); one scan over the words' popcounts gives, per word,
 // the offsets of its marked vertices in hlist and of its marked non-seeds in
 // the candidate list, so both lists come out in ascending vertex id without
 // touching n-sized arrays.  Counts are packed as (hop-1 << 32) | candidates.
-constexpr int kBitsThreads = 256;
-constexpr int kBitsPerThread = 1;                               // words per thread
-constexpr int kBitsWords = kBitsThreads * kBitsPerThread;       // words per block
-
-// One pass over the seed rows: the hop-1 bit of every element, and per seed
+// One pass over the seed rows: the seeds' bits, the hop-1 bit of every element, and per seed
 // the sum of len(h) over row(s) for the packed-size upper bound (uacc).
 // deg[y] (DeltaOverlay::degree) is at least the overlay row length of y (a
 // tombstone removes at least one base entry), so the sums stay upper bounds.
 __global__ void __launch_bounds__(kLbThreads, MF_LB_MIN_BLOCKS) k_lb_hop1_bound(GraphView g, const int32_t* deg, const int32_t* seeds,
                                                               const int64_t* offs, int64_t ns, uint32_t* hbits,
-                                                              unsigned long long* uacc, unsigned long long* work) {
+                                                              uint32_t* sbits, unsigned long long* uacc,
+                                                              unsigned long long* work) {
   pdl_wait();
   pdl_trigger();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += (int64_t)gridDim.x * blockDim.x)
+    atomicOr(sbits + (seeds[i] >> 5), 1u << (seeds[i] & 31));
   int64_t cur = -1;
   unsigned long long acc = 0;
   const int64_t vis = lb_rows(g, seeds, offs, ns, [&](int64_t i, int32_t, int32_t y) {
@@ -377,93 +381,32 @@ __global__ void __launch_bounds__(kLbThreads, MF_LB_MIN_BLOCKS) k_lb_hop1_bound(
   add_work(work, vis);
 }
 
-__global__ void k_seed_bits(const int32_t* seeds, int64_t ns, uint32_t* sbits) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < ns) atomicOr(sbits + (seeds[i] >> 5), 1u << (seeds[i] & 31));
-}
+// The scan's items are the bitmap words: load counts a word, out writes the
+// word's vertices at the word's prefix.  The total goes to cnt[0], and the
+// bound's sum (cnt[1]) starts at zero.
+struct BitsCount {
+  const uint32_t* hbits;
+  const uint32_t* sbits;
+  __device__ __forceinline__ int64_t operator()(int64_t w) const {
+    const uint32_t m = hbits[w];
+    return ((int64_t)__popc(m) << 32) | (int64_t)__popc(m & ~sbits[w]);
+  }
+};
 
-__device__ __forceinline__ int64_t bits_count4(const uint32_t* hbits, const uint32_t* sbits, int64_t w0,
-                                               int64_t words) {
-  int64_t h = 0, c = 0;
-  for (int j = 0; j < kBitsPerThread; ++j) {
-    const int64_t w = w0 + j;
-    if (w < words) {
-      const uint32_t m = hbits[w];
-      h += __popc(m);
-      c += __popc(m & ~sbits[w]);
+struct BitsLists {
+  const uint32_t* hbits;
+  const uint32_t* sbits;
+  int64_t words, cap;
+  int32_t* hlist;
+  int32_t* cands;
+  int64_t* cnt;
+  __device__ __forceinline__ void operator()(int64_t w, int64_t prefix) const {
+    if (w == words) {
+      cnt[0] = prefix;
+      cnt[1] = 0;
+      return;
     }
-  }
-  return (h << 32) | c;
-}
-
-// Block-wide exclusive scan of one int64 per thread (kBitsThreads threads).
-__device__ __forceinline__ int64_t bits_block_scan(int64_t x, int64_t* s_warp, int64_t* total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int64_t inc = x;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += y;
-  }
-  if (lane == 31) s_warp[wid] = inc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t run = 0;
-    for (int w = 0; w < kBitsThreads / 32; ++w) { const int64_t y = s_warp[w]; s_warp[w] = run; run += y; }
-    s_warp[kBitsThreads / 32] = run;
-  }
-  __syncthreads();
-  const int64_t r = s_warp[wid] + inc - x;
-  *total = s_warp[kBitsThreads / 32];
-  __syncthreads();
-  return r;
-}
-
-__global__ void __launch_bounds__(kBitsThreads) k_bits_reduce(const uint32_t* hbits, const uint32_t* sbits,
-                                                              int64_t words, int64_t* block_sums) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ int64_t s_warp[kBitsThreads / 32 + 1];
-  const int64_t w0 = (int64_t)blockIdx.x * kBitsWords + (int64_t)threadIdx.x * kBitsPerThread;
-  int64_t total = 0;
-  bits_block_scan(bits_count4(hbits, sbits, w0, words), s_warp, &total);
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-// Exclusive scan of the block sums in place (one block; loops for any count);
-// the grand total goes to *total.
-__global__ void __launch_bounds__(kBitsThreads) k_bits_scan_sums(int64_t* block_sums, int64_t nblocks,
-                                                                 int64_t* total) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ int64_t s_warp[kBitsThreads / 32 + 1];
-  int64_t carry = 0;
-  for (int64_t b0 = 0; b0 < nblocks; b0 += kBitsThreads) {
-    const int64_t b = b0 + threadIdx.x;
-    const int64_t x = b < nblocks ? block_sums[b] : 0;
-    int64_t t = 0;
-    const int64_t e = bits_block_scan(x, s_warp, &t);
-    if (b < nblocks) block_sums[b] = carry + e;
-    carry += t;
-  }
-  if (threadIdx.x == 0) *total = carry;
-}
-
-__global__ void __launch_bounds__(kBitsThreads) k_bits_compact(const uint32_t* hbits, const uint32_t* sbits,
-                                                               int64_t words, const int64_t* block_offs, int64_t cap,
-                                                               int64_t ns, int32_t* hlist, int32_t* cands,
-                                                               int32_t* v2i) {
-  pdl_wait();
-  pdl_trigger();
-  __shared__ int64_t s_warp[kBitsThreads / 32 + 1];
-  const int64_t w0 = (int64_t)blockIdx.x * kBitsWords + (int64_t)threadIdx.x * kBitsPerThread;
-  int64_t total = 0;
-  const int64_t off = block_offs[blockIdx.x] + bits_block_scan(bits_count4(hbits, sbits, w0, words), s_warp, &total);
-  int64_t ph = off >> 32, pc = off & 0xffffffffll;
-  for (int j = 0; j < kBitsPerThread; ++j) {
-    const int64_t w = w0 + j;
-    if (w >= words) break;
+    int64_t ph = prefix >> 32, pc = prefix & 0xffffffffll;
     uint32_t m = hbits[w];
     const uint32_t sm = sbits[w];
     while (m) {
@@ -472,24 +415,12 @@ __global__ void __launch_bounds__(kBitsThreads) k_bits_compact(const uint32_t* h
       const int32_t x = (int32_t)(w * 32 + b);
       hlist[ph++] = x;
       if (!((sm >> b) & 1u)) {
-        if (pc < cap) {
-          cands[pc] = x;
-          if (v2i) v2i[x] = (int32_t)(ns + pc);
-        }
+        if (pc < cap) cands[pc] = x;
         ++pc;
       }
     }
   }
-}
-
-// Row map of the candidates (rows ns .. ns + nct - 1), once the previous
-// sub-batch has cleared its rows.
-__global__ void k_cand_v2i(const int32_t* cands, int64_t nct, int64_t ns, int32_t* v2i) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nct) v2i[cands[i]] = (int32_t)(ns + i);
-}
+};
 
 // ---- packed sizes ---------------------------------------------------------------
 
@@ -499,13 +430,20 @@ __global__ void k_cand_v2i(const int32_t* cands, int64_t nct, int64_t ns, int32_
 // The candidate count comes from the hop-1 compaction on the device (low 32
 // bits of *hop_counts, capped at capc), so the bound needs no host round trip
 // after the hop-1 stage.  Grid-stride over the ns + nct rows.
-__global__ void k_bound_finish(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* cands,
-                               const int64_t* hop_counts, int64_t capc, const unsigned long long* uacc,
-                               const int64_t* n2cache, const uint32_t* n2stamp, const int64_t* n2bound,
-                               const uint32_t* n2bstamp, uint32_t stamp, unsigned long long* out) {
+// The front ends here: both bitmaps and the seeds' sums go back to zero for
+// the next front, and the last block writes the counts and the bound (cnt[0],
+// cnt[1]) to the host's pinned words.
+__global__ void k_bound_finish(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t* cnt,
+                               int64_t capc, unsigned long long* uacc, const int64_t* n2cache,
+                               const uint32_t* n2stamp, const int64_t* n2bound, const uint32_t* n2bstamp,
+                               uint32_t stamp, uint32_t* bits, int64_t bit_words, int64_t* host) {
   pdl_wait();
   pdl_trigger();
-  const int64_t nct = min((int64_t)(*hop_counts & 0xffffffffll), capc);
+  unsigned long long* out = reinterpret_cast<unsigned long long*>(cnt + 1);
+  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < bit_words;
+       w += (int64_t)gridDim.x * blockDim.x)
+    bits[w] = 0;
+  const int64_t nct = min((int64_t)(cnt[0] & 0xffffffffll), capc);
   const int64_t rows = ns + nct;
   unsigned long long b = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += (int64_t)gridDim.x * blockDim.x) {
@@ -520,12 +458,26 @@ __global__ void k_bound_finish(GraphView g, const int32_t* seeds, int64_t ns, co
         if (e > (unsigned long long)g.n) e = (unsigned long long)g.n;
         b += e;
       }
+      uacc[i] = 0;
     } else {
       b += (unsigned long long)row_len(g, cands[i - ns]);
     }
   }
   for (int o = 16; o > 0; o >>= 1) b += __shfl_down_sync(0xffffffffu, b, o);
-  if ((threadIdx.x & 31) == 0 && b) atomicAdd(out, b);
+  __shared__ unsigned long long s_b[32];
+  if ((threadIdx.x & 31) == 0) s_b[threadIdx.x >> 5] = b;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b += s_b[w];
+    if (b) atomicAdd(out, b);
+    __threadfence();
+    unsigned long long* done = out + 1;
+    if (atomicAdd(done, 1ull) == gridDim.x - 1) {
+      *done = 0;
+      host[0] = cnt[0];
+      host[1] = (int64_t)atomicAdd(out, 0ull);
+    }
+  }
 }
 
 // Seeds whose exact size is cached for this batch take it; the others are
@@ -1616,15 +1568,17 @@ __global__ void k_first_chunks(GraphView g, P pred, unsigned long long* firstpos
 
 // Per row: early return when the row's own vertex already has an id
 // (src/misfit/misfit.cu:224); the other rows are listed (row index and
-// vertex) for the first-existing-id searches.
+// vertex) for the first-existing-id searches.  The candidates also take their
+// place in the row map here (rows ns .. ns + nct - 1).
 __global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, const int32_t* cid,
-                           int32_t* rowcid, uint8_t* creates, int32_t* live_i, int32_t* live_v,
+                           int32_t* v2i, int32_t* rowcid, uint8_t* creates, int32_t* live_i, int32_t* live_v,
                            unsigned long long* nlive) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ns + nct) return;
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
+  if (i >= ns) v2i[x] = (int32_t)i;
   if (cid[x] != -1) {
     rowcid[i] = kSkip;
     creates[i] = 0;
@@ -1727,16 +1681,24 @@ __global__ void k_need_decide(GraphView g, const int32_t* need, const int32_t* n
 // New cluster ids by ascending row index; the seed rows that write (not
 // skipped) also take phase 1 of the clustering write here: bval[s] = max tag
 // of those rows with s = their own vertex (the rest of phase 1 is
-// k_lb_push_seed).  A skipped row stays skipped whatever its id.
+// k_lb_push_seed).  A skipped row stays skipped whatever its id.  The
+// candidates that write set their bit for the pull (ncbits, null when the
+// candidates' ids are pushed); k_clear takes the bits back.
 __global__ void k_new_ids(int64_t rows, const int64_t* pos, int32_t* rowcid, const int32_t* seeds, int64_t ns,
-                          uint32_t epoch, uint32_t* bval) {
+                          const int32_t* cands, uint32_t epoch, uint32_t* bval, uint32_t* ncbits) {
   pdl_wait();
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= rows) return;
   const int32_t rc = rowcid[i];
   if (rc == -1) rowcid[i] = (int32_t)pos[i];
-  if (i < ns && rc != kSkip) atomicMax(bval + seeds[i], (epoch << kRowBits) | (uint32_t)i);
+  if (rc == kSkip) return;
+  if (i < ns) {
+    atomicMax(bval + seeds[i], (epoch << kRowBits) | (uint32_t)i);
+  } else if (ncbits) {
+    const int32_t x = cands[i - ns];
+    atomicOr(ncbits + (x >> 5), 1u << (x & 31));
+  }
 }
 
 // The pushes are reductions whose results are not read back, so they issue
@@ -1830,16 +1792,6 @@ struct PullArgs {
 
 __device__ __forceinline__ bool pull_nonskip(const PullArgs& a, int32_t c) {
   return (__ldg(a.ncbits + (c >> 5)) >> (c & 31)) & 1u;
-}
-
-// Bits of the non-skipped candidates (rows ns .. ns+nct-1) for the pull pass.
-__global__ void k_cand_bits(const int32_t* cands, int64_t nct, int64_t ns, const int32_t* rowcid, uint32_t* bits) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nct || rowcid[ns + i] == kSkip) return;
-  const int32_t c = cands[i];
-  atomicOr(bits + (c >> 5), 1u << (c & 31));
 }
 
 __device__ __forceinline__ void pull_finish(const PullArgs& a, int32_t y, int32_t best) {
@@ -1973,6 +1925,66 @@ __global__ void k_assign(const int32_t* u, const int32_t* v, int64_t p, int64_t 
   const unsigned long long k = atomicAdd(count, 1ull);
   keys[k] = ((uint64_t)c << tbits) | (uint64_t)(((1u << tbits) - 1u) - (uint32_t)t);
   vals[k] = (uint32_t)t;
+}
+
+// The assignment of a sub-batch whose edges fit one commit block of the repair
+// (kRoundCap), in one launch: the assigned edges, ordered by (cluster
+// ascending, index descending), and the start of the repair -- both result
+// pairs' first buffers to "no write", the round words (see SpecArgs::dyn) and
+// the deferral counters to zero.  The counts stay on the device (dyn[4] edges,
+// dyn[5] cluster count).  A thread takes the edge with the index len - 1 - tid,
+// so a stable sort on the cluster alone gives the order.
+__global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const int32_t* v, int64_t p, int len,
+                                                       const int32_t* cid, const int64_t* ccp, int cbits,
+                                                       uint32_t* order, int32_t* w0, int32_t* w1, int64_t* dyn,
+                                                       int64_t* counts) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ uint64_t sk[1024];
+  __shared__ uint32_t sv[1024];
+  __shared__ uint32_t cnt[32 * sort_detail::kDigits];
+  __shared__ uint32_t dbase[sort_detail::kDigits];
+  __shared__ uint32_t sw[32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, warps = blockDim.x >> 5;
+  const int64_t cc = *ccp;
+  const int t = len - 1 - tid;
+  int32_t c = -1;
+  if (t >= 0) {
+    c = cid[u[p + t]];
+    if (c == -1) c = cid[v[p + t]];
+  }
+  const bool take = c >= 0 && (int64_t)c < min(cc, kMaxBatchEdges);
+  const unsigned mask = __ballot_sync(0xffffffffu, take);
+  if (lane == 0) sw[w] = __popc(mask);
+  __syncthreads();
+  uint32_t x = lane < warps ? sw[lane] : 0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const uint32_t before = w > 0 ? __shfl_sync(0xffffffffu, x, w - 1) : 0;
+  const int n = (int)__shfl_sync(0xffffffffu, x, 31);
+  const uint32_t slot = before + __popc(mask & ((1u << lane) - 1u));
+  if (take) {
+    sk[slot] = (uint64_t)(uint32_t)c;
+    sv[slot] = (uint32_t)t;
+  }
+  __syncthreads();
+  uint64_t key[1] = {tid < n ? sk[tid] : 0};
+  uint32_t val[1] = {tid < n ? sv[tid] : 0};
+  __syncthreads();
+  sort_detail::block_sort<1>(false, key, val, n, 0, cbits, sk, sv, cnt, dbase, sw);
+  if (tid < n) {
+    order[tid] = val[0];
+    w0[tid] = -1;
+    w1[tid] = -1;
+  }
+  if (tid < 4) dyn[tid] = 0;
+  if (tid < 6) counts[tid] = 0;
+  if (tid == 0) {
+    dyn[4] = n;
+    dyn[5] = cc;
+  }
 }
 
 // ---- repair -------------------------------------------------------------------------------
@@ -2236,7 +2248,8 @@ struct SpecArgs {
   int64_t pre_cap;
   // rounds queued without a host read-back: [0] first pending position,
   // [1] entries of the view, [2] 1 once no position changed, [3] rounds run
-  // (k_spec_round keeps them); p0 and view.nkeys above are then ignored
+  // (k_spec_round keeps them), [4] positions; p0, cnt and view.nkeys above are
+  // then ignored
   int64_t* dyn = nullptr;
 };
 
@@ -2247,6 +2260,7 @@ __device__ __forceinline__ bool spec_dyn_load(SpecArgs& a) {
   if (a.dyn[2] != 0) return false;
   a.p0 = a.dyn[0];
   a.view.nkeys = a.dyn[1];
+  a.cnt = a.dyn[4];
   return true;
 }
 
@@ -2853,8 +2867,8 @@ __device__ __forceinline__ int round_scan(int x, int* s_warp, int* total) {
   return r;
 }
 
-// Start of a queued repair: both result pairs' first buffers to "no
-// write", the round words and the deferral counters to zero, in one launch.
+// Start of a queued repair of a larger sub-batch that assigned few edges: as
+// k_assign_small leaves it.
 __global__ void k_repair_init(int32_t* w0, int32_t* w1, int64_t cnt, int64_t* dyn, int64_t* counts) {
   pdl_wait();
   pdl_trigger();
@@ -2864,6 +2878,7 @@ __global__ void k_repair_init(int32_t* w0, int32_t* w1, int64_t cnt, int64_t* dy
     w1[i] = -1;
   }
   if (i < 4) dyn[i] = 0;
+  if (i == 4) dyn[4] = cnt;
   if (i < 6) counts[i] = 0;
 }
 
@@ -2879,6 +2894,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
   if (!spec_dyn_load(sa)) return;
   if (sa.dyn != nullptr) {
     p0 = sa.p0;
+    cnt = sa.cnt;
     nview_old = sa.view.nkeys;
   }
   __shared__ uint64_t s_keys[kRoundWrites];
@@ -2990,7 +3006,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
 }
 
 __global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, int32_t* cid,
-                        int32_t* v2i) {
+                        int32_t* v2i, uint32_t* ncbits) {
   pdl_wait();
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2998,6 +3014,7 @@ __global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, 
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
   cid[x] = -1;
   v2i[x] = -1;
+  if (ncbits && i >= ns) ncbits[x >> 5] = 0;
 }
 
 template <typename T>
@@ -3049,49 +3066,47 @@ void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>
 }
 
 // Buffers of both fronts at their largest sizes for a batch of m updates, so
-// that no front allocates while another stream may use its memory.
-void front_reserve(mf_ctx* c, int64_t m) {
+// that no front allocates while another stream may use its memory.  Bitmaps,
+// sums and counters start at zero, and every front leaves them so.
+void front_reserve(mf_ctx* c, int64_t m, bool clear) {
+  cudaStream_t s = c->stream;
   const int64_t words = ((int64_t)c->n + 31) / 32;
-  const int64_t bblocks = (words + kBitsWords - 1) / kBitsWords;
   const int64_t max_ns = 2 * std::min<int64_t>(m, kMaxBatchEdges);
+  auto zeroed = [&](auto& buf, int64_t count) {
+    const bool grown = buf.cap < count;
+    buf.reserve(count);
+    if (grown || clear) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
+  };
   for (auto& f : c->front) {
-    f.bits.reserve(std::max<int64_t>(2 * words, 1));
-    f.bits_sums.reserve(bblocks + 1);
-    f.uacc.reserve(std::max<int64_t>(max_ns, 1));
+    zeroed(f.bits, std::max<int64_t>(2 * words, 1));
+    zeroed(f.uacc, std::max<int64_t>(max_ns, 1));
+    zeroed(f.cnt, 3);
     f.hlist.reserve(std::max<int32_t>(c->n, 1));
     f.cands.reserve(kMaxRows);
     f.lb_offs.reserve(2 * max_ns + 2);
-    f.cnt.reserve(2);
   }
 }
 
 // Front of a sub-batch with `ns` seeds: hop-1 and seed bitmaps, the hop-1
 // list and the candidate list in ascending id (no row map yet), and the
 // packed-size upper bound; cnt[0] = (hop-1 << 32 | candidates), cnt[1] =
-// bound.  Everything on stream `st`; it reads only the graph, the seeds and
+// bound, both also in the pinned words `host` once the stream has passed the
+// front.  Everything on stream `st`; it reads only the graph, the seeds and
 // the per-batch size caches.
-void front_compute(mf_ctx* c, Front& f, const int32_t* seeds, int64_t ns, cudaStream_t st) {
+void front_compute(mf_ctx* c, Front& f, const int32_t* seeds, int64_t ns, cudaStream_t st, int64_t* host) {
   const GraphView g = c->view();
-  const int32_t n = c->n;
-  const int64_t words = ((int64_t)n + 31) / 32;
-  const int64_t bblocks = (words + kBitsWords - 1) / kBitsWords;
+  const int64_t words = ((int64_t)c->n + 31) / 32;
   uint32_t* hbits = f.bits.p;
   uint32_t* sbits = f.bits.p + words;
-  MF_CUDA(cudaMemsetAsync(hbits, 0, sizeof(uint32_t) * (size_t)(2 * words), st));
-  MF_CUDA(cudaMemsetAsync(f.uacc.p, 0, sizeof(unsigned long long) * (size_t)std::max<int64_t>(ns, 1), st));
-  MF_CUDA(cudaMemsetAsync(f.cnt.p + 1, 0, sizeof(int64_t), st));
   row_offsets_into(c, seeds, ns, f.lb_offs, f.ws, st);
-  MF_K(launch_pdl(k_lb_hop1_bound, lb_grid(c, k_lb_hop1_bound), kTB, 0, st, g, c->deg.p, seeds, f.lb_offs.p, ns, hbits, f.uacc.p,
-                                                                    c->work.p + 2 * kStHop1));
-  if (ns > 0) MF_K(launch_pdl(k_seed_bits, grid_for(ns), kTB, 0, st, seeds, ns, sbits));
+  MF_K(launch_pdl(k_lb_hop1_bound, lb_grid(c, k_lb_hop1_bound), kTB, 0, st, g, c->deg.p, seeds, f.lb_offs.p, ns, hbits,
+                  sbits, f.uacc.p, c->work.p + 2 * kStHop1));
   const int64_t capc = std::max<int64_t>(0, kMaxRows - ns);
-  MF_K(launch_pdl(k_bits_reduce, (unsigned)bblocks, kBitsThreads, 0, st, hbits, sbits, words, f.bits_sums.p));
-  MF_K(launch_pdl(k_bits_scan_sums, 1, kBitsThreads, 0, st, f.bits_sums.p, bblocks, f.cnt.p));
-  MF_K(launch_pdl(k_bits_compact, (unsigned)bblocks, kBitsThreads, 0, st, hbits, sbits, words, f.bits_sums.p, capc, ns,
-                                                                  f.hlist.p, f.cands.p, nullptr));
-  MF_K(launch_pdl(k_bound_finish, lb_grid(c, k_bound_finish), kTB, 0, st, 
-      g, seeds, ns, f.cands.p, f.cnt.p, capc, f.uacc.p, c->n2cache.p, c->n2stamp.p, c->n2bound.p, c->n2bstamp.p,
-      c->n2batch, reinterpret_cast<unsigned long long*>(f.cnt.p + 1)));
+  scan_detail::scan_exclusive_to(BitsCount{hbits, sbits},
+                                 BitsLists{hbits, sbits, words, capc, f.hlist.p, f.cands.p, f.cnt.p}, words, f.ws, st);
+  const unsigned grid = std::min(lb_grid(c, k_bound_finish), grid_for(std::max<int64_t>(ns + c->n, 2 * words)));
+  MF_K(launch_pdl(k_bound_finish, grid, kTB, 0, st, g, seeds, ns, f.cands.p, f.cnt.p, capc, f.uacc.p, c->n2cache.p,
+                  c->n2stamp.p, c->n2bound.p, c->n2bstamp.p, c->n2batch, f.bits.p, 2 * words, host));
 }
 
 double host_ms() {
@@ -3452,19 +3467,8 @@ bool host_rounds_forced() {
   return forced;
 }
 
-// Repair of one sub-batch: c->vals holds the order (sub-batch indices),
-// nproc entries.  Returns the number of speculative rounds.
-int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t ns) {
-  cudaStream_t s = c->stream;
-  int64_t* h = c->h_counters;
-  unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
-  const uint32_t* order = c->vals.p;
-  if (sequential_repair_forced()) {
-    RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order, nproc, ns, c->v2i.p, c->mis.p};
-    MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
-    MF_CUDA(cudaGetLastError());
-    return 0;
-  }
+// The repair's buffers for up to nproc edges.
+void repair_reserve(mf_ctx* c, int64_t nproc) {
   c->rp_w0.reserve(nproc);
   c->rp_w1.reserve(nproc);
   c->rp_n0.reserve(nproc);
@@ -3487,16 +3491,40 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     MF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
     c->big_grid = 4 * sms;
   }
+}
+
+// The rounds of a sub-batch may be queued with their start, view and count on
+// the device.
+bool queued_rounds(int64_t most) { return most <= kRoundCap && !host_rounds_forced() && !debug_counters(); }
+
+// Repair of one sub-batch: c->vals holds the order (sub-batch indices),
+// nproc entries.  With `prepared`, k_assign_small has made the order and the
+// start, nproc is an upper bound, and the read-back of the rounds brings the
+// edge and cluster counts (h[62], h[63]).  Returns the number of speculative
+// rounds.
+int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t ns, bool prepared) {
+  cudaStream_t s = c->stream;
+  int64_t* h = c->h_counters;
+  unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
+  const uint32_t* order = c->vals.p;
+  if (sequential_repair_forced()) {
+    RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order, nproc, ns, c->v2i.p, c->mis.p};
+    MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
+    MF_CUDA(cudaGetLastError());
+    return 0;
+  }
+  repair_reserve(c, nproc);
   const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
   int64_t p0 = 0, nview = 0, rounds = 0;
-  if (nproc <= kRoundCap && !host_rounds_forced() && !debug_counters()) {
+  if (prepared || queued_rounds(nproc)) {
     // Every round fits one commit block: rounds are queued kRoundsPerSync at
     // a time and read back once; a queued round finds its start and view on
     // the device and does nothing once the repair is done.  Round r writes
     // into one pair of result buffers and compares with the other, in turn.
     int64_t* dyn = c->counters.p + 58;
-    MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 6)), kTB, 0, s, c->rp_w0.p, c->rp_w1.p, nproc,
-                    dyn, c->counters.p + 24));
+    if (!prepared)
+      MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 6)), kTB, 0, s, c->rp_w0.p, c->rp_w1.p, nproc,
+                      dyn, c->counters.p + 24));
     std::optional<StageScope> dsc;
     int64_t queued = 0;
     while (true) {
@@ -3521,7 +3549,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
         MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, o0, o1, r0, r1, (int64_t)0, nproc, c->bins.p, p, order,
                         c->rp_keys.p, c->rp_vals.p, (int64_t)0, c->mis.p, ucnt + 20, a, c->big_best.p));
       }
-      MF_CUDA(cudaMemcpyAsync(h + 58, dyn, sizeof(int64_t) * 4, cudaMemcpyDeviceToHost, s));
+      MF_CUDA(cudaMemcpyAsync(h + 58, dyn, sizeof(int64_t) * 6, cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
       dsc.reset();
       if (h[60] != 0) break;
@@ -3529,6 +3557,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
         // round limit: the rest in order by the sequential kernel
         p0 = h[58];
         nview = h[59];
+        nproc = h[62];
         if (nview > 0) MF_K(k_spec_clear_flags<<<grid_for(nview), kTB, 0, s>>>(c->rp_keys.p, nview, c->mis.p));
         RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, c->v2i.p, c->mis.p};
         MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
@@ -3651,8 +3680,16 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(cnt);
   int64_t* h = c->h_counters;
 
+  // a batch that failed midway leaves scratch that must be zero between
+  // batches; the next one clears it whole
+  const bool dirty = c->mid_batch;
+  if (dirty) {
+    MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
+    if (c->akill.cap > 0) MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
+  }
   std::optional<StageScope> sc;
   sc.emplace(c, kStOverlay);
+  c->mid_batch = true;
   apply_overlay(c, in, m);
   sc.reset();
   if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
@@ -3752,6 +3789,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   MF_CUDA(cudaEventSynchronize(c->ev_a));
   if (c->h_plan[1] != 0) {
     MF_CUDA(cudaStreamSynchronize(s));
+    c->mid_batch = dirty;
     MF_FAIL(MF_EINVAL, "update endpoints must be distinct vertex ids in [0, n)");
   }
   swap_overlay(c, c->h_plan[2], c->h_plan[3]);
@@ -3767,10 +3805,11 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   // previous sub-batch on the second stream for large graphs; for small ones
   // the stream switch costs more than the front, which then runs inline.
   const bool overlap_fronts = c->n >= (1 << 20);
-  front_reserve(c, m);
+  front_reserve(c, m, dirty);
   int cur = 0;
   bool front_on_b = false;
-  front_compute(c, c->front[0], c->seeds_all.p, seed_end.empty() ? 0 : seed_end[0], s);
+  front_compute(c, c->front[0], c->seeds_all.p, seed_end.empty() ? 0 : seed_end[0], s, h + kFrontSlot);
+  MF_CUDA(cudaEventRecord(c->ev_b, s));
 
   int64_t p = 0;
   while (p < m) {
@@ -3781,8 +3820,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
 
     // ---- seeds (first appearance) of this sub-batch into their rows
     sc.emplace(c, kStSeeds);
-    if (ns > 0)
-      MF_K(launch_pdl(k_seed_rows, grid_for(ns), kTB, 0, s, c->seeds_all.p + seed_base, ns, c->seeds.p, c->v2i.p));
+    MF_K(launch_pdl(k_seed_rows, grid_for(ns), kTB, 0, s, c->seeds_all.p + seed_base, ns, c->seeds.p, c->v2i.p, ucnt));
     const int64_t max_before = c->max_csr;
 
     // ---- hop-1 set and size bound: this sub-batch's front (computed on the
@@ -3797,26 +3835,19 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     std::swap(c->cands, fr.cands);
 
     // ---- packed sizes (upper bound) and MAX_CSR_ELEMENTS growth.  The
-    // hop-1 counts and the bound: a front computed on the second stream
-    // copied them to its own host slot there, and by now has long finished,
-    // so this stream keeps its queue; otherwise one round trip here.
+    // front wrote its counts and bound to its pinned words; one computed while
+    // the previous sub-batch ran has long finished, and this stream keeps its
+    // queue.
     sc.emplace(c, kStSizes);
-    if (front_on_b) {
-      MF_CUDA(cudaEventSynchronize(c->ev_b));
-      h[2] = h[kFrontSlot + 2 * cur];
-      h[3] = h[kFrontSlot + 2 * cur + 1];
-    } else {
-      MF_CUDA(cudaMemcpyAsync(h + 2, fr.cnt.p, sizeof(int64_t) * 2, cudaMemcpyDeviceToHost, s));
-      MF_CUDA(cudaStreamSynchronize(s));
-    }
-    h[4] = h[3];
+    MF_CUDA(cudaEventSynchronize(c->ev_b));
+    h[2] = h[kFrontSlot + 2 * cur];
+    h[4] = h[kFrontSlot + 2 * cur + 1];
     h[3] = h[2] & 0xffffffffll;
     h[2] = h[2] >> 32;
     const int64_t nh = h[2];
     const int64_t capc = std::max<int64_t>(0, kMaxRows - ns);
     const int64_t nct = std::min<int64_t>(h[3], capc);
     const int64_t rows = ns + nct;
-    if (nct > 0) MF_K(launch_pdl(k_cand_v2i, grid_for(nct), kTB, 0, s, c->cands.p, nct, ns, c->v2i.p));
     int64_t packed = -1;
     int64_t cand_total = h[4];   // entries of the candidate rows: the bound, exact below if sized
     const bool exact = h[4] >= c->max_csr;
@@ -3888,14 +3919,15 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
         MF_CUDA(cudaEventRecord(c->ev_a, s));
         MF_CUDA(cudaStreamWaitEvent(c->stream_b, c->ev_a, 0));
         g_alloc_stream = c->stream_b;   // any scratch the front's scans grow belongs to its stream
-        front_compute(c, c->front[cur ^ 1], c->seeds_all.p + seed_base_next, ns_next, c->stream_b);
-        MF_CUDA(cudaMemcpyAsync(h + kFrontSlot + 2 * (cur ^ 1), c->front[cur ^ 1].cnt.p, sizeof(int64_t) * 2,
-                                cudaMemcpyDeviceToHost, c->stream_b));
+        front_compute(c, c->front[cur ^ 1], c->seeds_all.p + seed_base_next, ns_next, c->stream_b,
+                      h + kFrontSlot + 2 * (cur ^ 1));
         g_alloc_stream = s;
         MF_CUDA(cudaEventRecord(c->ev_b, c->stream_b));
         front_on_b = true;
       } else {
-        front_compute(c, c->front[cur ^ 1], c->seeds_all.p + seed_base_next, ns_next, s);
+        front_compute(c, c->front[cur ^ 1], c->seeds_all.p + seed_base_next, ns_next, s,
+                      h + kFrontSlot + 2 * (cur ^ 1));
+        MF_CUDA(cudaEventRecord(c->ev_b, s));
       }
     }
 
@@ -3908,15 +3940,13 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     c->mq_idx.reserve(std::max<int64_t>(ns, 1));
     c->mq_v.reserve(std::max<int64_t>(ns, 1));
     c->mq_base.reserve(std::max<int64_t>(ns, 1));
-    // [33] live rows, [34] need seeds, [35] their neighbours, [36] the pull's
-    // long rows; [48, 49], [51, 52], [53, 54] the queues of the three
-    // first-hit searches, [50] the chunk queue of the need seeds' rows, [55]
-    // the assignment's count
-    MF_CUDA(cudaMemsetAsync(cnt + 33, 0, sizeof(int64_t) * 4, s));
-    MF_CUDA(cudaMemsetAsync(cnt + 48, 0, sizeof(int64_t) * 8, s));
+    // counters, zeroed by k_seed_rows: [33] live rows, [34] need seeds, [35]
+    // their neighbours, [36] the pull's long rows; [48, 49], [51, 52], [53, 54]
+    // the queues of the three first-hit searches, [50] the chunk queue of the
+    // need seeds' rows, [55] the assignment's count
     const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
-    MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->rowcid.p,
-                                                    c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
+    MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
+                    c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
     c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
     MF_K(launch_pdl(k_cid_bits, warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s, c->cid.p, n,
                     c->cidbits.p));
@@ -3933,10 +3963,29 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     first_hits(c, c->needv.p, ucnt + 34, ns, HasF1{c->f1.p}, ucnt + 53);
     MF_K(launch_pdl(k_need_decide, lb_grid(c, k_need_decide), kTB, 0, s, g, c->need.p, c->needv.p, ucnt + 34, c->fpos.p,
                                                                  c->f1.p, c->rowcid.p, c->creates.p));
+    // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
+    // it reads (as many per vertex as in the last batch that pulled); the
+    // push at most 12 B per entry of the candidate rows plus the 8 B per
+    // vertex of its finalising pass.  With cand_push 0 the push is taken
+    // when that bound is under half the pull's estimate (sparse candidate
+    // rows on a large graph, where the pull walks most rows to their end).
+    bool use_pull = c->symmetric && c->rows_sorted && c->tune.cand_push != 1;
+    if (use_pull && c->tune.cand_push == 0) {
+      const double push_b = 12.0 * (double)cand_total + 8.0 * (double)n;
+      const double pull_b = (28.0 + 4.0 * c->pull_visit_ratio) * (double)n;
+      if (2.0 * push_b < pull_b) use_pull = false;
+    }
+    if (use_pull) {
+      const int64_t nwords = std::max<int64_t>(((int64_t)n + 31) / 32, 1);
+      const bool grown = c->ncbits.cap < nwords;
+      c->ncbits.reserve(nwords);
+      if (grown || (dirty && c->pull_runs == 0))
+        MF_CUDA(cudaMemsetAsync(c->ncbits.p, 0, sizeof(uint32_t) * (size_t)c->ncbits.cap, s));
+    }
+    uint32_t* ncbits = use_pull ? c->ncbits.p : nullptr;
     scan_exclusive_u8(c->creates.p, c->i64b.p, rows, c->ws, s);
-    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, rows, c->i64b.p, c->rowcid.p, c->seeds.p, ns, ep,
-                    c->bval.p));
-    MF_CUDA(cudaMemcpyAsync(h + 7, c->i64b.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, rows, c->i64b.p, c->rowcid.p, c->seeds.p, ns, c->cands.p, ep,
+                    c->bval.p, ncbits));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
     row_offsets(c, c->seeds.p, ns, kCntSeedRows, ns, ep);
@@ -3957,27 +4006,10 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                                                                  c->wval.p, wk_extra + 1));
     sc.emplace(c, kStPush);
     if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
-    // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
-    // it reads (as many per vertex as in the last batch that pulled); the
-    // push at most 12 B per entry of the candidate rows plus the 8 B per
-    // vertex of its finalising pass.  With cand_push 0 the push is taken
-    // when that bound is under half the pull's estimate (sparse candidate
-    // rows on a large graph, where the pull walks most rows to their end).
-    bool use_pull = c->symmetric && c->rows_sorted && c->tune.cand_push != 1;
-    if (use_pull && c->tune.cand_push == 0) {
-      const double push_b = 12.0 * (double)cand_total + 8.0 * (double)n;
-      const double pull_b = (28.0 + 4.0 * c->pull_visit_ratio) * (double)n;
-      if (2.0 * push_b < pull_b) use_pull = false;
-    }
     sc.emplace(c, use_pull ? kStPull : kStPush);
     if (use_pull) {
       ++c->pull_runs;
       c->pull_long.reserve(std::max<int32_t>(n, 1));
-      const int64_t nwords = ((int64_t)n + 31) / 32;
-      c->ncbits.reserve(std::max<int64_t>(nwords, 1));
-      MF_CUDA(cudaMemsetAsync(c->ncbits.p, 0, sizeof(uint32_t) * (size_t)nwords, s));   // [36] zeroed above
-      if (nct > 0)
-        MF_K(launch_pdl(k_cand_bits, grid_for(nct), kTB, 0, s, c->cands.p, nct, ns, c->rowcid.p, c->ncbits.p));
       const PullArgs pa{g,  c->v2i.p, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
                         ucnt + 36, wk_extra + 2, c->tune.pull_long};
       MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
@@ -4007,23 +4039,39 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       if (packed >= 0) tr->row_len = fetch(c->rowlens.p, rows, s);
     }
 
-    // ---- assignment + order (cluster ascending, index descending)
+    // ---- assignment + order (cluster ascending, index descending), then the
+    // repair (it times itself: rounds vs grid-wide searches).  A sub-batch
+    // whose edges fit one commit block is assigned and ordered by one launch,
+    // and the host first hears of it when it reads the rounds back.
     sc.emplace(c, kStAssign);
-    const int tbits = bits_for(std::max<int64_t>(q - p - 1, 1));   // the sub-batch index of an edge
-    MF_K(launch_pdl(k_assign, grid_for(q - p), kTB, 0, s, c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows, tbits,
-                    c->keys.p, c->vals.p, ucnt + 55));
-    MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaStreamSynchronize(s));
-    const int64_t cc = h[7];
-    const int64_t limit = std::min<int64_t>(cc, kMaxBatchEdges);
-    const int64_t nproc = h[9];
+    int64_t nproc, cc;
+    if (queued_rounds(q - p) && !sequential_repair_forced()) {
+      repair_reserve(c, q - p);
+      const unsigned threads = q - p <= 256 ? 256 : 1024;
+      MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)(q - p), c->cid.p, c->i64b.p + rows,
+                      bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1)), c->vals.p, c->rp_w0.p,
+                      c->rp_w1.p, c->counters.p + 58, c->counters.p + 24));
+      sc.reset();
+      const int64_t rounds = repair(c, g, p, q - p, ns, true);
+      nproc = h[62];
+      cc = h[63];
+      if (nproc > 0) c->stats.repair_rounds += rounds;
+    } else {
+      const int tbits = bits_for(std::max<int64_t>(q - p - 1, 1));   // the sub-batch index of an edge
+      MF_CUDA(cudaMemcpyAsync(h + 7, c->i64b.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      MF_K(launch_pdl(k_assign, grid_for(q - p), kTB, 0, s, c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows, tbits,
+                      c->keys.p, c->vals.p, ucnt + 55));
+      MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      MF_CUDA(cudaStreamSynchronize(s));
+      cc = h[7];
+      const int64_t limit = std::min<int64_t>(cc, kMaxBatchEdges);
+      nproc = h[9];
+      radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, tbits + bits_for(std::max<int64_t>(limit, 1)), c->ws,
+                                s);
+      sc.reset();
+      if (nproc > 0) c->stats.repair_rounds += repair(c, g, p, nproc, ns, false);
+    }
     if (tr) tr->hdr[6] = cc;
-    radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, tbits + bits_for(std::max<int64_t>(limit, 1)), c->ws,
-                              s);
-
-    // ---- repair (times itself: rounds vs grid-wide searches)
-    sc.reset();
-    if (nproc > 0) c->stats.repair_rounds += repair(c, g, p, nproc, ns);
     sc.reset();
     if (tr) {
       tr->hdr[7] = nproc;
@@ -4035,7 +4083,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
 
     // ---- clear (mapped vertices only)
     sc.emplace(c, kStClear);
-    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p));
+    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
+                    ncbits));
     MF_CUDA(cudaGetLastError());
 
     sc.reset();
@@ -4050,6 +4099,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     cur ^= 1;
   }
   if (front_on_b) MF_CUDA(cudaStreamSynchronize(c->stream_b));
+  c->mid_batch = false;
   c->stats.max_csr = c->max_csr;
   if (c->profile & 4) {
     MF_CUDA(cudaMemcpyAsync(h + 56, cnt + 56, sizeof(int64_t) * 2, cudaMemcpyDeviceToHost, s));
