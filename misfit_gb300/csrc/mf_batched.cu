@@ -426,6 +426,7 @@ void apply_batches(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
       const int64_t i = kitems[j].idx;
       mf_ctx* c = ctxs[i];
       const int64_t* out = E.h_out + cta::kOutWords * j;
+      c->max_row = -1;   // the kernel does not keep track of the longest row
       if (out[cta::kOutStatus] != 0) {
         bad_items.push_back(i);
         continue;

@@ -590,6 +590,9 @@ struct mf_ctx {
   mf::DBuf<int64_t> aoff, aoff_alt;
   mf::DBuf<int32_t> aadj, aown, aadj_alt, aown_alt;
   int64_t a_total = 0;
+  // no row has more positions (base and added); -1: not known, the next plain
+  // batch looks
+  int64_t max_row = -1;
 
   mf::DBuf<uint8_t> mis;
   mf::DBuf<int32_t> cid, v2i;
@@ -858,9 +861,10 @@ constexpr int64_t kSmallBatch = 4096;
 constexpr int kCntBad = 2 * kStCount + 8;        // lines with invalid endpoints
 constexpr int kCntAppended = kCntBad + 1;        // entries added to the overlay
 constexpr int kCntKilled = kCntBad + 2;          // added entries that go
+constexpr int kCntMaxRow = kCntBad + 3;          // longest row of the lines' vertices, or more
 constexpr int kWorkWords = kCntBad + 8;
 // The batch plan in pinned memory: [0] sub-batches, [1] invalid lines, [2, 3]
-// appended and killed entries, from [8] the first kPlanHost {cut, estimate,
+// appended and killed entries, [4] kCntMaxRow, from [8] the first kPlanHost {cut, estimate,
 // seed end} records.
 constexpr int64_t kPlanHost = 160;
 constexpr int64_t kPlanWords = 8 + 3 * kPlanHost;

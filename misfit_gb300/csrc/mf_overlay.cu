@@ -41,6 +41,20 @@ __global__ void k_base_degree(const int64_t* nindex, int32_t n, int32_t* deg) {
   if (x < n) deg[x] = (int32_t)(nindex[x + 1] - nindex[x]);
 }
 
+// The longest row (base and added positions).
+__global__ void k_max_row(GraphView g, unsigned long long* out) {
+  const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  long long len = x < g.n ? (long long)row_positions(g, (int32_t)x) : 0;
+  for (int o = 16; o > 0; o >>= 1) len = max(len, __shfl_xor_sync(0xffffffffu, len, o));
+  __shared__ long long s_len[kTB / 32];
+  if ((threadIdx.x & 31) == 0) s_len[threadIdx.x >> 5] = len;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kTB / 32; ++w) len = max(len, s_len[w]);
+    atomicMax(out, (unsigned long long)len);
+  }
+}
+
 // Rows non-decreasing?  (Sorted rows allow binary search for a neighbour.)
 // Load-balanced over all entries: each entry compares with its predecessor
 // in the same row.  flags[0] cleared on a descent.
@@ -346,8 +360,10 @@ __global__ void k_apply_pairs(GraphView g, uint32_t* live, int32_t* dead, int32_
   }
   if (appended) {
     app_line[last_seq] = 1;
-    atomicAdd(adelta + a, 1);
-    atomicAdd(adelta + b, 1);
+    // at least the new length of either row (other pairs may take entries yet)
+    const long long la = row_positions(g, a) + atomicAdd(adelta + a, 1) + 1;
+    const long long lb = row_positions(g, b) + atomicAdd(adelta + b, 1) + 1;
+    atomicMax(cnt + (kCntMaxRow - kCntBad), (unsigned long long)max(la, lb));
     ++da;
     ++db;
     atomicAdd(cnt + (kCntAppended - kCntBad), 2ull);
@@ -668,6 +684,7 @@ void upload_base(mf_ctx* c, int32_t n, const int64_t* nindex, const int32_t* nli
     c->symmetric = true;
   }
   c->max_csr = initial_max_csr(n, c->header_edges);
+  c->max_row = -1;
 }
 
 // The n-sized scratch with its initial values: no row mapped (v2i = -1),
@@ -734,6 +751,7 @@ void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m) {
                                              c->vals.p, c->slot_keys.p, c->slot_vals.p, c->work.p + kCntBad));
     pairs = radix_group_pairs(c->keys.p, c->vals.p, m, gbits, c->ws, s);
   }
+  if (c->max_row < 0) MF_K(k_max_row<<<grid_for(c->n), kTB, 0, s>>>(c->view(), c->work.p + kCntMaxRow));
   MF_K(launch_pdl(k_apply_pairs, grid_for(m), kTB, 0, s, c->view(), c->live.p, c->dead.p, c->rcnt.p, c->deg.p,
                   c->rows_sorted, pairs.keys, pairs.vals, m, nbits, gbits, c->bu.p, c->bv.p, c->bins.p, c->adelta.p,
                   c->akill.p, c->app_line.p, c->work.p + kCntBad));

@@ -160,7 +160,7 @@ __device__ int64_t plan_cuts(const int32_t* u, const int32_t* v, const int32_t* 
 // Header of the plan in pinned memory (see kPlanWords).
 __device__ __forceinline__ void plan_header(int64_t count, const unsigned long long* bc, int64_t* host) {
   host[0] = count;
-  for (int k = 0; k < 3; ++k) host[1 + k] = (int64_t)bc[k];
+  for (int k = 0; k < 4; ++k) host[1 + k] = (int64_t)bc[k];
 }
 
 __device__ __forceinline__ void plan_record(int64_t k, const int64_t* cuts, const int64_t* ests, int64_t seed_end,
@@ -1764,6 +1764,218 @@ __global__ void k_lb_push_cand(GraphView g, const int32_t* cands, const int64_t*
   add_work(work, vis);
 }
 
+// ---- short rows ----------------------------------------------------------------------
+// On a graph whose rows all have at most kShortRow positions (meshes, random
+// graphs) a row is one small group's work: eight lanes read it, sixteen
+// positions a step, from its first position, and no prefix of row lengths, queue
+// of open rows or second and third level is needed.  Each kernel here stands
+// for two to nine launches of the general path (a row-length scan and a
+// load-balanced walk each; probe, warp and chunk levels of a first-hit
+// search), which on such graphs last as long as their launches: 1,003 lines
+// on a mesh of 99,991 vertices ran 46 launches of 2.5 to 16 us a sub-batch.  A
+// lane reads at most kShortRow / 8 positions of a row in turn, and in
+// k_need_short a whole row, which sets the limit.
+constexpr int64_t kShortRow = 128;
+constexpr int kGroup = 8;   // lanes per row
+
+struct ShortRow {
+  int64_t b0, a0;
+  int32_t nb, np;   // base positions, all positions
+  bool filt;
+};
+
+__device__ __forceinline__ ShortRow short_row(const GraphView& g, int32_t x) {
+  ShortRow r;
+  r.b0 = g.nindex[x];
+  r.nb = (int32_t)(g.nindex[x + 1] - r.b0);
+  r.a0 = g.aoff[x];
+  r.np = r.nb + (int32_t)(g.aoff[x + 1] - r.a0);
+  r.filt = g.dead[x] != 0;
+  return r;
+}
+
+__device__ __forceinline__ int32_t short_elem(const GraphView& g, const ShortRow& r, int32_t k) {
+  if (k >= r.np) return -1;
+  if (k >= r.nb) return g.aadj[r.a0 + (k - r.nb)];
+  return !r.filt || live_at(g.live, r.b0 + k) ? __ldg(g.nlist + r.b0 + k) : -1;
+}
+
+// f(y) for this lane's share of the live elements of row r.
+template <class F>
+__device__ __forceinline__ int64_t short_each(const GraphView& g, const ShortRow& r, F f) {
+  int64_t visited = 0;
+  for (int32_t k = threadIdx.x & (kGroup - 1); k < r.np; k += 2 * kGroup) {
+    const int32_t y0 = short_elem(g, r, k), y1 = short_elem(g, r, k + kGroup);
+    if (y0 >= 0) { f(y0); ++visited; }
+    if (y1 >= 0) { f(y1); ++visited; }
+  }
+  return visited;
+}
+
+__device__ __forceinline__ int64_t group_id() {
+  return ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kGroup;
+}
+
+__device__ __forceinline__ void add_work_if(unsigned long long* work, int64_t visited) {
+  if (work) add_work(work, visited);
+}
+
+// k_lb_hop1_bound without the prefix.
+__global__ void k_hop1_short(GraphView g, const int32_t* deg, const int32_t* seeds, int64_t ns, uint32_t* hbits,
+                             uint32_t* sbits, unsigned long long* uacc, unsigned long long* work) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = group_id();
+  unsigned long long acc = 0;
+  int64_t vis = 0;
+  const bool lead = (threadIdx.x & (kGroup - 1)) == 0;
+  if (i < ns) {
+    const int32_t s = seeds[i];
+    if (lead) atomicOr(sbits + (s >> 5), 1u << (s & 31));
+    vis = short_each(g, short_row(g, s), [&](int32_t y) {
+      const uint32_t bit = 1u << (y & 31);
+      acc += (unsigned long long)__ldg(deg + y);
+      if (!(hbits[y >> 5] & bit)) atomicOr(hbits + (y >> 5), bit);
+    });
+  }
+  for (int o = 1; o < kGroup; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (i < ns && lead) uacc[i] = acc;
+  add_work_if(work, vis);
+}
+
+// k_row_skip, the first-hit search of the rows and k_live_decide: the group
+// tests the ids themselves, so no bitmap of them is built.
+__global__ void k_first_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct,
+                              const int32_t* cid, int32_t* v2i, int32_t* rowcid, uint8_t* creates, int32_t* need,
+                              int32_t* needv, unsigned long long* nneed) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = group_id();
+  const int gl = threadIdx.x & (kGroup - 1);
+  const int g0 = threadIdx.x & 31 & ~(kGroup - 1);   // the group's first lane
+  const bool valid = i < ns + nct;
+  const int32_t x = valid ? (i < ns ? seeds[i] : cands[i - ns]) : 0;
+  const int32_t own = valid ? cid[x] : 0;
+  bool open = valid && own == -1;
+  ShortRow r{};
+  if (open) r = short_row(g, x);
+  int32_t id = -1;
+  for (int32_t k0 = 0; __any_sync(0xffffffffu, open && k0 < r.np); k0 += 2 * kGroup) {
+    int32_t y[2], c[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) y[q] = open ? short_elem(g, r, k0 + q * kGroup + gl) : -1;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) c[q] = y[q] >= 0 ? cid[y[q]] : -1;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const unsigned m = (__ballot_sync(0xffffffffu, c[q] != -1) >> g0) & ((1u << kGroup) - 1u);
+      const int32_t first = __shfl_sync(0xffffffffu, c[q], m ? g0 + __ffs(m) - 1 : 0);
+      if (open && m) {
+        id = first;
+        open = false;
+      }
+    }
+  }
+  if (!valid || gl != 0) return;
+  if (i >= ns) v2i[x] = (int32_t)i;
+  rowcid[i] = own != -1 ? kSkip : id;
+  creates[i] = own == -1 && id == -1 ? 1 : 0;
+  if (own == -1 && id == -1 && i < ns) {
+    const unsigned long long u = atomicAdd(nneed, 1ull);
+    need[u] = (int32_t)i;
+    needv[u] = x;
+  }
+}
+
+// The hop-2 part of the seeds without an id in their own row: the id of the
+// first element with one in the first row(h), h over row(s) in order, that has
+// any.  One warp per seed, one h per lane.
+__global__ void k_need_short(GraphView g, const int32_t* need, const int32_t* needv, const unsigned long long* dcnt,
+                             const int32_t* cid, int32_t* rowcid, uint8_t* creates) {
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int64_t cnt = (int64_t)*dcnt, nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t u = warp_id(); u < cnt; u += nw) {
+    const ShortRow r = short_row(g, needv[u]);
+    for (int32_t k0 = 0; k0 < r.np; k0 += 32) {
+      const int32_t h = short_elem(g, r, k0 + lane);
+      int32_t id = -1;
+      if (h >= 0) {
+        const ShortRow rh = short_row(g, h);
+        for (int32_t j0 = 0; j0 < rh.np && id == -1; j0 += 8) {
+          int32_t y[8], c[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) y[q] = short_elem(g, rh, j0 + q);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) c[q] = y[q] >= 0 ? cid[y[q]] : -1;
+#pragma unroll
+          for (int q = 7; q >= 0; --q)
+            if (c[q] != -1) id = c[q];
+        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, id != -1);
+      if (m) {
+        id = __shfl_sync(0xffffffffu, id, __ffs(m) - 1);
+        if (lane == 0) {
+          rowcid[need[u]] = id;
+          creates[need[u]] = 0;
+        }
+        break;
+      }
+    }
+  }
+}
+
+// k_lb_push_seed without the prefix.
+__global__ void k_push_seed_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* rowcid, uint32_t epoch,
+                                  uint32_t* bval, unsigned long long* work) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = group_id();
+  int64_t vis = 0;
+  if (i < ns && rowcid[i] != kSkip) {
+    const uint32_t tag = (epoch << kRowBits) | (uint32_t)i;
+    vis = short_each(g, short_row(g, seeds[i]), [&](int32_t y) { push_w(bval, y, tag); });
+  }
+  add_work_if(work, vis);
+}
+
+// k_self_push, both k_lb_push_hop passes and (nct > 0) k_lb_push_cand: all of
+// them only raise wval, so their order does not matter.
+__global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* hlist, int64_t nh,
+                                 const int32_t* cands, int64_t nct, const int32_t* v2i, const int32_t* rowcid,
+                                 uint32_t epoch, const uint32_t* bval, uint32_t* wval, unsigned long long* work_hop,
+                                 unsigned long long* work_cand) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t i = group_id();
+  int64_t vis = 0;
+  bool cand = false;
+  if (i < ns + nh) {
+    const int32_t x = i < ns ? seeds[i] : hlist[i - ns];
+    const uint32_t tag = bval[x];
+    if ((tag >> kRowBits) == epoch) {
+      if ((threadIdx.x & (kGroup - 1)) == 0) push_w(wval, x, tag);
+      bool use = true;   // as RowCounts: seeds push as seeds, a writing candidate dominates its row
+      if (i >= ns) {
+        const int32_t vi = v2i[x];
+        use = !(vi >= 0 && ((int64_t)vi < ns || rowcid[vi] != kSkip));
+      }
+      if (use) vis = short_each(g, short_row(g, x), [&](int32_t y) { push_w(wval, y, tag); });
+    }
+  } else if (i < ns + nh + nct) {
+    const int64_t k = i - ns - nh;
+    cand = true;
+    if (rowcid[ns + k] != kSkip) {
+      const uint32_t tag = (epoch << kRowBits) | (uint32_t)(ns + k);
+      vis = short_each(g, short_row(g, cands[k]), [&](int32_t y) { push_w(wval, y, tag); });
+    }
+  }
+  add_work_if(work_hop, cand ? 0 : vis);
+  add_work_if(work_cand, cand ? vis : 0);
+}
+
 // Pull form of the candidate writes (symmetric graphs with sorted base rows).
 // The candidate rows that write are the non-skipped ones, and their tags
 // grow with the candidate's vertex id (candidates are packed in ascending
@@ -3098,9 +3310,14 @@ void front_compute(mf_ctx* c, Front& f, const int32_t* seeds, int64_t ns, cudaSt
   const int64_t words = ((int64_t)c->n + 31) / 32;
   uint32_t* hbits = f.bits.p;
   uint32_t* sbits = f.bits.p + words;
-  row_offsets_into(c, seeds, ns, f.lb_offs, f.ws, st);
-  MF_K(launch_pdl(k_lb_hop1_bound, lb_grid(c, k_lb_hop1_bound), kTB, 0, st, g, c->deg.p, seeds, f.lb_offs.p, ns, hbits,
-                  sbits, f.uacc.p, c->work.p + 2 * kStHop1));
+  if (c->max_row <= kShortRow) {
+    MF_K(launch_pdl(k_hop1_short, grid_for(ns * kGroup), kTB, 0, st, g, c->deg.p, seeds, ns, hbits, sbits, f.uacc.p,
+                    c->profile ? c->work.p + 2 * kStHop1 : nullptr));
+  } else {
+    row_offsets_into(c, seeds, ns, f.lb_offs, f.ws, st);
+    MF_K(launch_pdl(k_lb_hop1_bound, lb_grid(c, k_lb_hop1_bound), kTB, 0, st, g, c->deg.p, seeds, f.lb_offs.p, ns, hbits,
+                    sbits, f.uacc.p, c->work.p + 2 * kStHop1));
+  }
   const int64_t capc = std::max<int64_t>(0, kMaxRows - ns);
   scan_detail::scan_exclusive_to(BitsCount{hbits, sbits},
                                  BitsLists{hbits, sbits, words, capc, f.hlist.p, f.cands.p, f.cnt.p}, words, f.ws, st);
@@ -3435,6 +3652,39 @@ void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, 
     c->dbg_first[3] += (int64_t)(v[2] >> kChunkShift);
     c->dbg_first[4] += (int64_t)(v[2] & kChunkMask);
   }
+}
+
+// The clustering read of a sub-batch by the general path (rows of any length):
+// row ids and creation flags of the ns + nct rows into c->rowcid / c->creates.
+void cluster_read(mf_ctx* c, const GraphView& g, int64_t ns, int64_t nct, uint32_t ep, std::optional<StageScope>& sc) {
+  cudaStream_t s = c->stream;
+  const int32_t n = c->n;
+  const int64_t rows = ns + nct;
+  unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
+  c->live_i.reserve(std::max<int64_t>(rows, 1));
+  c->live_v.reserve(std::max<int64_t>(rows, 1));
+  c->mq_idx.reserve(std::max<int64_t>(ns, 1));
+  c->mq_v.reserve(std::max<int64_t>(ns, 1));
+  c->mq_base.reserve(std::max<int64_t>(ns, 1));
+  const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
+  MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
+                  c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
+  c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
+  MF_K(launch_pdl(k_cid_bits, warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s, c->cid.p, n,
+                  c->cidbits.p));
+  const HasCidBit has_cid{c->cidbits.p};
+  first_hits(c, c->live_v.p, ucnt + 33, rows, has_cid, ucnt + 48);
+  MF_K(launch_pdl(k_live_decide, lb_grid(c, k_live_decide), kTB, 0, s, g, c->live_i.p, c->live_v.p, ucnt + 33, ns,
+                                                               c->fpos.p, c->cid.p, c->rowcid.p, c->creates.p,
+                                                               c->seeds.p, c->need.p, c->needv.p, ucnt + 34, mq));
+  sc.emplace(c, kStFirstNeed);
+  MF_K(launch_pdl(k_mark_need, lb_grid(c, k_mark_need), kTB, 0, s, g, mq, ep, c->nmark.p, c->nlist_need.p, ucnt + 35));
+  first_hits(c, c->nlist_need.p, ucnt + 35, n, has_cid, ucnt + 51);
+  MF_K(launch_pdl(k_f1_finish, lb_grid(c, k_f1_finish), kTB, 0, s, g, c->nlist_need.p, ucnt + 35, c->fpos.p, c->cid.p,
+                                                           c->f1.p));
+  first_hits(c, c->needv.p, ucnt + 34, ns, HasF1{c->f1.p}, ucnt + 53);
+  MF_K(launch_pdl(k_need_decide, lb_grid(c, k_need_decide), kTB, 0, s, g, c->need.p, c->needv.p, ucnt + 34, c->fpos.p,
+                                                               c->f1.p, c->rowcid.p, c->creates.p));
 }
 
 void next_epoch(mf_ctx* c) {
@@ -3793,6 +4043,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     MF_FAIL(MF_EINVAL, "update endpoints must be distinct vertex ids in [0, n)");
   }
   swap_overlay(c, c->h_plan[2], c->h_plan[3]);
+  c->max_row = std::max(c->max_row, c->h_plan[4]);
   c->stats = mf_batch_stats{};
   c->stats.updates = m;
   c->stats.packed_total = -1;
@@ -3933,36 +4184,22 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
 
     // ---- clustering (bulk-synchronous); counts stay on the device
     sc.emplace(c, kStFirst);
-    c->live_i.reserve(std::max<int64_t>(rows, 1));
-    c->live_v.reserve(std::max<int64_t>(rows, 1));
-    c->need.reserve(std::max<int64_t>(ns, 1));
-    c->needv.reserve(std::max<int64_t>(ns, 1));
-    c->mq_idx.reserve(std::max<int64_t>(ns, 1));
-    c->mq_v.reserve(std::max<int64_t>(ns, 1));
-    c->mq_base.reserve(std::max<int64_t>(ns, 1));
     // counters, zeroed by k_seed_rows: [33] live rows, [34] need seeds, [35]
     // their neighbours, [36] the pull's long rows; [48, 49], [51, 52], [53, 54]
     // the queues of the three first-hit searches, [50] the chunk queue of the
     // need seeds' rows, [55] the assignment's count
-    const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
-    MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
-                    c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
-    c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
-    MF_K(launch_pdl(k_cid_bits, warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s, c->cid.p, n,
-                    c->cidbits.p));
-    const HasCidBit has_cid{c->cidbits.p};
-    first_hits(c, c->live_v.p, ucnt + 33, rows, has_cid, ucnt + 48);
-    MF_K(launch_pdl(k_live_decide, lb_grid(c, k_live_decide), kTB, 0, s, g, c->live_i.p, c->live_v.p, ucnt + 33, ns,
-                                                                 c->fpos.p, c->cid.p, c->rowcid.p, c->creates.p,
-                                                                 c->seeds.p, c->need.p, c->needv.p, ucnt + 34, mq));
-    sc.emplace(c, kStFirstNeed);
-    MF_K(launch_pdl(k_mark_need, lb_grid(c, k_mark_need), kTB, 0, s, g, mq, ep, c->nmark.p, c->nlist_need.p, ucnt + 35));
-    first_hits(c, c->nlist_need.p, ucnt + 35, n, has_cid, ucnt + 51);
-    MF_K(launch_pdl(k_f1_finish, lb_grid(c, k_f1_finish), kTB, 0, s, g, c->nlist_need.p, ucnt + 35, c->fpos.p, c->cid.p,
-                                                             c->f1.p));
-    first_hits(c, c->needv.p, ucnt + 34, ns, HasF1{c->f1.p}, ucnt + 53);
-    MF_K(launch_pdl(k_need_decide, lb_grid(c, k_need_decide), kTB, 0, s, g, c->need.p, c->needv.p, ucnt + 34, c->fpos.p,
-                                                                 c->f1.p, c->rowcid.p, c->creates.p));
+    c->need.reserve(std::max<int64_t>(ns, 1));
+    c->needv.reserve(std::max<int64_t>(ns, 1));
+    const bool short_rows = c->max_row <= kShortRow;
+    if (short_rows) {
+      MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->cands.p, nct, c->cid.p,
+                      c->v2i.p, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
+      sc.emplace(c, kStFirstNeed);
+      MF_K(launch_pdl(k_need_short, std::min(warps_grid(ns), lb_grid(c, k_need_short)), kTB, 0, s, g, c->need.p,
+                      c->needv.p, ucnt + 34, c->cid.p, c->rowcid.p, c->creates.p));
+    } else {
+      cluster_read(c, g, ns, nct, ep, sc);
+    }
     // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
     // it reads (as many per vertex as in the last batch that pulled); the
     // push at most 12 B per entry of the candidate rows plus the 8 B per
@@ -3988,24 +4225,36 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                     c->bval.p, ncbits));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
-    row_offsets(c, c->seeds.p, ns, kCntSeedRows, ns, ep);
-    MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
-    MF_K(launch_pdl(k_self_push, grid_for(ns + nh), kTB, 0, s, c->seeds.p, ns, c->hlist.p, nh, ep, c->bval.p,
-                    c->wval.p));
-    row_offsets(c, c->seeds.p, ns, kCntSeedPushers, ns, ep);
-    const unsigned long long dbg0 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
-    sc.emplace(c, kStPushHop);
-    MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p,
-                                                                 c->wval.p, wk_extra + 1));
-    sc.emplace(c, kStPush);
-    if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg0);
-    row_offsets(c, c->hlist.p, nh, kCntHopPushers, ns, ep);
-    const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
-    sc.emplace(c, kStPushHop);
-    MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->hlist.p, c->lb_offs.p, nh, ep, c->bval.p,
-                                                                 c->wval.p, wk_extra + 1));
-    sc.emplace(c, kStPush);
-    if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
+    if (short_rows) {
+      // the elements are counted for the profiler only
+      unsigned long long* wk = c->profile ? wk_extra : nullptr;
+      MF_K(launch_pdl(k_push_seed_short, grid_for(ns * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->rowcid.p, ep, c->bval.p,
+                      wk));
+      sc.emplace(c, kStPushHop);
+      const int64_t npc = use_pull ? 0 : nct;
+      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->hlist.p, nh,
+                      c->cands.p, npc, c->v2i.p, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
+                      wk ? wk + 3 : nullptr));
+    } else {
+      row_offsets(c, c->seeds.p, ns, kCntSeedRows, ns, ep);
+      MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
+      MF_K(launch_pdl(k_self_push, grid_for(ns + nh), kTB, 0, s, c->seeds.p, ns, c->hlist.p, nh, ep, c->bval.p,
+                      c->wval.p));
+      row_offsets(c, c->seeds.p, ns, kCntSeedPushers, ns, ep);
+      const unsigned long long dbg0 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
+      sc.emplace(c, kStPushHop);
+      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p,
+                                                                   c->wval.p, wk_extra + 1));
+      sc.emplace(c, kStPush);
+      if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg0);
+      row_offsets(c, c->hlist.p, nh, kCntHopPushers, ns, ep);
+      const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
+      sc.emplace(c, kStPushHop);
+      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->hlist.p, c->lb_offs.p, nh, ep, c->bval.p,
+                                                                   c->wval.p, wk_extra + 1));
+      sc.emplace(c, kStPush);
+      if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
+    }
     sc.emplace(c, use_pull ? kStPull : kStPush);
     if (use_pull) {
       ++c->pull_runs;
@@ -4013,14 +4262,17 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       const PullArgs pa{g,  c->v2i.p, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
                         ucnt + 36, wk_extra + 2, c->tune.pull_long};
       MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
-      MF_K(launch_pdl(k_pull_cand_long, lb_grid(c, k_pull_cand_long), kTB, 0, s, pa));
+      if (c->max_row > c->tune.pull_long)
+        MF_K(launch_pdl(k_pull_cand_long, lb_grid(c, k_pull_cand_long), kTB, 0, s, pa));
       // per vertex: row bounds (8 B of nindex, 8 B of aoff), tombstone count,
       // tag and id (4 B each); the row entries read are counted on the device
       if (c->profile) c->stage_bytes[kStPull] += 28.0 * (double)n;
     } else {
-      row_offsets(c, c->cands.p, nct, kCntCandRows, ns, ep);
-      MF_K(launch_pdl(k_lb_push_cand, lb_grid(c, k_lb_push_cand), kTB, 0, s, g, c->cands.p, c->lb_offs.p, nct, ns, ep, c->wval.p,
-                                                     wk_extra + 3));
+      if (!short_rows) {
+        row_offsets(c, c->cands.p, nct, kCntCandRows, ns, ep);
+        MF_K(launch_pdl(k_lb_push_cand, lb_grid(c, k_lb_push_cand), kTB, 0, s, g, c->cands.p, c->lb_offs.p, nct, ns, ep,
+                        c->wval.p, wk_extra + 3));
+      }
       MF_K(launch_pdl(k_finalize_all, grid_for(((int64_t)n + 3) / 4), kTB, 0, s, c->wval.p, n, ep, c->rowcid.p, c->cid.p));
     }
     c->touched_total += n;

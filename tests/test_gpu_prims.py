@@ -95,3 +95,39 @@ def test_plan_cuts(gb, m, max_csr):
         assert g.max_csr == orc.max_csr
         assert np.array_equal(g.get_mis(), orc.get_mis())
         assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
+
+
+@pytest.mark.parametrize("hub,push", [(120, 0), (126, 0), (127, 1), (128, 0), (129, 1), (140, 2)])
+def test_row_length_limit_of_short_kernels(gb, hub, push):
+    """Graphs of rows up to 128 positions take the group-per-row kernels, longer ones the general path: a hub row
+    that starts at `hub` entries and grows by a few every batch crosses the line; every stage equals the oracle's."""
+    import oracle as O
+    n = 1500
+    rng = np.random.default_rng(hub)
+    nindex, nlist = W.er_graph(n, 5, hub)
+    lo, hi = W.undirected_pairs(n, nindex, nlist)
+    keep = (lo != 7) & (hi != 7)
+    others = rng.permutation(np.delete(np.arange(n), 7))
+    nindex, nlist = W.csr_from_pairs(n, np.concatenate([lo[keep], np.full(hub, 7)]),
+                                     np.concatenate([hi[keep], others[:hub]]))
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    stream = W.ToggleStream(n, nindex, nlist, hub)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        g.set_tuning(cand_push=push)
+        for x in (g, orc):
+            x.set_mis(mis)
+            x.trace(True)
+        for b in range(4):
+            u, v, ins = stream.next_batch(150, with_flags=True)
+            more = others[hub + 2 * b:hub + 2 * b + 2].astype(np.int32)
+            u, v = np.concatenate([u, more]), np.concatenate([v, np.full(2, 7, np.int32)])
+            ins = np.concatenate([ins, np.ones(2, np.uint8)])
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            a, b2 = g.trace_records(), orc.trace_records()
+            assert len(a) == len(b2)
+            for x, y in zip(a, b2):
+                for field in (1, 2, 3, 4, 5):
+                    assert np.array_equal(x[field], y[field]), field
+            assert np.array_equal(g.get_mis(), orc.get_mis())
