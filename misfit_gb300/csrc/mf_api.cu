@@ -67,6 +67,16 @@ bool pdl_on() {
   return on;
 }
 
+void raise_smem_limit(int device, const void* kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> raised;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& have = raised[{device, kernel}];
+  if (have >= bytes) return;
+  MF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  have = bytes;
+}
+
 bool ktime_on() {
   static const bool on = [] {
     const char* e = std::getenv("MISFIT_GB_KTIME");
@@ -196,7 +206,7 @@ mf_ctx* new_ctx(int gpu) {
     MF_CUDA(cudaMallocHost(&c->h_counters, sizeof(int64_t) * (64 + mf::kPlanWords) + 9 * (size_t)mf::kSmallBatch));
     c->h_plan = c->h_counters + 64;
     c->h_stage = reinterpret_cast<uint8_t*>(c->h_plan + mf::kPlanWords);
-    c->counters.reserve(64);
+    c->counters.reserve(mf::kCounterWords);
   } catch (...) {
     release_all(c);
     delete c;

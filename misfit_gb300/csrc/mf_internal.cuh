@@ -98,6 +98,13 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 bool pdl_on();
 
+void raise_smem_limit(int device, const void* kernel, size_t bytes);
+// Raises a kernel's dynamic shared memory limit to `bytes`, once per device.
+template <typename... KArgs>
+void raise_smem(int device, void (*kernel)(KArgs...), size_t bytes) {
+  raise_smem_limit(device, reinterpret_cast<const void*>(kernel), bytes);
+}
+
 template <typename... KArgs, typename... Args>
 void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg{};
@@ -631,6 +638,7 @@ struct mf_ctx {
   mf::DBuf<int32_t> big_r;
   mf::DBuf<unsigned long long> big_best;
   int big_grid = 0;
+  int64_t repair_last = 2;   // rounds of the last queued repair
   mf::DBuf<uint32_t> bitmaps;   // per-CTA vertex bitmaps for exact 2-hop sizes
   int64_t bitmap_words = 0;
   int bitmap_ctas = 0;
@@ -848,6 +856,7 @@ struct StageScope {
 
 // mf_overlay.cu
 void upload_base(mf_ctx* c, int32_t n, const int64_t* nindex, const int32_t* nlist, int64_t nnz);
+constexpr int64_t kCounterWords = 72;   // device counters of a context
 // A batch's lines, readable by the device (device memory or pinned host memory).
 struct BatchIn {
   const int32_t* u;

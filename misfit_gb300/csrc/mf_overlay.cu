@@ -14,7 +14,6 @@
 // three-state machine none / added / tombstoned that insertEdge, removeEdge,
 // un_tombstone and forget_delta_edge implement, core/FlashGraph.h:196-275).
 #include <algorithm>
-#include <atomic>
 #include <mutex>
 
 #include "mf_internal.cuh"
@@ -260,16 +259,8 @@ __global__ void __launch_bounds__(1024) k_small_input(BatchIn in, int m, int32_t
 template <int Items>
 void small_input(mf_ctx* c, const BatchIn& in, int m, int threads, int nbits, int gbits) {
   const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * sort_detail::kDigits * 4;
-  if (smem > 48 * 1024) {
-    // raised once per device for this kernel
-    static std::atomic<unsigned long long> raised{0};
-    const unsigned long long bit = 1ull << (c->device & 63);
-    if (c->device > 63 || !(raised.load(std::memory_order_acquire) & bit)) {
-      MF_CUDA(cudaFuncSetAttribute(k_small_input<Items>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   Items * 1024 * 12 + 32 * sort_detail::kDigits * 4));
-      raised.fetch_or(bit, std::memory_order_release);
-    }
-  }
+  if (smem > 48 * 1024)
+    raise_smem(c->device, k_small_input<Items>, Items * 1024 * 12 + 32 * sort_detail::kDigits * 4);
   MF_K(k_small_input<Items><<<2, threads, smem, c->stream>>>(
       in, m, c->n, nbits, gbits, c->bu.p, c->bv.p, c->bins.p, c->app_line.p, c->keys.p, c->vals.p, c->slot_keys.p,
       c->slot_vals.p, c->prev.p, c->work.p + kCntBad));
@@ -710,7 +701,7 @@ void alloc_vertex_scratch(mf_ctx* c) {
     MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
   }
   c->epoch = 0;
-  c->counters.reserve(64);
+  c->counters.reserve(kCounterWords);
 }
 
 void flag_updates(mf_ctx* c, int64_t m) {

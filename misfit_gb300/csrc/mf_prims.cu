@@ -8,7 +8,6 @@
 // per digit, each tile finding its place by a decoupled look-back per digit
 // (Adinets and Merrill, "Onesweep", 2022).
 #include <algorithm>
-#include <atomic>
 
 #include "mf_scan.cuh"
 #include "mf_sort.cuh"
@@ -60,16 +59,9 @@ template <int Items, bool Mixed>
 void sort_block(uint64_t* keys, uint32_t* vals, int n, int threads, int first_bit, int end_bit, cudaStream_t s) {
   const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * kDigits * 4;
   if (smem > 48 * 1024) {
-    // raised once per device for this kernel
-    static std::atomic<unsigned long long> raised{0};
     int dev = 0;
     MF_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (dev > 63 || !(raised.load(std::memory_order_acquire) & bit)) {
-      MF_CUDA(cudaFuncSetAttribute(k_sort_block<Items, Mixed>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   Items * 1024 * 12 + 32 * kDigits * 4));
-      raised.fetch_or(bit, std::memory_order_release);
-    }
+    raise_smem(dev, k_sort_block<Items, Mixed>, Items * 1024 * 12 + 32 * kDigits * 4);
   }
   MF_K(launch_pdl(k_sort_block<Items, Mixed>, 1, (unsigned)threads, smem, s, keys, vals, n, first_bit, end_bit));
 }

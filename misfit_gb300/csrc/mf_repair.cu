@@ -2141,15 +2141,18 @@ __global__ void k_assign(const int32_t* u, const int32_t* v, int64_t p, int64_t 
 
 // The assignment of a sub-batch whose edges fit one commit block of the repair
 // (kRoundCap), in one launch: the assigned edges, ordered by (cluster
-// ascending, index descending), and the start of the repair -- both result
-// pairs' first buffers to "no write", the round words (see SpecArgs::dyn) and
-// the deferral counters to zero.  The counts stay on the device (dyn[4] edges,
-// dyn[5] cluster count).  A thread takes the edge with the index len - 1 - tid,
-// so a stable sort on the cluster alone gives the order.
+// ascending, index descending), and the start of the repair: the guessed
+// writes as the last round's results and as the view (see the speculative
+// repair), the round words (SpecArgs::dyn) and the deferral counters to zero.
+// The counts stay on the device (dyn[4] edges, dyn[5] cluster count).  A thread
+// takes the edge with the index len - 1 - tid, so a stable sort on the cluster
+// alone gives the order.  The guessed writes, a few of the edges, are ordered
+// by counting the smaller ones.
 __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const int32_t* v, int64_t p, int len,
-                                                       const int32_t* cid, const int64_t* ccp, int cbits,
-                                                       uint32_t* order, int32_t* w0, int32_t* w1, int64_t* dyn,
-                                                       int64_t* counts) {
+                                                       const uint8_t* ins, const int32_t* cid, const int64_t* ccp,
+                                                       int cbits, uint32_t* order, int32_t* w0, int32_t* w1,
+                                                       uint8_t* mis, uint64_t* view_keys, uint32_t* view_vals,
+                                                       int64_t* dyn, int64_t* counts) {
   pdl_wait();
   pdl_trigger();
   __shared__ uint64_t sk[1024];
@@ -2186,16 +2189,44 @@ __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const i
   uint32_t val[1] = {tid < n ? sv[tid] : 0};
   __syncthreads();
   sort_detail::block_sort<1>(false, key, val, n, 0, cbits, sk, sv, cnt, dbase, sw);
+  int32_t r = -1;
   if (tid < n) {
+    const int64_t j = p + val[0];
+    const int32_t a = u[j], b = v[j];
     order[tid] = val[0];
-    w0[tid] = -1;
+    if (ins[j] && (mis[a] & 1) && (mis[b] & 1)) r = max(a, b);
+    w0[tid] = r;
     w1[tid] = -1;
   }
-  if (tid < 4) dyn[tid] = 0;
+  const unsigned rmask = __ballot_sync(0xffffffffu, r >= 0);
+  if (lane == 0) sw[w] = __popc(rmask);
+  __syncthreads();   // also: every member byte is read
+  x = lane < warps ? sw[lane] : 0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const uint32_t rbefore = w > 0 ? __shfl_sync(0xffffffffu, x, w - 1) : 0;
+  const int nview = (int)__shfl_sync(0xffffffffu, x, 31);
+  const uint64_t mine = ((uint64_t)(uint32_t)r << 32) | (uint64_t)tid;
+  if (r >= 0) sk[rbefore + __popc(rmask & ((1u << lane) - 1u))] = mine;
+  __syncthreads();
+  if (r >= 0) {
+    int rank = 0;
+    for (int k = 0; k < nview; ++k) rank += sk[k] < mine;
+    view_keys[rank] = mine;
+    view_vals[rank] = 0;
+    mis[r] |= 2;
+  }
   if (tid < 6) counts[tid] = 0;
   if (tid == 0) {
+    dyn[0] = 0;
+    dyn[1] = nview;
+    dyn[2] = 0;
+    dyn[3] = 0;
     dyn[4] = n;
     dyn[5] = cc;
+    dyn[6] = 0;
   }
 }
 
@@ -2412,6 +2443,13 @@ __global__ void __launch_bounds__(1024) k_repair_sequential(RepairArgs a) {
 // it.  Independent edges settle in the same round; a chain of k dependent
 // edges needs k rounds.  After kMaxRounds rounds the remainder is walked by
 // the sequential kernel.
+// The queued rounds start from a guess: every insert whose ends are both
+// members now removes its larger end and nothing joins.  The first round sees
+// these writes as its view and is compared with them, so a sub-batch whose
+// guess holds (no vertex joins: the common case next to hubs) is done after one
+// round instead of two.  And when a round differs from the last only by
+// vertices that joined, the next round keeps every "nothing eligible": the
+// members it saw have only grown, and more members make nothing eligible.
 
 constexpr int kMaxRounds = 48;
 constexpr int kRoundsPerSync = 2;   // small rounds queued per host read-back
@@ -2460,9 +2498,13 @@ struct SpecArgs {
   int64_t pre_cap;
   // rounds queued without a host read-back: [0] first pending position,
   // [1] entries of the view, [2] 1 once no position changed, [3] rounds run
-  // (k_spec_round keeps them), [4] positions; p0, cnt and view.nkeys above are
-  // then ignored
+  // (k_spec_round keeps them), [4] positions, [5] cluster count, [6] 1 when the
+  // view differs from the last round's only by vertices that joined; p0, cnt
+  // and view.nkeys above are then ignored
   int64_t* dyn = nullptr;
+  const int32_t* prev0 = nullptr;   // the last round's out0 and out1 (with dyn)
+  const int32_t* prev1 = nullptr;
+  bool grown = false;               // dyn[6]
 };
 
 // A queued round's start and view from the device; false once the repair
@@ -2473,6 +2515,7 @@ __device__ __forceinline__ bool spec_dyn_load(SpecArgs& a) {
   a.p0 = a.dyn[0];
   a.view.nkeys = a.dyn[1];
   a.cnt = a.dyn[4];
+  a.grown = a.dyn[6] != 0;
   return true;
 }
 
@@ -2791,7 +2834,7 @@ __global__ void k_spec_eval(SpecArgs a, int64_t* chunk_pre, unsigned long long* 
         const int32_t r = x > y ? x : y;
         o0 = r;
         mem.self0 = r;
-        if (a.v2i[r] >= 0) o1 = w_first_eligible(a, mem, r);
+        if (a.v2i[r] >= 0 && !(a.grown && a.prev0[pos] == r && a.prev1[pos] == -1)) o1 = w_first_eligible(a, mem, r);
       }
     } else if (mx != my) {
       const int32_t yy = mx ? y : x, keep = mx ? x : y;
@@ -3079,19 +3122,28 @@ __device__ __forceinline__ int round_scan(int x, int* s_warp, int* total) {
   return r;
 }
 
-// Start of a queued repair of a larger sub-batch that assigned few edges: as
-// k_assign_small leaves it.
-__global__ void k_repair_init(int32_t* w0, int32_t* w1, int64_t cnt, int64_t* dyn, int64_t* counts) {
+// Start of a larger queued repair: the guessed writes, the round words and the
+// deferral counters; k_spec_round_large makes the view of them.
+__global__ void k_repair_init(const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t p, const uint32_t* order,
+                              const uint8_t* mis, int32_t* w0, int32_t* w1, int64_t cnt, int64_t* dyn,
+                              int64_t* counts) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cnt) {
-    w0[i] = -1;
+    const int64_t j = p + order[i];
+    const int32_t a = u[j], b = v[j];
+    w0[i] = ins[j] && (mis[a] & 1) && (mis[b] & 1) ? max(a, b) : -1;
     w1[i] = -1;
   }
-  if (i < 4) dyn[i] = 0;
-  if (i == 4) dyn[4] = cnt;
+  if (i < 7) dyn[i] = i == 4 ? cnt : 0;
   if (i < 6) counts[i] = 0;
+}
+
+// Whether a changed result leaves the members grown: an insert that found a
+// vertex to join after the same removal, or a delete whose vertex now joins.
+__device__ __forceinline__ bool only_joins(bool ins, int32_t a, int32_t b, int32_t ra, int32_t rb) {
+  return ins ? (a >= 0 && a == ra && rb < 0 && b >= 0) : (ra < 0 && a >= 0);
 }
 
 __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0, const int32_t* n1, const int32_t* r0,
@@ -3100,7 +3152,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
                                                               uint64_t* view_keys, uint32_t* view_vals,
                                                               int64_t nview_old, uint8_t* m,
                                                               unsigned long long* out, SpecArgs sa,
-                                                              const unsigned long long* best) {
+                                                              const unsigned long long* best, int64_t* host) {
   pdl_wait();
   pdl_trigger();
   if (!spec_dyn_load(sa)) return;
@@ -3113,13 +3165,17 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
   __shared__ uint32_t s_vals[kRoundWrites];
   __shared__ int s_warp[33];
   __shared__ unsigned long long s_f;
+  __shared__ int s_grown;
   const int tid = threadIdx.x;
   // answers of the edges whose hop-2 search ran grid-wide (k_big_scan)
   const int64_t nbig = (int64_t)*sa.big_count;
   for (int64_t i = tid; i < nbig; i += kRoundThreads) big_finalize_one(sa, best, i);
   __syncthreads();
   const int64_t pending = cnt - p0;
-  if (tid == 0) s_f = (unsigned long long)cnt;
+  if (tid == 0) {
+    s_f = (unsigned long long)cnt;
+    s_grown = 1;
+  }
   __syncthreads();
   // first changed position; this round's writes into shared memory
   int32_t a = -1, b = -1;
@@ -3127,7 +3183,12 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
   if (tid < pending) {
     a = n0[pos];
     b = n1[pos];
-    if (a != r0[pos] || b != r1[pos]) atomicMin(&s_f, (unsigned long long)pos);
+    const int32_t ra = r0[pos], rb = r1[pos];
+    if (a != ra || b != rb) {
+      atomicMin(&s_f, (unsigned long long)pos);
+      if (!only_joins(ins[p + order[pos]] != 0, a, b, ra, rb)) s_grown = 0;
+    }
+    if (a == b) a = -1;   // a removed vertex that joins again: the join is the later write
   }
   int nk = 0;
   const int off = round_scan((a >= 0) + (b >= 0), s_warp, &nk);
@@ -3212,8 +3273,141 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round(const int32_t* n0,
       sa.dyn[1] = nview;
       sa.dyn[2] = (int64_t)f >= cnt ? 1 : 0;
       sa.dyn[3] += 1;
+      sa.dyn[6] = s_grown;
+      for (int k = 0; k < 6; ++k) sa.big_count[k] = 0;   // deferrals, prefix use, queue (2), spare, done
+      for (int k = 0; k < 6; ++k) host[k] = sa.dyn[k];
+    }
+  }
+}
+
+// k_spec_round for up to kLargeCap pending positions, queued rounds only: the
+// writes, kLargeWrites at most, are compacted in position order, so one stable
+// sort on the vertex orders them.  With `init` the results are the guessed
+// writes (r0, r1), nothing is committed, and every write goes into the view.
+// More writes than that: dyn[2] = 2 and nothing is changed (the host goes on
+// with its own rounds).
+// It replaces about ten launches and two host waits a round; one block's sort
+// and its passes over the positions bound it.
+constexpr int kLargeCap = 16384;
+constexpr int kLargeItems = 8;
+constexpr int kLargeWrites = kLargeItems * kRoundThreads;
+constexpr size_t kLargeSmem = (size_t)kLargeWrites * 12 + (size_t)(kRoundThreads / 32) * sort_detail::kDigits * 4;
+
+__global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa, const unsigned long long* best,
+                                                                    bool init, int nbits, uint64_t* view_keys,
+                                                                    uint32_t* view_vals, uint8_t* m, int64_t* host) {
+  pdl_wait();
+  pdl_trigger();
+  if (!spec_dyn_load(sa)) return;
+  extern __shared__ __align__(16) unsigned char round_smem[];
+  uint64_t* sk = reinterpret_cast<uint64_t*>(round_smem);
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + kLargeWrites);
+  uint32_t* cnts = sv + kLargeWrites;
+  __shared__ uint32_t s_dbase[sort_detail::kDigits];
+  __shared__ uint32_t s_sw[sort_detail::kDigits / 32];
+  __shared__ int s_warp[33];
+  __shared__ unsigned long long s_f;
+  __shared__ int s_grown;
+  const int tid = threadIdx.x;
+  const int32_t* n0 = init ? sa.prev0 : sa.out0;
+  const int32_t* n1 = init ? sa.prev1 : sa.out1;
+  if (!init) {
+    const int64_t nbig = (int64_t)*sa.big_count;
+    for (int64_t i = tid; i < nbig; i += kRoundThreads) big_finalize_one(sa, best, i);
+  }
+  if (tid == 0) {
+    s_f = (unsigned long long)sa.cnt;
+    s_grown = 1;
+  }
+  __syncthreads();
+  int nk = 0;
+  for (int64_t base = sa.p0; base < sa.cnt; base += kRoundThreads) {
+    const int64_t pos = base + tid;
+    int32_t a = -1, b = -1;
+    bool ins = false;
+    if (pos < sa.cnt) {
+      a = n0[pos];
+      b = n1[pos];
+      ins = sa.ins[sa.p + sa.order[pos]] != 0;
+      const int32_t ra = sa.prev0[pos], rb = sa.prev1[pos];
+      if (a != ra || b != rb) {
+        atomicMin(&s_f, (unsigned long long)pos);
+        if (!only_joins(ins, a, b, ra, rb)) s_grown = 0;
+      }
+      if (a == b) a = -1;   // a removed vertex that joins again: the join is the later write
+    }
+    int total = 0;
+    int k = nk + round_scan((a >= 0) + (b >= 0), s_warp, &total);
+    if (a >= 0) {
+      if (k < kLargeWrites) {
+        sk[k] = ((uint64_t)(uint32_t)a << 32) | (uint64_t)pos;
+        sv[k] = ins ? 0u : 1u;
+      }
+      ++k;
+    }
+    if (b >= 0 && k < kLargeWrites) {
+      sk[k] = ((uint64_t)(uint32_t)b << 32) | (uint64_t)pos;
+      sv[k] = 1u;
+    }
+    nk += total;
+  }
+  __syncthreads();
+  if (nk > kLargeWrites) {
+    if (tid == 0) {
+      sa.dyn[2] = 2;
+      for (int k = 0; k < 6; ++k) host[k] = sa.dyn[k];
+    }
+    return;
+  }
+  if (nk > 1) {
+    const int at = (tid >> 5) * 32 * kLargeItems + (tid & 31);
+    uint64_t key[kLargeItems];
+    uint32_t val[kLargeItems];
+#pragma unroll
+    for (int r = 0; r < kLargeItems; ++r) {
+      key[r] = at + r * 32 < nk ? sk[at + r * 32] : 0;
+      val[r] = at + r * 32 < nk ? sv[at + r * 32] : 0;
+    }
+    __syncthreads();
+    sort_detail::block_sort<kLargeItems>(false, key, val, nk, 32, 32 + nbits, sk, sv, cnts, s_dbase, s_sw);
+  }
+  for (int64_t k = tid; k < sa.view.nkeys; k += kRoundThreads) m[view_keys[k] >> 32] &= 1;
+  __syncthreads();
+  const unsigned long long f = s_f;
+  const int64_t last = init ? -1 : min((int64_t)f, sa.cnt - 1);
+  for (int k = tid; k < nk; k += kRoundThreads) {
+    const uint64_t key = sk[k];
+    if ((int64_t)(key & 0xffffffffull) > last) continue;
+    if (k + 1 < nk) {
+      const uint64_t nx = sk[k + 1];
+      if ((nx >> 32) == (key >> 32) && (int64_t)(nx & 0xffffffffull) <= last) continue;
+    }
+    m[key >> 32] = (uint8_t)sv[k];
+  }
+  __syncthreads();
+  int nview = 0;
+  for (int base = 0; base < nk; base += kRoundThreads) {
+    const int k = base + tid;
+    const bool keep = k < nk && (int64_t)(sk[k] & 0xffffffffull) > last;
+    int total = 0;
+    const int at = nview + round_scan((int)keep, s_warp, &total);
+    if (keep) {
+      m[sk[k] >> 32] |= 2;
+      view_keys[at] = sk[k];
+      view_vals[at] = sv[k];
+    }
+    nview += total;
+  }
+  if (tid == 0) {
+    sa.dyn[1] = nview;
+    if (!init) {
+      sa.dyn[0] = (int64_t)f + 1;
+      sa.dyn[2] = (int64_t)f >= sa.cnt ? 1 : 0;
+      sa.dyn[3] += 1;
+      sa.dyn[6] = s_grown;
       for (int k = 0; k < 6; ++k) sa.big_count[k] = 0;   // deferrals, prefix use, queue (2), spare, done
     }
+    for (int k = 0; k < 6; ++k) host[k] = sa.dyn[k];
   }
 }
 
@@ -3743,9 +3937,9 @@ void repair_reserve(mf_ctx* c, int64_t nproc) {
   }
 }
 
-// The rounds of a sub-batch may be queued with their start, view and count on
-// the device.
-bool queued_rounds(int64_t most) { return most <= kRoundCap && !host_rounds_forced() && !debug_counters(); }
+// The rounds of a sub-batch of at most `most` edges may be queued with their
+// start, view and count on the device.
+bool queued_rounds(int64_t most) { return most <= kLargeCap && !host_rounds_forced() && !debug_counters(); }
 
 // Repair of one sub-batch: c->vals holds the order (sub-batch indices),
 // nproc entries.  With `prepared`, k_assign_small has made the order and the
@@ -3767,28 +3961,36 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
   const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
   int64_t p0 = 0, nview = 0, rounds = 0;
   if (prepared || queued_rounds(nproc)) {
-    // Every round fits one commit block: rounds are queued kRoundsPerSync at
-    // a time and read back once; a queued round finds its start and view on
-    // the device and does nothing once the repair is done.  Round r writes
-    // into one pair of result buffers and compares with the other, in turn.
+    // Every round fits one commit block: rounds are queued up to kRoundsPerSync
+    // at a time (one, while the last sub-batch needed only one) and read back
+    // once; a queued round finds its start and view on the device and does
+    // nothing once the repair is done.  Round r writes into one pair of result
+    // buffers and compares with the other, in turn.
     int64_t* dyn = c->counters.p + 58;
-    if (!prepared)
-      MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 6)), kTB, 0, s, c->rp_w0.p, c->rp_w1.p, nproc,
-                      dyn, c->counters.p + 24));
     std::optional<StageScope> dsc;
+    auto args = [&](int64_t round) {
+      const bool even = (round & 1) == 0;
+      SpecArgs a{g, c->bu.p, c->bv.p, c->bins.p, p, order, 0, nproc, ns, c->v2i.p,
+                 View{c->mis.p, c->rp_keys.p, c->rp_vals.p, 0}, even ? c->rp_n0.p : c->rp_w0.p,
+                 even ? c->rp_n1.p : c->rp_w1.p, c->tune.big_threshold, ucnt + 24, c->big_pos.p, c->big_r.p,
+                 c->big_off.p, c->big_nr.p, c->big_pre.p, ucnt + 25, c->big_pre.cap, dyn,
+                 even ? c->rp_w0.p : c->rp_n0.p, even ? c->rp_w1.p : c->rp_n1.p};
+      return a;
+    };
+    if (!prepared) {
+      raise_smem(c->device, k_spec_round_large, kLargeSmem);
+      dsc.emplace(c, kStRepair);
+      MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 7)), kTB, 0, s, c->bu.p, c->bv.p, c->bins.p, p,
+                      order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, dyn, c->counters.p + 24));
+      MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, args(0), c->big_best.p, true, nbits,
+                      c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
+    }
     int64_t queued = 0;
     while (true) {
-      const int64_t k = std::min<int64_t>(kRoundsPerSync, kMaxRounds - queued);
+      const int64_t most = queued == 0 && c->repair_last <= 1 ? 1 : kRoundsPerSync;
+      const int64_t k = std::min<int64_t>(most, kMaxRounds - queued);
       for (int64_t j = 0; j < k; ++j, ++queued) {
-        const bool even = (queued & 1) == 0;
-        int32_t* o0 = even ? c->rp_n0.p : c->rp_w0.p;
-        int32_t* o1 = even ? c->rp_n1.p : c->rp_w1.p;
-        int32_t* r0 = even ? c->rp_w0.p : c->rp_n0.p;
-        int32_t* r1 = even ? c->rp_w1.p : c->rp_n1.p;
-        SpecArgs a{g, c->bu.p, c->bv.p, c->bins.p, p, order, 0, nproc, ns, c->v2i.p,
-                   View{c->mis.p, c->rp_keys.p, c->rp_vals.p, 0}, o0, o1, c->tune.big_threshold, ucnt + 24,
-                   c->big_pos.p, c->big_r.p, c->big_off.p, c->big_nr.p, c->big_pre.p, ucnt + 25, c->big_pre.cap,
-                   dyn};
+        const SpecArgs a = args(queued);
         dsc.emplace(c, kStRepair);
         MF_K(launch_pdl(k_spec_eval, warps_grid(nproc), kTB, 0, s, a, c->big_chunks.p, c->big_best.p, ucnt + 26,
                         reinterpret_cast<unsigned int*>(ucnt + 29)));
@@ -3796,13 +3998,21 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
         MF_K(launch_pdl(k_big_scan, (unsigned)c->big_grid, kBigChunk, 0, s, a, c->big_chunks.p, c->big_best.p,
                         ucnt + 26));
         dsc.emplace(c, kStRepair);
-        MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, o0, o1, r0, r1, (int64_t)0, nproc, c->bins.p, p, order,
-                        c->rp_keys.p, c->rp_vals.p, (int64_t)0, c->mis.p, ucnt + 20, a, c->big_best.p));
+        if (prepared)
+          MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, a.out0, a.out1, a.prev0, a.prev1, (int64_t)0, nproc,
+                          c->bins.p, p, order, c->rp_keys.p, c->rp_vals.p, (int64_t)0, c->mis.p, ucnt + 20, a,
+                          c->big_best.p, h + 58));
+        else
+          MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, a, c->big_best.p, false, nbits,
+                          c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
       }
-      MF_CUDA(cudaMemcpyAsync(h + 58, dyn, sizeof(int64_t) * 6, cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
       dsc.reset();
-      if (h[60] != 0) break;
+      if (h[60] == 1) {
+        c->repair_last = h[61];
+        return h[61];
+      }
+      if (h[60] == 2) break;   // too many writes for one block
       if (queued >= kMaxRounds) {
         // round limit: the rest in order by the sequential kernel
         p0 = h[58];
@@ -3812,13 +4022,23 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
         RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, c->v2i.p, c->mis.p};
         MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
         MF_CUDA(cudaGetLastError());
-        break;
+        return h[61];
       }
     }
-    return h[61];
+    // on with host-driven rounds from the last one that was committed
+    p0 = h[58];
+    nview = h[59];
+    rounds = h[61];
+    c->repair_last = kRoundsPerSync;
+    if (rounds & 1) {
+      std::swap(c->rp_w0, c->rp_n0);
+      std::swap(c->rp_w1, c->rp_n1);
+    }
   }
-  MF_CUDA(cudaMemsetAsync(c->rp_w0.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
-  MF_CUDA(cudaMemsetAsync(c->rp_w1.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
+  if (rounds == 0 && nview == 0) {   // else the last results and the view stand as they are
+    MF_CUDA(cudaMemsetAsync(c->rp_w0.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
+    MF_CUDA(cudaMemsetAsync(c->rp_w1.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
+  }
   int64_t dbg_big = 0, dbg_chunks = 0, dbg_scanned = 0;
   std::optional<StageScope> rsc;
   rsc.emplace(c, kStRepair);
@@ -3848,7 +4068,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
       // the round, one host round trip
       MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, c->rp_n0.p, c->rp_n1.p, c->rp_w0.p, c->rp_w1.p, p0, nproc, c->bins.p,
                                                     p, order, c->rp_keys.p, c->rp_vals.p, nview, c->mis.p, ucnt + 20,
-                                                    a, c->big_best.p));
+                                                    a, c->big_best.p, static_cast<int64_t*>(nullptr)));
       MF_CUDA(cudaMemcpyAsync(h + 20, c->counters.p + 20, sizeof(int64_t) * 2, cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
       const int64_t f = h[20];
@@ -4297,12 +4517,13 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // and the host first hears of it when it reads the rounds back.
     sc.emplace(c, kStAssign);
     int64_t nproc, cc;
-    if (queued_rounds(q - p) && !sequential_repair_forced()) {
+    if (q - p <= kRoundCap && queued_rounds(q - p) && !sequential_repair_forced()) {
       repair_reserve(c, q - p);
       const unsigned threads = q - p <= 256 ? 256 : 1024;
-      MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)(q - p), c->cid.p, c->i64b.p + rows,
-                      bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1)), c->vals.p, c->rp_w0.p,
-                      c->rp_w1.p, c->counters.p + 58, c->counters.p + 24));
+      MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)(q - p), c->bins.p, c->cid.p,
+                      c->i64b.p + rows, bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1)),
+                      c->vals.p, c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, c->counters.p + 58,
+                      c->counters.p + 24));
       sc.reset();
       const int64_t rounds = repair(c, g, p, q - p, ns, true);
       nproc = h[62];

@@ -131,3 +131,41 @@ def test_row_length_limit_of_short_kernels(gb, hub, push):
                 for field in (1, 2, 3, 4, 5):
                     assert np.array_equal(x[field], y[field]), field
             assert np.array_equal(g.get_mis(), orc.get_mis())
+
+
+# one block commits up to 1,024 edges, another up to 16,384 edges with up to 8,192 writes; more go to host-driven rounds
+@pytest.mark.parametrize("m,writes", [(1000, 900), (1024, 1024), (1025, 1025), (1100, 600), (8300, 8192), (8300, 8193),
+                                      (16384, 5000), (16385, 5000), (9000, 9000)])
+def test_repair_commit_blocks(gb, m, writes):
+    """One sub-batch of m edges, `writes` of them inserts that join two members (each removes one), the rest inserts
+    around them: dependent chains, joins and plain removals; order, membership and ids equal the oracle's."""
+    import oracle as O
+    n = 45000
+    rng = np.random.default_rng(m + writes)
+    # pairs (2k, 2k + 1) with k < n / 4: one member, one covered vertex; the rest isolated members
+    k = np.arange(n // 4)
+    nindex, nlist = W.csr_from_pairs(n, 2 * k, 2 * k + 1)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    members = rng.permutation(np.nonzero(mis)[0])
+    a, b = members[0:2 * writes:2], members[1:2 * writes:2]   # disjoint pairs of members
+    short = writes - a.size
+    extra = m - a.size
+    u = np.concatenate([a, rng.choice(members, extra)])
+    v = np.concatenate([b, rng.integers(0, n, extra)])
+    assert short >= 0
+    ok = u != v
+    u, v = u[ok].astype(np.int32), v[ok].astype(np.int32)
+    p = rng.permutation(u.size)
+    u, v = u[p], v[p]
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for x in (g, orc):
+            x.max_csr = 1 << 40
+            x.set_mis(mis)
+        for batch in range(2):
+            ins = orc.flag_updates(u, v)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            assert g.stats()["sub_batches"] == 1
+            assert np.array_equal(g.get_mis(), orc.get_mis())
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
