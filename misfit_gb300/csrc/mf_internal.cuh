@@ -648,6 +648,7 @@ struct mf_ctx {
   mf::DBuf<uint32_t> dense_bits;      // per dense seed bitmaps (exact sizes)
   mf::DBuf<int64_t> dense_light;      // per dense seed light volume (size bound)
   mf::DBuf<int32_t> pull_long;        // vertices with long rows for the warp pull pass
+  mf::DBuf<int32_t> tails;            // last two entries of each base row (large graphs, made on first use)
   mf::DBuf<uint32_t> ncbits;          // non-skipped candidate bits for the pull pass
   // exact 2-hop sizes by row passes: seed masks per vertex and their filter
   // bits, the huge rows' chunk ORs, neighbourhood volumes, chunk tasks, the
@@ -754,7 +755,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->cid); f(c->v2i); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
   f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
-  f(c->pull_long); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
+  f(c->pull_long); f(c->tails); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
   f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);

@@ -674,6 +674,7 @@ void upload_base(mf_ctx* c, int32_t n, const int64_t* nindex, const int32_t* nli
     c->rows_sorted = true;
     c->symmetric = true;
   }
+  c->tails.release();   // of another base
   c->max_csr = initial_max_csr(n, c->header_edges);
   c->max_row = -1;
 }

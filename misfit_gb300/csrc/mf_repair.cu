@@ -47,6 +47,7 @@ namespace {
 constexpr int kTB = 256;
 static_assert(kTB == kLbThreads, "lb_rows kernels run kLbThreads-thread blocks");
 constexpr int32_t kSkip = -2;
+constexpr int32_t kTailsMin = 1 << 20;   // vertices from which the pull uses row tails
 // host counter slots [kFrontSlot + 2f, +1]: front f's counts, copied on the
 // stream that computed it
 constexpr int kFrontSlot = 10;
@@ -1683,9 +1684,10 @@ __global__ void k_need_decide(GraphView g, const int32_t* need, const int32_t* n
 // of those rows with s = their own vertex (the rest of phase 1 is
 // k_lb_push_seed).  A skipped row stays skipped whatever its id.  The
 // candidates that write set their bit for the pull (ncbits, null when the
-// candidates' ids are pushed); k_clear takes the bits back.
+// candidates' ids are pushed; k_clear takes the bits back) and leave their id
+// where one load finds it (newcid).
 __global__ void k_new_ids(int64_t rows, const int64_t* pos, int32_t* rowcid, const int32_t* seeds, int64_t ns,
-                          const int32_t* cands, uint32_t epoch, uint32_t* bval, uint32_t* ncbits) {
+                          const int32_t* cands, uint32_t epoch, uint32_t* bval, uint32_t* ncbits, int32_t* newcid) {
   pdl_wait();
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1698,6 +1700,7 @@ __global__ void k_new_ids(int64_t rows, const int64_t* pos, int32_t* rowcid, con
   } else if (ncbits) {
     const int32_t x = cands[i - ns];
     atomicOr(ncbits + (x >> 5), 1u << (x & 31));
+    newcid[x] = rc == -1 ? (int32_t)pos[i] : rc;
   }
 }
 
@@ -2000,21 +2003,52 @@ struct PullArgs {
   unsigned long long* nlong;
   unsigned long long* work;
   int64_t pull_long;              // rows longer than this go to the warp pass
+  const int2* tail;               // last two entries of each base row (.y the last, -1 where the row ends), or null
+  const int32_t* newcid;          // cluster id of each non-skipped candidate
 };
 
 __device__ __forceinline__ bool pull_nonskip(const PullArgs& a, int32_t c) {
   return (__ldg(a.ncbits + (c >> 5)) >> (c & 31)) & 1u;
 }
 
+// The last two entries of every base row.  The pull is bound by random
+// sectors: consecutive rows' ends lie about a row apart, so each costs a
+// 32-byte sector of DRAM for the one or two entries that decide most rows.
+// As an array of its own those entries are one coalesced read.
+__global__ void k_row_tails(const int64_t* nindex, const int32_t* nlist, int32_t n, int2* tail) {
+  const int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (y >= n) return;
+  const int64_t b = nindex[y], e = nindex[y + 1];
+  tail[y] = make_int2(e - b >= 2 ? nlist[e - 2] : -1, e - b >= 1 ? nlist[e - 1] : -1);
+}
+
+// Counts of one block into *work by one atomic (a warp's atomic each made
+// n / 32 of them on one address).
+__device__ __forceinline__ void add_work_block(unsigned long long* work, int64_t visited) {
+  __shared__ int s_visited;
+  if (threadIdx.x == 0) s_visited = 0;
+  __syncthreads();
+  int v = (int)visited;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(&s_visited, v);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_visited) atomicAdd(work, (unsigned long long)s_visited);
+}
+
 __device__ __forceinline__ void pull_finish(const PullArgs& a, int32_t y, int32_t best) {
   if (best >= 0) {
-    a.cid[y] = a.rowcid[a.v2i[best]];
+    a.cid[y] = a.newcid[best];
   } else {
     const uint32_t t = a.wval[y];
     if ((t >> kRowBits) == a.epoch) a.cid[y] = a.rowcid[t & kRowMask];
   }
 }
 
+// One vertex per thread.  With row tails (a.tail), an unchanged row is first
+// tried by its last two entries; the rows they leave open, and changed ones,
+// read their bounds and walk.  R-MAT scale 22 (2.4 M rows of any length, 330,000
+// candidates): 168 us by the bounds alone.
+template <bool Tails>
 __global__ void k_pull_cand(PullArgs a) {
   pdl_wait();
   pdl_trigger();
@@ -2023,32 +2057,60 @@ __global__ void k_pull_cand(PullArgs a) {
   int64_t visited = 0;
   if (yi < g.n) {
     const int32_t y = (int32_t)yi;
-    const int64_t b = g.nindex[y], e = g.nindex[y + 1];
     const int64_t ab = g.aoff[y], ae = g.aoff[y + 1];
-    if ((e - b) + (ae - ab) > a.pull_long) {
-      a.longv[atomicAdd(a.nlong, 1ull)] = y;
-    } else {
-      int32_t best = -1;
-      for (int64_t k = ab; k < ae; ++k) {
-        const int32_t c = g.aadj[k];
-        ++visited;
-        if (c > best && pull_nonskip(a, c)) best = c;
-      }
-      const bool filt = g.dead[y] != 0;
-      for (int64_t k = e - 1; k >= b; --k) {
-        const int32_t c = __ldg(g.nlist + k);
-        ++visited;
-        if (c <= best) break;
-        if (filt && !live_at(g.live, k)) continue;
-        if (pull_nonskip(a, c)) {
-          best = c;
-          break;
+    const bool filt = g.dead[y] != 0;
+    int skip = 0;        // entries at the row's end that are no candidates
+    bool done = false;
+    int32_t best = -1;
+    if (Tails) {
+      const int2 t = a.tail[y];
+      if (!filt && ab == ae) {
+        if (t.y < 0) {
+          done = true;
+        } else if (pull_nonskip(a, t.y)) {
+          best = t.y;
+          done = true;
+          visited = 1;
+        } else if (t.x < 0) {
+          done = true;
+          visited = 1;
+        } else if (pull_nonskip(a, t.x)) {
+          best = t.x;
+          done = true;
+          visited = 2;
+        } else {
+          skip = 2;
+          visited = 2;
         }
       }
+    }
+    if (done) {
       pull_finish(a, y, best);
+    } else {
+      const int64_t b = g.nindex[y], e = g.nindex[y + 1];
+      if ((e - b) + (ae - ab) > a.pull_long) {
+        a.longv[atomicAdd(a.nlong, 1ull)] = y;
+      } else {
+        for (int64_t k = ab; k < ae; ++k) {
+          const int32_t c = g.aadj[k];
+          ++visited;
+          if (c > best && pull_nonskip(a, c)) best = c;
+        }
+        for (int64_t k = e - 1 - skip; k >= b; --k) {
+          const int32_t c = __ldg(g.nlist + k);
+          ++visited;
+          if (c <= best) break;
+          if (filt && !live_at(g.live, k)) continue;
+          if (pull_nonskip(a, c)) {
+            best = c;
+            break;
+          }
+        }
+        pull_finish(a, y, best);
+      }
     }
   }
-  add_work(a.work, visited);
+  add_work_block(a.work, visited);
 }
 
 // The long rows: the warp takes the maximum over the added part, then walks
@@ -4432,6 +4494,13 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       const double pull_b = (28.0 + 4.0 * c->pull_visit_ratio) * (double)n;
       if (2.0 * push_b < pull_b) use_pull = false;
     }
+    // Row tails where the rows are too many for L2 to hold what the pull reads
+    // (made once per base; on smaller graphs the rows' ends come from L2).
+    const bool tails = use_pull && n >= kTailsMin;
+    if (tails && c->tails.cap < 2 * (int64_t)n) {
+      c->tails.reserve(2 * (int64_t)n);
+      MF_K(k_row_tails<<<grid_for(n), kTB, 0, s>>>(c->nindex.p, c->nlist.p, n, reinterpret_cast<int2*>(c->tails.p)));
+    }
     if (use_pull) {
       const int64_t nwords = std::max<int64_t>(((int64_t)n + 31) / 32, 1);
       const bool grown = c->ncbits.cap < nwords;
@@ -4442,7 +4511,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     uint32_t* ncbits = use_pull ? c->ncbits.p : nullptr;
     scan_exclusive_u8(c->creates.p, c->i64b.p, rows, c->ws, s);
     MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, rows, c->i64b.p, c->rowcid.p, c->seeds.p, ns, c->cands.p, ep,
-                    c->bval.p, ncbits));
+                    c->bval.p, ncbits, c->f1.p));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
     if (short_rows) {
@@ -4480,8 +4549,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       ++c->pull_runs;
       c->pull_long.reserve(std::max<int32_t>(n, 1));
       const PullArgs pa{g,  c->v2i.p, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
-                        ucnt + 36, wk_extra + 2, c->tune.pull_long};
-      MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
+                        ucnt + 36, wk_extra + 2, c->tune.pull_long, reinterpret_cast<const int2*>(c->tails.p), c->f1.p};
+      if (tails) MF_K(launch_pdl(k_pull_cand<true>, grid_for(n), kTB, 0, s, pa));
+      else MF_K(launch_pdl(k_pull_cand<false>, grid_for(n), kTB, 0, s, pa));
       if (c->max_row > c->tune.pull_long)
         MF_K(launch_pdl(k_pull_cand_long, lb_grid(c, k_pull_cand_long), kTB, 0, s, pa));
       // per vertex: row bounds (8 B of nindex, 8 B of aoff), tombstone count,
