@@ -648,7 +648,7 @@ struct mf_ctx {
   mf::DBuf<uint32_t> dense_bits;      // per dense seed bitmaps (exact sizes)
   mf::DBuf<int64_t> dense_light;      // per dense seed light volume (size bound)
   mf::DBuf<int32_t> pull_long;        // vertices with long rows for the warp pull pass
-  mf::DBuf<int32_t> tails;            // last two entries of each base row (large graphs, made on first use)
+  mf::DBuf<int32_t> tails;            // last four entries of each base row (large graphs, made on first use)
   mf::DBuf<uint32_t> ncbits;          // non-skipped candidate bits for the pull pass
   // exact 2-hop sizes by row passes: seed masks per vertex and their filter
   // bits, the huge rows' chunk ORs, neighbourhood volumes, chunk tasks, the

@@ -2003,7 +2003,7 @@ struct PullArgs {
   unsigned long long* nlong;
   unsigned long long* work;
   int64_t pull_long;              // rows longer than this go to the warp pass
-  const int2* tail;               // last two entries of each base row (.y the last, -1 where the row ends), or null
+  const int4* tail;               // last four entries of each base row (.w the last, -1 where the row ends), or null
   const int32_t* newcid;          // cluster id of each non-skipped candidate
 };
 
@@ -2011,15 +2011,16 @@ __device__ __forceinline__ bool pull_nonskip(const PullArgs& a, int32_t c) {
   return (__ldg(a.ncbits + (c >> 5)) >> (c & 31)) & 1u;
 }
 
-// The last two entries of every base row.  The pull is bound by random
+// The last four entries of every base row.  The pull is bound by random
 // sectors: consecutive rows' ends lie about a row apart, so each costs a
-// 32-byte sector of DRAM for the one or two entries that decide most rows.
-// As an array of its own those entries are one coalesced read.
-__global__ void k_row_tails(const int64_t* nindex, const int32_t* nlist, int32_t n, int2* tail) {
+// 32-byte sector of DRAM for the few entries that decide most rows.  As an
+// array of its own those entries are one coalesced read.
+__global__ void k_row_tails(const int64_t* nindex, const int32_t* nlist, int32_t n, int4* tail) {
   const int64_t y = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (y >= n) return;
   const int64_t b = nindex[y], e = nindex[y + 1];
-  tail[y] = make_int2(e - b >= 2 ? nlist[e - 2] : -1, e - b >= 1 ? nlist[e - 1] : -1);
+  auto at = [&](int64_t k) { return k >= b ? nlist[k] : -1; };
+  tail[y] = make_int4(at(e - 4), at(e - 3), at(e - 2), at(e - 1));
 }
 
 // Counts of one block into *work by one atomic (a warp's atomic each made
@@ -2044,71 +2045,121 @@ __device__ __forceinline__ void pull_finish(const PullArgs& a, int32_t y, int32_
   }
 }
 
-// One vertex per thread.  With row tails (a.tail), an unchanged row is first
-// tried by its last two entries; the rows they leave open, and changed ones,
-// read their bounds and walk.  R-MAT scale 22 (2.4 M rows of any length, 330,000
-// candidates): 168 us by the bounds alone.
-template <bool Tails>
+// The row of y by its bounds: the added part, then the base part from its end
+// (less `skip` entries known to be no candidates).
+__device__ __forceinline__ int64_t pull_walk(const PullArgs& a, int32_t y, int64_t ab, int64_t ae, bool filt, int skip) {
+  const GraphView& g = a.g;
+  const int64_t b = g.nindex[y], e = g.nindex[y + 1];
+  if ((e - b) + (ae - ab) > a.pull_long) {
+    a.longv[atomicAdd(a.nlong, 1ull)] = y;
+    return 0;
+  }
+  int64_t visited = 0;
+  int32_t best = -1;
+  for (int64_t k = ab; k < ae; ++k) {
+    const int32_t c = g.aadj[k];
+    ++visited;
+    if (c > best && pull_nonskip(a, c)) best = c;
+  }
+  for (int64_t k = e - 1 - skip; k >= b; --k) {
+    const int32_t c = __ldg(g.nlist + k);
+    ++visited;
+    if (c <= best) break;
+    if (filt && !live_at(g.live, k)) continue;
+    if (pull_nonskip(a, c)) {
+      best = c;
+      break;
+    }
+  }
+  pull_finish(a, y, best);
+  return visited;
+}
+
 __global__ void k_pull_cand(PullArgs a) {
   pdl_wait();
   pdl_trigger();
-  const GraphView& g = a.g;
   const int64_t yi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t visited = 0;
-  if (yi < g.n) {
+  if (yi < a.g.n) {
     const int32_t y = (int32_t)yi;
-    const int64_t ab = g.aoff[y], ae = g.aoff[y + 1];
-    const bool filt = g.dead[y] != 0;
-    int skip = 0;        // entries at the row's end that are no candidates
-    bool done = false;
-    int32_t best = -1;
-    if (Tails) {
-      const int2 t = a.tail[y];
-      if (!filt && ab == ae) {
-        if (t.y < 0) {
-          done = true;
-        } else if (pull_nonskip(a, t.y)) {
-          best = t.y;
-          done = true;
-          visited = 1;
-        } else if (t.x < 0) {
-          done = true;
-          visited = 1;
-        } else if (pull_nonskip(a, t.x)) {
-          best = t.x;
-          done = true;
-          visited = 2;
-        } else {
-          skip = 2;
-          visited = 2;
-        }
-      }
+    visited = pull_walk(a, y, a.g.aoff[y], a.g.aoff[y + 1], a.g.dead[y] != 0, 0);
+  }
+  add_work_block(a.work, visited);
+}
+
+// The same by row tails: a row without tombstones and with few added entries
+// is first tried by its added part and its last four base entries; the rows they
+// leave open read their bounds and walk.  Two vertices per thread, each step's
+// loads issued for both.  R-MAT scale 22 (2.4 M rows, 330,000 candidates), ncu
+// with cold caches: 168 us by the bounds alone, 88 us with the last two entries
+// and one vertex per thread, 80 us with two, 71 us with four entries; walking the
+// open rows in a launch of their own, eight lanes each, took 48 + 38 us.
+constexpr int kPullPer = 2;
+constexpr int64_t kPullAdded = 16;
+
+__global__ void __launch_bounds__(kTB) k_pull_tails(PullArgs a) {
+  pdl_wait();
+  pdl_trigger();
+  const GraphView& g = a.g;
+  const int64_t y0 = (int64_t)blockIdx.x * blockDim.x * kPullPer + threadIdx.x;
+  int64_t ab[kPullPer], ae[kPullPer];
+  int4 t[kPullPer];
+  bool filt[kPullPer], in[kPullPer];
+  int64_t visited = 0;
+#pragma unroll
+  for (int q = 0; q < kPullPer; ++q) {
+    const int64_t y = y0 + (int64_t)q * blockDim.x;
+    in[q] = y < g.n;
+    ab[q] = in[q] ? g.aoff[y] : 0;
+    ae[q] = in[q] ? g.aoff[y + 1] : 0;
+    t[q] = in[q] ? a.tail[y] : make_int4(-1, -1, -1, -1);
+    filt[q] = in[q] && g.dead[y] != 0;
+  }
+  bool hit1[kPullPer], hit2[kPullPer];
+#pragma unroll
+  for (int q = 0; q < kPullPer; ++q) {
+    hit1[q] = t[q].w >= 0 && pull_nonskip(a, t[q].w);
+    hit2[q] = t[q].z >= 0 && pull_nonskip(a, t[q].z);
+  }
+#pragma unroll
+  for (int q = 0; q < kPullPer; ++q) {
+    if (!in[q]) continue;
+    const int32_t y = (int32_t)(y0 + (int64_t)q * blockDim.x);
+    if (filt[q] || ae[q] - ab[q] > kPullAdded) {
+      visited += pull_walk(a, y, ab[q], ae[q], filt[q], 0);
+      continue;
     }
-    if (done) {
-      pull_finish(a, y, best);
-    } else {
-      const int64_t b = g.nindex[y], e = g.nindex[y + 1];
-      if ((e - b) + (ae - ab) > a.pull_long) {
-        a.longv[atomicAdd(a.nlong, 1ull)] = y;
-      } else {
-        for (int64_t k = ab; k < ae; ++k) {
-          const int32_t c = g.aadj[k];
+    int32_t best = -1;
+    for (int64_t k = ab[q]; k < ae[q]; ++k) {
+      const int32_t c = g.aadj[k];
+      ++visited;
+      if (c > best && pull_nonskip(a, c)) best = c;
+    }
+    // the base part is sorted: an entry at or below the best one ends it
+    bool open = false;
+    if (t[q].w > best) {
+      ++visited;
+      if (hit1[q]) {
+        best = t[q].w;
+      } else if (t[q].z > best) {
+        ++visited;
+        if (hit2[q]) {
+          best = t[q].z;
+        } else if (t[q].y > best) {
+          const bool h3 = pull_nonskip(a, t[q].y);
+          const bool h4 = t[q].x >= 0 && pull_nonskip(a, t[q].x);
           ++visited;
-          if (c > best && pull_nonskip(a, c)) best = c;
-        }
-        for (int64_t k = e - 1 - skip; k >= b; --k) {
-          const int32_t c = __ldg(g.nlist + k);
-          ++visited;
-          if (c <= best) break;
-          if (filt && !live_at(g.live, k)) continue;
-          if (pull_nonskip(a, c)) {
-            best = c;
-            break;
+          if (h3) {
+            best = t[q].y;
+          } else if (t[q].x > best) {
+            ++visited;
+            if (h4) best = t[q].x; else open = true;
           }
         }
-        pull_finish(a, y, best);
       }
     }
+    if (open) visited += pull_walk(a, y, ab[q], ae[q], false, 4);
+    else pull_finish(a, y, best);
   }
   add_work_block(a.work, visited);
 }
@@ -4497,9 +4548,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // Row tails where the rows are too many for L2 to hold what the pull reads
     // (made once per base; on smaller graphs the rows' ends come from L2).
     const bool tails = use_pull && n >= kTailsMin;
-    if (tails && c->tails.cap < 2 * (int64_t)n) {
-      c->tails.reserve(2 * (int64_t)n);
-      MF_K(k_row_tails<<<grid_for(n), kTB, 0, s>>>(c->nindex.p, c->nlist.p, n, reinterpret_cast<int2*>(c->tails.p)));
+    if (tails && c->tails.cap < 4 * (int64_t)n) {
+      c->tails.reserve(4 * (int64_t)n);
+      MF_K(k_row_tails<<<grid_for(n), kTB, 0, s>>>(c->nindex.p, c->nlist.p, n, reinterpret_cast<int4*>(c->tails.p)));
     }
     if (use_pull) {
       const int64_t nwords = std::max<int64_t>(((int64_t)n + 31) / 32, 1);
@@ -4549,9 +4600,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       ++c->pull_runs;
       c->pull_long.reserve(std::max<int32_t>(n, 1));
       const PullArgs pa{g,  c->v2i.p, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
-                        ucnt + 36, wk_extra + 2, c->tune.pull_long, reinterpret_cast<const int2*>(c->tails.p), c->f1.p};
-      if (tails) MF_K(launch_pdl(k_pull_cand<true>, grid_for(n), kTB, 0, s, pa));
-      else MF_K(launch_pdl(k_pull_cand<false>, grid_for(n), kTB, 0, s, pa));
+                        ucnt + 36, wk_extra + 2, c->tune.pull_long, reinterpret_cast<const int4*>(c->tails.p), c->f1.p};
+      if (tails) MF_K(launch_pdl(k_pull_tails, grid_for(n, kTB * kPullPer), kTB, 0, s, pa));
+      else MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
       if (c->max_row > c->tune.pull_long)
         MF_K(launch_pdl(k_pull_cand_long, lb_grid(c, k_pull_cand_long), kTB, 0, s, pa));
       // per vertex: row bounds (8 B of nindex, 8 B of aoff), tombstone count,
