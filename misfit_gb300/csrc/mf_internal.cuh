@@ -638,7 +638,7 @@ struct mf_ctx {
   mf::DBuf<int32_t> big_r;
   mf::DBuf<unsigned long long> big_best;
   int big_grid = 0;
-  int64_t repair_last = 2;   // rounds of the last queued repair
+  uint32_t repair_more = 1;   // bit k: the queued repair k before the last took more than one round
   mf::DBuf<uint32_t> bitmaps;   // per-CTA vertex bitmaps for exact 2-hop sizes
   int64_t bitmap_words = 0;
   int bitmap_ctas = 0;
@@ -660,6 +660,7 @@ struct mf_ctx {
   // sub-batch plan of the current batch: cuts, estimates, seed lists
   mf::DBuf<int64_t> plan_cuts, plan_ests, plan_send, plan_pos;
   mf::DBuf<uint8_t> plan_flags;
+  mf::DBuf<int32_t> plan_edges;   // int4 per edge of a larger batch
   mf::DBuf<int32_t> seeds_all;
   // first-hit chunk queue (rows) and the need seeds' chunk queue
   mf::DBuf<int32_t> rq_idx, rq_v, mq_idx, mq_v;
@@ -755,7 +756,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->cid); f(c->v2i); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
   f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
-  f(c->pull_long); f(c->tails); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
+  f(c->pull_long); f(c->tails); f(c->plan_edges); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
   f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);

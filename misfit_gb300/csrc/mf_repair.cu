@@ -80,16 +80,40 @@ __device__ __forceinline__ int64_t warp_id() {
 // k, ests[k] = estimate of the edges before the cut; returns the count.
 //
 // The windows form one serial chain, so their latency bounds it.  The edges'
-// degrees and previous occurrences are gathered into shared memory kCutChunk
-// edges at a time, so that a window (or the next sub-batch's, which starts
-// inside the last one) is a shared-memory read, two warp scans and two
-// barriers.
+// degrees and previous occurrences come into shared memory kCutChunk edges at
+// a time, so that a window (or the next sub-batch's, which starts inside the
+// last one) is a shared-memory read, two warp scans and two barriers.  For more
+// than kSmallBatch lines the whole grid gathers them into one array first: one
+// SM took 5 us to gather a chunk's 4,096 random degrees (128 us for 50,000 lines).
 constexpr int kCutThreads = 1024;
 constexpr int kCutChunk = 2 * kCutThreads;
 
-__device__ int64_t plan_cuts(const int32_t* u, const int32_t* v, const int32_t* prev, const int32_t* deg, int64_t m,
-                             int64_t p0, int64_t maxcsr, int64_t* cuts, int64_t* ests) {
-  __shared__ int4 s_edge[kCutChunk];   // previous edge of u and of v, deg[u], deg[v]
+// What the estimate needs of edge j: previous edges of u and of v, deg[u], deg[v].
+struct GatherEdge {
+  const int32_t* u;
+  const int32_t* v;
+  const int32_t* prev;
+  const int32_t* deg;
+  __device__ __forceinline__ int4 operator()(int64_t j) const {
+    const int2 pe = *reinterpret_cast<const int2*>(prev + 2 * j);
+    return make_int4(pe.x, pe.y, deg[u[j]], deg[v[j]]);
+  }
+};
+struct PackedEdge {
+  const int4* e;
+  __device__ __forceinline__ int4 operator()(int64_t j) const { return e[j]; }
+};
+
+__global__ void k_pack_edges(GatherEdge edge, int64_t m, int4* out, const unsigned long long* bad) {
+  pdl_wait();
+  pdl_trigger();
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < m && *bad == 0) out[j] = edge(j);
+}
+
+template <class E>
+__device__ int64_t plan_cuts(E edge, int64_t m, int64_t p0, int64_t maxcsr, int64_t* cuts, int64_t* ests) {
+  __shared__ int4 s_edge[kCutChunk];
   __shared__ int64_t s_warp[2][kCutThreads / 32];
   __shared__ unsigned long long s_cut[2];
   __shared__ int64_t s_est;
@@ -107,10 +131,7 @@ __device__ int64_t plan_cuts(const int32_t* u, const int32_t* v, const int32_t* 
         c0 = p + t0;
         c1 = min(c0 + kCutChunk, m);
         __syncthreads();
-        for (int64_t j = c0 + tid; j < c1; j += kCutThreads) {
-          const int2 pe = *reinterpret_cast<const int2*>(prev + 2 * j);
-          s_edge[j - c0] = make_int4(pe.x, pe.y, deg[u[j]], deg[v[j]]);
-        }
+        for (int64_t j = c0 + tid; j < c1; j += kCutThreads) s_edge[j - c0] = edge(j);
         __syncthreads();
       }
       const int64_t t = t0 + tid;
@@ -172,13 +193,12 @@ __device__ __forceinline__ void plan_record(int64_t k, const int64_t* cuts, cons
   host[8 + 3 * k + 2] = seed_end;
 }
 
-__global__ void __launch_bounds__(kCutThreads) k_cuts(const int32_t* u, const int32_t* v, const int32_t* prev,
-                                                      const int32_t* deg, int64_t m, int64_t p0, int64_t maxcsr,
+__global__ void __launch_bounds__(kCutThreads) k_cuts(const int4* edges, int64_t m, int64_t p0, int64_t maxcsr,
                                                       int64_t* cuts, int64_t* ests, unsigned long long* count,
                                                       const unsigned long long* bc, int64_t* host) {
   pdl_wait();
   pdl_trigger();
-  const int64_t k = bc[0] != 0 ? 0 : plan_cuts(u, v, prev, deg, m, p0, maxcsr, cuts, ests);
+  const int64_t k = bc[0] != 0 ? 0 : plan_cuts(PackedEdge{edges}, m, p0, maxcsr, cuts, ests);
   if (threadIdx.x == 0) {
     *count = (unsigned long long)k;
     plan_header(k, bc, host);
@@ -202,7 +222,7 @@ __global__ void __launch_bounds__(kCutThreads) k_plan_small(const int32_t* u, co
   }
   __shared__ int s_warp[33];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int64_t count = plan_cuts(u, v, prev, deg, m, p0, maxcsr, cuts, ests);
+  const int64_t count = plan_cuts(GatherEdge{u, v, prev, deg}, m, p0, maxcsr, cuts, ests);
   __syncthreads();
   int64_t carry = 0;
   const int64_t slots = 2 * (m - p0);
@@ -2234,23 +2254,42 @@ __global__ void k_finalize_all(const uint32_t* wval, int32_t n, uint32_t epoch, 
 
 // ---- assignment and order ------------------------------------------------------------
 
-// The cluster count (*ccp, the new-id scan total) comes from the device; ids
-// at or beyond min(cluster_count, MAX_BATCH_SIZE) are dropped.
-__global__ void k_assign(const int32_t* u, const int32_t* v, int64_t p, int64_t len, const int32_t* cid,
-                         const int64_t* ccp, int tbits, uint64_t* keys, uint32_t* vals, unsigned long long* count) {
-  pdl_wait();
-  pdl_trigger();
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= len) return;
-  const int64_t limit = min(*ccp, kMaxBatchEdges);
-  const int64_t j = p + t;
-  int32_t c = cid[u[j]];
-  if (c == -1) c = cid[v[j]];
-  if (c < 0 || (int64_t)c >= limit) return;
-  const unsigned long long k = atomicAdd(count, 1ull);
-  keys[k] = ((uint64_t)c << tbits) | (uint64_t)(((1u << tbits) - 1u) - (uint32_t)t);
-  vals[k] = (uint32_t)t;
-}
+// The assigned edges of a larger sub-batch, by the library's scan: item i is
+// the edge with the index len - 1 - i, so the keys come out in descending
+// index and a stable sort on the cluster alone gives the order.  The cluster
+// count (*ccp, the new-id scan total) comes from the device; ids at or beyond
+// min(cluster_count, MAX_BATCH_SIZE) are dropped.
+struct AssignFlag {
+  const int32_t* u;
+  const int32_t* v;
+  int64_t p, len;
+  const int32_t* cid;
+  const int64_t* ccp;
+  __device__ __forceinline__ int32_t cluster(int64_t i) const {
+    const int64_t j = p + len - 1 - i;
+    int32_t c = cid[u[j]];
+    if (c == -1) c = cid[v[j]];
+    return c >= 0 && (int64_t)c < min(*ccp, kMaxBatchEdges) ? c : -1;
+  }
+  __device__ __forceinline__ int64_t operator()(int64_t i) const { return cluster(i) >= 0 ? 1 : 0; }
+};
+
+struct AssignOut {
+  AssignFlag edge;
+  uint64_t* keys;
+  uint32_t* vals;
+  unsigned long long* count;
+  __device__ __forceinline__ void operator()(int64_t i, int64_t at) const {
+    if (i == edge.len) {
+      *count = (unsigned long long)at;
+      return;
+    }
+    const int32_t c = edge.cluster(i);
+    if (c < 0) return;
+    keys[at] = (uint64_t)(uint32_t)c;
+    vals[at] = (uint32_t)(edge.len - 1 - i);
+  }
+};
 
 // The assignment of a sub-batch whose edges fit one commit block of the repair
 // (kRoundCap), in one launch: the assigned edges, ordered by (cluster
@@ -3406,6 +3445,22 @@ constexpr int kLargeItems = 8;
 constexpr int kLargeWrites = kLargeItems * kRoundThreads;
 constexpr size_t kLargeSmem = (size_t)kLargeWrites * 12 + (size_t)(kRoundThreads / 32) * sort_detail::kDigits * 4;
 
+// The nk writes in shared memory ordered by vertex (stable).
+template <int Items>
+__device__ __noinline__ void sort_writes(int nk, int nbits, uint64_t* sk, uint32_t* sv, uint32_t* cnt, uint32_t* dbase,
+                                         uint32_t* sw) {
+  const int at = (threadIdx.x >> 5) * 32 * Items + (threadIdx.x & 31);
+  uint64_t key[Items];
+  uint32_t val[Items];
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    key[r] = at + r * 32 < nk ? sk[at + r * 32] : 0;
+    val[r] = at + r * 32 < nk ? sv[at + r * 32] : 0;
+  }
+  __syncthreads();
+  sort_detail::block_sort<Items>(false, key, val, nk, 32, 32 + nbits, sk, sv, cnt, dbase, sw);
+}
+
 __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa, const unsigned long long* best,
                                                                     bool init, int nbits, uint64_t* view_keys,
                                                                     uint32_t* view_vals, uint8_t* m, int64_t* host) {
@@ -3434,33 +3489,45 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa,
   }
   __syncthreads();
   int nk = 0;
-  for (int64_t base = sa.p0; base < sa.cnt; base += kRoundThreads) {
-    const int64_t pos = base + tid;
-    int32_t a = -1, b = -1;
-    bool ins = false;
-    if (pos < sa.cnt) {
-      a = n0[pos];
-      b = n1[pos];
-      ins = sa.ins[sa.p + sa.order[pos]] != 0;
-      const int32_t ra = sa.prev0[pos], rb = sa.prev1[pos];
-      if (a != ra || b != rb) {
+  constexpr int kPer = 4;   // consecutive positions per thread and step
+  for (int64_t base = sa.p0; base < sa.cnt; base += kRoundThreads * kPer) {
+    const int64_t pos0 = base + (int64_t)tid * kPer;
+    int32_t a[kPer], b[kPer];
+    bool ins[kPer];
+    int writes = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      const int64_t pos = pos0 + q;
+      const bool in = pos < sa.cnt;
+      a[q] = in ? n0[pos] : -1;
+      b[q] = in ? n1[pos] : -1;
+      ins[q] = in && sa.ins[sa.p + sa.order[pos]] != 0;
+      const int32_t ra = in ? sa.prev0[pos] : -1, rb = in ? sa.prev1[pos] : -1;
+      if (a[q] != ra || b[q] != rb) {
         atomicMin(&s_f, (unsigned long long)pos);
-        if (!only_joins(ins, a, b, ra, rb)) s_grown = 0;
+        if (!only_joins(ins[q], a[q], b[q], ra, rb)) s_grown = 0;
       }
-      if (a == b) a = -1;   // a removed vertex that joins again: the join is the later write
+      if (a[q] == b[q]) a[q] = -1;   // a removed vertex that joins again: the join is the later write
+      writes += (a[q] >= 0) + (b[q] >= 0);
     }
     int total = 0;
-    int k = nk + round_scan((a >= 0) + (b >= 0), s_warp, &total);
-    if (a >= 0) {
-      if (k < kLargeWrites) {
-        sk[k] = ((uint64_t)(uint32_t)a << 32) | (uint64_t)pos;
-        sv[k] = ins ? 0u : 1u;
+    int k = nk + round_scan(writes, s_warp, &total);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+      if (a[q] >= 0) {
+        if (k < kLargeWrites) {
+          sk[k] = ((uint64_t)(uint32_t)a[q] << 32) | (uint64_t)(pos0 + q);
+          sv[k] = ins[q] ? 0u : 1u;
+        }
+        ++k;
       }
-      ++k;
-    }
-    if (b >= 0 && k < kLargeWrites) {
-      sk[k] = ((uint64_t)(uint32_t)b << 32) | (uint64_t)pos;
-      sv[k] = 1u;
+      if (b[q] >= 0) {
+        if (k < kLargeWrites) {
+          sk[k] = ((uint64_t)(uint32_t)b[q] << 32) | (uint64_t)(pos0 + q);
+          sv[k] = 1u;
+        }
+        ++k;
+      }
     }
     nk += total;
   }
@@ -3472,18 +3539,11 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa,
     }
     return;
   }
-  if (nk > 1) {
-    const int at = (tid >> 5) * 32 * kLargeItems + (tid & 31);
-    uint64_t key[kLargeItems];
-    uint32_t val[kLargeItems];
-#pragma unroll
-    for (int r = 0; r < kLargeItems; ++r) {
-      key[r] = at + r * 32 < nk ? sk[at + r * 32] : 0;
-      val[r] = at + r * 32 < nk ? sv[at + r * 32] : 0;
-    }
-    __syncthreads();
-    sort_detail::block_sort<kLargeItems>(false, key, val, nk, 32, 32 + nbits, sk, sv, cnts, s_dbase, s_sw);
-  }
+  // the fewest items per thread that hold the writes
+  if (nk > 4 * kRoundThreads) sort_writes<8>(nk, nbits, sk, sv, cnts, s_dbase, s_sw);
+  else if (nk > 2 * kRoundThreads) sort_writes<4>(nk, nbits, sk, sv, cnts, s_dbase, s_sw);
+  else if (nk > kRoundThreads) sort_writes<2>(nk, nbits, sk, sv, cnts, s_dbase, s_sw);
+  else if (nk > 1) sort_writes<1>(nk, nbits, sk, sv, cnts, s_dbase, s_sw);
   for (int64_t k = tid; k < sa.view.nkeys; k += kRoundThreads) m[view_keys[k] >> 32] &= 1;
   __syncthreads();
   const unsigned long long f = s_f;
@@ -4075,8 +4135,9 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
   int64_t p0 = 0, nview = 0, rounds = 0;
   if (prepared || queued_rounds(nproc)) {
     // Every round fits one commit block: rounds are queued up to kRoundsPerSync
-    // at a time (one, while the last sub-batch needed only one) and read back
-    // once; a queued round finds its start and view on the device and does
+    // at a time (one, while the last four sub-batches needed only one: a queued
+    // round that is not needed costs 6 us, one that was not queued a wait) and
+    // read back once; a queued round finds its start and view on the device and does
     // nothing once the repair is done.  Round r writes into one pair of result
     // buffers and compares with the other, in turn.
     int64_t* dyn = c->counters.p + 58;
@@ -4100,7 +4161,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     }
     int64_t queued = 0;
     while (true) {
-      const int64_t most = queued == 0 && c->repair_last <= 1 ? 1 : kRoundsPerSync;
+      const int64_t most = queued == 0 && (c->repair_more & 15u) == 0 ? 1 : kRoundsPerSync;
       const int64_t k = std::min<int64_t>(most, kMaxRounds - queued);
       for (int64_t j = 0; j < k; ++j, ++queued) {
         const SpecArgs a = args(queued);
@@ -4122,7 +4183,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
       MF_CUDA(cudaStreamSynchronize(s));
       dsc.reset();
       if (h[60] == 1) {
-        c->repair_last = h[61];
+        c->repair_more = (c->repair_more << 1) | (h[61] > 1 ? 1u : 0u);
         return h[61];
       }
       if (h[60] == 2) break;   // too many writes for one block
@@ -4142,7 +4203,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     p0 = h[58];
     nview = h[59];
     rounds = h[61];
-    c->repair_last = kRoundsPerSync;
+    c->repair_more = (c->repair_more << 1) | 1u;
     if (rounds & 1) {
       std::swap(c->rp_w0, c->rp_n0);
       std::swap(c->rp_w1, c->rp_n1);
@@ -4322,8 +4383,11 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                       c->plan_cuts.p, c->plan_ests.p, c->plan_send.p, c->seeds_all.p, bc, c->h_plan));
       return;
     }
-    MF_K(launch_pdl(k_cuts, 1, kCutThreads, 0, s, c->bu.p, c->bv.p, c->prev.p, c->deg.p, m, p0, c->max_csr,
-                    c->plan_cuts.p, c->plan_ests.p, kcount, bc, c->h_plan));
+    c->plan_edges.reserve(4 * m);
+    int4* edges = reinterpret_cast<int4*>(c->plan_edges.p);
+    MF_K(launch_pdl(k_pack_edges, grid_for(m), kTB, 0, s, GatherEdge{c->bu.p, c->bv.p, c->prev.p, c->deg.p}, m, edges,
+                    bc));
+    MF_K(launch_pdl(k_cuts, 1, kCutThreads, 0, s, edges, m, p0, c->max_csr, c->plan_cuts.p, c->plan_ests.p, kcount, bc, c->h_plan));
     MF_K(launch_pdl(k_plan_seed_flags, grid_for(nslots), kTB, 0, s, c->prev.p, c->plan_cuts.p, kcount, m, p0,
                     c->plan_flags.p));
     scan_exclusive_u8(c->plan_flags.p, c->plan_pos.p, nslots, c->ws, s);
@@ -4546,7 +4610,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       if (2.0 * push_b < pull_b) use_pull = false;
     }
     // Row tails where the rows are too many for L2 to hold what the pull reads
-    // (made once per base; on smaller graphs the rows' ends come from L2).
+    // (made once per base; on smaller graphs the rows' ends come from L2: at
+    // 10^6 vertices of degree 20 the pull took 60 us without and 70 us with them).
     const bool tails = use_pull && n >= kTailsMin;
     if (tails && c->tails.cap < 4 * (int64_t)n) {
       c->tails.reserve(4 * (int64_t)n);
@@ -4651,17 +4716,15 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       cc = h[63];
       if (nproc > 0) c->stats.repair_rounds += rounds;
     } else {
-      const int tbits = bits_for(std::max<int64_t>(q - p - 1, 1));   // the sub-batch index of an edge
       MF_CUDA(cudaMemcpyAsync(h + 7, c->i64b.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      MF_K(launch_pdl(k_assign, grid_for(q - p), kTB, 0, s, c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows, tbits,
-                      c->keys.p, c->vals.p, ucnt + 55));
+      const AssignFlag af{c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows};
+      scan_detail::scan_exclusive_to(af, AssignOut{af, c->keys.p, c->vals.p, ucnt + 55}, q - p, c->ws, s);
       MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
       cc = h[7];
       const int64_t limit = std::min<int64_t>(cc, kMaxBatchEdges);
       nproc = h[9];
-      radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, tbits + bits_for(std::max<int64_t>(limit, 1)), c->ws,
-                                s);
+      radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, bits_for(std::max<int64_t>(limit, 1)), c->ws, s);
       sc.reset();
       if (nproc > 0) c->stats.repair_rounds += repair(c, g, p, nproc, ns, false);
     }
