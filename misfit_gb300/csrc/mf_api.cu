@@ -232,6 +232,7 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   c->work.reserve(mf::kWorkWords);
   c->touched_total = 0;
   c->pull_runs = 0;
+  c->end_recorded = false;
   MF_CUDA(cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long) * mf::kWorkWords, s));
   MF_CUDA(cudaEventRecord(c->ev0, s));
   if (m > 0) {
@@ -243,7 +244,7 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
     c->stats.row_degree_total = -1;
     c->traces.clear();
   }
-  MF_CUDA(cudaEventRecord(c->ev1, s));
+  if (!c->end_recorded) MF_CUDA(cudaEventRecord(c->ev1, s));
   MF_CUDA(cudaEventSynchronize(c->ev1));
   float ms = 0.f;
   MF_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));

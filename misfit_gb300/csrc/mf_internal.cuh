@@ -732,6 +732,7 @@ struct mf_ctx {
   // counts the ones not yet collected
   mf::AsyncQueue* aq = nullptr;
   bool pending = false;
+  bool end_recorded = false;   // ev1 stands behind the batch's last work
   bool mid_batch = false;   // a batch began and has not ended: zeroed scratch may not be zero
   // load-balancing settings (mf_set_tuning); they move work between kernels,
   // never a result

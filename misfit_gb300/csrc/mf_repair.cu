@@ -47,6 +47,7 @@ namespace {
 constexpr int kTB = 256;
 static_assert(kTB == kLbThreads, "lb_rows kernels run kLbThreads-thread blocks");
 constexpr int32_t kSkip = -2;
+constexpr int64_t kUncountedRows = 1 << 19;   // most rows a sub-batch may be launched for before its count is known
 constexpr int32_t kTailsMin = 1 << 20;   // vertices from which the pull uses row tails
 // host counter slots [kFrontSlot + 2f, +1]: front f's counts, copied on the
 // stream that computed it
@@ -367,6 +368,23 @@ __device__ __forceinline__ void add_work(unsigned long long* work, int64_t visit
   for (int o = 16; o > 0; o >>= 1) visited += __shfl_down_sync(0xffffffffu, visited, o);
   if ((threadIdx.x & 31) == 0 && visited) atomicAdd(work, (unsigned long long)visited);
 }
+
+// The counts of a sub-batch's front where they are first known, on the device:
+// kernels sized by an upper bound read them there.
+struct HopCounts {
+  const int64_t* cnt;   // [0] hop-1 << 32 | candidates
+  int64_t capc;         // most candidate rows
+  __device__ __forceinline__ int64_t hop1() const { return *cnt >> 32; }
+  __device__ __forceinline__ int64_t cands() const { return min((int64_t)(*cnt & 0xffffffffll), capc); }
+};
+
+// Creation flags of the rows that exist, zero up to the scan's bound.
+struct CreatesUpTo {
+  const uint8_t* creates;
+  int64_t ns;
+  HopCounts hc;
+  __device__ __forceinline__ int64_t operator()(int64_t i) const { return i < ns + hc.cands() ? creates[i] : 0; }
+};
 
 // ---- hop-1 set as a bitmap ----------------------------------------------------------
 // The hop-1 marks of a sub-batch go into a bitmap (hbits) and the seeds into
@@ -1706,12 +1724,12 @@ __global__ void k_need_decide(GraphView g, const int32_t* need, const int32_t* n
 // candidates that write set their bit for the pull (ncbits, null when the
 // candidates' ids are pushed; k_clear takes the bits back) and leave their id
 // where one load finds it (newcid).
-__global__ void k_new_ids(int64_t rows, const int64_t* pos, int32_t* rowcid, const int32_t* seeds, int64_t ns,
+__global__ void k_new_ids(HopCounts hc, const int64_t* pos, int32_t* rowcid, const int32_t* seeds, int64_t ns,
                           const int32_t* cands, uint32_t epoch, uint32_t* bval, uint32_t* ncbits, int32_t* newcid) {
   pdl_wait();
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows) return;
+  if (i >= ns + hc.cands()) return;
   const int32_t rc = rowcid[i];
   if (rc == -1) rowcid[i] = (int32_t)pos[i];
   if (rc == kSkip) return;
@@ -1868,7 +1886,7 @@ __global__ void k_hop1_short(GraphView g, const int32_t* deg, const int32_t* see
 
 // k_row_skip, the first-hit search of the rows and k_live_decide: the group
 // tests the ids themselves, so no bitmap of them is built.
-__global__ void k_first_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct,
+__global__ void k_first_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* cands, HopCounts hc,
                               const int32_t* cid, int32_t* v2i, int32_t* rowcid, uint8_t* creates, int32_t* need,
                               int32_t* needv, unsigned long long* nneed) {
   pdl_wait();
@@ -1876,7 +1894,7 @@ __global__ void k_first_short(GraphView g, const int32_t* seeds, int64_t ns, con
   const int64_t i = group_id();
   const int gl = threadIdx.x & (kGroup - 1);
   const int g0 = threadIdx.x & 31 & ~(kGroup - 1);   // the group's first lane
-  const bool valid = i < ns + nct;
+  const bool valid = i < ns + hc.cands();
   const int32_t x = valid ? (i < ns ? seeds[i] : cands[i - ns]) : 0;
   const int32_t own = valid ? cid[x] : 0;
   bool open = valid && own == -1;
@@ -1964,15 +1982,16 @@ __global__ void k_push_seed_short(GraphView g, const int32_t* seeds, int64_t ns,
   add_work_if(work, vis);
 }
 
-// k_self_push, both k_lb_push_hop passes and (nct > 0) k_lb_push_cand: all of
-// them only raise wval, so their order does not matter.
-__global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* hlist, int64_t nh,
-                                 const int32_t* cands, int64_t nct, const int32_t* v2i, const int32_t* rowcid,
-                                 uint32_t epoch, const uint32_t* bval, uint32_t* wval, unsigned long long* work_hop,
+// k_self_push, both k_lb_push_hop passes and (with_cands) k_lb_push_cand: all
+// of them only raise wval, so their order does not matter.
+__global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* hlist,
+                                 const int32_t* cands, HopCounts hc, bool with_cands, const int32_t* v2i,
+                                 const int32_t* rowcid, uint32_t epoch, const uint32_t* bval, uint32_t* wval, unsigned long long* work_hop,
                                  unsigned long long* work_cand) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = group_id();
+  const int64_t nh = hc.hop1(), nct = with_cands ? hc.cands() : 0;
   int64_t vis = 0;
   bool cand = false;
   if (i < ns + nh) {
@@ -2379,6 +2398,80 @@ __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const i
     dyn[4] = n;
     dyn[5] = cc;
     dyn[6] = 0;
+  }
+}
+
+// The same for sub-batches of up to Items * 1024 edges: assignment and order by
+// one block, several edges a thread; k_repair_init and k_spec_round_large make
+// the repair's start.  order[0 .. dyn[4]).
+constexpr int64_t kAssignBlock = 8192;
+
+template <int Items>
+__global__ void __launch_bounds__(1024) k_assign_block(const int32_t* u, const int32_t* v, int64_t p, int len,
+                                                       const int32_t* cid, const int64_t* ccp, int cbits,
+                                                       uint32_t* order, int64_t* dyn) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) unsigned char as_smem[];
+  __shared__ uint32_t dbase[sort_detail::kDigits];
+  __shared__ uint32_t sw[32];
+  constexpr int cap = Items * 1024;
+  uint64_t* sk = reinterpret_cast<uint64_t*>(as_smem);
+  uint32_t* sv = reinterpret_cast<uint32_t*>(sk + cap);
+  uint32_t* cnt = sv + cap;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int at = w * 32 * Items + lane;
+  const int64_t cc = *ccp;
+  int32_t c[Items];
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    const int t = len - 1 - (at + r * 32);
+    c[r] = t >= 0 ? cid[u[p + t]] : -1;
+  }
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    const int t = len - 1 - (at + r * 32);
+    if (t >= 0 && c[r] == -1) c[r] = cid[v[p + t]];
+    if ((int64_t)c[r] >= min(cc, kMaxBatchEdges)) c[r] = -1;
+  }
+  uint32_t mine = 0;
+#pragma unroll
+  for (int r = 0; r < Items; ++r) mine += __popc(__ballot_sync(0xffffffffu, c[r] >= 0));
+  if (lane == 0) sw[w] = mine;
+  __syncthreads();
+  uint32_t x = sw[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  uint32_t slot = w > 0 ? __shfl_sync(0xffffffffu, x, w - 1) : 0;
+  const int n = (int)__shfl_sync(0xffffffffu, x, 31);
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    const unsigned mask = __ballot_sync(0xffffffffu, c[r] >= 0);
+    if (c[r] >= 0) {
+      const uint32_t k = slot + __popc(mask & ((1u << lane) - 1u));
+      sk[k] = (uint64_t)(uint32_t)c[r];
+      sv[k] = (uint32_t)(len - 1 - (at + r * 32));
+    }
+    slot += __popc(mask);
+  }
+  __syncthreads();
+  uint64_t key[Items];
+  uint32_t val[Items];
+#pragma unroll
+  for (int r = 0; r < Items; ++r) {
+    key[r] = at + r * 32 < n ? sk[at + r * 32] : 0;
+    val[r] = at + r * 32 < n ? sv[at + r * 32] : 0;
+  }
+  __syncthreads();
+  sort_detail::block_sort<Items>(false, key, val, n, 0, cbits, sk, sv, cnt, dbase, sw);
+#pragma unroll
+  for (int r = 0; r < Items; ++r)
+    if (at + r * 32 < n) order[at + r * 32] = val[r];
+  if (tid == 0) {
+    dyn[4] = n;
+    dyn[5] = cc;
   }
 }
 
@@ -3277,10 +3370,11 @@ __device__ __forceinline__ int round_scan(int x, int* s_warp, int* total) {
 // Start of a larger queued repair: the guessed writes, the round words and the
 // deferral counters; k_spec_round_large makes the view of them.
 __global__ void k_repair_init(const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t p, const uint32_t* order,
-                              const uint8_t* mis, int32_t* w0, int32_t* w1, int64_t cnt, int64_t* dyn,
+                              const uint8_t* mis, int32_t* w0, int32_t* w1, int64_t cnt, bool counted, int64_t* dyn,
                               int64_t* counts) {
   pdl_wait();
   pdl_trigger();
+  if (counted) cnt = dyn[4];   // k_assign_block's count
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cnt) {
     const int64_t j = p + order[i];
@@ -3288,7 +3382,7 @@ __global__ void k_repair_init(const int32_t* u, const int32_t* v, const uint8_t*
     w0[i] = ins[j] && (mis[a] & 1) && (mis[b] & 1) ? max(a, b) : -1;
     w1[i] = -1;
   }
-  if (i < 7) dyn[i] = i == 4 ? cnt : 0;
+  if (i < 7 && !(counted && (i == 4 || i == 5))) dyn[i] = i == 4 ? cnt : 0;
   if (i < 6) counts[i] = 0;
 }
 
@@ -3584,12 +3678,16 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa,
   }
 }
 
-__global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, int32_t* cid,
-                        int32_t* v2i, uint32_t* ncbits) {
+// Mapped vertices back to no row and no id.  Queued behind the repair's rounds
+// before the host knows whether they were enough: with `done`, nothing happens
+// unless the repair's word says so.
+__global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, HopCounts hc, int32_t* cid,
+                        int32_t* v2i, uint32_t* ncbits, const int64_t* done) {
   pdl_wait();
   pdl_trigger();
+  if (done && *done != 1) return;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ns + nct) return;
+  if (i >= ns + hc.cands()) return;
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
   cid[x] = -1;
   v2i[x] = -1;
@@ -4114,12 +4212,22 @@ void repair_reserve(mf_ctx* c, int64_t nproc) {
 // start, view and count on the device.
 bool queued_rounds(int64_t most) { return most <= kLargeCap && !host_rounds_forced() && !debug_counters(); }
 
+// How a sub-batch's edges reach the repair: counted on the host, or assigned
+// and ordered by one block with the count on the device (nproc is then an
+// upper bound, and the read-back of the rounds brings the edge and cluster
+// counts, h[62] and h[63]) -- k_assign_small with the repair's start,
+// k_assign_block without it.
+enum class Assigned { kCounted, kSmall, kBlock };
+
 // Repair of one sub-batch: c->vals holds the order (sub-batch indices),
-// nproc entries.  With `prepared`, k_assign_small has made the order and the
-// start, nproc is an upper bound, and the read-back of the rounds brings the
-// edge and cluster counts (h[62], h[63]).  Returns the number of speculative
-// rounds.
-int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t ns, bool prepared) {
+// nproc entries.  queue_clear(done) is called behind every set of queued
+// rounds; *cleared tells whether the last such clear took effect.  Returns the
+// number of speculative rounds.
+template <class F>
+int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t ns, Assigned how, F&& queue_clear,
+               bool* cleared) {
+  const bool prepared = how == Assigned::kSmall;
+  *cleared = false;
   cudaStream_t s = c->stream;
   int64_t* h = c->h_counters;
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
@@ -4133,7 +4241,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
   repair_reserve(c, nproc);
   const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
   int64_t p0 = 0, nview = 0, rounds = 0;
-  if (prepared || queued_rounds(nproc)) {
+  if (how != Assigned::kCounted || queued_rounds(nproc)) {
     // Every round fits one commit block: rounds are queued up to kRoundsPerSync
     // at a time (one, while the last four sub-batches needed only one: a queued
     // round that is not needed costs 6 us, one that was not queued a wait) and
@@ -4155,7 +4263,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
       raise_smem(c->device, k_spec_round_large, kLargeSmem);
       dsc.emplace(c, kStRepair);
       MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 7)), kTB, 0, s, c->bu.p, c->bv.p, c->bins.p, p,
-                      order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, dyn, c->counters.p + 24));
+                      order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, how == Assigned::kBlock, dyn, c->counters.p + 24));
       MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, args(0), c->big_best.p, true, nbits,
                       c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
     }
@@ -4180,9 +4288,11 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
           MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, a, c->big_best.p, false, nbits,
                           c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
       }
-      MF_CUDA(cudaStreamSynchronize(s));
       dsc.reset();
+      queue_clear(dyn + 2);
+      MF_CUDA(cudaStreamSynchronize(s));
       if (h[60] == 1) {
+        *cleared = true;
         c->repair_more = (c->repair_more << 1) | (h[61] > 1 ? 1u : 0u);
         return h[61];
       }
@@ -4203,6 +4313,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     p0 = h[58];
     nview = h[59];
     rounds = h[61];
+    nproc = h[62];
     c->repair_more = (c->repair_more << 1) | 1u;
     if (rounds & 1) {
       std::swap(c->rp_w0, c->rp_n0);
@@ -4487,14 +4598,39 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // the previous sub-batch ran has long finished, and this stream keeps its
     // queue.
     sc.emplace(c, kStSizes);
-    MF_CUDA(cudaEventSynchronize(c->ev_b));
-    h[2] = h[kFrontSlot + 2 * cur];
-    h[4] = h[kFrontSlot + 2 * cur + 1];
-    h[3] = h[2] & 0xffffffffll;
-    h[2] = h[2] >> 32;
-    const int64_t nh = h[2];
+    const bool short_rows = c->max_row <= kShortRow;
     const int64_t capc = std::max<int64_t>(0, kMaxRows - ns);
-    const int64_t nct = std::min<int64_t>(h[3], capc);
+    const HopCounts hc{fr.cnt.p, capc};
+    // Most that the counts and the packed size can be, by the longest row.  A
+    // small graph's or a small batch's packed size is far below the limit:
+    // then nothing on the host depends on the counts, and a front still in
+    // flight is not waited for (the kernels read its counts on the device), as
+    // long as the grids sized by the bound stay small (10^6 rows to clear, scan
+    // and tag cost more than the wait).
+    const double longest = (double)c->max_row;
+    const double most_hop = std::min((double)n, (double)ns * longest);
+    const double most_packed = (double)ns * std::min((double)n, 1.0 + longest + longest * longest) +
+                               (double)(c->nnz + c->a_total);
+    bool exact_counts = true;
+    if (short_rows && !c->trace && !(c->profile & 4) && most_packed < (double)c->max_csr &&
+        (double)ns + most_hop <= (double)kUncountedRows) {
+      const cudaError_t ready = cudaEventQuery(c->ev_b);
+      if (ready != cudaSuccess && ready != cudaErrorNotReady) MF_CUDA(ready);
+      exact_counts = ready == cudaSuccess;
+    } else {
+      MF_CUDA(cudaEventSynchronize(c->ev_b));
+    }
+    if (exact_counts) {
+      h[2] = h[kFrontSlot + 2 * cur];
+      h[4] = h[kFrontSlot + 2 * cur + 1];
+      h[3] = h[2] & 0xffffffffll;
+      h[2] = h[2] >> 32;
+    } else {
+      h[2] = h[3] = (int64_t)most_hop;
+      h[4] = std::min((int64_t)(most_hop * longest), c->nnz + c->a_total);
+    }
+    const int64_t nh = h[2];
+    const int64_t nct = std::min<int64_t>(h[3], capc);   // nh, nct, rows: upper bounds without exact_counts
     const int64_t rows = ns + nct;
     int64_t packed = -1;
     int64_t cand_total = h[4];   // entries of the candidate rows: the bound, exact below if sized
@@ -4587,9 +4723,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // need seeds' rows, [55] the assignment's count
     c->need.reserve(std::max<int64_t>(ns, 1));
     c->needv.reserve(std::max<int64_t>(ns, 1));
-    const bool short_rows = c->max_row <= kShortRow;
     if (short_rows) {
-      MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->cands.p, nct, c->cid.p,
+      MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->cands.p, hc, c->cid.p,
                       c->v2i.p, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
       sc.emplace(c, kStFirstNeed);
       MF_K(launch_pdl(k_need_short, std::min(warps_grid(ns), lb_grid(c, k_need_short)), kTB, 0, s, g, c->need.p,
@@ -4625,8 +4760,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
         MF_CUDA(cudaMemsetAsync(c->ncbits.p, 0, sizeof(uint32_t) * (size_t)c->ncbits.cap, s));
     }
     uint32_t* ncbits = use_pull ? c->ncbits.p : nullptr;
-    scan_exclusive_u8(c->creates.p, c->i64b.p, rows, c->ws, s);
-    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, rows, c->i64b.p, c->rowcid.p, c->seeds.p, ns, c->cands.p, ep,
+    scan_exclusive_with(CreatesUpTo{c->creates.p, ns, hc}, c->i64b.p, rows, c->ws, s);
+    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, hc, c->i64b.p, c->rowcid.p, c->seeds.p, ns, c->cands.p, ep,
                     c->bval.p, ncbits, c->f1.p));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
@@ -4637,8 +4772,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                       wk));
       sc.emplace(c, kStPushHop);
       const int64_t npc = use_pull ? 0 : nct;
-      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->hlist.p, nh,
-                      c->cands.p, npc, c->v2i.p, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
+      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->hlist.p,
+                      c->cands.p, hc, !use_pull, c->v2i.p, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
                       wk ? wk + 3 : nullptr));
     } else {
       row_offsets(c, c->seeds.p, ns, kCntSeedRows, ns, ep);
@@ -4701,24 +4836,49 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // repair (it times itself: rounds vs grid-wide searches).  A sub-batch
     // whose edges fit one commit block is assigned and ordered by one launch,
     // and the host first hears of it when it reads the rounds back.
+    // The mapped vertices are cleared behind the queued rounds, and the last
+    // sub-batch's end of the batch is recorded behind that.
+    const bool last = q >= m && !c->exact;
+    auto queue_clear = [&](const int64_t* done) {
+      StageScope csc(c, kStClear);
+      MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, hc, c->cid.p, c->v2i.p, ncbits,
+                      done));
+      if (last) MF_CUDA(cudaEventRecord(c->ev1, s));
+    };
     sc.emplace(c, kStAssign);
     int64_t nproc, cc;
-    if (q - p <= kRoundCap && queued_rounds(q - p) && !sequential_repair_forced()) {
-      repair_reserve(c, q - p);
-      const unsigned threads = q - p <= 256 ? 256 : 1024;
-      MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)(q - p), c->bins.p, c->cid.p,
-                      c->i64b.p + rows, bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1)),
-                      c->vals.p, c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, c->counters.p + 58,
-                      c->counters.p + 24));
+    bool cleared = false;
+    const int64_t len = q - p;
+    if (len <= kAssignBlock && queued_rounds(len) && !sequential_repair_forced()) {
+      repair_reserve(c, len);
+      const int cbits = bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1));
+      int64_t* dyn = c->counters.p + 58;
+      const int64_t* ccp = c->i64b.p + rows;
+      if (len <= kRoundCap) {
+        const unsigned threads = len <= 256 ? 256 : 1024;
+        MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)len, c->bins.p, c->cid.p, ccp, cbits,
+                        c->vals.p, c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, dyn,
+                        c->counters.p + 24));
+      } else {
+        auto launch = [&](auto kernel, int items) {
+          const size_t smem = (size_t)items * 1024 * 12 + 32 * sort_detail::kDigits * 4;
+          raise_smem(c->device, kernel, smem);
+          MF_K(launch_pdl(kernel, 1, 1024, smem, s, c->bu.p, c->bv.p, p, (int)len, c->cid.p, ccp, cbits, c->vals.p, dyn));
+        };
+        if (len <= 2048) launch(k_assign_block<2>, 2);
+        else if (len <= 4096) launch(k_assign_block<4>, 4);
+        else launch(k_assign_block<8>, 8);
+      }
       sc.reset();
-      const int64_t rounds = repair(c, g, p, q - p, ns, true);
+      const int64_t rounds = repair(c, g, p, len, ns, len <= kRoundCap ? Assigned::kSmall : Assigned::kBlock, queue_clear,
+                                    &cleared);
       nproc = h[62];
       cc = h[63];
       if (nproc > 0) c->stats.repair_rounds += rounds;
     } else {
       MF_CUDA(cudaMemcpyAsync(h + 7, c->i64b.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      const AssignFlag af{c->bu.p, c->bv.p, p, q - p, c->cid.p, c->i64b.p + rows};
-      scan_detail::scan_exclusive_to(af, AssignOut{af, c->keys.p, c->vals.p, ucnt + 55}, q - p, c->ws, s);
+      const AssignFlag af{c->bu.p, c->bv.p, p, len, c->cid.p, c->i64b.p + rows};
+      scan_detail::scan_exclusive_to(af, AssignOut{af, c->keys.p, c->vals.p, ucnt + 55}, len, c->ws, s);
       MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
       cc = h[7];
@@ -4726,7 +4886,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       nproc = h[9];
       radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, bits_for(std::max<int64_t>(limit, 1)), c->ws, s);
       sc.reset();
-      if (nproc > 0) c->stats.repair_rounds += repair(c, g, p, nproc, ns, false);
+      if (nproc > 0)
+        c->stats.repair_rounds += repair(c, g, p, nproc, ns, Assigned::kCounted, queue_clear, &cleared);
     }
     if (tr) tr->hdr[6] = cc;
     sc.reset();
@@ -4737,17 +4898,15 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       for (size_t i = 0; i < ord.size(); ++i) tr->order[i] = (int32_t)(p + ord[i]);
       tr->mis_after = fetch(c->mis.p, n, s);
     }
-
-    // ---- clear (mapped vertices only)
-    sc.emplace(c, kStClear);
-    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
-                    ncbits));
+    if (!cleared) queue_clear(nullptr);
+    if (last) c->end_recorded = true;
     MF_CUDA(cudaGetLastError());
+    const int64_t ncands = std::min<int64_t>(h[kFrontSlot + 2 * cur] & 0xffffffffll, capc);   // the front is past
 
     sc.reset();
     c->stats.sub_batches += 1;
     c->stats.seeds += ns;
-    c->stats.candidates += nct;
+    c->stats.candidates += ncands;
     c->stats.clusters += cc;
     c->stats.processed_edges += nproc;
     p = q;
