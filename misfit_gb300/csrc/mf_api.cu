@@ -156,6 +156,8 @@ void release_all(mf_ctx* c) {
   if (c->h_counters) cudaFreeHost(c->h_counters);
   c->h_counters = c->h_plan = nullptr;
   c->h_stage = nullptr;
+  if (c->h_read) cudaFreeHost(c->h_read);
+  c->h_read = nullptr;
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   c->ev_pool.clear();
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -726,11 +728,7 @@ int mf_greedy_mis(mf_ctx* c, uint8_t* out, int64_t n) {
   return guarded([&] {
     need(c && out && n == c->n, MF_EINVAL, "output must have n entries");
     bind(c);
-    mf::DBuf<uint8_t> d;
-    d.reserve(std::max<int64_t>(n, 1));
-    mf::greedy_mis(c, d.p);
-    if (n > 0) MF_CUDA(cudaMemcpy(out, d.p, (size_t)n, cudaMemcpyDeviceToHost));
-    d.release();
+    mf::greedy_mis(c, out);
   });
 }
 

@@ -727,6 +727,10 @@ struct mf_ctx {
   // records, and the staged input of a small batch
   int64_t* h_plan = nullptr;
   uint8_t* h_stage = nullptr;
+  // batch files parsed on the device: text, line starts, pinned read chunks
+  mf::DBuf<char> txt;
+  mf::DBuf<int64_t> txt_begin;
+  char* h_read = nullptr;
   // the pipelined engine: batches enqueued by mf_apply_batch_async run in
   // order on this context's worker thread (made on first use); `pending`
   // counts the ones not yet collected
@@ -751,7 +755,7 @@ template <class F>
 void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->nindex); f(c->aoff); f(c->aoff_alt); f(c->i64a); f(c->i64b); f(c->rowlens); f(c->rp_pos);
   f(c->big_pos); f(c->big_off); f(c->big_nr); f(c->big_chunks); f(c->big_pre); f(c->dense_light);
-  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base); f(c->atail);
+  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base); f(c->atail); f(c->txt_begin); f(c->txt);
   f(c->n2cache); f(c->n2bound); f(c->un_cnt); f(c->counters); f(c->lb_offs);
   f(c->nlist); f(c->dead); f(c->rcnt); f(c->deg); f(c->aadj); f(c->aown); f(c->aadj_alt); f(c->aown_alt);
   f(c->cid); f(c->v2i); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
@@ -893,7 +897,7 @@ void flag_updates_noalloc(mf_ctx* c, const int32_t* u, const int32_t* v, int64_t
 void noalloc_refresh(int device);   // scratch address of the no-allocation flags, looked up again
 void compact_graph(mf_ctx* c, std::vector<int64_t>& nindex_out, std::vector<int32_t>& nlist_out);
 void rebase(mf_ctx* c);
-void greedy_mis(mf_ctx* c, uint8_t* d_out);
+void greedy_mis(mf_ctx* c, uint8_t* out);       // to host memory
 void check_mis(mf_ctx* c, int64_t* viol, int64_t* uncovered);
 void exact_fixup(mf_ctx* c);                       // exact-MIS mode after a batch
 // mf_parse.cu: batch file -> c->bu / c->bv (valid lines, file order); returns the count

@@ -169,3 +169,59 @@ def test_repair_commit_blocks(gb, m, writes):
             assert g.stats()["sub_batches"] == 1
             assert np.array_equal(g.get_mis(), orc.get_mis())
             assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
+
+
+def _greedy_graphs():
+    yield "one", 1, *W.csr_from_pairs(2, [0], [1])
+    for n in (31, 32, 33, 257, 3000):
+        yield "path", n, *W.csr_from_pairs(n, np.arange(n - 1), np.arange(1, n))        # one chain through every tile
+        yield "back", n, *W.csr_from_pairs(n, np.arange(n - 1), np.full(n - 1, n - 1))  # everything below one vertex
+    yield "er", 20000, *W.er_graph(20000, 9, 3)
+    yield "rmat", 4096, *W.rmat_graph(12, 12, 3)[1]
+
+
+@pytest.mark.parametrize("kind,n,nindex,nlist", [pytest.param(*g, id="%s%d" % g[:2]) for g in _greedy_graphs()])
+def test_greedy_passes(gb, kind, n, nindex, nlist):
+    """The seed MIS of the base graph and of an evolved overlay, and the exact mode's completion (the same passes)."""
+    import oracle as O
+    orc = O.Oracle.from_csr(nindex, nlist)
+    n = nindex.size - 1
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        assert np.array_equal(g.greedy_mis(), O.greedy_mis(nindex, nlist))
+        for x in (g, orc):
+            x.set_mis(np.zeros(n, np.uint8))
+            x.set_exact(True)
+        rng = np.random.default_rng(n)
+        m = min(400, 3 * n)
+        for _ in range(2):
+            u = rng.integers(0, n, m).astype(np.int32)
+            v = ((u + rng.integers(1, max(n, 2), m)) % n).astype(np.int32)
+            keep = u != v
+            u, v = u[keep], v[keep]
+            ins = rng.integers(0, 2, u.size).astype(np.uint8)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            assert np.array_equal(g.get_mis(), orc.get_mis())
+        orc.greedy_current()   # into the oracle's membership
+        assert np.array_equal(g.greedy_mis(), orc.get_mis())
+
+
+def test_parse_long_lines_over_read_chunks(gb, tmp_path):
+    """Files longer than the read chunks, lines longer than a scan word, blank lines, no newline at the end."""
+    rng = np.random.default_rng(1)
+    with gb.Graph.from_csr(*W.er_graph(500, 6, 3)) as g:
+        for size, tail in ((256 << 10, ""), (512 << 10, "\n"), ((768 << 10) + 5, "1 2")):
+            parts, at = [], 0
+            while at < size:
+                kind = rng.integers(0, 4)
+                a, b = rng.integers(0, 600, 2)
+                line = ("%d %d" % (a, b), "%d\t%d %s" % (a, b, "x" * rng.integers(1, 200)), "", "%% %d" % a)[kind]
+                parts.append(line)
+                at += len(line) + 1
+            path = str(tmp_path / "1.mtx")
+            with open(path, "w") as f:
+                f.write("\n".join(parts)[:size] + tail)
+            u, v = gb.read_batch_file(path, 500)
+            du, dv, di = g.parse_batch_file(path)
+            assert u.size > 1000
+            assert np.array_equal(du, u) and np.array_equal(dv, v) and np.array_equal(di, g.flag_updates(u, v))
