@@ -15,6 +15,7 @@
 // equal mf_apply_batch's, and a graph can alternate between the two paths.
 #include <algorithm>
 #include <chrono>
+#include <cmath>
 #include <climits>
 #include <cstdio>
 #include <cstdlib>
@@ -197,6 +198,55 @@ int run_path_items(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
   return status;
 }
 
+// Which of the batches within the kernel's limits run in it.  One CTA makes its
+// vertex passes and walks its rows alone, so its time grows with both far
+// faster than the multi-launch path's, which spreads them over the GPU; but up
+// to two CTAs per SM run at once, while the path's threads overlap by about
+// three.  Measured at the default block (milliseconds; the estimates below
+// follow these):
+//   lines, vertices, mean degree    one CTA   multi-launch
+//   10, 680,622, 27                    3.8       0.19
+//   69, 1,514, 26                      2.4       0.12
+//   954, 12,520, 14                    5.2       0.15
+//   1,418, 15,424, 6                   3.9       0.16
+//   8,000, 100,000, 16                46         0.34
+// So the longest items move to the path as long as an item's own time in the
+// kernel exceeds what the path then has to do.  Small graphs stay while their
+// item is short: steps of many of them are what the kernel is for.
+constexpr double kCtaStays = 3.25;          // ms
+constexpr int32_t kCtaStaysVertices = 4096;
+constexpr double kPathOverlap = 3.0;
+
+double cta_ms(const mf_ctx* c, int64_t m) {
+  const double row = 1.0 + (c->n > 0 ? (double)(c->nnz + c->a_total) / c->n : 0.0);
+  return 0.1 + 4e-6 * (double)c->n + std::max(0.010 * std::sqrt((double)m) * row, 3.6e-4 * (double)m * row);
+}
+
+double path_ms(const mf_ctx* c, int64_t m) { return (0.11 + 2.3e-5 * (double)m + 1e-7 * (double)c->n) / kPathOverlap; }
+
+void route_items(mf_ctx* const* ctxs, const int64_t* m, std::vector<mf::KernelItem>& kernel, std::vector<int64_t>& path) {
+  using mf::KernelItem;
+  double path_total = 0.0;
+  for (int64_t i : path) path_total += path_ms(ctxs[i], m[i]);
+  std::vector<std::pair<double, int64_t>> by_time;   // (one-CTA time, batch)
+  for (const KernelItem& k : kernel) by_time.emplace_back(cta_ms(ctxs[k.idx], m[k.idx]), k.idx);
+  std::sort(by_time.rbegin(), by_time.rend());
+  std::vector<int64_t> moved;
+  for (const auto& t : by_time) {
+    const double after = path_total + path_ms(ctxs[t.second], m[t.second]);
+    if (t.first <= after) break;
+    if (t.first <= kCtaStays && ctxs[t.second]->n <= kCtaStaysVertices) continue;
+    path_total = after;
+    moved.push_back(t.second);
+  }
+  if (moved.empty()) return;
+  std::sort(moved.begin(), moved.end());
+  kernel.erase(std::remove_if(kernel.begin(), kernel.end(),
+                              [&](const KernelItem& k) { return std::binary_search(moved.begin(), moved.end(), k.idx); }),
+               kernel.end());
+  path.insert(path.end(), moved.begin(), moved.end());
+}
+
 void apply_batches(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* const* v, const uint8_t* const* ins,
                    const int64_t* m, int64_t count, const mf_batched_opts& o, mf_batched_stats* st) {
   using namespace mf;
@@ -254,6 +304,7 @@ void apply_batches(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
       path_items.push_back(i);
     }
   }
+  route_items(ctxs, m, kitems, path_items);
   std::sort(kitems.begin(), kitems.end(), [](const KernelItem& a, const KernelItem& b) { return a.cost > b.cost; });
   stats.kernel_items = (int64_t)kitems.size();
   stats.path_items = (int64_t)path_items.size();
