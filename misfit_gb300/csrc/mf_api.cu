@@ -167,6 +167,13 @@ void release_all(mf_ctx* c) {
     cudaStreamDestroy(c->stream_b);
   }
   c->stream_b = nullptr;
+  if (c->stream_r) {
+    cudaStreamSynchronize(c->stream_r);
+    cudaStreamDestroy(c->stream_r);
+  }
+  c->stream_r = nullptr;
+  if (c->ev_s) cudaEventDestroy(c->ev_s);
+  if (c->ev_r) cudaEventDestroy(c->ev_r);
   if (c->ev_a) cudaEventDestroy(c->ev_a);
   if (c->ev_b) cudaEventDestroy(c->ev_b);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -203,6 +210,7 @@ mf_ctx* new_ctx(int gpu) {
     MF_CUDA(cudaStreamCreateWithFlags(&c->stream_b, cudaStreamNonBlocking));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_a, cudaEventDisableTiming));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_b, cudaEventDisableTiming));
+    MF_CUDA(cudaEventCreateWithFlags(&c->ev_r, cudaEventDisableTiming));
     mf::note_alloc();
     // one pinned block: 64 counter words, the batch plan, a small batch's lines
     MF_CUDA(cudaMallocHost(&c->h_counters, sizeof(int64_t) * (64 + mf::kPlanWords) + 9 * (size_t)mf::kSmallBatch));

@@ -675,6 +675,13 @@ struct mf_ctx {
   mf::Front front[2];                 // current and next sub-batch fronts
   cudaStream_t stream_b = nullptr;    // the fronts of later sub-batches run here
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
+  // repairs that overlap the next sub-batch (batches of more than one): their
+  // stream, and the second set of seeds, row map and edge order
+  cudaStream_t stream_r = nullptr;
+  cudaEvent_t ev_s = nullptr, ev_r = nullptr;   // ev_r: the last queued rounds, on either stream
+  mf::DBuf<int32_t> v2i_b, seeds_b;
+  mf::DBuf<uint32_t> vals_b;
+  mf::Scratch ws_r;                   // the repair's scans and sorts
   mf::DBuf<int64_t> n2cache;           // exact 2-hop sizes of this batch's rows
   mf::DBuf<uint32_t> n2stamp;          // batch stamp of each cached size
   mf::DBuf<int64_t> n2bound;           // tighter upper bounds of this batch's 2-hop sizes
@@ -758,13 +765,13 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base); f(c->atail); f(c->txt_begin); f(c->txt);
   f(c->n2cache); f(c->n2bound); f(c->un_cnt); f(c->counters); f(c->lb_offs);
   f(c->nlist); f(c->dead); f(c->rcnt); f(c->deg); f(c->aadj); f(c->aown); f(c->aadj_alt); f(c->aown_alt);
-  f(c->cid); f(c->v2i); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
+  f(c->cid); f(c->v2i); f(c->v2i_b); f(c->seeds_b); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
   f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
   f(c->pull_long); f(c->tails); f(c->plan_edges); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
-  f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
+  f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->vals_b); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
   f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->ncbits); f(c->n2stamp);
   f(c->n2bstamp); f(c->nmark); f(c->cidbits);
   f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
@@ -775,6 +782,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->p2_cnt);
   f(c->ws.hist); f(c->ws.sort_status); f(c->ws.keys_alt);
   f(c->ws.vals_alt); f(c->ws.scan_status);
+  f(c->ws_r.hist); f(c->ws_r.sort_status); f(c->ws_r.keys_alt); f(c->ws_r.vals_alt); f(c->ws_r.scan_status);
   for (auto& fr : c->front) {
     f(fr.bits); f(fr.uacc); f(fr.hlist); f(fr.cands); f(fr.lb_offs); f(fr.cnt);
     f(fr.ws.hist); f(fr.ws.sort_status); f(fr.ws.keys_alt);

@@ -2319,11 +2319,14 @@ struct AssignOut {
 // takes the edge with the index len - 1 - tid, so a stable sort on the cluster
 // alone gives the order.  The guessed writes, a few of the edges, are ordered
 // by counting the smaller ones.
+// As two launches (kAssign, then kGuess) where the guess has to wait for the
+// last sub-batch's repair; `got` then carries the two counts between them.
+template <bool kAssign, bool kGuess>
 __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const int32_t* v, int64_t p, int len,
                                                        const uint8_t* ins, const int32_t* cid, const int64_t* ccp,
                                                        int cbits, uint32_t* order, int32_t* w0, int32_t* w1,
                                                        uint8_t* mis, uint64_t* view_keys, uint32_t* view_vals,
-                                                       int64_t* dyn, int64_t* counts) {
+                                                       int64_t* dyn, int64_t* counts, int64_t* got) {
   pdl_wait();
   pdl_trigger();
   __shared__ uint64_t sk[1024];
@@ -2332,39 +2335,55 @@ __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const i
   __shared__ uint32_t dbase[sort_detail::kDigits];
   __shared__ uint32_t sw[32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, warps = blockDim.x >> 5;
-  const int64_t cc = *ccp;
-  const int t = len - 1 - tid;
-  int32_t c = -1;
-  if (t >= 0) {
-    c = cid[u[p + t]];
-    if (c == -1) c = cid[v[p + t]];
+  int64_t cc = 0;
+  int n = 0;
+  uint32_t val[1] = {0};
+  if (kAssign) {
+    cc = *ccp;
+    const int t = len - 1 - tid;
+    int32_t c = -1;
+    if (t >= 0) {
+      c = cid[u[p + t]];
+      if (c == -1) c = cid[v[p + t]];
+    }
+    const bool take = c >= 0 && (int64_t)c < min(cc, kMaxBatchEdges);
+    const unsigned mask = __ballot_sync(0xffffffffu, take);
+    if (lane == 0) sw[w] = __popc(mask);
+    __syncthreads();
+    uint32_t x = lane < warps ? sw[lane] : 0;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const uint32_t before = w > 0 ? __shfl_sync(0xffffffffu, x, w - 1) : 0;
+    n = (int)__shfl_sync(0xffffffffu, x, 31);
+    const uint32_t slot = before + __popc(mask & ((1u << lane) - 1u));
+    if (take) {
+      sk[slot] = (uint64_t)(uint32_t)c;
+      sv[slot] = (uint32_t)t;
+    }
+    __syncthreads();
+    uint64_t key[1] = {tid < n ? sk[tid] : 0};
+    val[0] = tid < n ? sv[tid] : 0;
+    __syncthreads();
+    sort_detail::block_sort<1>(false, key, val, n, 0, cbits, sk, sv, cnt, dbase, sw);
+    if (tid < n) order[tid] = val[0];
+    if (!kGuess) {
+      if (tid == 0) {
+        got[0] = n;
+        got[1] = cc;
+      }
+      return;
+    }
+  } else {
+    n = (int)got[0];
+    cc = got[1];
+    if (tid < n) val[0] = order[tid];
   }
-  const bool take = c >= 0 && (int64_t)c < min(cc, kMaxBatchEdges);
-  const unsigned mask = __ballot_sync(0xffffffffu, take);
-  if (lane == 0) sw[w] = __popc(mask);
-  __syncthreads();
-  uint32_t x = lane < warps ? sw[lane] : 0;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  const uint32_t before = w > 0 ? __shfl_sync(0xffffffffu, x, w - 1) : 0;
-  const int n = (int)__shfl_sync(0xffffffffu, x, 31);
-  const uint32_t slot = before + __popc(mask & ((1u << lane) - 1u));
-  if (take) {
-    sk[slot] = (uint64_t)(uint32_t)c;
-    sv[slot] = (uint32_t)t;
-  }
-  __syncthreads();
-  uint64_t key[1] = {tid < n ? sk[tid] : 0};
-  uint32_t val[1] = {tid < n ? sv[tid] : 0};
-  __syncthreads();
-  sort_detail::block_sort<1>(false, key, val, n, 0, cbits, sk, sv, cnt, dbase, sw);
   int32_t r = -1;
   if (tid < n) {
     const int64_t j = p + val[0];
     const int32_t a = u[j], b = v[j];
-    order[tid] = val[0];
     if (ins[j] && (mis[a] & 1) && (mis[b] & 1)) r = max(a, b);
     w0[tid] = r;
     w1[tid] = -1;
@@ -2372,7 +2391,7 @@ __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const i
   const unsigned rmask = __ballot_sync(0xffffffffu, r >= 0);
   if (lane == 0) sw[w] = __popc(rmask);
   __syncthreads();   // also: every member byte is read
-  x = lane < warps ? sw[lane] : 0;
+  uint32_t x = lane < warps ? sw[lane] : 0;
   for (int o = 1; o < 32; o <<= 1) {
     const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
     if (lane >= o) x += y;
@@ -2403,13 +2422,13 @@ __global__ void __launch_bounds__(1024) k_assign_small(const int32_t* u, const i
 
 // The same for sub-batches of up to Items * 1024 edges: assignment and order by
 // one block, several edges a thread; k_repair_init and k_spec_round_large make
-// the repair's start.  order[0 .. dyn[4]).
+// the repair's start.  order[0 .. got[0]); got[1] the cluster count.
 constexpr int64_t kAssignBlock = 8192;
 
 template <int Items>
 __global__ void __launch_bounds__(1024) k_assign_block(const int32_t* u, const int32_t* v, int64_t p, int len,
                                                        const int32_t* cid, const int64_t* ccp, int cbits,
-                                                       uint32_t* order, int64_t* dyn) {
+                                                       uint32_t* order, int64_t* got) {
   pdl_wait();
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char as_smem[];
@@ -2470,8 +2489,8 @@ __global__ void __launch_bounds__(1024) k_assign_block(const int32_t* u, const i
   for (int r = 0; r < Items; ++r)
     if (at + r * 32 < n) order[at + r * 32] = val[r];
   if (tid == 0) {
-    dyn[4] = n;
-    dyn[5] = cc;
+    got[0] = n;
+    got[1] = cc;
   }
 }
 
@@ -3370,11 +3389,11 @@ __device__ __forceinline__ int round_scan(int x, int* s_warp, int* total) {
 // Start of a larger queued repair: the guessed writes, the round words and the
 // deferral counters; k_spec_round_large makes the view of them.
 __global__ void k_repair_init(const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t p, const uint32_t* order,
-                              const uint8_t* mis, int32_t* w0, int32_t* w1, int64_t cnt, bool counted, int64_t* dyn,
-                              int64_t* counts) {
+                              const uint8_t* mis, int32_t* w0, int32_t* w1, int64_t cnt, const int64_t* got,
+                              int64_t* dyn, int64_t* counts) {
   pdl_wait();
   pdl_trigger();
-  if (counted) cnt = dyn[4];   // k_assign_block's count
+  if (got) cnt = got[0];   // k_assign_block's count
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cnt) {
     const int64_t j = p + order[i];
@@ -3382,7 +3401,7 @@ __global__ void k_repair_init(const int32_t* u, const int32_t* v, const uint8_t*
     w0[i] = ins[j] && (mis[a] & 1) && (mis[b] & 1) ? max(a, b) : -1;
     w1[i] = -1;
   }
-  if (i < 7 && !(counted && (i == 4 || i == 5))) dyn[i] = i == 4 ? cnt : 0;
+  if (i < 7) dyn[i] = i == 4 ? cnt : i == 5 && got ? got[1] : 0;
   if (i < 6) counts[i] = 0;
 }
 
@@ -3680,17 +3699,20 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa,
 
 // Mapped vertices back to no row and no id.  Queued behind the repair's rounds
 // before the host knows whether they were enough: with `done`, nothing happens
-// unless the repair's word says so.
+// unless the repair's word says so.  Null arrays are left alone: where the
+// repair overlaps the next sub-batch, the ids are cleared at once (and the
+// counts kept for the other call), the row map behind the repair.
 __global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, HopCounts hc, int32_t* cid,
-                        int32_t* v2i, uint32_t* ncbits, const int64_t* done) {
+                        int32_t* v2i, uint32_t* ncbits, const int64_t* done, int64_t* keep) {
   pdl_wait();
   pdl_trigger();
   if (done && *done != 1) return;
+  if (keep && blockIdx.x == 0 && threadIdx.x == 0) *keep = *hc.cnt;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ns + hc.cands()) return;
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
-  cid[x] = -1;
-  v2i[x] = -1;
+  if (cid) cid[x] = -1;
+  if (v2i) v2i[x] = -1;
   if (ncbits && i >= ns) ncbits[x >> 5] = 0;
 }
 
@@ -3721,10 +3743,11 @@ unsigned lb_grid(mf_ctx* c, K kernel) {
 }
 
 // Row-position prefix of list[0..cnt) for lb_rows into c->lb_offs.
-void row_offsets(mf_ctx* c, const int32_t* list, int64_t cnt, int kind, int64_t ns, uint32_t epoch) {
+void row_offsets(mf_ctx* c, const int32_t* list, int64_t cnt, int kind, int64_t ns, uint32_t epoch,
+                 const int32_t* v2i) {
   cudaStream_t s = c->stream;
   c->lb_offs.reserve(cnt + 1);
-  scan_exclusive_with(RowCounts{c->view(), list, kind, c->rowcid.p, ns, c->bval.p, epoch, c->v2i.p}, c->lb_offs.p, cnt,
+  scan_exclusive_with(RowCounts{c->view(), list, kind, c->rowcid.p, ns, c->bval.p, epoch, v2i}, c->lb_offs.p, cnt,
                       c->ws, s);
 }
 
@@ -3988,7 +4011,7 @@ void exact_sizes(mf_ctx* c, int64_t ns, uint32_t ep, bool bound_only) {
   // collect the heavy members of the seeds' closed neighbourhoods not cached yet
   h[30] = c->heavy_used;
   MF_CUDA(cudaMemcpyAsync(c->counters.p + 30, h + 30, sizeof(int64_t), cudaMemcpyHostToDevice, s));
-  row_offsets(c, c->seeds.p, ns, kCntAll, ns, ep);
+  row_offsets(c, c->seeds.p, ns, kCntAll, ns, ep, c->v2i.p);
   MF_K(k_heavy_collect<<<lb_grid(c, k_heavy_collect), kTB, 0, s>>>(g, c->seeds.p, c->lb_offs.p, ns, thr, c->heavy_slot.p,
                                                   c->heavy_list.p,
                                                   reinterpret_cast<unsigned long long*>(c->counters.p) + 30));
@@ -4003,7 +4026,7 @@ void exact_sizes(mf_ctx* c, int64_t ns, uint32_t ep, bool bound_only) {
     if (build_to > from) {
       MF_CUDA(cudaMemsetAsync(c->heavy_bits.p + from * words, 0,
                               sizeof(uint32_t) * (size_t)((build_to - from) * words), s));
-      row_offsets(c, c->heavy_list.p + from, build_to - from, kCntAll, ns, ep);
+      row_offsets(c, c->heavy_list.p + from, build_to - from, kCntAll, ns, ep, c->v2i.p);
       MF_K(k_heavy_build<<<lb_grid(c, k_heavy_build), kTB, 0, s>>>(g, c->heavy_list.p + from, c->lb_offs.p, build_to - from, from,
                                                      words, c->heavy_bits.p));
     }
@@ -4121,7 +4144,8 @@ void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, 
 
 // The clustering read of a sub-batch by the general path (rows of any length):
 // row ids and creation flags of the ns + nct rows into c->rowcid / c->creates.
-void cluster_read(mf_ctx* c, const GraphView& g, int64_t ns, int64_t nct, uint32_t ep, std::optional<StageScope>& sc) {
+void cluster_read(mf_ctx* c, const GraphView& g, const int32_t* seeds, int64_t ns, int64_t nct, int32_t* v2i,
+                  uint32_t ep, std::optional<StageScope>& sc) {
   cudaStream_t s = c->stream;
   const int32_t n = c->n;
   const int64_t rows = ns + nct;
@@ -4132,7 +4156,7 @@ void cluster_read(mf_ctx* c, const GraphView& g, int64_t ns, int64_t nct, uint32
   c->mq_v.reserve(std::max<int64_t>(ns, 1));
   c->mq_base.reserve(std::max<int64_t>(ns, 1));
   const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
-  MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, nct, c->cid.p, c->v2i.p,
+  MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, seeds, ns, c->cands.p, nct, c->cid.p, v2i,
                   c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
   c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
   MF_K(launch_pdl(k_cid_bits, warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s, c->cid.p, n,
@@ -4141,7 +4165,7 @@ void cluster_read(mf_ctx* c, const GraphView& g, int64_t ns, int64_t nct, uint32
   first_hits(c, c->live_v.p, ucnt + 33, rows, has_cid, ucnt + 48);
   MF_K(launch_pdl(k_live_decide, lb_grid(c, k_live_decide), kTB, 0, s, g, c->live_i.p, c->live_v.p, ucnt + 33, ns,
                                                                c->fpos.p, c->cid.p, c->rowcid.p, c->creates.p,
-                                                               c->seeds.p, c->need.p, c->needv.p, ucnt + 34, mq));
+                                                               seeds, c->need.p, c->needv.p, ucnt + 34, mq));
   sc.emplace(c, kStFirstNeed);
   MF_K(launch_pdl(k_mark_need, lb_grid(c, k_mark_need), kTB, 0, s, g, mq, ep, c->nmark.p, c->nlist_need.p, ucnt + 35));
   first_hits(c, c->nlist_need.p, ucnt + 35, n, has_cid, ucnt + 51);
@@ -4212,114 +4236,189 @@ void repair_reserve(mf_ctx* c, int64_t nproc) {
 // start, view and count on the device.
 bool queued_rounds(int64_t most) { return most <= kLargeCap && !host_rounds_forced() && !debug_counters(); }
 
-// How a sub-batch's edges reach the repair: counted on the host, or assigned
-// and ordered by one block with the count on the device (nproc is then an
-// upper bound, and the read-back of the rounds brings the edge and cluster
-// counts, h[62] and h[63]) -- k_assign_small with the repair's start,
-// k_assign_block without it.
-enum class Assigned { kCounted, kSmall, kBlock };
+// How a sub-batch's edges reach the repair: counted on the host (kCounted), or
+// assigned and ordered by one block with the counts on the device -- with the
+// repair's start (kStarted), without it (kSmall, up to kRoundCap edges; kBlock).
+// The job's nproc is then an upper bound, and the read-back of the rounds
+// brings the edge and cluster counts.
+enum class Assigned { kCounted, kStarted, kSmall, kBlock };
 
-// Repair of one sub-batch: c->vals holds the order (sub-batch indices),
-// nproc entries.  queue_clear(done) is called behind every set of queued
-// rounds; *cleared tells whether the last such clear took effect.  Returns the
-// number of speculative rounds.
-template <class F>
-int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t ns, Assigned how, F&& queue_clear,
-               bool* cleared) {
-  const bool prepared = how == Assigned::kSmall;
-  *cleared = false;
-  cudaStream_t s = c->stream;
-  int64_t* h = c->h_counters;
-  unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
-  const uint32_t* order = c->vals.p;
-  if (sequential_repair_forced()) {
-    RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order, nproc, ns, c->v2i.p, c->mis.p};
+// The repair of one sub-batch on stream s: order holds its edges (sub-batch
+// indices).  start() queues the first rounds and behind them the clear of the
+// row map, which takes effect if they suffice; finish() waits for them and does
+// what is left.  Between the two the caller may queue the next sub-batch's
+// clustering on another stream: it reads neither the membership nor this
+// sub-batch's row map.
+struct Repair {
+  mf_ctx* c = nullptr;
+  GraphView g{};
+  cudaStream_t s = nullptr;
+  int64_t p = 0, nproc = 0, ns = 0;
+  Assigned how = Assigned::kCounted;
+  const uint32_t* order = nullptr;
+  const int64_t* got = nullptr;    // device words of the one-block assignments
+  int64_t cc = 0;                  // clusters (kCounted)
+  // the clear
+  const int32_t* seeds = nullptr;
+  const int32_t* cands = nullptr;
+  HopCounts hc{};
+  int64_t rows = 0;                // upper bound of the rows
+  int32_t* v2i = nullptr;
+  int32_t* cid = nullptr;          // null: cleared already
+  uint32_t* ncbits = nullptr;
+  bool last = false;               // the batch ends with it: ev1 behind the clear
+  int64_t queued = 0;
+  bool in_flight = false;
+
+  bool queues() const { return how != Assigned::kCounted || queued_rounds(nproc); }
+
+  void queue_clear(const int64_t* done) {
+    StageScope csc(c, kStClear);
+    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, seeds, ns, cands, hc, cid, v2i, ncbits, done,
+                    static_cast<int64_t*>(nullptr)));
+    if (last) MF_CUDA(cudaEventRecord(c->ev1, s));
+  }
+
+  SpecArgs args(int64_t round) const {
+    const bool even = (round & 1) == 0;
+    unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
+    return SpecArgs{g, c->bu.p, c->bv.p, c->bins.p, p, order, 0, nproc, ns, v2i,
+                    View{c->mis.p, c->rp_keys.p, c->rp_vals.p, 0}, even ? c->rp_n0.p : c->rp_w0.p,
+                    even ? c->rp_n1.p : c->rp_w1.p, c->tune.big_threshold, ucnt + 24, c->big_pos.p, c->big_r.p,
+                    c->big_off.p, c->big_nr.p, c->big_pre.p, ucnt + 25, c->big_pre.cap, c->counters.p + 58,
+                    even ? c->rp_w0.p : c->rp_n0.p, even ? c->rp_w1.p : c->rp_n1.p};
+  }
+
+  bool small() const { return how == Assigned::kStarted || how == Assigned::kSmall; }
+  int vertex_bits() const { return bits_for(std::max<int32_t>(c->n - 1, 1)); }
+
+  // Every round fits one commit block: rounds are queued up to kRoundsPerSync
+  // at a time (one, while the last four sub-batches needed only one: a queued
+  // round that is not needed costs 6 us, one that was not queued a wait) and
+  // read back once; a queued round finds its start and view on the device and
+  // does nothing once the repair is done.  Round r writes into one pair of
+  // result buffers and compares with the other, in turn.
+  void queue_rounds() {
+    int64_t* h = c->h_counters;
+    unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
+    std::optional<StageScope> dsc;
+    const int64_t most = queued == 0 && (c->repair_more & 15u) == 0 ? 1 : kRoundsPerSync;
+    const int64_t k = std::min<int64_t>(most, kMaxRounds - queued);
+    for (int64_t j = 0; j < k; ++j, ++queued) {
+      const SpecArgs a = args(queued);
+      dsc.emplace(c, kStRepair);
+      MF_K(launch_pdl(k_spec_eval, warps_grid(nproc), kTB, 0, s, a, c->big_chunks.p, c->big_best.p, ucnt + 26,
+                      reinterpret_cast<unsigned int*>(ucnt + 29)));
+      dsc.emplace(c, kStRepairBig);
+      MF_K(launch_pdl(k_big_scan, (unsigned)c->big_grid, kBigChunk, 0, s, a, c->big_chunks.p, c->big_best.p,
+                      ucnt + 26));
+      dsc.emplace(c, kStRepair);
+      if (small())
+        MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, a.out0, a.out1, a.prev0, a.prev1, (int64_t)0, nproc,
+                        c->bins.p, p, order, c->rp_keys.p, c->rp_vals.p, (int64_t)0, c->mis.p, ucnt + 20, a,
+                        c->big_best.p, h + 58));
+      else
+        MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, a, c->big_best.p, false, vertex_bits(),
+                        c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
+    }
+    dsc.reset();
+    queue_clear(c->counters.p + 58 + 2);
+    MF_CUDA(cudaEventRecord(c->ev_r, s));
+    MF_CUDA(cudaGetLastError());
+  }
+
+  void start() {
+    in_flight = true;
+    if (sequential_repair_forced() || !queues()) return;   // all of it in finish()
+    int64_t* dyn = c->counters.p + 58;
+    if (how == Assigned::kSmall) {
+      MF_K(launch_pdl(k_assign_small<false, true>, 1, nproc <= 256 ? 256 : 1024, 0, s, c->bu.p, c->bv.p, p, (int)nproc,
+                      c->bins.p, static_cast<const int32_t*>(nullptr), static_cast<const int64_t*>(nullptr), 0,
+                      const_cast<uint32_t*>(order), c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, dyn,
+                      c->counters.p + 24, const_cast<int64_t*>(got)));
+    } else if (!small()) {
+      raise_smem(c->device, k_spec_round_large, kLargeSmem);
+      StageScope isc(c, kStRepair);
+      MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 7)), kTB, 0, s, c->bu.p, c->bv.p, c->bins.p, p,
+                      order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, got, dyn, c->counters.p + 24));
+      MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, args(0), c->big_best.p, true, vertex_bits(),
+                      c->rp_keys.p, c->rp_vals.p, c->mis.p, c->h_counters + 58));
+    }
+    queue_rounds();
+  }
+
+  void finish();
+  int64_t host_rounds(int64_t p0, int64_t nview, int64_t rounds);
+  void sequential(int64_t p0) {
+    RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, v2i, c->mis.p};
     MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
     MF_CUDA(cudaGetLastError());
-    return 0;
   }
-  repair_reserve(c, nproc);
-  const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
-  int64_t p0 = 0, nview = 0, rounds = 0;
-  if (how != Assigned::kCounted || queued_rounds(nproc)) {
-    // Every round fits one commit block: rounds are queued up to kRoundsPerSync
-    // at a time (one, while the last four sub-batches needed only one: a queued
-    // round that is not needed costs 6 us, one that was not queued a wait) and
-    // read back once; a queued round finds its start and view on the device and does
-    // nothing once the repair is done.  Round r writes into one pair of result
-    // buffers and compares with the other, in turn.
-    int64_t* dyn = c->counters.p + 58;
-    std::optional<StageScope> dsc;
-    auto args = [&](int64_t round) {
-      const bool even = (round & 1) == 0;
-      SpecArgs a{g, c->bu.p, c->bv.p, c->bins.p, p, order, 0, nproc, ns, c->v2i.p,
-                 View{c->mis.p, c->rp_keys.p, c->rp_vals.p, 0}, even ? c->rp_n0.p : c->rp_w0.p,
-                 even ? c->rp_n1.p : c->rp_w1.p, c->tune.big_threshold, ucnt + 24, c->big_pos.p, c->big_r.p,
-                 c->big_off.p, c->big_nr.p, c->big_pre.p, ucnt + 25, c->big_pre.cap, dyn,
-                 even ? c->rp_w0.p : c->rp_n0.p, even ? c->rp_w1.p : c->rp_n1.p};
-      return a;
-    };
-    if (!prepared) {
-      raise_smem(c->device, k_spec_round_large, kLargeSmem);
-      dsc.emplace(c, kStRepair);
-      MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 7)), kTB, 0, s, c->bu.p, c->bv.p, c->bins.p, p,
-                      order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, how == Assigned::kBlock, dyn, c->counters.p + 24));
-      MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, args(0), c->big_best.p, true, nbits,
-                      c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
-    }
-    int64_t queued = 0;
-    while (true) {
-      const int64_t most = queued == 0 && (c->repair_more & 15u) == 0 ? 1 : kRoundsPerSync;
-      const int64_t k = std::min<int64_t>(most, kMaxRounds - queued);
-      for (int64_t j = 0; j < k; ++j, ++queued) {
-        const SpecArgs a = args(queued);
-        dsc.emplace(c, kStRepair);
-        MF_K(launch_pdl(k_spec_eval, warps_grid(nproc), kTB, 0, s, a, c->big_chunks.p, c->big_best.p, ucnt + 26,
-                        reinterpret_cast<unsigned int*>(ucnt + 29)));
-        dsc.emplace(c, kStRepairBig);
-        MF_K(launch_pdl(k_big_scan, (unsigned)c->big_grid, kBigChunk, 0, s, a, c->big_chunks.p, c->big_best.p,
-                        ucnt + 26));
-        dsc.emplace(c, kStRepair);
-        if (prepared)
-          MF_K(launch_pdl(k_spec_round, 1, kRoundThreads, 0, s, a.out0, a.out1, a.prev0, a.prev1, (int64_t)0, nproc,
-                          c->bins.p, p, order, c->rp_keys.p, c->rp_vals.p, (int64_t)0, c->mis.p, ucnt + 20, a,
-                          c->big_best.p, h + 58));
-        else
-          MF_K(launch_pdl(k_spec_round_large, 1, kRoundThreads, kLargeSmem, s, a, c->big_best.p, false, nbits,
-                          c->rp_keys.p, c->rp_vals.p, c->mis.p, h + 58));
-      }
-      dsc.reset();
-      queue_clear(dyn + 2);
-      MF_CUDA(cudaStreamSynchronize(s));
+};
+
+void Repair::finish() {
+  in_flight = false;
+  int64_t* h = c->h_counters;
+  int64_t rounds = 0;
+  bool cleared = false;
+  if (sequential_repair_forced()) {
+    if (nproc > 0) sequential(0);
+  } else if (queues()) {
+    for (;;) {
+      MF_CUDA(cudaEventSynchronize(c->ev_r));
+      rounds = h[61];
+      nproc = h[62];
+      if (how != Assigned::kCounted) cc = h[63];
       if (h[60] == 1) {
-        *cleared = true;
-        c->repair_more = (c->repair_more << 1) | (h[61] > 1 ? 1u : 0u);
-        return h[61];
+        cleared = true;
+        c->repair_more = (c->repair_more << 1) | (rounds > 1 ? 1u : 0u);
+        break;
       }
-      if (h[60] == 2) break;   // too many writes for one block
+      if (h[60] == 2) {
+        // too many writes for one block: on with host-driven rounds from the
+        // last one that was committed
+        c->repair_more = (c->repair_more << 1) | 1u;
+        if (rounds & 1) {
+          std::swap(c->rp_w0, c->rp_n0);
+          std::swap(c->rp_w1, c->rp_n1);
+        }
+        rounds = host_rounds(h[58], h[59], rounds);
+        break;
+      }
       if (queued >= kMaxRounds) {
         // round limit: the rest in order by the sequential kernel
-        p0 = h[58];
-        nview = h[59];
-        nproc = h[62];
-        if (nview > 0) MF_K(k_spec_clear_flags<<<grid_for(nview), kTB, 0, s>>>(c->rp_keys.p, nview, c->mis.p));
-        RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, c->v2i.p, c->mis.p};
-        MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
-        MF_CUDA(cudaGetLastError());
-        return h[61];
+        if (h[59] > 0) MF_K(k_spec_clear_flags<<<grid_for(h[59]), kTB, 0, s>>>(c->rp_keys.p, h[59], c->mis.p));
+        sequential(h[58]);
+        break;
       }
+      queue_rounds();
     }
-    // on with host-driven rounds from the last one that was committed
-    p0 = h[58];
-    nview = h[59];
-    rounds = h[61];
-    nproc = h[62];
-    c->repair_more = (c->repair_more << 1) | 1u;
-    if (rounds & 1) {
-      std::swap(c->rp_w0, c->rp_n0);
-      std::swap(c->rp_w1, c->rp_n1);
-    }
+  } else if (nproc > 0) {
+    rounds = host_rounds(0, 0, 0);
   }
+  if (!cleared) {
+    queue_clear(nullptr);
+    MF_CUDA(cudaEventRecord(c->ev_r, s));
+    MF_CUDA(cudaEventSynchronize(c->ev_r));   // the row map is free, and so are the host words
+  }
+  if (nproc > 0) c->stats.repair_rounds += rounds;
+  c->stats.clusters += cc;
+  c->stats.processed_edges += nproc;
+}
+
+// Rounds read back one by one (more than kLargeCap edges, or more writes than
+// one block holds), from position p0 with nview entries of the view.
+int64_t Repair::host_rounds(int64_t p0, int64_t nview, int64_t rounds) {
+  int64_t* h = c->h_counters;
+  unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
+  const int nbits = vertex_bits();
+  // scratch that grows here belongs to the repair's stream
+  Scratch& ws = c->ws_r;
+  struct AllocOn {
+    cudaStream_t before = g_alloc_stream;
+    explicit AllocOn(cudaStream_t s) { g_alloc_stream = s; }
+    ~AllocOn() { g_alloc_stream = before; }
+  } alloc_on(s);
   if (rounds == 0 && nview == 0) {   // else the last results and the view stand as they are
     MF_CUDA(cudaMemsetAsync(c->rp_w0.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
     MF_CUDA(cudaMemsetAsync(c->rp_w1.p, 0xFF, sizeof(int32_t) * (size_t)nproc, s));
@@ -4330,7 +4429,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
   while (p0 < nproc) {
     if (rounds >= kMaxRounds) {
       if (nview > 0) MF_K(k_spec_clear_flags<<<grid_for(nview), kTB, 0, s>>>(c->rp_keys.p, nview, c->mis.p));
-      RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, c->v2i.p, c->mis.p};
+      RepairArgs ra{g, c->bu.p, c->bv.p, c->bins.p, p, order + p0, nproc - p0, ns, v2i, c->mis.p};
       MF_K(k_repair_sequential<<<1, 1024, 0, s>>>(ra));
       MF_CUDA(cudaGetLastError());
       break;
@@ -4338,7 +4437,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     ++rounds;
     const int64_t pending = nproc - p0;
     MF_CUDA(cudaMemsetAsync(c->counters.p + 24, 0, sizeof(int64_t) * 6, s));  // deferrals, prefix use, queue, done
-    SpecArgs a{g, c->bu.p, c->bv.p, c->bins.p, p, order, p0, nproc, ns, c->v2i.p,
+    SpecArgs a{g, c->bu.p, c->bv.p, c->bins.p, p, order, p0, nproc, ns, v2i,
                View{c->mis.p, c->rp_keys.p, c->rp_vals.p, nview}, c->rp_n0.p, c->rp_n1.p,
                c->tune.big_threshold, ucnt + 24, c->big_pos.p, c->big_r.p, c->big_off.p, c->big_nr.p,
                c->big_pre.p, ucnt + 25, c->big_pre.cap};
@@ -4380,7 +4479,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
                                                                  nproc, ucnt + 20));
     // all writes of this round, sorted by (vertex, position)
     MF_K(k_spec_count<<<grid_for(pending), kTB, 0, s>>>(c->rp_n0.p, c->rp_n1.p, p0, nproc, c->rp_u8.p));
-    scan_exclusive_u8(c->rp_u8.p, c->rp_pos.p, pending, c->ws, s);
+    scan_exclusive_u8(c->rp_u8.p, c->rp_pos.p, pending, ws, s);
     MF_CUDA(cudaMemcpyAsync(h + 21, c->rp_pos.p + pending, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaMemcpyAsync(h + 20, c->counters.p + 20, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     MF_K(k_spec_fill<<<grid_for(pending), kTB, 0, s>>>(c->rp_n0.p, c->rp_n1.p, c->rp_pos.p, p0, nproc, c->bu.p,
@@ -4399,7 +4498,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
       dbg_scanned += (int64_t)q[3];
     }
     // the writes are in position order already: a stable sort on the vertex
-    radix_sort_pairs_in_place(c->rp_keys2.p, c->rp_vals2.p, nk, 32, 32 + nbits, c->ws, s);
+    radix_sort_pairs_in_place(c->rp_keys2.p, c->rp_vals2.p, nk, 32, 32 + nbits, ws, s);
     if (nview > 0) MF_K(k_spec_clear_flags<<<grid_for(nview), kTB, 0, s>>>(c->rp_keys.p, nview, c->mis.p));
     const uint64_t last = (uint64_t)std::min<int64_t>(f, nproc - 1);
     if (nk > 0) MF_K(k_spec_commit<<<grid_for(nk), kTB, 0, s>>>(c->rp_keys2.p, c->rp_vals2.p, nk, last, c->mis.p));
@@ -4407,7 +4506,7 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
     nview = 0;
     if (nk > 0) {
       MF_K(k_spec_keep_flags<<<grid_for(nk), kTB, 0, s>>>(c->rp_keys2.p, nk, last, c->mis.p, c->rp_u8.p));
-      scan_exclusive_u8(c->rp_u8.p, c->rp_pos.p, nk, c->ws, s);
+      scan_exclusive_u8(c->rp_u8.p, c->rp_pos.p, nk, ws, s);
       MF_K(k_spec_compact<<<grid_for(nk), kTB, 0, s>>>(c->rp_keys2.p, c->rp_vals2.p, c->rp_u8.p, c->rp_pos.p, nk,
                                                          c->rp_keys.p, c->rp_vals.p));
       MF_CUDA(cudaMemcpyAsync(h + 22, c->rp_pos.p + nk, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -4428,6 +4527,25 @@ int64_t repair(mf_ctx* c, const GraphView& g, int64_t p, int64_t nproc, int64_t 
 
 }  // namespace
 
+namespace {
+
+// The second set of what a repair shares with its sub-batch's clustering, and
+// the repair's stream.
+void pipe_reserve(mf_ctx* c, int64_t m) {
+  if (!c->stream_r) {
+    MF_CUDA(cudaStreamCreateWithFlags(&c->stream_r, cudaStreamNonBlocking));
+    MF_CUDA(cudaEventCreateWithFlags(&c->ev_s, cudaEventDisableTiming));
+  }
+  if (c->v2i_b.cap < c->n) {
+    c->v2i_b.reserve(c->n);
+    MF_CUDA(cudaMemsetAsync(c->v2i_b.p, 0xFF, sizeof(int32_t) * (size_t)c->v2i_b.cap, c->stream));
+  }
+  c->seeds_b.reserve(c->seeds.cap);
+  c->vals_b.reserve(2 * m);
+}
+
+}  // namespace
+
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
   const int32_t n = c->n;
@@ -4439,6 +4557,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   // batches; the next one clears it whole
   const bool dirty = c->mid_batch;
   if (dirty) {
+    if (c->stream_r) MF_CUDA(cudaStreamSynchronize(c->stream_r));
     MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
     if (c->akill.cap > 0) MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
   }
@@ -4570,8 +4689,26 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   front_compute(c, c->front[0], c->seeds_all.p, seed_end.empty() ? 0 : seed_end[0], s, h + kFrontSlot);
   MF_CUDA(cudaEventRecord(c->ev_b, s));
 
+  // With more than one sub-batch, a sub-batch's repair runs on its own stream
+  // while the next one clusters: what both need (seeds, row map, edge order)
+  // alternates between two sets.  Traces and per-stage times keep one stream.
+  const bool pipe = cuts.size() > 1 && !c->trace && (c->profile & 3) != 1 && !debug_counters() && !debug_launches() &&
+                    !sequential_repair_forced() && !host_rounds_forced();
+  if (pipe) pipe_reserve(c, m);
+  Repair job;      // the repair in flight
+  int64_t sub = 0;
+
   int64_t p = 0;
-  while (p < m) {
+  for (; p < m; ++sub) {
+    const bool odd = pipe && (sub & 1) != 0;
+    if (pipe && sub > 0) {
+      std::swap(c->seeds, c->seeds_b);
+      std::swap(c->v2i, c->v2i_b);
+      std::swap(c->vals, c->vals_b);
+    }
+    int32_t* const v2i = c->v2i.p;
+    int32_t* const seeds = c->seeds.p;
+    uint32_t* const order = c->vals.p;
     if (kidx >= cuts.size()) MF_FAIL(MF_ESTATE, "sub-batch plan ended before the batch");
     const int64_t q = cuts[kidx];
     const int64_t est = ests[kidx];
@@ -4579,7 +4716,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
 
     // ---- seeds (first appearance) of this sub-batch into their rows
     sc.emplace(c, kStSeeds);
-    MF_K(launch_pdl(k_seed_rows, grid_for(ns), kTB, 0, s, c->seeds_all.p + seed_base, ns, c->seeds.p, c->v2i.p, ucnt));
+    MF_K(launch_pdl(k_seed_rows, grid_for(ns), kTB, 0, s, c->seeds_all.p + seed_base, ns, seeds, v2i, ucnt));
     const int64_t max_before = c->max_csr;
 
     // ---- hop-1 set and size bound: this sub-batch's front (computed on the
@@ -4612,7 +4749,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     const double most_packed = (double)ns * std::min((double)n, 1.0 + longest + longest * longest) +
                                (double)(c->nnz + c->a_total);
     bool exact_counts = true;
-    if (short_rows && !c->trace && !(c->profile & 4) && most_packed < (double)c->max_csr &&
+    if (short_rows && !pipe && !c->trace && !(c->profile & 4) && most_packed < (double)c->max_csr &&
         (double)ns + most_hop <= (double)kUncountedRows) {
       const cudaError_t ready = cudaEventQuery(c->ev_b);
       if (ready != cudaSuccess && ready != cudaErrorNotReady) MF_CUDA(ready);
@@ -4724,13 +4861,13 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     c->need.reserve(std::max<int64_t>(ns, 1));
     c->needv.reserve(std::max<int64_t>(ns, 1));
     if (short_rows) {
-      MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->cands.p, hc, c->cid.p,
-                      c->v2i.p, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
+      MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, seeds, ns, c->cands.p, hc, c->cid.p,
+                      v2i, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
       sc.emplace(c, kStFirstNeed);
       MF_K(launch_pdl(k_need_short, std::min(warps_grid(ns), lb_grid(c, k_need_short)), kTB, 0, s, g, c->need.p,
                       c->needv.p, ucnt + 34, c->cid.p, c->rowcid.p, c->creates.p));
     } else {
-      cluster_read(c, g, ns, nct, ep, sc);
+      cluster_read(c, g, seeds, ns, nct, v2i, ep, sc);
     }
     // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
     // it reads (as many per vertex as in the last batch that pulled); the
@@ -4761,33 +4898,33 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     }
     uint32_t* ncbits = use_pull ? c->ncbits.p : nullptr;
     scan_exclusive_with(CreatesUpTo{c->creates.p, ns, hc}, c->i64b.p, rows, c->ws, s);
-    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, hc, c->i64b.p, c->rowcid.p, c->seeds.p, ns, c->cands.p, ep,
+    MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, hc, c->i64b.p, c->rowcid.p, seeds, ns, c->cands.p, ep,
                     c->bval.p, ncbits, c->f1.p));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
     if (short_rows) {
       // the elements are counted for the profiler only
       unsigned long long* wk = c->profile ? wk_extra : nullptr;
-      MF_K(launch_pdl(k_push_seed_short, grid_for(ns * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->rowcid.p, ep, c->bval.p,
+      MF_K(launch_pdl(k_push_seed_short, grid_for(ns * kGroup), kTB, 0, s, g, seeds, ns, c->rowcid.p, ep, c->bval.p,
                       wk));
       sc.emplace(c, kStPushHop);
       const int64_t npc = use_pull ? 0 : nct;
-      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, c->seeds.p, ns, c->hlist.p,
-                      c->cands.p, hc, !use_pull, c->v2i.p, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
+      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, seeds, ns, c->hlist.p,
+                      c->cands.p, hc, !use_pull, v2i, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
                       wk ? wk + 3 : nullptr));
     } else {
-      row_offsets(c, c->seeds.p, ns, kCntSeedRows, ns, ep);
-      MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
-      MF_K(launch_pdl(k_self_push, grid_for(ns + nh), kTB, 0, s, c->seeds.p, ns, c->hlist.p, nh, ep, c->bval.p,
+      row_offsets(c, seeds, ns, kCntSeedRows, ns, ep, v2i);
+      MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
+      MF_K(launch_pdl(k_self_push, grid_for(ns + nh), kTB, 0, s, seeds, ns, c->hlist.p, nh, ep, c->bval.p,
                       c->wval.p));
-      row_offsets(c, c->seeds.p, ns, kCntSeedPushers, ns, ep);
+      row_offsets(c, seeds, ns, kCntSeedPushers, ns, ep, v2i);
       const unsigned long long dbg0 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
       sc.emplace(c, kStPushHop);
-      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->seeds.p, c->lb_offs.p, ns, ep, c->bval.p,
+      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p,
                                                                    c->wval.p, wk_extra + 1));
       sc.emplace(c, kStPush);
       if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg0);
-      row_offsets(c, c->hlist.p, nh, kCntHopPushers, ns, ep);
+      row_offsets(c, c->hlist.p, nh, kCntHopPushers, ns, ep, v2i);
       const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
       sc.emplace(c, kStPushHop);
       MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->hlist.p, c->lb_offs.p, nh, ep, c->bval.p,
@@ -4799,7 +4936,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     if (use_pull) {
       ++c->pull_runs;
       c->pull_long.reserve(std::max<int32_t>(n, 1));
-      const PullArgs pa{g,  c->v2i.p, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
+      const PullArgs pa{g,  v2i, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
                         ucnt + 36, wk_extra + 2, c->tune.pull_long, reinterpret_cast<const int4*>(c->tails.p), c->f1.p};
       if (tails) MF_K(launch_pdl(k_pull_tails, grid_for(n, kTB * kPullPer), kTB, 0, s, pa));
       else MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
@@ -4810,7 +4947,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       if (c->profile) c->stage_bytes[kStPull] += 28.0 * (double)n;
     } else {
       if (!short_rows) {
-        row_offsets(c, c->cands.p, nct, kCntCandRows, ns, ep);
+        row_offsets(c, c->cands.p, nct, kCntCandRows, ns, ep, v2i);
         MF_K(launch_pdl(k_lb_push_cand, lb_grid(c, k_lb_push_cand), kTB, 0, s, g, c->cands.p, c->lb_offs.p, nct, ns, ep,
                         c->wval.p, wk_extra + 3));
       }
@@ -4826,80 +4963,101 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       tr = &c->traces.back();
       tr->hdr[0] = p; tr->hdr[1] = q; tr->hdr[2] = ns; tr->hdr[3] = nct; tr->hdr[4] = packed;
       tr->hdr[5] = c->max_csr; tr->hdr[8] = rows; tr->hdr[9] = est;   // hdr[6] after the assignment
-      tr->seeds = fetch(c->seeds.p, ns, s);
+      tr->seeds = fetch(seeds, ns, s);
       tr->cands = fetch(c->cands.p, nct, s);
       tr->cid_after = fetch(c->cid.p, n, s);
       if (packed >= 0) tr->row_len = fetch(c->rowlens.p, rows, s);
     }
 
     // ---- assignment + order (cluster ascending, index descending), then the
-    // repair (it times itself: rounds vs grid-wide searches).  A sub-batch
-    // whose edges fit one commit block is assigned and ordered by one launch,
-    // and the host first hears of it when it reads the rounds back.
-    // The mapped vertices are cleared behind the queued rounds, and the last
-    // sub-batch's end of the batch is recorded behind that.
-    const bool last = q >= m && !c->exact;
-    auto queue_clear = [&](const int64_t* done) {
-      StageScope csc(c, kStClear);
-      MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, c->seeds.p, ns, c->cands.p, hc, c->cid.p, c->v2i.p, ncbits,
-                      done));
-      if (last) MF_CUDA(cudaEventRecord(c->ev1, s));
-    };
+    // repair (it times itself: rounds vs grid-wide searches).  A sub-batch of
+    // up to kAssignBlock edges is assigned and ordered by one launch, and the
+    // host first hears of it when it reads the rounds back.
     sc.emplace(c, kStAssign);
-    int64_t nproc, cc;
-    bool cleared = false;
     const int64_t len = q - p;
+    Repair next;
+    next.c = c;
+    next.g = g;
+    next.p = p;
+    next.nproc = len;
+    next.ns = ns;
+    next.order = order;
+    next.seeds = seeds;
+    next.cands = c->cands.p;
+    next.hc = hc;
+    next.rows = rows;
+    next.v2i = v2i;
+    next.last = q >= m && !c->exact;
+    const int64_t* ccp = c->i64b.p + rows;
     if (len <= kAssignBlock && queued_rounds(len) && !sequential_repair_forced()) {
-      repair_reserve(c, len);
+      if (!pipe) repair_reserve(c, len);
       const int cbits = bits_for(std::max<int64_t>(std::min<int64_t>(rows, kMaxBatchEdges), 1));
-      int64_t* dyn = c->counters.p + 58;
-      const int64_t* ccp = c->i64b.p + rows;
+      int64_t* got = c->counters.p + 66 + (odd ? 2 : 0);
+      next.got = got;
       if (len <= kRoundCap) {
+        next.how = pipe ? Assigned::kSmall : Assigned::kStarted;
         const unsigned threads = len <= 256 ? 256 : 1024;
-        MF_K(launch_pdl(k_assign_small, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)len, c->bins.p, c->cid.p, ccp, cbits,
-                        c->vals.p, c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, dyn,
-                        c->counters.p + 24));
+        auto launch = [&](auto kernel) {
+          MF_K(launch_pdl(kernel, 1, threads, 0, s, c->bu.p, c->bv.p, p, (int)len, c->bins.p, c->cid.p, ccp, cbits,
+                          order, c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, c->counters.p + 58,
+                          c->counters.p + 24, got));
+        };
+        if (pipe) launch(k_assign_small<true, false>);
+        else launch(k_assign_small<true, true>);
       } else {
+        next.how = Assigned::kBlock;
         auto launch = [&](auto kernel, int items) {
           const size_t smem = (size_t)items * 1024 * 12 + 32 * sort_detail::kDigits * 4;
           raise_smem(c->device, kernel, smem);
-          MF_K(launch_pdl(kernel, 1, 1024, smem, s, c->bu.p, c->bv.p, p, (int)len, c->cid.p, ccp, cbits, c->vals.p, dyn));
+          MF_K(launch_pdl(kernel, 1, 1024, smem, s, c->bu.p, c->bv.p, p, (int)len, c->cid.p, ccp, cbits, order, got));
         };
         if (len <= 2048) launch(k_assign_block<2>, 2);
         else if (len <= 4096) launch(k_assign_block<4>, 4);
         else launch(k_assign_block<8>, 8);
       }
-      sc.reset();
-      const int64_t rounds = repair(c, g, p, len, ns, len <= kRoundCap ? Assigned::kSmall : Assigned::kBlock, queue_clear,
-                                    &cleared);
-      nproc = h[62];
-      cc = h[63];
-      if (nproc > 0) c->stats.repair_rounds += rounds;
     } else {
-      MF_CUDA(cudaMemcpyAsync(h + 7, c->i64b.p + rows, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-      const AssignFlag af{c->bu.p, c->bv.p, p, len, c->cid.p, c->i64b.p + rows};
-      scan_detail::scan_exclusive_to(af, AssignOut{af, c->keys.p, c->vals.p, ucnt + 55}, len, c->ws, s);
+      MF_CUDA(cudaMemcpyAsync(h + 7, ccp, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+      const AssignFlag af{c->bu.p, c->bv.p, p, len, c->cid.p, ccp};
+      scan_detail::scan_exclusive_to(af, AssignOut{af, c->keys.p, order, ucnt + 55}, len, c->ws, s);
       MF_CUDA(cudaMemcpyAsync(h + 9, cnt + 55, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
       MF_CUDA(cudaStreamSynchronize(s));
-      cc = h[7];
-      const int64_t limit = std::min<int64_t>(cc, kMaxBatchEdges);
-      nproc = h[9];
-      radix_sort_pairs_in_place(c->keys.p, c->vals.p, nproc, 0, bits_for(std::max<int64_t>(limit, 1)), c->ws, s);
-      sc.reset();
-      if (nproc > 0)
-        c->stats.repair_rounds += repair(c, g, p, nproc, ns, Assigned::kCounted, queue_clear, &cleared);
+      next.cc = h[7];
+      const int64_t limit = std::min<int64_t>(next.cc, kMaxBatchEdges);
+      next.nproc = h[9];
+      radix_sort_pairs_in_place(c->keys.p, order, next.nproc, 0, bits_for(std::max<int64_t>(limit, 1)), c->ws, s);
     }
-    if (tr) tr->hdr[6] = cc;
     sc.reset();
+    if (pipe) {
+      // the ids are free for the next sub-batch; the row map once the repair is done
+      int64_t* keep = c->counters.p + 70 + (odd ? 1 : 0);
+      MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, seeds, ns, c->cands.p, hc, c->cid.p,
+                      static_cast<int32_t*>(nullptr), ncbits, static_cast<const int64_t*>(nullptr), keep));
+      next.hc = HopCounts{keep, capc};
+      next.s = c->stream_r;
+      if (job.in_flight) job.finish();
+      repair_reserve(c, std::max<int64_t>(next.nproc, 1));
+      MF_CUDA(cudaEventRecord(c->ev_s, s));
+      MF_CUDA(cudaStreamWaitEvent(c->stream_r, c->ev_s, 0));
+      job = next;
+      job.start();
+    } else {
+      next.s = s;
+      next.cid = c->cid.p;
+      next.ncbits = ncbits;
+      if (next.how == Assigned::kCounted) repair_reserve(c, std::max<int64_t>(next.nproc, 1));
+      job = next;
+      job.start();
+      job.finish();
+    }
     if (tr) {
-      tr->hdr[7] = nproc;
-      std::vector<uint32_t> ord = fetch(c->vals.p, nproc, s);
+      tr->hdr[6] = job.cc;
+      tr->hdr[7] = job.nproc;
+      std::vector<uint32_t> ord = fetch(order, job.nproc, s);
       tr->order.resize(ord.size());
       for (size_t i = 0; i < ord.size(); ++i) tr->order[i] = (int32_t)(p + ord[i]);
       tr->mis_after = fetch(c->mis.p, n, s);
     }
-    if (!cleared) queue_clear(nullptr);
-    if (last) c->end_recorded = true;
+    if (next.last) c->end_recorded = true;
     MF_CUDA(cudaGetLastError());
     const int64_t ncands = std::min<int64_t>(h[kFrontSlot + 2 * cur] & 0xffffffffll, capc);   // the front is past
 
@@ -4907,13 +5065,12 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     c->stats.sub_batches += 1;
     c->stats.seeds += ns;
     c->stats.candidates += ncands;
-    c->stats.clusters += cc;
-    c->stats.processed_edges += nproc;
     p = q;
     seed_base = seed_base_next;
     kidx = kidx_next;
     cur ^= 1;
   }
+  if (job.in_flight) job.finish();
   if (front_on_b) MF_CUDA(cudaStreamSynchronize(c->stream_b));
   c->mid_batch = false;
   c->stats.max_csr = c->max_csr;

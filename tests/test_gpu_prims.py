@@ -225,3 +225,45 @@ def test_parse_long_lines_over_read_chunks(gb, tmp_path):
             du, dv, di = g.parse_batch_file(path)
             assert u.size > 1000
             assert np.array_equal(du, u) and np.array_equal(dv, v) and np.array_equal(di, g.flag_updates(u, v))
+
+
+@pytest.mark.parametrize("kind,m,max_csr,exact", [
+    ("er", 600, 100000, False), ("er", 600, 100000, True),        # short rows, many sub-batches, growth on the way
+    ("rmat", 800, 300000, False), ("rmat", 800, 300000, True),    # long rows
+    ("sparse", 9000, 4000000, False),                             # sub-batches of 1,025 to 8,192 edges
+    ("sparse", 30000, 30000000, False),                           # of more than 8,192 (assigned over the grid)
+])
+def test_overlapped_repairs(gb, kind, m, max_csr, exact):
+    """Batches of several sub-batches without a trace, so that repairs overlap the next clustering; a batch refused in
+    between changes nothing.  Membership, ids, limit and counters equal the oracle's, and the row map is left clean."""
+    import oracle as O
+    if kind == "er":
+        nindex, nlist = W.er_graph(2000, 6, 5)
+    elif kind == "rmat":
+        nindex, nlist = W.rmat_graph(11, 8, 5)[1]
+    else:
+        nindex, nlist = W.er_graph(60000, 2, 5)
+    n = nindex.size - 1
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    stream = W.ToggleStream(n, nindex, nlist, 6)
+    subs = 0
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for x in (g, orc):
+            x.max_csr = max_csr
+            x.set_mis(mis)
+            x.set_exact(exact)
+        for k in range(3):
+            u, v, ins = stream.next_batch(m, with_flags=True)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            subs = max(subs, g.stats()["sub_batches"])
+            assert np.array_equal(g.get_mis(), orc.get_mis()), k
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), k
+            assert g.max_csr == orc.max_csr
+            bad = u.copy()
+            bad[-1] = n
+            with pytest.raises(gb.MisfitError):
+                g.apply_batch(bad, v, ins)
+            assert np.array_equal(g.get_mis(), orc.get_mis()) and np.array_equal(g.degrees(), orc.degrees())
+    assert subs > 1
