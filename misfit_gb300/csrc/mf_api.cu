@@ -152,6 +152,9 @@ void need(bool cond, int status, const char* msg) {
 }
 
 void release_all(mf_ctx* c) {
+  // a batch that failed midway may have left work on any of them
+  for (cudaStream_t t : {c->stream_b, c->stream_r})
+    if (t) cudaStreamSynchronize(t);
   mf::release_device_state(c);
   if (c->h_counters) cudaFreeHost(c->h_counters);
   c->h_counters = c->h_plan = nullptr;
@@ -167,10 +170,7 @@ void release_all(mf_ctx* c) {
     cudaStreamDestroy(c->stream_b);
   }
   c->stream_b = nullptr;
-  if (c->stream_r) {
-    cudaStreamSynchronize(c->stream_r);
-    cudaStreamDestroy(c->stream_r);
-  }
+  if (c->stream_r) cudaStreamDestroy(c->stream_r);
   c->stream_r = nullptr;
   if (c->ev_s) cudaEventDestroy(c->ev_s);
   if (c->ev_r) cudaEventDestroy(c->ev_r);

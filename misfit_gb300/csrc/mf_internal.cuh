@@ -328,8 +328,8 @@ struct NoAux {
   __device__ __forceinline__ uint32_t operator()(int64_t, int32_t) const { return 0u; }
 };
 
-template <class A, class F>
-__device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const int32_t* list, const int64_t* offs, int64_t cnt,
+template <class L, class A, class F>
+__device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const L& list, const int64_t* offs, int64_t cnt,
                                                A aux, F f) {
   __shared__ LbStage lb_stage[kLbWarps];
   const int lane = threadIdx.x & 31;

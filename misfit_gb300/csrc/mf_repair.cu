@@ -47,6 +47,7 @@ namespace {
 constexpr int kTB = 256;
 static_assert(kTB == kLbThreads, "lb_rows kernels run kLbThreads-thread blocks");
 constexpr int32_t kSkip = -2;
+constexpr int32_t kOverlapFronts = 1 << 16;   // vertices from which fronts run on the second stream
 constexpr int64_t kUncountedRows = 1 << 19;   // most rows a sub-batch may be launched for before its count is known
 constexpr int32_t kTailsMin = 1 << 20;   // vertices from which the pull uses row tails
 // host counter slots [kFrontSlot + 2f, +1]: front f's counts, copied on the
@@ -329,7 +330,7 @@ __global__ void k_seed_rows(const int32_t* seeds_all, int64_t ns, int32_t* seeds
 
 // Row-position counts for lb_rows; rows that must not be visited count 0.
 // kCntMarked: the rows i with marks[i] >= 0 (marks passed as rowcid).
-enum CountKind : int { kCntAll = 0, kCntSeedRows, kCntCandRows, kCntSeedPushers, kCntHopPushers, kCntMarked };
+enum CountKind : int { kCntAll = 0, kCntSeedRows, kCntCandRows, kCntPushers, kCntMarked };
 
 // The count of row i is computed inside the scan's tile load (RowCounts is
 // the scan's loader), so the prefix needs one launch and no count array.
@@ -342,23 +343,24 @@ struct RowCounts {
   const uint32_t* bval;
   uint32_t epoch;
   const int32_t* v2i;
+  const int32_t* hlist;   // kCntPushers: the rows from ns on
   __device__ __forceinline__ int64_t operator()(int64_t i) const {
-    const int32_t x = list[i];
+    const int32_t x = kind == kCntPushers && i >= ns ? hlist[i - ns] : list[i];
     bool use = true;
     if (kind == kCntSeedRows) {
       use = rowcid[i] != kSkip;
     } else if (kind == kCntCandRows) {
       use = rowcid[ns + i] != kSkip;
-    } else if (kind == kCntSeedPushers) {
-      use = (bval[x] >> kRowBits) == epoch;
     } else if (kind == kCntMarked) {
       use = rowcid[i] >= 0;
-    } else if (kind == kCntHopPushers) {
+    } else if (kind == kCntPushers) {
       use = (bval[x] >> kRowBits) == epoch;
-      const int32_t vi = v2i[x];
-      // seeds push in their own pass; a candidate row that writes its own tag
-      // over row(x) dominates bval[x] there (candidate tags are the larger)
-      if (vi >= 0 && ((int64_t)vi < ns || rowcid[vi] != kSkip)) use = false;
+      if (i >= ns) {
+        const int32_t vi = v2i[x];
+        // seeds push in their own place; a candidate row that writes its own tag
+        // over row(x) dominates bval[x] there (candidate tags are the larger)
+        if (vi >= 0 && ((int64_t)vi < ns || rowcid[vi] != kSkip)) use = false;
+      }
     }
     return use ? row_positions(g, x) : 0;
   }
@@ -1380,11 +1382,9 @@ struct HasCidBit {
 // nibbles together, and lane L stores the warp's word L.
 constexpr int64_t kCidBitsPerWarp = 1024;
 
-__global__ void k_cid_bits(const int32_t* cid, int32_t n, uint32_t* bits) {
-  pdl_wait();
-  pdl_trigger();
+__device__ __forceinline__ void cid_bits_warp(const int32_t* cid, int32_t n, uint32_t* bits, int64_t warp) {
   const int lane = threadIdx.x & 31;
-  const int64_t v0 = warp_id() * kCidBitsPerWarp;
+  const int64_t v0 = warp * kCidBitsPerWarp;
   if (v0 >= n) return;   // the whole warp
   uint32_t mine = 0;
 #pragma unroll
@@ -1609,11 +1609,16 @@ __global__ void k_first_chunks(GraphView g, P pred, unsigned long long* firstpos
 // (src/misfit/misfit.cu:224); the other rows are listed (row index and
 // vertex) for the first-existing-id searches.  The candidates also take their
 // place in the row map here (rows ns .. ns + nct - 1).
+// The blocks behind the first `row_blocks` build the id bitmap meanwhile.
 __global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, const int32_t* cid,
                            int32_t* v2i, int32_t* rowcid, uint8_t* creates, int32_t* live_i, int32_t* live_v,
-                           unsigned long long* nlive) {
+                           unsigned long long* nlive, unsigned row_blocks, int32_t n, uint32_t* bits) {
   pdl_wait();
   pdl_trigger();
+  if (blockIdx.x >= row_blocks) {
+    cid_bits_warp(cid, n, bits, ((int64_t)(blockIdx.x - row_blocks) * blockDim.x + threadIdx.x) >> 5);
+    return;
+  }
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ns + nct) return;
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
@@ -1663,10 +1668,15 @@ __global__ void k_live_decide(GraphView g, const int32_t* live_i, const int32_t*
 // order): after row(s), its first existing id is f1(h) of the first h of
 // row(s) that has one, f1(h) being the id of the first element of row(h)
 // with an id.  f1 is computed for the neighbours of the seeds that need it.
+// A chunk is the warp's eight windows: their elements, then their marks, then
+// their claims are in flight together, and the chunk's new entries take their
+// places by one atomic (a window at a time, with one each, took 20 us for
+// 65,000 entries).
 __global__ void k_mark_need(GraphView g, ChunkQueue mq, uint32_t epoch, uint32_t* nmark, int32_t* list,
                             unsigned long long* count) {
   pdl_wait();
   pdl_trigger();
+  constexpr int kWin = (int)(kFirstChunk / 32);
   const int lane = threadIdx.x & 31;
   const unsigned long long pk = *mq.packed;
   const int64_t rows = (int64_t)(pk >> kChunkShift), chunks = (int64_t)(pk & kChunkMask);
@@ -1675,12 +1685,39 @@ __global__ void k_mark_need(GraphView g, ChunkQueue mq, uint32_t epoch, uint32_t
     const int64_t slot = cq_slot(mq, rows, c);
     const int32_t x = mq.v[slot];
     const int64_t p0 = (c - mq.base[slot]) * kFirstChunk;
-    const int64_t nb = g.nindex[x + 1] - g.nindex[x];
-    const int64_t end = min(p0 + kFirstChunk, nb + (g.aoff[x + 1] - g.aoff[x]));
-    for (int64_t k = p0 + lane; k < end; k += 32) {
-      const int32_t y = row_elem(g, x, k, nb);
-      if (y >= 0 && nmark[y] != epoch && atomicExch(nmark + y, epoch) != epoch) list[atomicAdd(count, 1ull)] = y;
+    const int64_t b0 = g.nindex[x], nb = g.nindex[x + 1] - b0, a0 = g.aoff[x];
+    const int64_t end = min(p0 + kFirstChunk, nb + (g.aoff[x + 1] - a0));
+    const bool filt = g.dead[x] != 0;
+    int32_t y[kWin];
+#pragma unroll
+    for (int q = 0; q < kWin; ++q) {
+      const int64_t k = p0 + 32 * q + lane;
+      y[q] = -1;
+      if (k < nb && k < end) {
+        if (!filt || live_at(g.live, b0 + k)) y[q] = __ldg(g.nlist + b0 + k);
+      } else if (k < end) {
+        y[q] = g.aadj[a0 + (k - nb)];
+      }
     }
+    uint32_t seen[kWin];
+#pragma unroll
+    for (int q = 0; q < kWin; ++q) seen[q] = y[q] >= 0 ? nmark[y[q]] : epoch;
+    unsigned fresh = 0;   // bit q: this lane is the first to mark y[q]
+#pragma unroll
+    for (int q = 0; q < kWin; ++q)
+      if (seen[q] != epoch && atomicExch(nmark + y[q], epoch) != epoch) fresh |= 1u << q;
+    int mine = __popc(fresh), inc = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += t;
+    }
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    unsigned long long at = 0;
+    if (lane == 0 && total > 0) at = atomicAdd(count, (unsigned long long)total);
+    at = __shfl_sync(0xffffffffu, at, 0) + (unsigned long long)(inc - mine);
+#pragma unroll
+    for (int q = 0; q < kWin; ++q)
+      if ((fresh >> q) & 1u) list[at++] = y[q];
   }
 }
 
@@ -1769,21 +1806,17 @@ __global__ void k_lb_push_seed(GraphView g, const int32_t* seeds, const int64_t*
 
 // Phase 2: wval[y] = max over x with y in {x} u row(x) of bval[x] (the 2-hop
 // reach of the seed rows), and the candidate rows' own tags over row(c).
-// Every vertex of list a (cnt_a) and list b (cnt_b) pushes its own phase-1
-// tag, when it has one of this epoch, to itself (one launch for the seeds
-// and the hop-1 vertices).
-__global__ void k_self_push(const int32_t* a, int64_t cnt_a, const int32_t* b, int64_t cnt_b, uint32_t epoch,
-                            const uint32_t* bval, uint32_t* wval) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cnt_a + cnt_b) return;
-  const int32_t x = i < cnt_a ? a[i] : b[i - cnt_a];
-  const uint32_t t = bval[x];
-  if ((t >> kRowBits) == epoch) push_w(wval, x, t);
-}
+// The rows of the seeds and, behind them, of the hop-1 vertices: every vertex
+// with a tag of this epoch pushes it to itself, and to its row where the count
+// is not zero (all of it only raises wval, so one launch does it).
+struct TwoLists {
+  const int32_t* a;
+  const int32_t* b;
+  int64_t na;
+  __device__ __forceinline__ int32_t operator[](int64_t i) const { return i < na ? a[i] : b[i - na]; }
+};
 
-__global__ void __launch_bounds__(kLbThreads, MF_LB_MIN_BLOCKS) k_lb_push_hop(GraphView g, const int32_t* list, const int64_t* offs,
+__global__ void __launch_bounds__(kLbThreads, MF_LB_MIN_BLOCKS) k_lb_push_hop(GraphView g, TwoLists list, const int64_t* offs,
                                                             int64_t cnt, uint32_t epoch, const uint32_t* bval,
                                                             uint32_t* wval, unsigned long long* work) {
   pdl_wait();
@@ -1792,6 +1825,11 @@ __global__ void __launch_bounds__(kLbThreads, MF_LB_MIN_BLOCKS) k_lb_push_hop(Gr
   const int64_t vis = lb_rows_aux(
       g, list, offs, cnt, [&](int64_t, int32_t x) { return bval[x]; },
       [&](int64_t, int32_t, int32_t y, uint32_t t) { push_w(wval, y, t); });
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t x = list[i];
+    const uint32_t t = bval[x];
+    if ((t >> kRowBits) == epoch) push_w(wval, x, t);
+  }
   add_work(work, vis);
 }
 
@@ -1982,7 +2020,7 @@ __global__ void k_push_seed_short(GraphView g, const int32_t* seeds, int64_t ns,
   add_work_if(work, vis);
 }
 
-// k_self_push, both k_lb_push_hop passes and (with_cands) k_lb_push_cand: all
+// k_lb_push_hop and (with_cands) k_lb_push_cand without the prefix: all
 // of them only raise wval, so their order does not matter.
 __global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* hlist,
                                  const int32_t* cands, HopCounts hc, bool with_cands, const int32_t* v2i,
@@ -3747,14 +3785,14 @@ void row_offsets(mf_ctx* c, const int32_t* list, int64_t cnt, int kind, int64_t 
                  const int32_t* v2i) {
   cudaStream_t s = c->stream;
   c->lb_offs.reserve(cnt + 1);
-  scan_exclusive_with(RowCounts{c->view(), list, kind, c->rowcid.p, ns, c->bval.p, epoch, v2i}, c->lb_offs.p, cnt,
-                      c->ws, s);
+  scan_exclusive_with(RowCounts{c->view(), list, kind, c->rowcid.p, ns, c->bval.p, epoch, v2i, c->hlist.p}, c->lb_offs.p,
+                      cnt, c->ws, s);
 }
 
 // Row-position prefix of the rows i of list[0..cnt) with marks[i] >= 0.
 void row_offsets_marked(mf_ctx* c, const int32_t* list, const int32_t* marks, int64_t cnt) {
   c->lb_offs.reserve(cnt + 1);
-  scan_exclusive_with(RowCounts{c->view(), list, kCntMarked, marks, 0, c->bval.p, 0, c->v2i.p}, c->lb_offs.p, cnt,
+  scan_exclusive_with(RowCounts{c->view(), list, kCntMarked, marks, 0, c->bval.p, 0, c->v2i.p, nullptr}, c->lb_offs.p, cnt,
                       c->ws, c->stream);
 }
 
@@ -3762,7 +3800,7 @@ void row_offsets_marked(mf_ctx* c, const int32_t* list, const int32_t* marks, in
 void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>& offs, Scratch& ws,
                       cudaStream_t s) {
   offs.reserve(cnt + 1);
-  scan_exclusive_with(RowCounts{c->view(), list, kCntAll, c->rowcid.p, 0, c->bval.p, 0, c->v2i.p}, offs.p, cnt, ws, s);
+  scan_exclusive_with(RowCounts{c->view(), list, kCntAll, c->rowcid.p, 0, c->bval.p, 0, c->v2i.p, nullptr}, offs.p, cnt, ws, s);
 }
 
 // Buffers of both fronts at their largest sizes for a batch of m updates, so
@@ -3808,7 +3846,8 @@ void front_compute(mf_ctx* c, Front& f, const int32_t* seeds, int64_t ns, cudaSt
   }
   const int64_t capc = std::max<int64_t>(0, kMaxRows - ns);
   scan_detail::scan_exclusive_to(BitsCount{hbits, sbits},
-                                 BitsLists{hbits, sbits, words, capc, f.hlist.p, f.cands.p, f.cnt.p}, words, f.ws, st);
+                                 BitsLists{hbits, sbits, words, capc, f.hlist.p, f.cands.p, f.cnt.p}, words, f.ws, st,
+                                 1024);   // a word writes up to 32 vertices: one per thread
   const unsigned grid = std::min(lb_grid(c, k_bound_finish), grid_for(std::max<int64_t>(ns + c->n, 2 * words)));
   MF_K(launch_pdl(k_bound_finish, grid, kTB, 0, st, g, seeds, ns, f.cands.p, f.cnt.p, capc, f.uacc.p, c->n2cache.p,
                   c->n2stamp.p, c->n2bound.p, c->n2bstamp.p, c->n2batch, f.bits.p, 2 * words, host));
@@ -4156,11 +4195,11 @@ void cluster_read(mf_ctx* c, const GraphView& g, const int32_t* seeds, int64_t n
   c->mq_v.reserve(std::max<int64_t>(ns, 1));
   c->mq_base.reserve(std::max<int64_t>(ns, 1));
   const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
-  MF_K(launch_pdl(k_row_skip, grid_for(rows), kTB, 0, s, seeds, ns, c->cands.p, nct, c->cid.p, v2i,
-                  c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p, ucnt + 33));
   c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
-  MF_K(launch_pdl(k_cid_bits, warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s, c->cid.p, n,
-                  c->cidbits.p));
+  const unsigned row_blocks = grid_for(rows);
+  MF_K(launch_pdl(k_row_skip, row_blocks + warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s,
+                  seeds, ns, c->cands.p, nct, c->cid.p, v2i, c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p,
+                  ucnt + 33, row_blocks, n, c->cidbits.p));
   const HasCidBit has_cid{c->cidbits.p};
   first_hits(c, c->live_v.p, ucnt + 33, rows, has_cid, ucnt + 48);
   MF_K(launch_pdl(k_live_decide, lb_grid(c, k_live_decide), kTB, 0, s, g, c->live_i.p, c->live_v.p, ucnt + 33, ns,
@@ -4557,7 +4596,8 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   // batches; the next one clears it whole
   const bool dirty = c->mid_batch;
   if (dirty) {
-    if (c->stream_r) MF_CUDA(cudaStreamSynchronize(c->stream_r));
+    for (cudaStream_t t : {c->stream_b, c->stream_r})
+      if (t) MF_CUDA(cudaStreamSynchronize(t));
     MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
     if (c->akill.cap > 0) MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
   }
@@ -4680,9 +4720,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   const GraphView g = c->view();
 
   // the first sub-batch's front, on this stream.  Later fronts overlap the
-  // previous sub-batch on the second stream for large graphs; for small ones
-  // the stream switch costs more than the front, which then runs inline.
-  const bool overlap_fronts = c->n >= (1 << 20);
+  // previous sub-batch on the second stream; on small graphs the stream switch
+  // costs more than the front, which then runs inline.
+  const bool overlap_fronts = c->n >= kOverlapFronts;
   front_reserve(c, m, dirty);
   int cur = 0;
   bool front_on_b = false;
@@ -4915,20 +4955,11 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     } else {
       row_offsets(c, seeds, ns, kCntSeedRows, ns, ep, v2i);
       MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
-      MF_K(launch_pdl(k_self_push, grid_for(ns + nh), kTB, 0, s, seeds, ns, c->hlist.p, nh, ep, c->bval.p,
-                      c->wval.p));
-      row_offsets(c, seeds, ns, kCntSeedPushers, ns, ep, v2i);
-      const unsigned long long dbg0 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
-      sc.emplace(c, kStPushHop);
-      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p,
-                                                                   c->wval.p, wk_extra + 1));
-      sc.emplace(c, kStPush);
-      if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg0);
-      row_offsets(c, c->hlist.p, nh, kCntHopPushers, ns, ep, v2i);
+      row_offsets(c, seeds, ns + nh, kCntPushers, ns, ep, v2i);
       const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
       sc.emplace(c, kStPushHop);
-      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, c->hlist.p, c->lb_offs.p, nh, ep, c->bval.p,
-                                                                   c->wval.p, wk_extra + 1));
+      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, TwoLists{seeds, c->hlist.p, ns}, c->lb_offs.p,
+                      ns + nh, ep, c->bval.p, c->wval.p, wk_extra + 1));
       sc.emplace(c, kStPush);
       if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
     }

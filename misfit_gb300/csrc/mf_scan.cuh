@@ -237,12 +237,14 @@ void scan_lookback(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
 // k_scan_lookback.
 constexpr int64_t kSmallTiles = 192;
 
+// `small_tiles`: how many tiles of 256 before the 2,048-item ones (callers whose
+// items write lists of their own want more blocks).
 template <typename L, typename O>
-void scan_exclusive_to(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
+void scan_exclusive_to(L load, O out, int64_t n, Scratch& ws, cudaStream_t s, int64_t small_tiles = kSmallTiles) {
   if (n <= kSingleThreads) {
     const unsigned threads = (unsigned)((n + 31) & ~(int64_t)31);
     MF_K(launch_pdl(k_scan_single<L, O>, 1, threads, 0, s, load, n, out));
-  } else if (n <= kSmallTiles * 256) {
+  } else if (n <= small_tiles * 256) {
     scan_lookback<256, 1>(load, out, n, ws, s);
   } else {
     scan_lookback<512, 4>(load, out, n, ws, s);
