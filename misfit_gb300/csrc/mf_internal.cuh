@@ -328,9 +328,17 @@ struct NoAux {
   __device__ __forceinline__ uint32_t operator()(int64_t, int32_t) const { return 0u; }
 };
 
-template <class L, class A, class F>
-__device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const L& list, const int64_t* offs, int64_t cnt,
-                                               A aux, F f) {
+struct NoPre {
+  __device__ __forceinline__ uint32_t operator()(int32_t) const { return 0u; }
+};
+
+// pre(y) is what f needs to read for y (f gets it as its last argument): the
+// reads of all four windows are issued before any f runs.  Inside f they
+// would wait for one another, because an f that writes with atomics keeps the
+// next one's reads behind it.
+template <class L, class A, class R, class F>
+__device__ __forceinline__ int64_t lb_rows_pre(const GraphView& g, const L& list, const int64_t* offs, int64_t cnt,
+                                               A aux, R pre, F f) {
   __shared__ LbStage lb_stage[kLbWarps];
   const int lane = threadIdx.x & 31;
   LbStage& st = lb_stage[(threadIdx.x >> 5) & (kLbWarps - 1)];
@@ -424,11 +432,14 @@ __device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const L& list
           kr[q] = k;
         }
       }
+      decltype(pre(0)) pv[kLbUnroll];
+#pragma unroll
+      for (int q = 0; q < kLbUnroll; ++q) pv[q] = ok[q] ? pre(yv[q]) : decltype(pre(0)){};
 #pragma unroll
       for (int q = 0; q < kLbUnroll; ++q) {
         if (ok[q]) {
           ++visited;
-          f(ri + kr[q], st.x[kr[q]], yv[q], st.aux[kr[q]]);
+          f(ri + kr[q], st.x[kr[q]], yv[q], st.aux[kr[q]], pv[q]);
         }
       }
     }
@@ -436,6 +447,13 @@ __device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const L& list
     ri += 32;
   }
   return visited;
+}
+
+template <class L, class A, class F>
+__device__ __forceinline__ int64_t lb_rows_aux(const GraphView& g, const L& list, const int64_t* offs, int64_t cnt,
+                                               A aux, F f) {
+  return lb_rows_pre(g, list, offs, cnt, aux, NoPre{},
+                     [&](int64_t i, int32_t x, int32_t y, uint32_t a, uint32_t) { f(i, x, y, a); });
 }
 
 template <class F>
