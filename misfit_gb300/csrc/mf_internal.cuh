@@ -681,8 +681,7 @@ struct mf_ctx {
   mf::DBuf<int32_t> plan_edges;   // int4 per edge of a larger batch
   mf::DBuf<int32_t> seeds_all;
   // first-hit chunk queue (rows) and the need seeds' chunk queue
-  mf::DBuf<int32_t> rq_idx, rq_v, mq_idx, mq_v;
-  mf::DBuf<int64_t> mq_base;
+  mf::DBuf<int32_t> rq_idx, rq_v;
   mf::DBuf<uint8_t> xst, xleave;      // exact-MIS mode: completion states, leave flags
   // batched form (mf_batched.cu): per-vertex engine scratch kept between
   // batches (clustering-write tags, row map = -1, three zero bitmaps), its
@@ -722,7 +721,6 @@ struct mf_ctx {
   int64_t pull_runs = 0;
   mf::DBuf<unsigned long long> fpos;   // first-hit positions
   mf::DBuf<int32_t> un_idx, un_v, need, needv, live_i, live_v, nlist_need;
-  mf::DBuf<uint32_t> nmark;            // epoch marks: neighbours of seeds needing their hop-2 part
   mf::DBuf<int64_t> un_cnt;
   mf::DBuf<int64_t> counters;   // device counters
   int64_t* h_counters = nullptr;  // pinned mirror
@@ -780,18 +778,18 @@ template <class F>
 void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->nindex); f(c->aoff); f(c->aoff_alt); f(c->i64a); f(c->i64b); f(c->rowlens); f(c->rp_pos);
   f(c->big_pos); f(c->big_off); f(c->big_nr); f(c->big_chunks); f(c->big_pre); f(c->dense_light);
-  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->mq_base); f(c->atail); f(c->txt_begin); f(c->txt);
+  f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->atail); f(c->txt_begin); f(c->txt);
   f(c->n2cache); f(c->n2bound); f(c->un_cnt); f(c->counters); f(c->lb_offs);
   f(c->nlist); f(c->dead); f(c->rcnt); f(c->deg); f(c->aadj); f(c->aown); f(c->aadj_alt); f(c->aown_alt);
   f(c->cid); f(c->v2i); f(c->v2i_b); f(c->seeds_b); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
   f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
-  f(c->pull_long); f(c->tails); f(c->plan_edges); f(c->seeds_all); f(c->rq_idx); f(c->rq_v); f(c->mq_idx); f(c->mq_v);
+  f(c->pull_long); f(c->tails); f(c->plan_edges); f(c->seeds_all); f(c->rq_idx); f(c->rq_v);
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
   f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->vals_b); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
   f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->ncbits); f(c->n2stamp);
-  f(c->n2bstamp); f(c->nmark); f(c->cidbits);
+  f(c->n2bstamp); f(c->cidbits);
   f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
   f(c->xst); f(c->xleave); f(c->cta_vert); f(c->cta_ws);
   f(c->keys); f(c->slot_keys); f(c->rp_keys); f(c->rp_keys2);
@@ -831,7 +829,7 @@ inline void release_device_state(mf_ctx* c) {
 // and the n-sized vertex scratch (what a context needs between batches).
 inline void release_batch_scratch(mf_ctx* c) {
   const void* keep[] = {&c->nindex, &c->nlist, &c->live, &c->dead, &c->rcnt, &c->deg, &c->aoff, &c->aadj,
-                        &c->aown, &c->mis, &c->cid, &c->v2i, &c->bval, &c->wval, &c->f1, &c->nmark,
+                        &c->aown, &c->mis, &c->cid, &c->v2i, &c->bval, &c->wval, &c->f1,
                         &c->nlist_need, &c->touched, &c->hlist, &c->adelta, &c->aoff_alt, &c->counters,
                         &c->cta_vert};
   for_each_buffer(c, [&](auto& b) {

@@ -817,7 +817,6 @@ void alloc_vertex_scratch(mf_ctx* c) {
   c->bval.reserve(n);
   c->wval.reserve(n);
   c->f1.reserve(n);
-  c->nmark.reserve(n);
   c->nlist_need.reserve(n);
   c->touched.reserve(n);
   c->hlist.reserve(n);
@@ -826,7 +825,6 @@ void alloc_vertex_scratch(mf_ctx* c) {
     MF_CUDA(cudaMemsetAsync(c->v2i.p, 0xFF, sizeof(int32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->bval.p, 0, sizeof(uint32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->wval.p, 0, sizeof(uint32_t) * (size_t)n, s));
-    MF_CUDA(cudaMemsetAsync(c->nmark.p, 0, sizeof(uint32_t) * (size_t)n, s));
     MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
   }
   c->epoch = 0;

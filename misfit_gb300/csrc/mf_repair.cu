@@ -1424,7 +1424,6 @@ __device__ __forceinline__ void cid_bits_warp(const int32_t* cid, int32_t n, uin
 //      64-bit counter ((rows << 40) | chunks), so that the chunk bases grow
 //      with the row slots; a fixed grid of warps takes chunks, finds the row
 //      by binary search over the bases and keeps the minimum hit position.
-// The same chunk queue drives the marking of the need seeds' neighbours.
 constexpr int kProbe = 32;
 constexpr int64_t kFirstChunk = 256;
 constexpr int kChunkShift = 40;
@@ -1559,7 +1558,10 @@ __global__ void k_first_probe(GraphView g, const int32_t* list, const unsigned l
   }
 }
 
-template <class P>
+// kProbed: the rows that the probe left open, from position kProbe on; else
+// the rows of q.mid_v from their start (a search of few rows, which a thread
+// per row would keep waiting on one lane's chain of loads).
+template <bool kProbed, class P>
 __global__ void k_first_warp(GraphView g, P pred, unsigned long long* firstpos, FirstQueues q) {
   pdl_wait();
   pdl_trigger();
@@ -1567,15 +1569,16 @@ __global__ void k_first_warp(GraphView g, P pred, unsigned long long* firstpos, 
   const int64_t nmid = (int64_t)*q.mid_count;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   for (int64_t w = warp_id(); w < nmid; w += nw) {
-    const int32_t i = q.mid_idx[w];
+    const int32_t i = kProbed ? q.mid_idx[w] : (int32_t)w;
     const int32_t x = q.mid_v[w];
     const int64_t nb = g.nindex[x + 1] - g.nindex[x];
     const int64_t np = nb + (g.aoff[x + 1] - g.aoff[x]);
     const int64_t lim = np < q.bound ? np : q.bound;
-    const int64_t hit = warp_first_range(g, x, nb, kProbe, lim, pred);
-    if (hit >= 0) {
-      if (lane == 0) firstpos[i] = (unsigned long long)hit;
-    } else if (np > q.bound && lane == 0) {
+    const int64_t hit = warp_first_range(g, x, nb, kProbed ? kProbe : 0, lim, pred);
+    if (hit >= 0 || !kProbed) {
+      if (lane == 0) firstpos[i] = hit >= 0 ? (unsigned long long)hit : kNoPos;
+    }
+    if (hit < 0 && np > q.bound && lane == 0) {
       cq_push(q.rest, i, x, (np - q.bound + kFirstChunk - 1) / kFirstChunk);
     }
   }
@@ -1611,11 +1614,14 @@ __global__ void k_first_chunks(GraphView g, P pred, unsigned long long* firstpos
 // Per row: early return when the row's own vertex already has an id
 // (src/misfit/misfit.cu:224); the other rows are listed (row index and
 // vertex) for the first-existing-id searches.  The candidates also take their
-// place in the row map here (rows ns .. ns + nct - 1).
+// place in the row map here (rows ns .. ns + nct - 1).  Hop-1 vertices past
+// the last candidate row (more of them than rows: nh > 0) are listed as
+// rows -1, for their ids alone.
 // The blocks behind the first `row_blocks` build the id bitmap meanwhile.
-__global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, const int32_t* cid,
-                           int32_t* v2i, int32_t* rowcid, uint8_t* creates, int32_t* live_i, int32_t* live_v,
-                           unsigned long long* nlive, unsigned row_blocks, int32_t n, uint32_t* bits) {
+__global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cands, int64_t nct, const int32_t* hlist,
+                           int64_t nh, const int32_t* cid, int32_t* v2i, int32_t* rowcid, uint8_t* creates,
+                           int32_t* live_i, int32_t* live_v, unsigned long long* nlive, unsigned row_blocks, int32_t n,
+                           uint32_t* bits) {
   pdl_wait();
   pdl_trigger();
   if (blockIdx.x >= row_blocks) {
@@ -1623,7 +1629,16 @@ __global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cand
     return;
   }
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ns + nct) return;
+  if (i >= ns + nct + nh) return;
+  if (i >= ns + nct) {
+    const int32_t x = hlist[i - ns - nct];
+    const bool past = nct == 0 || x > cands[nct - 1];
+    if (!past || v2i[x] >= 0 || cid[x] != -1) return;
+    const unsigned long long k = atomicAdd(nlive, 1ull);
+    live_i[k] = -1;
+    live_v[k] = x;
+    return;
+  }
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
   if (i >= ns) v2i[x] = (int32_t)i;
   if (cid[x] != -1) {
@@ -1636,12 +1651,19 @@ __global__ void k_row_skip(const int32_t* seeds, int64_t ns, const int32_t* cand
   live_v[k] = x;
 }
 
-// The first existing id of row(x) in order, if any; seeds without one go on
-// to their hop-2 part (`need`), everything else without one creates a cluster.
+// The first existing id of row(x) in order, if any (f1[x], -1 without one);
+// seeds without one go on to their hop-2 part (`need`), every other row
+// without one creates a cluster.
+// A seed row is [s] ++ row(s) ++ row(h1) ++ row(h2) ++ ... (h over row(s) in
+// order): after row(s), its first existing id is f1(h) of the first h of
+// row(s) that has one.  No h of a row without an id has one itself, so each
+// was searched here as a seed's or a candidate's row, and f1 is known where
+// the hop-2 part reads it.  (The neighbours of those seeds were marked, listed
+// and searched again before: 80 us of a 350 us sub-batch on R-MAT scale 20.)
 __global__ void k_live_decide(GraphView g, const int32_t* live_i, const int32_t* live_v,
                               const unsigned long long* dcnt, int64_t ns, const unsigned long long* firstpos,
-                              const int32_t* cid, int32_t* rowcid, uint8_t* creates, const int32_t* seeds,
-                              int32_t* need, int32_t* needv, unsigned long long* nneed, ChunkQueue mq) {
+                              const int32_t* cid, int32_t* rowcid, uint8_t* creates, int32_t* f1, int32_t* need,
+                              int32_t* needv, unsigned long long* nneed) {
   pdl_wait();
   pdl_trigger();
   const int64_t cnt = (int64_t)*dcnt;
@@ -1649,90 +1671,16 @@ __global__ void k_live_decide(GraphView g, const int32_t* live_i, const int32_t*
     const int32_t i = live_i[k];
     const int32_t x = live_v[k];
     const unsigned long long fp = firstpos[k];
-    if (fp != kNoPos) {
-      rowcid[i] = cid[row_elem(g, x, (int64_t)fp, g.nindex[x + 1] - g.nindex[x])];
-      creates[i] = 0;
-      continue;
-    }
-    rowcid[i] = -1;
-    creates[i] = 1;
-    if (i < ns) {
+    const int32_t id = fp == kNoPos ? -1 : cid[row_elem(g, x, (int64_t)fp, g.nindex[x + 1] - g.nindex[x])];
+    f1[x] = id;
+    if (i < 0) continue;
+    rowcid[i] = id;
+    creates[i] = id == -1 ? 1 : 0;
+    if (id == -1 && i < ns) {
       const unsigned long long u = atomicAdd(nneed, 1ull);
       need[u] = i;
-      const int32_t s = seeds[i];
-      needv[u] = s;
-      const int64_t np = row_positions(g, s);
-      if (np > 0) cq_push(mq, (int32_t)u, s, (np + kFirstChunk - 1) / kFirstChunk);
+      needv[u] = x;
     }
-  }
-}
-
-// A seed row is [s] ++ row(s) ++ row(h1) ++ row(h2) ++ ... (h over row(s) in
-// order): after row(s), its first existing id is f1(h) of the first h of
-// row(s) that has one, f1(h) being the id of the first element of row(h)
-// with an id.  f1 is computed for the neighbours of the seeds that need it.
-// A chunk is the warp's eight windows: their elements, then their marks, then
-// their claims are in flight together, and the chunk's new entries take their
-// places by one atomic (a window at a time, with one each, took 20 us for
-// 65,000 entries).
-__global__ void k_mark_need(GraphView g, ChunkQueue mq, uint32_t epoch, uint32_t* nmark, int32_t* list,
-                            unsigned long long* count) {
-  pdl_wait();
-  pdl_trigger();
-  constexpr int kWin = (int)(kFirstChunk / 32);
-  const int lane = threadIdx.x & 31;
-  const unsigned long long pk = *mq.packed;
-  const int64_t rows = (int64_t)(pk >> kChunkShift), chunks = (int64_t)(pk & kChunkMask);
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t c = warp_id(); c < chunks; c += nw) {
-    const int64_t slot = cq_slot(mq, rows, c);
-    const int32_t x = mq.v[slot];
-    const int64_t p0 = (c - mq.base[slot]) * kFirstChunk;
-    const int64_t b0 = g.nindex[x], nb = g.nindex[x + 1] - b0, a0 = g.aoff[x];
-    const int64_t end = min(p0 + kFirstChunk, nb + (g.aoff[x + 1] - a0));
-    const bool filt = g.dead[x] != 0;
-    int32_t y[kWin];
-#pragma unroll
-    for (int q = 0; q < kWin; ++q) {
-      const int64_t k = p0 + 32 * q + lane;
-      y[q] = -1;
-      if (k < nb && k < end) {
-        if (!filt || live_at(g.live, b0 + k)) y[q] = __ldg(g.nlist + b0 + k);
-      } else if (k < end) {
-        y[q] = g.aadj[a0 + (k - nb)];
-      }
-    }
-    uint32_t seen[kWin];
-#pragma unroll
-    for (int q = 0; q < kWin; ++q) seen[q] = y[q] >= 0 ? nmark[y[q]] : epoch;
-    unsigned fresh = 0;   // bit q: this lane is the first to mark y[q]
-#pragma unroll
-    for (int q = 0; q < kWin; ++q)
-      if (seen[q] != epoch && atomicExch(nmark + y[q], epoch) != epoch) fresh |= 1u << q;
-    int mine = __popc(fresh), inc = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += t;
-    }
-    const int total = __shfl_sync(0xffffffffu, inc, 31);
-    unsigned long long at = 0;
-    if (lane == 0 && total > 0) at = atomicAdd(count, (unsigned long long)total);
-    at = __shfl_sync(0xffffffffu, at, 0) + (unsigned long long)(inc - mine);
-#pragma unroll
-    for (int q = 0; q < kWin; ++q)
-      if ((fresh >> q) & 1u) list[at++] = y[q];
-  }
-}
-
-__global__ void k_f1_finish(GraphView g, const int32_t* list, const unsigned long long* dcnt,
-                            const unsigned long long* firstpos, const int32_t* cid, int32_t* f1) {
-  pdl_wait();
-  pdl_trigger();
-  const int64_t cnt = (int64_t)*dcnt;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t x = list[i];
-    const unsigned long long fp = firstpos[i];
-    f1[x] = fp == kNoPos ? -1 : cid[row_elem(g, x, (int64_t)fp, g.nindex[x + 1] - g.nindex[x])];
   }
 }
 
@@ -1993,9 +1941,11 @@ __global__ void k_first_short(GraphView g, const int32_t* seeds, int64_t ns, con
 
 // The hop-2 part of the seeds without an id in their own row: the id of the
 // first element with one in the first row(h), h over row(s) in order, that has
-// any.  One warp per seed, one h per lane.
+// any.  One warp per seed, one h per lane.  A candidate's row was searched in
+// k_first_short and its id stands in rowcid; a seed's may be changing here, and
+// past the last candidate row there is none: those rows are read again.
 __global__ void k_need_short(GraphView g, const int32_t* need, const int32_t* needv, const unsigned long long* dcnt,
-                             const int32_t* cid, int32_t* rowcid, uint8_t* creates) {
+                             const int32_t* cid, const int32_t* v2i, int64_t ns, int32_t* rowcid, uint8_t* creates) {
   pdl_wait();
   pdl_trigger();
   const int lane = threadIdx.x & 31;
@@ -2005,7 +1955,10 @@ __global__ void k_need_short(GraphView g, const int32_t* need, const int32_t* ne
     for (int32_t k0 = 0; k0 < r.np; k0 += 32) {
       const int32_t h = short_elem(g, r, k0 + lane);
       int32_t id = -1;
-      if (h >= 0) {
+      const int32_t vh = h >= 0 ? v2i[h] : -1;
+      if (vh >= ns) {
+        id = rowcid[vh];
+      } else if (h >= 0) {
         const ShortRow rh = short_row(g, h);
         for (int32_t j0 = 0; j0 < rh.np && id == -1; j0 += 8) {
           int32_t y[8], c[8];
@@ -4180,10 +4133,7 @@ void exact_sizes(mf_ctx* c, int64_t ns, uint32_t ep, bool bound_only) {
 // First-hit search of `pred` over the rows of list[0 .. *dcnt) into c->fpos;
 // `upper` bounds *dcnt.  No host round trip: every level reads its count on
 // the device.
-template <class P>
-void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, int64_t upper, P pred,
-                unsigned long long* qcnt) {
-  cudaStream_t s = c->stream;
+FirstQueues first_queues(mf_ctx* c, int64_t upper, unsigned long long* qcnt) {
   const int64_t cap = std::max<int64_t>(upper, 1);
   c->fpos.reserve(cap);
   c->un_idx.reserve(cap);
@@ -4191,11 +4141,18 @@ void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, 
   c->un_cnt.reserve(cap);
   c->rq_idx.reserve(cap);
   c->rq_v.reserve(cap);
-  const FirstQueues q{c->un_idx.p, c->un_v.p, qcnt, ChunkQueue{c->rq_idx.p, c->rq_v.p, c->un_cnt.p, qcnt + 1},
-                      std::max<int64_t>(c->tune.first_bound, kProbe)};
+  return FirstQueues{c->un_idx.p, c->un_v.p, qcnt, ChunkQueue{c->rq_idx.p, c->rq_v.p, c->un_cnt.p, qcnt + 1},
+                     std::max<int64_t>(c->tune.first_bound, kProbe)};
+}
+
+template <class P>
+void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, int64_t upper, P pred,
+                unsigned long long* qcnt) {
+  cudaStream_t s = c->stream;
+  const FirstQueues q = first_queues(c, upper, qcnt);
   const GraphView g = c->view();
   MF_K(launch_pdl(k_first_probe<P>, lb_grid(c, k_first_probe<P>), kTB, 0, s, g, list, dcnt, pred, c->fpos.p, q));
-  MF_K(launch_pdl(k_first_warp<P>, lb_grid(c, k_first_warp<P>), kTB, 0, s, g, pred, c->fpos.p, q));
+  MF_K(launch_pdl(k_first_warp<true, P>, lb_grid(c, k_first_warp<true, P>), kTB, 0, s, g, pred, c->fpos.p, q));
   MF_K(launch_pdl(k_first_chunks<P>, lb_grid(c, k_first_chunks<P>), kTB, 0, s, g, pred, c->fpos.p, q));
   if (debug_counters()) {
     unsigned long long v[3] = {0, 0, 0};
@@ -4210,36 +4167,42 @@ void first_hits(mf_ctx* c, const int32_t* list, const unsigned long long* dcnt, 
   }
 }
 
+// The same for a list of few rows: a warp per row from its start.
+template <class P>
+void first_hits_few(mf_ctx* c, int32_t* list, unsigned long long* dcnt, int64_t upper, P pred,
+                    unsigned long long* qcnt) {
+  cudaStream_t s = c->stream;
+  FirstQueues q = first_queues(c, upper, qcnt);
+  q.mid_v = list;
+  q.mid_count = dcnt;
+  const GraphView g = c->view();
+  MF_K(launch_pdl(k_first_warp<false, P>, lb_grid(c, k_first_warp<false, P>), kTB, 0, s, g, pred, c->fpos.p, q));
+  MF_K(launch_pdl(k_first_chunks<P>, lb_grid(c, k_first_chunks<P>), kTB, 0, s, g, pred, c->fpos.p, q));
+}
+
 // The clustering read of a sub-batch by the general path (rows of any length):
 // row ids and creation flags of the ns + nct rows into c->rowcid / c->creates.
-void cluster_read(mf_ctx* c, const GraphView& g, const int32_t* seeds, int64_t ns, int64_t nct, int32_t* v2i,
-                  uint32_t ep, std::optional<StageScope>& sc) {
+// nh hop-1 vertices are in c->hlist; ncand of them are no seeds, and the first
+// nct of those have rows.
+void cluster_read(mf_ctx* c, const GraphView& g, const int32_t* seeds, int64_t ns, int64_t nh, int64_t ncand,
+                  int64_t nct, int32_t* v2i, std::optional<StageScope>& sc) {
   cudaStream_t s = c->stream;
   const int32_t n = c->n;
-  const int64_t rows = ns + nct;
+  const int64_t past = ncand > nct ? nh : 0;
+  const int64_t rows = ns + nct + past;
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
   c->live_i.reserve(std::max<int64_t>(rows, 1));
   c->live_v.reserve(std::max<int64_t>(rows, 1));
-  c->mq_idx.reserve(std::max<int64_t>(ns, 1));
-  c->mq_v.reserve(std::max<int64_t>(ns, 1));
-  c->mq_base.reserve(std::max<int64_t>(ns, 1));
-  const ChunkQueue mq{c->mq_idx.p, c->mq_v.p, c->mq_base.p, ucnt + 50};
   c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
   const unsigned row_blocks = grid_for(rows);
   MF_K(launch_pdl(k_row_skip, row_blocks + warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s,
-                  seeds, ns, c->cands.p, nct, c->cid.p, v2i, c->rowcid.p, c->creates.p, c->live_i.p, c->live_v.p,
-                  ucnt + 33, row_blocks, n, c->cidbits.p));
-  const HasCidBit has_cid{c->cidbits.p};
-  first_hits(c, c->live_v.p, ucnt + 33, rows, has_cid, ucnt + 48);
+                  seeds, ns, c->cands.p, nct, c->hlist.p, past, c->cid.p, v2i, c->rowcid.p, c->creates.p,
+                  c->live_i.p, c->live_v.p, ucnt + 33, row_blocks, n, c->cidbits.p));
+  first_hits(c, c->live_v.p, ucnt + 33, rows, HasCidBit{c->cidbits.p}, ucnt + 48);
   MF_K(launch_pdl(k_live_decide, lb_grid(c, k_live_decide), kTB, 0, s, g, c->live_i.p, c->live_v.p, ucnt + 33, ns,
-                                                               c->fpos.p, c->cid.p, c->rowcid.p, c->creates.p,
-                                                               seeds, c->need.p, c->needv.p, ucnt + 34, mq));
+                  c->fpos.p, c->cid.p, c->rowcid.p, c->creates.p, c->f1.p, c->need.p, c->needv.p, ucnt + 34));
   sc.emplace(c, kStFirstNeed);
-  MF_K(launch_pdl(k_mark_need, lb_grid(c, k_mark_need), kTB, 0, s, g, mq, ep, c->nmark.p, c->nlist_need.p, ucnt + 35));
-  first_hits(c, c->nlist_need.p, ucnt + 35, n, has_cid, ucnt + 51);
-  MF_K(launch_pdl(k_f1_finish, lb_grid(c, k_f1_finish), kTB, 0, s, g, c->nlist_need.p, ucnt + 35, c->fpos.p, c->cid.p,
-                                                           c->f1.p));
-  first_hits(c, c->needv.p, ucnt + 34, ns, HasF1{c->f1.p}, ucnt + 53);
+  first_hits_few(c, c->needv.p, ucnt + 34, ns, HasF1{c->f1.p}, ucnt + 53);
   MF_K(launch_pdl(k_need_decide, lb_grid(c, k_need_decide), kTB, 0, s, g, c->need.p, c->needv.p, ucnt + 34, c->fpos.p,
                                                                c->f1.p, c->rowcid.p, c->creates.p));
 }
@@ -4249,7 +4212,6 @@ void next_epoch(mf_ctx* c) {
     cudaStream_t s = c->stream;
     MF_CUDA(cudaMemsetAsync(c->bval.p, 0, sizeof(uint32_t) * (size_t)c->n, s));
     MF_CUDA(cudaMemsetAsync(c->wval.p, 0, sizeof(uint32_t) * (size_t)c->n, s));
-    MF_CUDA(cudaMemsetAsync(c->nmark.p, 0, sizeof(uint32_t) * (size_t)c->n, s));
     c->epoch = 0;
   }
   ++c->epoch;
@@ -4923,10 +4885,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
 
     // ---- clustering (bulk-synchronous); counts stay on the device
     sc.emplace(c, kStFirst);
-    // counters, zeroed by k_seed_rows: [33] live rows, [34] need seeds, [35]
-    // their neighbours, [36] the pull's long rows; [48, 49], [51, 52], [53, 54]
-    // the queues of the three first-hit searches, [50] the chunk queue of the
-    // need seeds' rows, [55] the assignment's count
+    // counters, zeroed by k_seed_rows: [33] live rows, [34] need seeds, [36]
+    // the pull's long rows; [48, 49], [53, 54] the queues of the two first-hit
+    // searches, [55] the assignment's count
     c->need.reserve(std::max<int64_t>(ns, 1));
     c->needv.reserve(std::max<int64_t>(ns, 1));
     if (short_rows) {
@@ -4934,9 +4895,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                       v2i, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
       sc.emplace(c, kStFirstNeed);
       MF_K(launch_pdl(k_need_short, std::min(warps_grid(ns), lb_grid(c, k_need_short)), kTB, 0, s, g, c->need.p,
-                      c->needv.p, ucnt + 34, c->cid.p, c->rowcid.p, c->creates.p));
+                      c->needv.p, ucnt + 34, c->cid.p, v2i, ns, c->rowcid.p, c->creates.p));
     } else {
-      cluster_read(c, g, seeds, ns, nct, v2i, ep, sc);
+      cluster_read(c, g, seeds, ns, nh, h[3], nct, v2i, sc);
     }
     // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
     // it reads (as many per vertex as in the last batch that pulled); the

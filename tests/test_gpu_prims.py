@@ -267,3 +267,63 @@ def test_overlapped_repairs(gb, kind, m, max_csr, exact):
                 g.apply_batch(bad, v, ins)
             assert np.array_equal(g.get_mis(), orc.get_mis()) and np.array_equal(g.degrees(), orc.degrees())
     assert subs > 1
+
+
+@pytest.mark.parametrize("zone", [30000, 1000])
+def test_vertices_past_the_last_candidate_row(gb, zone):
+    """A hub's row fills the sub-batch's 10^6 rows, so the neighbours of the other seeds (larger ids) have none, and
+    what the hop-2 part of those seeds reads of them comes without a row."""
+    import oracle as O
+    leaves = 1020000
+    n = leaves + 1 + zone
+    zi, zl = W.er_graph(zone, 3, zone)
+    lo, hi = W.undirected_pairs(zone, zi, zl)
+    nindex, nlist = W.csr_from_pairs(n, np.concatenate([np.zeros(leaves, np.int64), lo + leaves + 1]),
+                                     np.concatenate([np.arange(1, leaves + 1), hi + leaves + 1]))
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    stream = W.ToggleStream(zone, zi, zl, 3)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for x in (g, orc):
+            x.set_mis(mis)
+        for k in range(4):
+            u, v, ins = stream.next_batch(zone // 50, with_flags=True)
+            u, v = u + leaves + 1, v + leaves + 1
+            if k & 1:
+                u = np.append(u, 0).astype(np.int32)
+                v = np.append(v, leaves + k).astype(np.int32)
+                ins = np.append(ins, 1).astype(np.uint8)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            assert np.array_equal(g.get_mis(), orc.get_mis()), k
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), k
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, (1 << 20) + 1])
+def test_pull_by_row_tails(gb, n):
+    """From 2^20 vertices on the pull reads the rows' last entries first: rows shorter than a tail, tombstones at row
+    ends, rows with none, one and many added entries."""
+    import oracle as O
+    nindex, nlist = W.er_graph(n, 5, 7)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    rng = np.random.default_rng(n)
+    full = np.flatnonzero(np.diff(nindex) > 0)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        g.set_tuning(cand_push=2)
+        for x in (g, orc):
+            x.set_mis(mis)
+        for k in range(3):
+            a = rng.choice(full, 3000, replace=False)
+            last = nlist[nindex[a + 1] - 1]                       # deleted: the rows' last entries
+            w = rng.integers(0, n, 2000)
+            x = (w + 1 + rng.integers(0, n - 1, 2000)) % n        # added: anywhere,
+            hubs = np.repeat(a[:20], 25)                          # and 25 to each of 20 rows
+            y = (hubs + 1 + rng.integers(0, n - 1, hubs.size)) % n
+            u = np.concatenate([a, w, hubs]).astype(np.int32)
+            v = np.concatenate([last, x, y]).astype(np.int32)
+            ins = np.concatenate([np.zeros(a.size), np.ones(w.size + hubs.size)]).astype(np.uint8)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            assert np.array_equal(g.get_mis(), orc.get_mis()), k
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), k
