@@ -667,7 +667,7 @@ struct mf_ctx {
   mf::DBuf<int64_t> dense_light;      // per dense seed light volume (size bound)
   mf::DBuf<int32_t> pull_long;        // vertices with long rows for the warp pull pass
   mf::DBuf<int32_t> tails;            // last four entries of each base row (large graphs, made on first use)
-  mf::DBuf<uint32_t> ncbits;          // non-skipped candidate bits for the pull pass
+  mf::DBuf<uint2> pbits;              // the pull's bits: non-skipped candidates (.x), tagged vertices (.y)
   // exact 2-hop sizes by row passes: seed masks per vertex and their filter
   // bits, the huge rows' chunk ORs, neighbourhood volumes, chunk tasks, the
   // seed groups, huge-row slots, counters
@@ -788,7 +788,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->dense_idx); f(c->dense_hl); f(c->pair_d); f(c->pair_h); f(c->todo);
   f(c->un_idx); f(c->un_v); f(c->need); f(c->needv); f(c->live_i); f(c->live_v); f(c->nlist_need);
   f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->vals_b); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
-  f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->ncbits); f(c->n2stamp);
+  f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->pbits); f(c->n2stamp);
   f(c->n2bstamp); f(c->cidbits);
   f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
   f(c->xst); f(c->xleave); f(c->cta_vert); f(c->cta_ws);

@@ -1709,11 +1709,11 @@ __global__ void k_need_decide(GraphView g, const int32_t* need, const int32_t* n
 // skipped) also take phase 1 of the clustering write here: bval[s] = max tag
 // of those rows with s = their own vertex (the rest of phase 1 is
 // k_lb_push_seed).  A skipped row stays skipped whatever its id.  The
-// candidates that write set their bit for the pull (ncbits, null when the
-// candidates' ids are pushed; k_clear takes the bits back) and leave their id
-// where one load finds it (newcid).
+// candidates that write set their bit for the pull (pbits.x, pbits null when
+// the ids are pushed; k_clear takes the bits back) and leave their id
+// where one load finds it (newcid); pbits.y has the vertices with a tag.
 __global__ void k_new_ids(HopCounts hc, const int64_t* pos, int32_t* rowcid, const int32_t* seeds, int64_t ns,
-                          const int32_t* cands, uint32_t epoch, uint32_t* bval, uint32_t* ncbits, int32_t* newcid) {
+                          const int32_t* cands, uint32_t epoch, uint32_t* bval, uint2* pbits, int32_t* newcid) {
   pdl_wait();
   pdl_trigger();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1722,10 +1722,12 @@ __global__ void k_new_ids(HopCounts hc, const int64_t* pos, int32_t* rowcid, con
   if (rc == -1) rowcid[i] = (int32_t)pos[i];
   if (rc == kSkip) return;
   if (i < ns) {
-    atomicMax(bval + seeds[i], (epoch << kRowBits) | (uint32_t)i);
-  } else if (ncbits) {
+    const int32_t x = seeds[i];
+    atomicMax(bval + x, (epoch << kRowBits) | (uint32_t)i);
+    if (pbits) atomicOr(&pbits[x >> 5].y, 1u << (x & 31));
+  } else if (pbits) {
     const int32_t x = cands[i - ns];
-    atomicOr(ncbits + (x >> 5), 1u << (x & 31));
+    atomicOr(&pbits[x >> 5].x, 1u << (x & 31));
     newcid[x] = rc == -1 ? (int32_t)pos[i] : rc;
   }
 }
@@ -1748,12 +1750,22 @@ __device__ __forceinline__ void push_w(uint32_t* wval, int32_t y, uint32_t tag) 
 // Phase 1: bval[y] = max tag of the non-skipped seed rows with y in {s} u
 // row(s): the seeds themselves in k_new_ids, their rows here.
 
+// y's first tag of this epoch also sets its bit for the pull.
+__device__ __forceinline__ void push_b(uint32_t* bval, int32_t y, uint32_t have, uint32_t tag, uint2* pbits) {
+  if (have >= tag) return;
+  if (!pbits) {
+    atomicMax(bval + y, tag);
+  } else if ((atomicMax(bval + y, tag) >> kRowBits) != (tag >> kRowBits)) {
+    atomicOr(&pbits[y >> 5].y, 1u << (y & 31));
+  }
+}
+
 __global__ void k_lb_push_seed(GraphView g, const int32_t* seeds, const int64_t* offs, int64_t ns, uint32_t epoch,
-                               uint32_t* bval, unsigned long long* work) {
+                               uint32_t* bval, uint2* pbits, unsigned long long* work) {
   pdl_wait();
   pdl_trigger();
   const int64_t vis = lb_rows(g, seeds, offs, ns, [&](int64_t i, int32_t, int32_t y) {
-    push_w(bval, y, (epoch << kRowBits) | (uint32_t)i);
+    push_b(bval, y, bval[y], (epoch << kRowBits) | (uint32_t)i, pbits);
   });
   add_work(work, vis);
 }
@@ -1986,7 +1998,7 @@ __global__ void k_need_short(GraphView g, const int32_t* need, const int32_t* ne
 
 // k_lb_push_seed without the prefix.
 __global__ void k_push_seed_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* rowcid, uint32_t epoch,
-                                  uint32_t* bval, unsigned long long* work) {
+                                  uint32_t* bval, uint2* pbits, unsigned long long* work) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = group_id();
@@ -1994,21 +2006,21 @@ __global__ void k_push_seed_short(GraphView g, const int32_t* seeds, int64_t ns,
   if (i < ns && rowcid[i] != kSkip) {
     const uint32_t tag = (epoch << kRowBits) | (uint32_t)i;
     vis = short_each(g, short_row(g, seeds[i]), [&](int32_t y) { return bval[y]; },
-                     [&](int32_t y, uint32_t have) { push_over(bval, y, have, tag); });
+                     [&](int32_t y, uint32_t have) { push_b(bval, y, have, tag, pbits); });
   }
   add_work_if(work, vis);
 }
 
-// k_lb_push_hop and (with_cands) k_lb_push_cand without the prefix: all
-// of them only raise wval, so their order does not matter.
+// k_lb_push_hop and k_lb_push_cand without the prefix: all of them only raise
+// wval, so their order does not matter.
 __global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, const int32_t* hlist,
-                                 const int32_t* cands, HopCounts hc, bool with_cands, const int32_t* v2i,
+                                 const int32_t* cands, HopCounts hc, const int32_t* v2i,
                                  const int32_t* rowcid, uint32_t epoch, const uint32_t* bval, uint32_t* wval, unsigned long long* work_hop,
                                  unsigned long long* work_cand) {
   pdl_wait();
   pdl_trigger();
   const int64_t i = group_id();
-  const int64_t nh = hc.hop1(), nct = with_cands ? hc.cands() : 0;
+  const int64_t nh = hc.hop1(), nct = hc.cands();
   int64_t vis = 0;
   bool cand = false;
   if (i < ns + nh) {
@@ -2038,24 +2050,27 @@ __global__ void k_push_hop_short(GraphView g, const int32_t* seeds, int64_t ns, 
   add_work_if(work_cand, cand ? vis : 0);
 }
 
-// Pull form of the candidate writes (symmetric graphs with sorted base rows).
+// Pull form of the clustering write (symmetric graphs with sorted base rows).
 // The candidate rows that write are the non-skipped ones, and their tags
 // grow with the candidate's vertex id (candidates are packed in ascending
 // id), so the last writer of y among them is its largest-id non-skipped
 // candidate neighbour: the added part of row(y) is scanned, then the base
 // part from its end until the first such neighbour.  That tag dominates every
-// seed-row tag; without one, the pushed seed-row tag (wval) decides.
+// seed-row tag.  Without one the whole row has been walked, and the seed rows'
+// last writer is the largest of the tags (bval) of y and of row(y), taken on
+// the way: y is in {h} u row(h) exactly then.  (Pushing those tags from the
+// rows of the tagged vertices instead took, with its prefix, 96 us of a
+// sub-batch on R-MAT scale 22: their rows are the hubs', most of whose
+// elements have a writing candidate anyway.)
 // One thread per vertex; rows longer than a.pull_long positions (a tuning
 // setting, 2048 by default) go to a list that k_pull_cand_long finishes with
 // one warp per row.
 
 struct PullArgs {
   GraphView g;
-  const int32_t* v2i;
   const int32_t* rowcid;
-  const uint32_t* ncbits;         // bit c set <=> c is a non-skipped candidate
-  int64_t ns;
-  const uint32_t* wval;
+  const uint2* pbits;             // bit c of .x: c is a non-skipped candidate; of .y: c has a tag (bval)
+  const uint32_t* bval;
   uint32_t epoch;
   int32_t* cid;
   int32_t* longv;                 // rows left for the warp pass
@@ -2066,8 +2081,10 @@ struct PullArgs {
   const int32_t* newcid;          // cluster id of each non-skipped candidate
 };
 
-__device__ __forceinline__ bool pull_nonskip(const PullArgs& a, int32_t c) {
-  return (__ldg(a.ncbits + (c >> 5)) >> (c & 31)) & 1u;
+// Bit 0: c is a non-skipped candidate; bit 1: c has a tag.
+__device__ __forceinline__ uint32_t pull_bits(const PullArgs& a, int32_t c) {
+  const uint2 w = __ldg(a.pbits + (c >> 5));
+  return ((w.x >> (c & 31)) & 1u) | (((w.y >> (c & 31)) & 1u) << 1);
 }
 
 // The last four entries of every base row.  The pull is bound by random
@@ -2095,42 +2112,67 @@ __device__ __forceinline__ void add_work_block(unsigned long long* work, int64_t
   if (threadIdx.x == 0 && s_visited) atomicAdd(work, (unsigned long long)s_visited);
 }
 
-__device__ __forceinline__ void pull_finish(const PullArgs& a, int32_t y, int32_t best) {
+__device__ __forceinline__ void pull_finish(const PullArgs& a, int32_t y, int32_t best, uint32_t tag) {
   if (best >= 0) {
     a.cid[y] = a.newcid[best];
   } else {
-    const uint32_t t = a.wval[y];
-    if ((t >> kRowBits) == a.epoch) a.cid[y] = a.rowcid[t & kRowMask];
+    tag = max(tag, a.bval[y]);
+    if ((tag >> kRowBits) == a.epoch) a.cid[y] = a.rowcid[tag & kRowMask];
   }
 }
 
+// The added part of row(y): the largest non-skipped candidate, and the largest tag.
+__device__ __forceinline__ int32_t pull_added(const PullArgs& a, int64_t ab, int64_t ae, uint32_t* tag) {
+  int32_t best = -1;
+  for (int64_t k = ab; k < ae; ++k) {
+    const int32_t c = a.g.aadj[k];
+    const uint32_t m = pull_bits(a, c);
+    if ((m & 1u) && c > best) best = c;
+    if (m & 2u) *tag = max(*tag, a.bval[c]);
+  }
+  return best;
+}
+
 // The row of y by its bounds: the added part, then the base part from its end
-// (less `skip` entries known to be no candidates).
-__device__ __forceinline__ int64_t pull_walk(const PullArgs& a, int32_t y, int64_t ab, int64_t ae, bool filt, int skip) {
+// (less `skip` entries known to be no candidates, whose tags are in `tag`),
+// four entries a step.
+__device__ __forceinline__ int64_t pull_walk(const PullArgs& a, int32_t y, int64_t ab, int64_t ae, bool filt, int skip,
+                                             uint32_t tag) {
   const GraphView& g = a.g;
   const int64_t b = g.nindex[y], e = g.nindex[y + 1];
   if ((e - b) + (ae - ab) > a.pull_long) {
     a.longv[atomicAdd(a.nlong, 1ull)] = y;
     return 0;
   }
-  int64_t visited = 0;
-  int32_t best = -1;
-  for (int64_t k = ab; k < ae; ++k) {
-    const int32_t c = g.aadj[k];
-    ++visited;
-    if (c > best && pull_nonskip(a, c)) best = c;
-  }
-  for (int64_t k = e - 1 - skip; k >= b; --k) {
-    const int32_t c = __ldg(g.nlist + k);
-    ++visited;
-    if (c <= best) break;
-    if (filt && !live_at(g.live, k)) continue;
-    if (pull_nonskip(a, c)) {
-      best = c;
+  int64_t visited = ae - ab;
+  int32_t best = pull_added(a, ab, ae, &tag);
+  for (int64_t k = e - 1 - skip; k >= b; k -= 4) {
+    int32_t c[4];
+    uint32_t m[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c[q] = k - q >= b ? __ldg(g.nlist + k - q) : -1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      m[q] = c[q] > best ? pull_bits(a, c[q]) : 0u;
+      if (filt && m[q] && !live_at(g.live, k - q)) m[q] = 0u;
+    }
+    int32_t hit = -1;
+#pragma unroll
+    for (int q = 3; q >= 0; --q)
+      if (m[q] & 1u) hit = c[q];
+    visited += min((int64_t)4, k - b + 1);
+    if (hit >= 0) {
+      best = hit;
       break;
     }
+    if (c[3] <= best) {   // the rest is at or below the best one, or the row ends
+      if (best >= 0) break;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (best < 0 && (m[q] & 2u)) tag = max(tag, a.bval[c[q]]);
   }
-  pull_finish(a, y, best);
+  pull_finish(a, y, best, tag);
   return visited;
 }
 
@@ -2141,7 +2183,7 @@ __global__ void k_pull_cand(PullArgs a) {
   int64_t visited = 0;
   if (yi < a.g.n) {
     const int32_t y = (int32_t)yi;
-    visited = pull_walk(a, y, a.g.aoff[y], a.g.aoff[y + 1], a.g.dead[y] != 0, 0);
+    visited = pull_walk(a, y, a.g.aoff[y], a.g.aoff[y + 1], a.g.dead[y] != 0, 0, 0u);
   }
   add_work_block(a.work, visited);
 }
@@ -2174,51 +2216,58 @@ __global__ void __launch_bounds__(kTB) k_pull_tails(PullArgs a) {
     t[q] = in[q] ? a.tail[y] : make_int4(-1, -1, -1, -1);
     filt[q] = in[q] && g.dead[y] != 0;
   }
-  bool hit1[kPullPer], hit2[kPullPer];
+  uint32_t m1[kPullPer], m2[kPullPer];
 #pragma unroll
   for (int q = 0; q < kPullPer; ++q) {
-    hit1[q] = t[q].w >= 0 && pull_nonskip(a, t[q].w);
-    hit2[q] = t[q].z >= 0 && pull_nonskip(a, t[q].z);
+    m1[q] = t[q].w >= 0 ? pull_bits(a, t[q].w) : 0u;
+    m2[q] = t[q].z >= 0 ? pull_bits(a, t[q].z) : 0u;
   }
 #pragma unroll
   for (int q = 0; q < kPullPer; ++q) {
     if (!in[q]) continue;
     const int32_t y = (int32_t)(y0 + (int64_t)q * blockDim.x);
     if (filt[q] || ae[q] - ab[q] > kPullAdded) {
-      visited += pull_walk(a, y, ab[q], ae[q], filt[q], 0);
+      visited += pull_walk(a, y, ab[q], ae[q], filt[q], 0, 0u);
       continue;
     }
-    int32_t best = -1;
-    for (int64_t k = ab[q]; k < ae[q]; ++k) {
-      const int32_t c = g.aadj[k];
-      ++visited;
-      if (c > best && pull_nonskip(a, c)) best = c;
-    }
+    uint32_t tag = 0;
+    int32_t best = pull_added(a, ab[q], ae[q], &tag);
+    visited += ae[q] - ab[q];
     // the base part is sorted: an entry at or below the best one ends it
     bool open = false;
     if (t[q].w > best) {
       ++visited;
-      if (hit1[q]) {
+      if (m1[q] & 1u) {
         best = t[q].w;
       } else if (t[q].z > best) {
         ++visited;
-        if (hit2[q]) {
+        if (m2[q] & 1u) {
           best = t[q].z;
         } else if (t[q].y > best) {
-          const bool h3 = pull_nonskip(a, t[q].y);
-          const bool h4 = t[q].x >= 0 && pull_nonskip(a, t[q].x);
+          const uint32_t m3 = pull_bits(a, t[q].y);
+          const uint32_t m4 = t[q].x >= 0 ? pull_bits(a, t[q].x) : 0u;
           ++visited;
-          if (h3) {
+          if (m3 & 1u) {
             best = t[q].y;
-          } else if (t[q].x > best) {
-            ++visited;
-            if (h4) best = t[q].x; else open = true;
+          } else {
+            if (t[q].x > best) {
+              ++visited;
+              if (m4 & 1u) best = t[q].x; else open = true;
+            }
+            if (best < 0) {
+              if (m3 & 2u) tag = max(tag, a.bval[t[q].y]);
+              if (m4 & 2u) tag = max(tag, a.bval[t[q].x]);
+            }
           }
         }
       }
+      if (best < 0) {
+        if (m1[q] & 2u) tag = max(tag, a.bval[t[q].w]);
+        if (m2[q] & 2u) tag = max(tag, a.bval[t[q].z]);
+      }
     }
-    if (open) visited += pull_walk(a, y, ab[q], ae[q], false, 4);
-    else pull_finish(a, y, best);
+    if (open) visited += pull_walk(a, y, ab[q], ae[q], false, 4, tag);
+    else pull_finish(a, y, best, tag);
   }
   add_work_block(a.work, visited);
 }
@@ -2241,10 +2290,13 @@ __global__ void k_pull_cand_long(PullArgs a) {
     const int64_t b = g.nindex[y], e = g.nindex[y + 1];
     const int64_t ab = g.aoff[y], ae = g.aoff[y + 1];
     int32_t best = -1;
+    uint32_t tag = 0;
     for (int64_t k = ab + lane; k < ae; k += 32) {
       const int32_t c = g.aadj[k];
       ++visited;
-      if (c > best && pull_nonskip(a, c)) best = c;
+      const uint32_t m = pull_bits(a, c);
+      if ((m & 1u) && c > best) best = c;
+      if (m & 2u) tag = max(tag, a.bval[c]);
     }
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
     const bool filt = g.dead[y] != 0;
@@ -2256,7 +2308,9 @@ __global__ void k_pull_cand_long(PullArgs a) {
         c = __ldg(g.nlist + k);
         ++visited;
         above = c > best;
-        hit = above && (!filt || live_at(g.live, k)) && pull_nonskip(a, c);
+        const uint32_t m = above && (!filt || live_at(g.live, k)) ? pull_bits(a, c) : 0u;
+        hit = m & 1u;
+        if (best < 0 && (m & 2u)) tag = max(tag, a.bval[c]);
       }
       const unsigned hm = __ballot_sync(0xffffffffu, hit);
       if (hm) {
@@ -2265,7 +2319,8 @@ __global__ void k_pull_cand_long(PullArgs a) {
       }
       if (__ballot_sync(0xffffffffu, above) != 0xffffffffu) break;  // the rest is <= best
     }
-    if (lane == 0) pull_finish(a, y, best);
+    for (int o = 16; o > 0; o >>= 1) tag = max(tag, __shfl_xor_sync(0xffffffffu, tag, o));
+    if (lane == 0) pull_finish(a, y, best, tag);
   }
   add_work(a.work, visited);
 }
@@ -3723,7 +3778,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_spec_round_large(SpecArgs sa,
 // repair overlaps the next sub-batch, the ids are cleared at once (and the
 // counts kept for the other call), the row map behind the repair.
 __global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, HopCounts hc, int32_t* cid,
-                        int32_t* v2i, uint32_t* ncbits, const int64_t* done, int64_t* keep) {
+                        int32_t* v2i, uint2* pbits, const int64_t* done, int64_t* keep) {
   pdl_wait();
   pdl_trigger();
   if (done && *done != 1) return;
@@ -3733,7 +3788,7 @@ __global__ void k_clear(const int32_t* seeds, int64_t ns, const int32_t* cands, 
   const int32_t x = i < ns ? seeds[i] : cands[i - ns];
   if (cid) cid[x] = -1;
   if (v2i) v2i[x] = -1;
-  if (ncbits && i >= ns) ncbits[x >> 5] = 0;
+  if (pbits) pbits[x >> 5] = make_uint2(0u, 0u);
 }
 
 template <typename T>
@@ -4295,7 +4350,7 @@ struct Repair {
   int64_t rows = 0;                // upper bound of the rows
   int32_t* v2i = nullptr;
   int32_t* cid = nullptr;          // null: cleared already
-  uint32_t* ncbits = nullptr;
+  uint2* pbits = nullptr;
   bool last = false;               // the batch ends with it: ev1 behind the clear
   int64_t queued = 0;
   bool in_flight = false;
@@ -4304,7 +4359,7 @@ struct Repair {
 
   void queue_clear(const int64_t* done) {
     StageScope csc(c, kStClear);
-    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, seeds, ns, cands, hc, cid, v2i, ncbits, done,
+    MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, seeds, ns, cands, hc, cid, v2i, pbits, done,
                     static_cast<int64_t*>(nullptr)));
     if (last) MF_CUDA(cudaEventRecord(c->ev1, s));
   }
@@ -4921,43 +4976,32 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     }
     if (use_pull) {
       const int64_t nwords = std::max<int64_t>(((int64_t)n + 31) / 32, 1);
-      const bool grown = c->ncbits.cap < nwords;
-      c->ncbits.reserve(nwords);
+      const bool grown = c->pbits.cap < nwords;
+      c->pbits.reserve(nwords);
       if (grown || (dirty && c->pull_runs == 0))
-        MF_CUDA(cudaMemsetAsync(c->ncbits.p, 0, sizeof(uint32_t) * (size_t)c->ncbits.cap, s));
+        MF_CUDA(cudaMemsetAsync(c->pbits.p, 0, sizeof(uint2) * (size_t)c->pbits.cap, s));
     }
-    uint32_t* ncbits = use_pull ? c->ncbits.p : nullptr;
+    uint2* pbits = use_pull ? c->pbits.p : nullptr;
     scan_exclusive_with(CreatesUpTo{c->creates.p, ns, hc}, c->i64b.p, rows, c->ws, s);
     MF_K(launch_pdl(k_new_ids, grid_for(rows), kTB, 0, s, hc, c->i64b.p, c->rowcid.p, seeds, ns, c->cands.p, ep,
-                    c->bval.p, ncbits, c->f1.p));
+                    c->bval.p, pbits, c->f1.p));
     sc.emplace(c, kStPush);
     unsigned long long* wk_extra = c->work.p + 2 * kStCount;   // [0] seed, [1] hop, [2] candidate pushes
+    // the elements of the short kernels are counted for the profiler only
+    unsigned long long* wk = c->profile ? wk_extra : nullptr;
     if (short_rows) {
-      // the elements are counted for the profiler only
-      unsigned long long* wk = c->profile ? wk_extra : nullptr;
       MF_K(launch_pdl(k_push_seed_short, grid_for(ns * kGroup), kTB, 0, s, g, seeds, ns, c->rowcid.p, ep, c->bval.p,
-                      wk));
-      sc.emplace(c, kStPushHop);
-      const int64_t npc = use_pull ? 0 : nct;
-      MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + npc) * kGroup), kTB, 0, s, g, seeds, ns, c->hlist.p,
-                      c->cands.p, hc, !use_pull, v2i, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
-                      wk ? wk + 3 : nullptr));
+                      pbits, wk));
     } else {
       row_offsets(c, seeds, ns, kCntSeedRows, ns, ep, v2i);
-      MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p, wk_extra + 0));
-      row_offsets(c, seeds, ns + nh, kCntPushers, ns, ep, v2i);
-      const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
-      sc.emplace(c, kStPushHop);
-      MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, TwoLists{seeds, c->hlist.p, ns}, c->lb_offs.p,
-                      ns + nh, ep, c->bval.p, c->wval.p, wk_extra + 1));
-      sc.emplace(c, kStPush);
-      if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
+      MF_K(launch_pdl(k_lb_push_seed, lb_grid(c, k_lb_push_seed), kTB, 0, s, g, seeds, c->lb_offs.p, ns, ep, c->bval.p,
+                      pbits, wk_extra + 0));
     }
     sc.emplace(c, use_pull ? kStPull : kStPush);
     if (use_pull) {
       ++c->pull_runs;
       c->pull_long.reserve(std::max<int32_t>(n, 1));
-      const PullArgs pa{g,  v2i, c->rowcid.p, c->ncbits.p, ns, c->wval.p, ep, c->cid.p, c->pull_long.p,
+      const PullArgs pa{g, c->rowcid.p, c->pbits.p, c->bval.p, ep, c->cid.p, c->pull_long.p,
                         ucnt + 36, wk_extra + 2, c->tune.pull_long, reinterpret_cast<const int4*>(c->tails.p), c->f1.p};
       if (tails) MF_K(launch_pdl(k_pull_tails, grid_for(n, kTB * kPullPer), kTB, 0, s, pa));
       else MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
@@ -4967,7 +5011,20 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       // tag and id (4 B each); the row entries read are counted on the device
       if (c->profile) c->stage_bytes[kStPull] += 28.0 * (double)n;
     } else {
-      if (!short_rows) {
+      if (short_rows) {
+        sc.emplace(c, kStPushHop);
+        MF_K(launch_pdl(k_push_hop_short, grid_for((ns + nh + nct) * kGroup), kTB, 0, s, g, seeds, ns, c->hlist.p,
+                        c->cands.p, hc, v2i, c->rowcid.p, ep, c->bval.p, c->wval.p, wk ? wk + 1 : nullptr,
+                        wk ? wk + 3 : nullptr));
+        sc.emplace(c, kStPush);
+      } else {
+        row_offsets(c, seeds, ns + nh, kCntPushers, ns, ep, v2i);
+        const unsigned long long dbg1 = debug_launches() ? debug_counter(c, wk_extra + 1) : 0;
+        sc.emplace(c, kStPushHop);
+        MF_K(launch_pdl(k_lb_push_hop, lb_grid(c, k_lb_push_hop), kTB, 0, s, g, TwoLists{seeds, c->hlist.p, ns},
+                        c->lb_offs.p, ns + nh, ep, c->bval.p, c->wval.p, wk_extra + 1));
+        sc.emplace(c, kStPush);
+        if (debug_launches()) debug_push_hop(c, wk_extra + 1, dbg1);
         row_offsets(c, c->cands.p, nct, kCntCandRows, ns, ep, v2i);
         MF_K(launch_pdl(k_lb_push_cand, lb_grid(c, k_lb_push_cand), kTB, 0, s, g, c->cands.p, c->lb_offs.p, nct, ns, ep,
                         c->wval.p, wk_extra + 3));
@@ -5052,7 +5109,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       // the ids are free for the next sub-batch; the row map once the repair is done
       int64_t* keep = c->counters.p + 70 + (odd ? 1 : 0);
       MF_K(launch_pdl(k_clear, grid_for(rows), kTB, 0, s, seeds, ns, c->cands.p, hc, c->cid.p,
-                      static_cast<int32_t*>(nullptr), ncbits, static_cast<const int64_t*>(nullptr), keep));
+                      static_cast<int32_t*>(nullptr), pbits, static_cast<const int64_t*>(nullptr), keep));
       next.hc = HopCounts{keep, capc};
       next.s = c->stream_r;
       if (job.in_flight) job.finish();
@@ -5064,7 +5121,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     } else {
       next.s = s;
       next.cid = c->cid.p;
-      next.ncbits = ncbits;
+      next.pbits = pbits;
       if (next.how == Assigned::kCounted) repair_reserve(c, std::max<int64_t>(next.nproc, 1));
       job = next;
       job.start();
