@@ -1461,21 +1461,32 @@ __device__ __forceinline__ int64_t cq_slot(const ChunkQueue& q, int64_t rows, in
   return lo;
 }
 
-// Warp-cooperative: first position k in [k0, k1) of row(x) (nb base
-// positions, then the added entries) whose element is live and satisfies
-// pred, or -1.  Steps of one, two, then four 32-position windows: the
-// windows of a step are loaded before any is tested, so each lane has up to
-// four element loads (then four predicate loads) in flight; the answer is
-// the lowest hit of the first window that has one.
+// The bounds of a row: nb base positions, np with the added entries.
+struct RowRef {
+  int64_t b0, a0, nb, np;
+  bool filt;
+};
+
+__device__ __forceinline__ RowRef row_ref(const GraphView& g, int32_t x) {
+  RowRef r;
+  r.b0 = g.nindex[x];
+  r.a0 = g.aoff[x];
+  r.nb = g.nindex[x + 1] - r.b0;
+  r.np = r.nb + (g.aoff[x + 1] - r.a0);
+  r.filt = g.dead[x] != 0;
+  return r;
+}
+
+// Warp-cooperative: first position k in [k0, k1) of the row whose element is
+// live and satisfies pred, or -1.  Steps of four 32-position windows: they
+// are loaded before any is tested, so each lane has up to four element loads
+// (then four predicate loads) in flight; the answer is the lowest hit of the
+// first window that has one.
 template <class P>
-__device__ __forceinline__ int64_t warp_first_range(const GraphView& g, int32_t x, int64_t nb, int64_t k0, int64_t k1,
+__device__ __forceinline__ int64_t warp_first_range(const GraphView& g, const RowRef& r, int64_t k0, int64_t k1,
                                                     P pred) {
   const int lane = threadIdx.x & 31;
-  const int64_t b0 = g.nindex[x];
-  const int64_t a0 = g.aoff[x];
-  const bool filt = g.dead[x] != 0;
-  int nwin = 1;   // windows per step: 1, 2, then 4 (a hit is often early)
-  for (int64_t base = k0; base < k1; base += 32 * nwin, nwin = nwin < 4 ? 2 * nwin : 4) {
+  for (int64_t base = k0; base < k1; base += 128) {
     int32_t y[4];
     bool live[4];
 #pragma unroll
@@ -1483,12 +1494,12 @@ __device__ __forceinline__ int64_t warp_first_range(const GraphView& g, int32_t 
       const int64_t k = base + 32 * q + lane;
       y[q] = -1;
       live[q] = false;
-      if (q < nwin && k < k1) {
-        if (k < nb) {
-          y[q] = __ldg(g.nlist + b0 + k);
-          live[q] = !filt || live_at(g.live, b0 + k);
+      if (k < k1) {
+        if (k < r.nb) {
+          y[q] = __ldg(g.nlist + r.b0 + k);
+          live[q] = !r.filt || live_at(g.live, r.b0 + k);
         } else {
-          y[q] = g.aadj[a0 + (k - nb)];
+          y[q] = g.aadj[r.a0 + (k - r.nb)];
           live[q] = true;
         }
       }
@@ -1568,19 +1579,28 @@ __global__ void k_first_warp(GraphView g, P pred, unsigned long long* firstpos, 
   const int lane = threadIdx.x & 31;
   const int64_t nmid = (int64_t)*q.mid_count;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t w = warp_id(); w < nmid; w += nw) {
+  // While a row is scanned, the next one's bounds and the one after's vertex
+  // are on their way.
+  int64_t w = warp_id();
+  if (w >= nmid) return;
+  int32_t x = q.mid_v[w];
+  int32_t xn = w + nw < nmid ? q.mid_v[w + nw] : x;
+  RowRef r = row_ref(g, x);
+  for (; w < nmid; w += nw) {
     const int32_t i = kProbed ? q.mid_idx[w] : (int32_t)w;
-    const int32_t x = q.mid_v[w];
-    const int64_t nb = g.nindex[x + 1] - g.nindex[x];
-    const int64_t np = nb + (g.aoff[x + 1] - g.aoff[x]);
-    const int64_t lim = np < q.bound ? np : q.bound;
-    const int64_t hit = warp_first_range(g, x, nb, kProbed ? kProbe : 0, lim, pred);
+    const RowRef rn = row_ref(g, xn);
+    const int32_t xnn = w + 2 * nw < nmid ? q.mid_v[w + 2 * nw] : xn;
+    const int64_t lim = r.np < q.bound ? r.np : q.bound;
+    const int64_t hit = warp_first_range(g, r, kProbed ? kProbe : 0, lim, pred);
     if (hit >= 0 || !kProbed) {
       if (lane == 0) firstpos[i] = hit >= 0 ? (unsigned long long)hit : kNoPos;
     }
-    if (hit < 0 && np > q.bound && lane == 0) {
-      cq_push(q.rest, i, x, (np - q.bound + kFirstChunk - 1) / kFirstChunk);
+    if (hit < 0 && r.np > q.bound && lane == 0) {
+      cq_push(q.rest, i, x, (r.np - q.bound + kFirstChunk - 1) / kFirstChunk);
     }
+    x = xn;
+    xn = xnn;
+    r = rn;
   }
 }
 
@@ -1603,10 +1623,9 @@ __global__ void k_first_chunks(GraphView g, P pred, unsigned long long* firstpos
     if (lane == 0) fp = *(volatile const unsigned long long*)(firstpos + i);
     fp = __shfl_sync(0xffffffffu, fp, 0);
     if (fp <= (unsigned long long)p0) continue;
-    const int64_t nb = g.nindex[x + 1] - g.nindex[x];
-    const int64_t np = nb + (g.aoff[x + 1] - g.aoff[x]);
-    const int64_t end = min(p0 + kFirstChunk, np);
-    const int64_t hit = warp_first_range(g, x, nb, p0, end, pred);
+    const RowRef r = row_ref(g, x);
+    const int64_t end = min(p0 + kFirstChunk, r.np);
+    const int64_t hit = warp_first_range(g, r, p0, end, pred);
     if (hit >= 0 && lane == 0) atomicMin(firstpos + i, (unsigned long long)hit);
   }
 }
