@@ -275,8 +275,8 @@ void mf_free(void* p);
 const char* mf_stage_name(int stage);
 /* on = 1: every later batch records CUDA events around each stage on the
  * context's stream; times accumulate until mf_profile_reset.  on = 2: only
- * the k_lb_push_hop launches (the "push_hop" stage) and the candidates'
- * pull (the "pull" stage: k_cand_bits, k_pull_cand, k_pull_cand_long) are
+ * the hop push (the "push_hop" stage, in the sub-batches that push) and the
+ * pull (the "pull" stage: k_pull_tails or k_pull_cand, k_pull_cand_long) are
  * timed, six event records per sub-batch instead of about fifty.  on = 0: off.
  * Adding 4 (on = 4, 5, 6) also counts each batch's algorithmic work
  * (mf_batch_stats.packed_total / row_degree_total): every sub-batch then
@@ -378,13 +378,14 @@ int mf_pool_set_budget(mf_pool* pool, int64_t hbm_budget);
  * repair, clear -- with no host round trip.  The step (batch upload, queue
  * reset, the kernel, the read-back of the per-graph results) is captured
  * and launched as one CUDA graph.  Larger batches, graphs above the vertex
- * limit and contexts in exact-MIS mode take the multi-launch path
+ * limit, contexts in exact-MIS mode and batches that would keep one CTA busy
+ * for longer than all of these take together go through the multi-launch path
  * (mf_apply_batch, from up to 8 host threads, each graph on its own stream)
  * while the persistent kernel runs. */
 typedef struct mf_batched_opts {
   int block;                  /* threads per persistent CTA: 64..1024, a multiple of 32 (default 512) */
   int ctas_per_sm;            /* persistent CTAs per SM (default 2) */
-  int64_t max_cta_updates;    /* batches of at most this many lines take the kernel (default 8192) */
+  int64_t max_cta_updates;    /* batches of at most this many lines may take the kernel (default 8192) */
   int32_t max_cta_vertices;   /* ... on graphs of at most this many vertices (default 2^20) */
   int use_graph;              /* 1: capture the step as a CUDA graph (default), 0: plain launches */
   int path_threads;           /* host threads driving the batches above the kernel's limits, each

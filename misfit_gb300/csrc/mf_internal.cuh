@@ -134,9 +134,9 @@ enum Stage : int {
   kStClear,         // clear of mapped vertices
   kStExact,         // exact 2-hop sizes (heavy bitmaps) and limit growth
   kStRepairBig,     // MIS repair: grid-wide hop-2 searches
-  kStPushHop,       // the k_lb_push_hop launches alone (part of the clustering write)
+  kStPushHop,       // the hop push of the sub-batches that push (part of the clustering write)
   kStFirstNeed,     // clustering read, seeds without an id in their own row (the hop-2 part)
-  kStPull,          // clustering write, the candidate rows' ids (pull or push + finalize)
+  kStPull,          // clustering write, the pull of the sub-batches that pull
   kStCount
 };
 extern const char* const kStageNames[kStCount];
