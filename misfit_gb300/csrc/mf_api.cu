@@ -166,11 +166,10 @@ void release_all(mf_ctx* c) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->stream_b) {
-    cudaStreamSynchronize(c->stream_b);
-    cudaStreamDestroy(c->stream_b);
+    mf::return_stream(c->device, c->stream_b);
   }
   c->stream_b = nullptr;
-  if (c->stream_r) cudaStreamDestroy(c->stream_r);
+  if (c->stream_r) mf::return_stream(c->device, c->stream_r);
   c->stream_r = nullptr;
   if (c->ev_s) cudaEventDestroy(c->ev_s);
   if (c->ev_r) cudaEventDestroy(c->ev_r);
@@ -207,7 +206,6 @@ mf_ctx* new_ctx(int gpu) {
     }
     MF_CUDA(cudaEventCreate(&c->ev0));
     MF_CUDA(cudaEventCreate(&c->ev1));
-    MF_CUDA(cudaStreamCreateWithFlags(&c->stream_b, cudaStreamNonBlocking));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_a, cudaEventDisableTiming));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_b, cudaEventDisableTiming));
     MF_CUDA(cudaEventCreateWithFlags(&c->ev_r, cudaEventDisableTiming));
@@ -256,6 +254,11 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   }
   if (!c->end_recorded) MF_CUDA(cudaEventRecord(c->ev1, s));
   MF_CUDA(cudaEventSynchronize(c->ev1));
+  for (cudaStream_t* t : {&c->stream_b, &c->stream_r})
+    if (*t) {
+      mf::return_stream(c->device, *t);
+      *t = nullptr;
+    }
   float ms = 0.f;
   MF_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->stats.device_ms = ms;

@@ -690,7 +690,7 @@ struct mf_ctx {
   uint32_t cta_epoch = 0;
   bool exact = false;                  // exact-MIS mode on
   mf::Front front[2];                 // current and next sub-batch fronts
-  cudaStream_t stream_b = nullptr;    // the fronts of later sub-batches run here
+  cudaStream_t stream_b = nullptr;    // the fronts of later sub-batches run here (lent for a batch, as stream_r)
   cudaEvent_t ev_a = nullptr, ev_b = nullptr;
   // repairs that overlap the next sub-batch (batches of more than one): their
   // stream, and the second set of seeds, row map and edge order
@@ -927,6 +927,9 @@ void exact_fixup(mf_ctx* c);                       // exact-MIS mode after a bat
 // mf_parse.cu: batch file -> c->bu / c->bv (valid lines, file order); returns the count
 int64_t parse_batch_file_device(mf_ctx* c, const char* path);
 // mf_repair.cu
+// Side streams of a device: borrowed for a batch, returned when it has ended.
+cudaStream_t borrow_stream(int device);
+void return_stream(int device, cudaStream_t t);
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m);
 int64_t initial_max_csr(int32_t n, uint64_t edges);
 }  // namespace mf

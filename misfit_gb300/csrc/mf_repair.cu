@@ -3862,6 +3862,10 @@ void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>
 // Buffers of both fronts at their largest sizes for a batch of m updates, so
 // that no front allocates while another stream may use its memory.  Bitmaps,
 // sums and counters start at zero, and every front leaves them so.
+// Candidates are distinct vertices, so a small graph needs few rows.  (10^6 for
+// every graph were tens of MB a context, whatever its size.)
+int64_t max_cands(const mf_ctx* c) { return std::min<int64_t>(kMaxRows, std::max<int32_t>(c->n, 1)); }
+
 void front_reserve(mf_ctx* c, int64_t m, bool clear) {
   cudaStream_t s = c->stream;
   const int64_t words = ((int64_t)c->n + 31) / 32;
@@ -3876,7 +3880,7 @@ void front_reserve(mf_ctx* c, int64_t m, bool clear) {
     zeroed(f.uacc, std::max<int64_t>(max_ns, 1));
     zeroed(f.cnt, 3);
     f.hlist.reserve(std::max<int32_t>(c->n, 1));
-    f.cands.reserve(kMaxRows);
+    f.cands.reserve(max_cands(c));
     f.lb_offs.reserve(2 * max_ns + 2);
   }
 }
@@ -4636,10 +4640,8 @@ namespace {
 // The second set of what a repair shares with its sub-batch's clustering, and
 // the repair's stream.
 void pipe_reserve(mf_ctx* c, int64_t m) {
-  if (!c->stream_r) {
-    MF_CUDA(cudaStreamCreateWithFlags(&c->stream_r, cudaStreamNonBlocking));
-    MF_CUDA(cudaEventCreateWithFlags(&c->ev_s, cudaEventDisableTiming));
-  }
+  if (!c->stream_r) c->stream_r = borrow_stream(c->device);
+  if (!c->ev_s) MF_CUDA(cudaEventCreateWithFlags(&c->ev_s, cudaEventDisableTiming));
   if (c->v2i_b.cap < c->n) {
     c->v2i_b.reserve(c->n);
     MF_CUDA(cudaMemsetAsync(c->v2i_b.p, 0xFF, sizeof(int32_t) * (size_t)c->v2i_b.cap, c->stream));
@@ -4649,6 +4651,36 @@ void pipe_reserve(mf_ctx* c, int64_t m) {
 }
 
 }  // namespace
+
+// The side streams of a batch are lent for its length.  A stream's first work
+// costs milliseconds when hundreds of contexts each bring their own: the first
+// batch of 256 open contexts took 7.7 ms each with two of them per context.
+// As many exist as were ever out at once; they are not destroyed, because
+// buffers keep the stream that they were allocated on.
+namespace {
+std::mutex g_side_mu;
+std::unordered_map<int, std::vector<cudaStream_t>> g_side_idle;
+}  // namespace
+
+cudaStream_t borrow_stream(int device) {
+  {
+    std::lock_guard<std::mutex> lock(g_side_mu);
+    auto& idle = g_side_idle[device];
+    if (!idle.empty()) {
+      const cudaStream_t t = idle.back();
+      idle.pop_back();
+      return t;
+    }
+  }
+  cudaStream_t t = nullptr;
+  MF_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+  return t;
+}
+
+void return_stream(int device, cudaStream_t t) {
+  std::lock_guard<std::mutex> lock(g_side_mu);
+  g_side_idle[device].push_back(t);
+}
 
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
@@ -4693,10 +4725,10 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   c->i64b.reserve(big);
   c->u8a.reserve(big);
   c->seeds.reserve(2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->cands.reserve(kMaxRows);
-  c->rowcid.reserve(kMaxRows + 2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->creates.reserve(kMaxRows + 2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->rowlens.reserve(kMaxRows + 2 * std::min<int64_t>(m, kMaxBatchEdges) + 1);
+  c->cands.reserve(max_cands(c));
+  c->rowcid.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges));
+  c->creates.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges));
+  c->rowlens.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges) + 1);
 
   // ---- sub-batch plan: cuts, estimates and seed lists of the whole batch
   // from p0 (re-planned from the next sub-batch when MAX_CSR_ELEMENTS grows)
@@ -4942,6 +4974,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       if (kidx_next >= cuts.size()) MF_FAIL(MF_ESTATE, "sub-batch plan ended before the batch");
       const int64_t ns_next = seed_end[kidx_next] - seed_base_next;
       if (overlap_fronts) {
+        if (!c->stream_b) c->stream_b = borrow_stream(c->device);
         MF_CUDA(cudaEventRecord(c->ev_a, s));
         MF_CUDA(cudaStreamWaitEvent(c->stream_b, c->ev_a, 0));
         g_alloc_stream = c->stream_b;   // any scratch the front's scans grow belongs to its stream
