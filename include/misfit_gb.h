@@ -153,7 +153,10 @@ int mf_flag_updates_noalloc(mf_ctx* ctx, const int32_t* u, const int32_t* v, int
  * Replaces processBatchGPUVertexClustering (src/misfit/misfit.cu:704-730)
  * with GPUVertexClusteringGraph::processBatchWithVertexClustering
  * (:468-692).  u, v: 0-based endpoints, u != v, both < n; ins: the flags.
- * Host arrays; returns when the batch is complete on the device. */
+ * Host arrays; returns when the batch is complete on the device.
+ * A batch that fails with MF_ENOMEM has changed nothing, or its links are all
+ * in the graph and part of it is not repaired; the context goes on from there
+ * (mf_greedy_mis and mf_set_mis give it a whole membership again). */
 int mf_apply_batch(mf_ctx* ctx, const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t m);
 
 /* Same with device-resident inputs (device pointers, m entries each). */

@@ -32,6 +32,7 @@ thread_local std::string g_error;
 std::atomic<long long> g_launches{0};
 std::atomic<long long> g_allocs{0};
 thread_local cudaStream_t g_alloc_stream = nullptr;
+thread_local long long* g_fail_alloc = nullptr;
 
 namespace {
 struct KTimes {
@@ -196,6 +197,7 @@ mf_ctx* new_ctx(int gpu) {
         c->exact_cap_pairs = pr > 0 ? std::max<long long>(4096, pr) : 0;
       }
     }
+    if (const char* e = std::getenv("MISFIT_GB_FAIL_ALLOC")) c->fail_alloc = std::max<long long>(0, std::atoll(e));
     MF_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
     mf::g_alloc_stream = c->stream;
     // keep freed stream-ordered memory in this process's pool for reuse
@@ -234,6 +236,14 @@ void bind(const mf_ctx* c) {
   mf::g_alloc_stream = c->stream;
 }
 
+void return_side_streams(mf_ctx* c) {
+  for (cudaStream_t* t : {&c->stream_b, &c->stream_r})
+    if (*t) {
+      mf::return_stream(c->device, *t);
+      *t = nullptr;
+    }
+}
+
 // One batch of m lines.  Invalid lines fail it before anything changes.
 void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
@@ -244,8 +254,19 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   MF_CUDA(cudaMemsetAsync(c->work.p, 0, sizeof(unsigned long long) * mf::kWorkWords, s));
   MF_CUDA(cudaEventRecord(c->ev0, s));
   if (m > 0) {
-    mf::process_batch(c, in, m);
-    if (c->exact) mf::exact_fixup(c);
+    struct FailAlloc {
+      explicit FailAlloc(long long* k) { mf::g_fail_alloc = k; }
+      ~FailAlloc() { mf::g_fail_alloc = nullptr; }
+    };
+    try {
+      FailAlloc fail(&c->fail_alloc);
+      mf::process_batch(c, in, m);
+      if (c->exact) mf::exact_fixup(c);
+    } catch (...) {
+      mf::abandon_batch(c);
+      return_side_streams(c);
+      throw;
+    }
   } else {
     c->stats = mf_batch_stats{};
     c->stats.packed_total = -1;
@@ -254,11 +275,7 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
   }
   if (!c->end_recorded) MF_CUDA(cudaEventRecord(c->ev1, s));
   MF_CUDA(cudaEventSynchronize(c->ev1));
-  for (cudaStream_t* t : {&c->stream_b, &c->stream_r})
-    if (*t) {
-      mf::return_stream(c->device, *t);
-      *t = nullptr;
-    }
+  return_side_streams(c);
   float ms = 0.f;
   MF_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
   c->stats.device_ms = ms;

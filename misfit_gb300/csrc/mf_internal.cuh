@@ -64,7 +64,13 @@ inline void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); 
 // Every device or pinned-host allocation of the library counts here
 // (mf_allocations), so that a caller can check that a call allocated nothing.
 extern std::atomic<long long> g_allocs;
-inline void note_alloc() { g_allocs.fetch_add(1, std::memory_order_relaxed); }
+// The allocation to refuse on this thread's batch (mf_ctx::fail_alloc), or null.
+extern thread_local long long* g_fail_alloc;
+inline void note_alloc() {
+  g_allocs.fetch_add(1, std::memory_order_relaxed);
+  if (g_fail_alloc != nullptr && *g_fail_alloc > 0 && --*g_fail_alloc == 0)
+    MF_FAIL(MF_ENOMEM, "allocation refused (MISFIT_GB_FAIL_ALLOC)");
+}
 // Per-kernel timing (MISFIT_GB_KTIME=1): the device is synchronised around
 // every launch and the host-timed milliseconds are summed per kernel name and
 // printed to stderr at exit.  Off by default; it slows everything down and is
@@ -535,6 +541,8 @@ struct SortedPairs {
 };
 SortedPairs radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
                              cudaStream_t s);
+// Room in the workspace for any of these sorts of up to n pairs.
+void reserve_sort(Scratch& ws, int64_t n, cudaStream_t s);
 // The same with the result always in keys/vals.
 void radix_sort_pairs_in_place(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
                                cudaStream_t s);
@@ -760,7 +768,10 @@ struct mf_ctx {
   mf::AsyncQueue* aq = nullptr;
   bool pending = false;
   bool end_recorded = false;   // ev1 stands behind the batch's last work
-  bool mid_batch = false;   // a batch began and has not ended: zeroed scratch may not be zero
+  bool mid_batch = false;   // a batch began and has not ended: its marks and maps may stand
+  // testing (MISFIT_GB_FAIL_ALLOC=k when the context is made): the k-th device
+  // allocation of its batches reports out of memory, once
+  long long fail_alloc = 0;
   // load-balancing settings (mf_set_tuning); they move work between kernels,
   // never a result
   mf_tuning tune = mf_tuning{2048, 2048, 64, 256, 0, 1};
@@ -908,6 +919,9 @@ constexpr int kWorkWords = kCntBad + 8;
 // seed end} records.
 constexpr int64_t kPlanHost = 160;
 constexpr int64_t kPlanWords = 8 + 3 * kPlanHost;
+// The buffers of the calls below, so that none of them allocates: between the
+// first and swap_overlay the graph is half changed and nothing may fail.
+void reserve_overlay(mf_ctx* c, int64_t m);
 // lines -> c->bu/bv/bins, endpoint slots by vertex, previous occurrences, and
 // the pairs' state changes (nothing changes when a line is invalid)
 void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m);
@@ -931,5 +945,7 @@ int64_t parse_batch_file_device(mf_ctx* c, const char* path);
 cudaStream_t borrow_stream(int device);
 void return_stream(int device, cudaStream_t t);
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m);
+// After a batch that threw: waits for what it queued, and takes back its marks.
+void abandon_batch(mf_ctx* c);
 int64_t initial_max_csr(int32_t n, uint64_t edges);
 }  // namespace mf

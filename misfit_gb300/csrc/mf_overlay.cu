@@ -837,6 +837,30 @@ void flag_updates(mf_ctx* c, int64_t m) {
   MF_CUDA(cudaGetLastError());
 }
 
+void reserve_overlay(mf_ctx* c, int64_t m) {
+  cudaStream_t s = c->stream;
+  const int64_t n = c->n, a = c->a_total, slots = 2 * m;
+  c->bu.reserve(m);
+  c->bv.reserve(m);
+  c->bins.reserve(m);
+  c->app_line.reserve(m);
+  c->keys.reserve(slots);
+  c->vals.reserve(slots);
+  c->slot_keys.reserve(slots);
+  c->slot_vals.reserve(slots);
+  c->prev.reserve(slots);
+  // grown with every mark cleared: the rebuild clears the ones it used
+  if (c->akill.grow(std::max<int64_t>(a, 1)))
+    MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
+  c->aadj_alt.grow(a + slots);
+  c->aown_alt.grow(a + slots);
+  c->aadj.reserve(std::max<int64_t>(a, 1));
+  c->aown.reserve(std::max<int64_t>(a, 1));
+  c->atail.grow(a + slots + 1);
+  reserve_sort(c->ws, slots, s);
+  scan_detail::reserve_scan(c->ws, n + a + slots, s);
+}
+
 void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
   const int nbits = bits_for(std::max<int32_t>(c->n - 1, 1));
@@ -844,18 +868,6 @@ void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m) {
   // needs: two 8-bit digits up to 2^13 lines and three up to 2^21, where the
   // pair itself has 2 * nbits bits (six digits at 2^22 vertices)
   const int gbits = std::min(64, (bits_for(m) + 3 + 7) / 8 * 8);
-  c->bu.reserve(m);
-  c->bv.reserve(m);
-  c->bins.reserve(m);
-  c->app_line.reserve(m);
-  c->keys.reserve(2 * m);
-  c->vals.reserve(2 * m);
-  c->slot_keys.reserve(2 * m);
-  c->slot_vals.reserve(2 * m);
-  c->prev.reserve(2 * m);
-  // grown with every mark cleared: the rebuild clears the ones it used
-  if (c->akill.grow(std::max<int64_t>(c->a_total, 1)))
-    MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
   SortedPairs pairs{c->keys.p, c->vals.p};
   if (m <= kSmallBatch) {
     const int slots = (int)(2 * m);
@@ -883,11 +895,6 @@ void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m) {
 void rebuild_added(mf_ctx* c, int64_t m) {
   cudaStream_t s = c->stream;
   const int64_t n = c->n, a = c->a_total, slots = 2 * m;
-  c->aadj_alt.grow(a + slots);
-  c->aown_alt.grow(a + slots);
-  c->aadj.reserve(std::max<int64_t>(a, 1));
-  c->aown.reserve(std::max<int64_t>(a, 1));
-  c->atail.grow(a + slots + 1);
   scan_exclusive_to(RebuildCounts{n, a, c->aoff.p, c->adelta.p, c->akill.p, c->slot_vals.p, c->app_line.p},
                     RebuildOut{n, c->aoff_alt.p, c->atail.p}, n + a + slots, c->ws, s);
   MF_K(launch_pdl(k_rebuild_added, grid_for(a + slots), kTB, 0, s, c->aoff.p, c->aadj.p, c->aown.p, a, c->aoff_alt.p,

@@ -184,6 +184,19 @@ __global__ void __launch_bounds__(kThreads) k_sort_pass(const uint64_t* keys, co
   }
 }
 
+void reserve_passes(Scratch& ws, int64_t n, cudaStream_t s) {
+  const int64_t tiles = (n + kTile - 1) / kTile;
+  ws.keys_alt.reserve(n);
+  ws.vals_alt.reserve(n);
+  ws.hist.reserve(kMaxPasses * kDigits);
+  if (ws.sort_status.cap < tiles * kDigits) {
+    ws.sort_status.reserve(tiles * kDigits);
+    // fresh memory may hold anything: no tag may match a later sequence number
+    MF_CUDA(cudaMemsetAsync(ws.sort_status.p, 0, sizeof(unsigned long long) * (size_t)ws.sort_status.cap, s));
+    ws.sort_seq = 0;
+  }
+}
+
 template <bool Mixed>
 SortedPairs sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,
                        cudaStream_t s) {
@@ -200,15 +213,7 @@ SortedPairs sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit,
   }
   const int64_t tiles = (n + kTile - 1) / kTile;
   const int passes = (end_bit - first_bit + 7) / 8;
-  ws.keys_alt.reserve(n);
-  ws.vals_alt.reserve(n);
-  ws.hist.reserve(kMaxPasses * kDigits);
-  if (ws.sort_status.cap < tiles * kDigits) {
-    ws.sort_status.reserve(tiles * kDigits);
-    // fresh memory may hold anything: no tag may match a later sequence number
-    MF_CUDA(cudaMemsetAsync(ws.sort_status.p, 0, sizeof(unsigned long long) * (size_t)ws.sort_status.cap, s));
-    ws.sort_seq = 0;
-  }
+  reserve_passes(ws, n, s);
   if (ws.sort_seq + kMaxPasses >= (1ull << 30)) {   // the tag's 30 bits are used up
     MF_CUDA(cudaMemsetAsync(ws.sort_status.p, 0, sizeof(unsigned long long) * (size_t)ws.sort_status.cap, s));
     ws.sort_seq = 0;
@@ -243,6 +248,10 @@ void scan_exclusive_i32(const int32_t* in, int64_t* out, int64_t n, Scratch& ws,
 }
 void scan_exclusive_u8(const uint8_t* in, int64_t* out, int64_t n, Scratch& ws, cudaStream_t s) {
   scan_exclusive(Loader<uint8_t>{in}, out, n, ws, s);
+}
+
+void reserve_sort(Scratch& ws, int64_t n, cudaStream_t s) {
+  if (n > kBlockSortMax) reserve_passes(ws, n, s);
 }
 
 SortedPairs radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit, int end_bit, Scratch& ws,

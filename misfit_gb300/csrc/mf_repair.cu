@@ -3866,14 +3866,14 @@ void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>
 // every graph were tens of MB a context, whatever its size.)
 int64_t max_cands(const mf_ctx* c) { return std::min<int64_t>(kMaxRows, std::max<int32_t>(c->n, 1)); }
 
-void front_reserve(mf_ctx* c, int64_t m, bool clear) {
+void front_reserve(mf_ctx* c, int64_t m) {
   cudaStream_t s = c->stream;
   const int64_t words = ((int64_t)c->n + 31) / 32;
   const int64_t max_ns = 2 * std::min<int64_t>(m, kMaxBatchEdges);
   auto zeroed = [&](auto& buf, int64_t count) {
     const bool grown = buf.cap < count;
     buf.reserve(count);
-    if (grown || clear) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
+    if (grown) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
   };
   for (auto& f : c->front) {
     zeroed(f.bits, std::max<int64_t>(2 * words, 1));
@@ -4683,6 +4683,88 @@ void return_stream(int device, cudaStream_t t) {
   g_side_idle[device].push_back(t);
 }
 
+namespace {
+
+// What a failed batch left where every batch expects none: the marks of the
+// overlay and of the fronts, the pull's bits, the row maps (with the ids of the
+// sub-batch in the current one, which its own clear would have taken), and the
+// repair's pending bits.  The ids that the clustering wrote elsewhere, the links
+// and the repairs that were committed stay.
+__global__ void k_leftovers(int32_t n, int32_t* v2i, int32_t* v2i_b, int32_t* cid, uint8_t* mis) {
+  const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= n) return;
+  if (v2i[x] >= 0) {
+    cid[x] = -1;
+    v2i[x] = -1;
+  }
+  if (v2i_b) v2i_b[x] = -1;
+  mis[x] &= 1;
+}
+
+void clear_leftovers(mf_ctx* c) {
+  cudaStream_t s = c->stream;
+  auto zero = [&](auto& buf) {
+    if (buf.cap > 0) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
+  };
+  zero(c->adelta);
+  zero(c->akill);
+  zero(c->pbits);
+  for (auto& f : c->front) {
+    zero(f.bits);
+    zero(f.uacc);
+    zero(f.cnt);
+  }
+  if (c->n > 0)
+    MF_K(k_leftovers<<<grid_for(c->n), kTB, 0, s>>>(c->n, c->v2i.p, c->v2i_b.cap > 0 ? c->v2i_b.p : nullptr, c->cid.p,
+                                                    c->mis.p));
+  MF_CUDA(cudaGetLastError());
+  MF_CUDA(cudaStreamSynchronize(s));
+  c->bitmap_ctas = 0;   // the exact sizes' bitmaps and slots are made anew
+  c->heavy_used = 0;
+  c->mid_batch = false;
+}
+
+// Buffers of the sub-batch plan and of one sub-batch's rows, at their largest.
+void reserve_plan(mf_ctx* c, int64_t m) {
+  const int64_t edges = std::min<int64_t>(m, kMaxBatchEdges), n1 = std::max<int32_t>(c->n, 1);
+  c->n2cache.reserve(n1);
+  c->n2stamp.reserve(n1);
+  c->n2bound.reserve(n1);
+  c->n2bstamp.reserve(n1);
+  c->i64a.reserve(2 * edges + c->n + 2);
+  c->i64b.reserve(2 * edges + c->n + 2);
+  c->u8a.reserve(2 * edges + c->n + 2);
+  c->seeds.reserve(2 * edges);
+  c->cands.reserve(max_cands(c));
+  c->rowcid.reserve(max_cands(c) + 2 * edges);
+  c->creates.reserve(max_cands(c) + 2 * edges);
+  c->rowlens.reserve(max_cands(c) + 2 * edges + 1);
+  c->plan_cuts.reserve(std::max<int64_t>(m, 1));
+  c->plan_ests.reserve(std::max<int64_t>(m, 1));
+  c->plan_send.reserve(std::max<int64_t>(m, 1));
+  c->plan_flags.reserve(2 * m);
+  c->plan_pos.reserve(2 * m + 1);
+  c->seeds_all.reserve(2 * m);
+  if (m > kSmallBatch) c->plan_edges.reserve(4 * m);
+}
+
+}  // namespace
+
+void abandon_batch(mf_ctx* c) {
+  // the lines in pinned memory, the buffers and the caller's arrays are free
+  // once nothing that was queued can still read them
+  for (cudaStream_t t : {c->stream, c->stream_b, c->stream_r})
+    if (t) cudaStreamSynchronize(t);
+  cudaGetLastError();   // a refused allocation is reported once
+  if (!c->mid_batch) return;
+  const std::string why = get_error();
+  try {
+    clear_leftovers(c);
+  } catch (...) {   // the device is lost; the next batch says so
+  }
+  set_error(why);
+}
+
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   cudaStream_t s = c->stream;
   const int32_t n = c->n;
@@ -4690,20 +4772,13 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(cnt);
   int64_t* h = c->h_counters;
 
-  // a batch that failed midway leaves scratch that must be zero between
-  // batches; the next one clears it whole
-  const bool dirty = c->mid_batch;
-  if (dirty) {
-    for (cudaStream_t t : {c->stream_b, c->stream_r})
-      if (t) MF_CUDA(cudaStreamSynchronize(t));
-    MF_CUDA(cudaMemsetAsync(c->adelta.p, 0, sizeof(int32_t) * (size_t)n, s));
-    if (c->akill.cap > 0) MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));
-  }
+  if (c->mid_batch) clear_leftovers(c);   // of a failed batch, where it could not do so itself
+  // every buffer that is needed before the batch's links are in the graph: up
+  // to here a batch that runs out of memory has changed nothing
+  reserve_overlay(c, m);
+  reserve_plan(c, m);
+  front_reserve(c, m);
   std::optional<StageScope> sc;
-  sc.emplace(c, kStOverlay);
-  c->mid_batch = true;
-  apply_overlay(c, in, m);
-  sc.reset();
   if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
 
   if (c->heavy_used > 0) {
@@ -4711,34 +4786,15 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     c->heavy_used = 0;
   }
   // exact 2-hop sizes stay valid for the rows of this batch only
-  c->n2cache.reserve(std::max<int32_t>(n, 1));
-  c->n2stamp.reserve(std::max<int32_t>(n, 1));
-  c->n2bound.reserve(std::max<int32_t>(n, 1));
-  c->n2bstamp.reserve(std::max<int32_t>(n, 1));
   if (c->n2batch == 0 || c->n2batch == 0xffffffffu) {
     MF_CUDA(cudaMemsetAsync(c->n2stamp.p, 0, sizeof(uint32_t) * (size_t)std::max<int32_t>(n, 1), s));
     MF_CUDA(cudaMemsetAsync(c->n2bstamp.p, 0, sizeof(uint32_t) * (size_t)std::max<int32_t>(n, 1), s));
     c->n2batch = 0;
   }
   ++c->n2batch;
-  const int64_t big = 2 * std::min<int64_t>(m, kMaxBatchEdges) + (int64_t)n + 2;
-  c->i64a.reserve(big);
-  c->i64b.reserve(big);
-  c->u8a.reserve(big);
-  c->seeds.reserve(2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->cands.reserve(max_cands(c));
-  c->rowcid.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->creates.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges));
-  c->rowlens.reserve(max_cands(c) + 2 * std::min<int64_t>(m, kMaxBatchEdges) + 1);
 
   // ---- sub-batch plan: cuts, estimates and seed lists of the whole batch
   // from p0 (re-planned from the next sub-batch when MAX_CSR_ELEMENTS grows)
-  c->plan_cuts.reserve(std::max<int64_t>(m, 1));
-  c->plan_ests.reserve(std::max<int64_t>(m, 1));
-  c->plan_send.reserve(std::max<int64_t>(m, 1));
-  c->plan_flags.reserve(2 * m);
-  c->plan_pos.reserve(2 * m + 1);
-  c->seeds_all.reserve(2 * m);
   std::vector<int64_t> cuts, ests, seed_end;
   size_t kidx = 0;
   int64_t seed_base = 0;
@@ -4751,7 +4807,6 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
                       c->plan_cuts.p, c->plan_ests.p, c->plan_send.p, c->seeds_all.p, bc, c->h_plan));
       return;
     }
-    c->plan_edges.reserve(4 * m);
     int4* edges = reinterpret_cast<int4*>(c->plan_edges.p);
     MF_K(launch_pdl(k_pack_edges, grid_for(m), kTB, 0, s, GatherEdge{c->bu.p, c->bv.p, c->prev.p, c->deg.p}, m, edges,
                     bc));
@@ -4792,6 +4847,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     plan_read();
     sc.reset();
   };
+  sc.emplace(c, kStOverlay);
+  c->mid_batch = true;
+  apply_overlay(c, in, m);
   // The plan of the whole batch, then the added arrays' rebuild: the host
   // waits for the plan alone, and the rebuild runs while it goes on.  The
   // header says whether the lines were valid (nothing has changed if not).
@@ -4804,7 +4862,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   MF_CUDA(cudaEventSynchronize(c->ev_a));
   if (c->h_plan[1] != 0) {
     MF_CUDA(cudaStreamSynchronize(s));
-    c->mid_batch = dirty;
+    c->mid_batch = false;
     MF_FAIL(MF_EINVAL, "update endpoints must be distinct vertex ids in [0, n)");
   }
   swap_overlay(c, c->h_plan[2], c->h_plan[3]);
@@ -4821,7 +4879,6 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   // previous sub-batch on the second stream; on small graphs the stream switch
   // costs more than the front, which then runs inline.
   const bool overlap_fronts = c->n >= kOverlapFronts;
-  front_reserve(c, m, dirty);
   int cur = 0;
   bool front_on_b = false;
   front_compute(c, c->front[0], c->seeds_all.p, seed_end.empty() ? 0 : seed_end[0], s, h + kFrontSlot);
@@ -5031,8 +5088,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       const int64_t nwords = std::max<int64_t>(((int64_t)n + 31) / 32, 1);
       const bool grown = c->pbits.cap < nwords;
       c->pbits.reserve(nwords);
-      if (grown || (dirty && c->pull_runs == 0))
-        MF_CUDA(cudaMemsetAsync(c->pbits.p, 0, sizeof(uint2) * (size_t)c->pbits.cap, s));
+      if (grown) MF_CUDA(cudaMemsetAsync(c->pbits.p, 0, sizeof(uint2) * (size_t)c->pbits.cap, s));
     }
     uint2* pbits = use_pull ? c->pbits.p : nullptr;
     scan_exclusive_with(CreatesUpTo{c->creates.p, ns, hc}, c->i64b.p, rows, c->ws, s);

@@ -215,14 +215,18 @@ __global__ void __launch_bounds__(Threads) k_scan_lookback(L load, int64_t n, O 
   if (t == (int64_t)gridDim.x - 1 && threadIdx.x == 0) out(n, excl + tot);
 }
 
-template <int Threads, int Items, typename L, typename O>
-void scan_lookback(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
-  const int64_t nb = (n + Threads * Items - 1) / (Threads * Items);
+inline void reserve_tiles(Scratch& ws, int64_t nb, cudaStream_t s) {
   if (ws.scan_status.cap < 2 * nb) {
     ws.scan_status.reserve(2 * nb);
     // fresh memory may hold anything: no tag may match a later sequence number
     MF_CUDA(cudaMemsetAsync(ws.scan_status.p, 0, sizeof(unsigned long long) * (size_t)ws.scan_status.cap, s));
   }
+}
+
+template <int Threads, int Items, typename L, typename O>
+void scan_lookback(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
+  const int64_t nb = (n + Threads * Items - 1) / (Threads * Items);
+  reserve_tiles(ws, nb, s);
   const unsigned long long seq = ++ws.scan_seq;
   MF_K(launch_pdl(k_scan_lookback<Threads, Items, L, O>, (unsigned)nb, Threads, 0, s, load, n, out,
                   reinterpret_cast<ulonglong2*>(ws.scan_status.p), seq));
@@ -236,6 +240,12 @@ void scan_lookback(L load, O out, int64_t n, Scratch& ws, cudaStream_t s) {
 // Measured on the row counts of a sub-batch (ncu, before -> after): see
 // k_scan_lookback.
 constexpr int64_t kSmallTiles = 192;
+
+// Room for the status words of any scan of up to n items with the default
+// split, so that the scan itself allocates nothing.
+inline void reserve_scan(Scratch& ws, int64_t n, cudaStream_t s) {
+  reserve_tiles(ws, std::max<int64_t>(kSmallTiles, (n + 2047) / 2048), s);
+}
 
 // `small_tiles`: how many tiles of 256 before the 2,048-item ones (callers whose
 // items write lists of their own want more blocks).
