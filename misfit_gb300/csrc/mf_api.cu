@@ -336,11 +336,25 @@ __global__ void k_validate(const int32_t* u, const int32_t* v, int64_t m, int32_
   if (a < 0 || a >= n || b < 0 || b >= n || a == b) atomicAdd(bad, 1ull);
 }
 
+// A batch's lines copied to the context's arrays.
+mf::BatchIn copied_input(mf_ctx* c, const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t m,
+                         cudaMemcpyKind kind) {
+  cudaStream_t s = c->stream;
+  c->bu.reserve(m);
+  c->bv.reserve(m);
+  c->bins.reserve(m);
+  if (m > 0) {
+    MF_CUDA(cudaMemcpyAsync(c->bu.p, u, sizeof(int32_t) * (size_t)m, kind, s));
+    MF_CUDA(cudaMemcpyAsync(c->bv.p, v, sizeof(int32_t) * (size_t)m, kind, s));
+    MF_CUDA(cudaMemcpyAsync(c->bins.p, ins, (size_t)m, kind, s));
+  }
+  return {c->bu.p, c->bv.p, c->bins.p};
+}
+
 // Host lines of a batch where the device can read them: a small batch in the
 // context's pinned block (no copy is queued; the caller's call runs to the
 // end of the batch before the block is used again), a larger one copied.
 mf::BatchIn host_input(mf_ctx* c, const int32_t* u, const int32_t* v, const uint8_t* ins, int64_t m) {
-  cudaStream_t s = c->stream;
   if (m <= mf::kSmallBatch) {
     int32_t* hu = reinterpret_cast<int32_t*>(c->h_stage);
     int32_t* hv = hu + mf::kSmallBatch;
@@ -352,13 +366,7 @@ mf::BatchIn host_input(mf_ctx* c, const int32_t* u, const int32_t* v, const uint
     }
     return {hu, hv, hi};
   }
-  c->bu.reserve(m);
-  c->bv.reserve(m);
-  c->bins.reserve(m);
-  MF_CUDA(cudaMemcpyAsync(c->bu.p, u, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
-  MF_CUDA(cudaMemcpyAsync(c->bv.p, v, sizeof(int32_t) * (size_t)m, cudaMemcpyHostToDevice, s));
-  MF_CUDA(cudaMemcpyAsync(c->bins.p, ins, (size_t)m, cudaMemcpyHostToDevice, s));
-  return {c->bu.p, c->bv.p, c->bins.p};
+  return copied_input(c, u, v, ins, m, cudaMemcpyHostToDevice);
 }
 
 // The pairs of a flag query into c->bu / c->bv, checked.
@@ -793,7 +801,9 @@ int mf_apply_batch_device(mf_ctx* c, const int32_t* d_u, const int32_t* d_v, con
     need(c && m >= 0 && (m == 0 || (d_u && d_v && d_ins)), MF_EINVAL, "bad arguments");
     need(!c->pending, MF_EINVAL, "asynchronous batches are pending; collect them (mf_collect / mf_sync) first");
     bind(c);
-    run_batch(c, mf::BatchIn{d_u, d_v, d_ins}, m);
+    // copied, so that any address that a copy can read will do: kernels would
+    // need 4-byte alignment and memory of this GPU
+    run_batch(c, copied_input(c, d_u, d_v, d_ins, m, cudaMemcpyDeviceToDevice), m);
   });
 }
 

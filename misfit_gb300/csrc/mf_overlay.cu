@@ -183,8 +183,8 @@ __global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, 
 
 // A small batch's input in one launch: block 0 stages and checks the lines and
 // groups the pairs, block 1 sorts the endpoint slots and finds the previous
-// occurrences.  Both read the lines where the caller's copy is (pinned host
-// memory or the device).  Latency of one block's sort bounds it; as separate
+// occurrences.  Both read the lines where they were staged (pinned host
+// memory, or the context's arrays).  Latency of one block's sort bounds it; as separate
 // launches (three copies, a check, key kernels, three sorts, k_prev) the same
 // work took 16 launches and two round trips to the host.
 template <int Items>

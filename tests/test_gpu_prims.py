@@ -327,3 +327,31 @@ def test_pull_by_row_tails(gb, n):
             orc.apply_batch(u, v, ins)
             assert np.array_equal(g.get_mis(), orc.get_mis()), k
             assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), k
+
+
+@pytest.mark.parametrize("m", [1, 700, 4096, 4097])
+@pytest.mark.parametrize("skew", [1, 2, 3])
+def test_device_lines_at_any_address(gb, m, skew):
+    """Device arrays that start between two words: the lines are copied, not read in place."""
+    import oracle as O
+    import torch
+    n = 3000
+    nindex, nlist = W.er_graph(n, 6, 2)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    stream = W.ToggleStream(n, nindex, nlist, m)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for x in (g, orc):
+            x.set_mis(mis)
+        for _ in range(2):
+            u, v, ins = stream.next_batch(m, with_flags=True)
+            raw = [np.zeros(a.nbytes + skew, np.uint8) for a in (u, v, ins)]
+            for r, a in zip(raw, (u, v, ins)):
+                r[skew:] = a.view(np.uint8)
+            dev = [torch.as_tensor(r, device="cuda") for r in raw]
+            torch.cuda.synchronize()
+            g.apply_batch_device(*(d.data_ptr() + skew for d in dev), u.size)
+            orc.apply_batch(u, v, ins)
+            assert np.array_equal(g.get_mis(), orc.get_mis())
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
+            assert np.array_equal(g.degrees(), orc.degrees())
