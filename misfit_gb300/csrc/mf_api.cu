@@ -68,16 +68,6 @@ bool pdl_on() {
   return on;
 }
 
-void raise_smem_limit(int device, const void* kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void*>, size_t> raised;
-  std::lock_guard<std::mutex> lock(mu);
-  size_t& have = raised[{device, kernel}];
-  if (have >= bytes) return;
-  MF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  have = bytes;
-}
-
 bool ktime_on() {
   static const bool on = [] {
     const char* e = std::getenv("MISFIT_GB_KTIME");

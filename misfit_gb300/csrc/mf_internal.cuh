@@ -104,12 +104,20 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 
 bool pdl_on();
 
-void raise_smem_limit(int device, const void* kernel, size_t bytes);
-// Raises a kernel's dynamic shared memory limit to `bytes`, once per device.
-template <typename... KArgs>
-void raise_smem(int device, void (*kernel)(KArgs...), size_t bytes) {
-  raise_smem_limit(device, reinterpret_cast<const void*>(kernel), bytes);
-}
+// Dynamic shared memory limits that were raised, kept with a context's
+// workspace: a device that is reset forgets them, and no workspace outlives
+// that.  Every caller raises a kernel to the same size.
+struct SmemLimits {
+  std::vector<const void*> raised;
+  template <typename... KArgs>
+  void raise(void (*kernel)(KArgs...), size_t bytes) {
+    const void* k = reinterpret_cast<const void*>(kernel);
+    for (const void* r : raised)
+      if (r == k) return;
+    MF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    raised.push_back(k);
+  }
+};
 
 template <typename... KArgs, typename... Args>
 void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
@@ -569,6 +577,7 @@ struct Scratch {
   DBuf<uint32_t> vals_alt;
   DBuf<unsigned long long> scan_status;   // look-back scan: {value, tag} per tile, tagged with scan_seq
   unsigned long long scan_seq = 0;
+  SmemLimits smem;
   void release() {
     scan_status.release();
     hist.release();

@@ -252,8 +252,7 @@ __global__ void __launch_bounds__(1024) k_small_input(BatchIn in, int m, int32_t
 template <int Items>
 void small_input(mf_ctx* c, const BatchIn& in, int m, int threads, int nbits, int gbits) {
   const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * sort_detail::kDigits * 4;
-  if (smem > 48 * 1024)
-    raise_smem(c->device, k_small_input<Items>, Items * 1024 * 12 + 32 * sort_detail::kDigits * 4);
+  if (smem > 48 * 1024) c->ws.smem.raise(k_small_input<Items>, Items * 1024 * 12 + 32 * sort_detail::kDigits * 4);
   MF_K(k_small_input<Items><<<2, threads, smem, c->stream>>>(
       in, m, c->n, nbits, gbits, c->bu.p, c->bv.p, c->bins.p, c->app_line.p, c->keys.p, c->vals.p, c->slot_keys.p,
       c->slot_vals.p, c->prev.p, c->work.p + kCntBad));

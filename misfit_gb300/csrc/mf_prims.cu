@@ -56,13 +56,10 @@ __global__ void __launch_bounds__(1024) k_sort_block(uint64_t* keys, uint32_t* v
 constexpr int kBlockSortMax = 8192;
 
 template <int Items, bool Mixed>
-void sort_block(uint64_t* keys, uint32_t* vals, int n, int threads, int first_bit, int end_bit, cudaStream_t s) {
+void sort_block(uint64_t* keys, uint32_t* vals, int n, int threads, int first_bit, int end_bit, Scratch& ws,
+                cudaStream_t s) {
   const size_t smem = (size_t)Items * threads * 12 + (size_t)(threads / 32) * kDigits * 4;
-  if (smem > 48 * 1024) {
-    int dev = 0;
-    MF_CUDA(cudaGetDevice(&dev));
-    raise_smem(dev, k_sort_block<Items, Mixed>, Items * 1024 * 12 + 32 * kDigits * 4);
-  }
+  if (smem > 48 * 1024) ws.smem.raise(k_sort_block<Items, Mixed>, Items * 1024 * 12 + 32 * kDigits * 4);
   MF_K(launch_pdl(k_sort_block<Items, Mixed>, 1, (unsigned)threads, smem, s, keys, vals, n, first_bit, end_bit));
 }
 
@@ -203,11 +200,11 @@ SortedPairs sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int first_bit,
   if (n <= 1) return {keys, vals};
   if (n <= kBlockSortMax) {
     // one to eight items a thread; 256 threads at least, one per digit
-    if (n <= 256) sort_block<1, Mixed>(keys, vals, (int)n, 256, first_bit, end_bit, s);
-    else if (n <= 1024) sort_block<1, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
-    else if (n <= 2048) sort_block<2, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
-    else if (n <= 4096) sort_block<4, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
-    else sort_block<8, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, s);
+    if (n <= 256) sort_block<1, Mixed>(keys, vals, (int)n, 256, first_bit, end_bit, ws, s);
+    else if (n <= 1024) sort_block<1, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, ws, s);
+    else if (n <= 2048) sort_block<2, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, ws, s);
+    else if (n <= 4096) sort_block<4, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, ws, s);
+    else sort_block<8, Mixed>(keys, vals, (int)n, 1024, first_bit, end_bit, ws, s);
     MF_CUDA(cudaGetLastError());
     return {keys, vals};
   }

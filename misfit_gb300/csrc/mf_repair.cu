@@ -4445,7 +4445,7 @@ struct Repair {
                       const_cast<uint32_t*>(order), c->rp_w0.p, c->rp_w1.p, c->mis.p, c->rp_keys.p, c->rp_vals.p, dyn,
                       c->counters.p + 24, const_cast<int64_t*>(got)));
     } else if (!small()) {
-      raise_smem(c->device, k_spec_round_large, kLargeSmem);
+      c->ws.smem.raise(k_spec_round_large, kLargeSmem);
       StageScope isc(c, kStRepair);
       MF_K(launch_pdl(k_repair_init, grid_for(std::max<int64_t>(nproc, 7)), kTB, 0, s, c->bu.p, c->bv.p, c->bins.p, p,
                       order, c->mis.p, c->rp_w0.p, c->rp_w1.p, nproc, got, dyn, c->counters.p + 24));
@@ -5195,7 +5195,7 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
         next.how = Assigned::kBlock;
         auto launch = [&](auto kernel, int items) {
           const size_t smem = (size_t)items * 1024 * 12 + 32 * sort_detail::kDigits * 4;
-          raise_smem(c->device, kernel, smem);
+          c->ws.smem.raise(kernel, smem);
           MF_K(launch_pdl(kernel, 1, 1024, smem, s, c->bu.p, c->bv.p, p, (int)len, c->cid.p, ccp, cbits, order, got));
         };
         if (len <= 2048) launch(k_assign_block<2>, 2);
