@@ -156,18 +156,17 @@ void release_all(mf_ctx* c) {
   c->ev_pool.clear();
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
-  if (c->stream_b) {
-    mf::return_stream(c->device, c->stream_b);
+  for (cudaStream_t* t : {&c->stream_b, &c->stream_r}) {
+    if (*t) mf::return_stream(c->device, *t);
+    *t = nullptr;
   }
-  c->stream_b = nullptr;
-  if (c->stream_r) mf::return_stream(c->device, c->stream_r);
-  c->stream_r = nullptr;
   if (c->ev_s) cudaEventDestroy(c->ev_s);
   if (c->ev_r) cudaEventDestroy(c->ev_r);
   if (c->ev_a) cudaEventDestroy(c->ev_a);
   if (c->ev_b) cudaEventDestroy(c->ev_b);
   if (c->stream) cudaStreamDestroy(c->stream);
   c->stream = nullptr;
+  mf::count_context(c->device, -1);
 }
 
 mf_ctx* new_ctx(int gpu) {
@@ -177,6 +176,7 @@ mf_ctx* new_ctx(int gpu) {
   MF_CUDA(cudaSetDevice(gpu));
   mf_ctx* c = new mf_ctx();
   c->device = gpu;
+  mf::count_context(gpu, 1);
   try {
     mf::noalloc_refresh(gpu);
     if (const char* e = std::getenv("MISFIT_GB_BIG_THRESHOLD")) c->tune.big_threshold = std::max<long long>(0, std::atoll(e));
@@ -226,9 +226,13 @@ void bind(const mf_ctx* c) {
   mf::g_alloc_stream = c->stream;
 }
 
+// The batch's side streams go back: the host has waited for all of its work.
 void return_side_streams(mf_ctx* c) {
   for (cudaStream_t* t : {&c->stream_b, &c->stream_r})
     if (*t) {
+      mf::for_each_buffer(c, [&](auto& b) {
+        if (b.s == *t) b.s = c->stream;
+      });
       mf::return_stream(c->device, *t);
       *t = nullptr;
     }

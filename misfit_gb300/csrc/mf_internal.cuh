@@ -950,7 +950,9 @@ void exact_fixup(mf_ctx* c);                       // exact-MIS mode after a bat
 // mf_parse.cu: batch file -> c->bu / c->bv (valid lines, file order); returns the count
 int64_t parse_batch_file_device(mf_ctx* c, const char* path);
 // mf_repair.cu
-// Side streams of a device: borrowed for a batch, returned when it has ended.
+// Side streams of a device: borrowed for a batch, returned when it has ended,
+// destroyed when its last context closes (count_context).
+void count_context(int device, int64_t change);
 cudaStream_t borrow_stream(int device);
 void return_stream(int device, cudaStream_t t);
 void process_batch(mf_ctx* c, const BatchIn& in, int64_t m);

@@ -4656,17 +4656,37 @@ void pipe_reserve(mf_ctx* c, int64_t m) {
 // costs milliseconds when hundreds of contexts each bring their own: the first
 // batch of 256 open contexts took 7.7 ms each with two of them per context,
 // 3.8 with lent ones.
-// As many exist as were ever out at once; they are not destroyed, because
-// buffers keep the stream that they were allocated on.
+// As many exist as were ever out at once while the device had contexts; the
+// last context that closes destroys them, so none outlives a device reset.
+// A batch gives its streams back when the host has waited for all of its
+// work, and the buffers that it allocated on them go over to the context's own
+// stream then (return_side_streams): no buffer is freed on a stream that
+// another context may hold, and within a batch a buffer of one of its streams
+// is freed on that stream, or after a host wait for its users.
 namespace {
+struct SideStreams {
+  int64_t contexts = 0;
+  std::vector<cudaStream_t> idle;
+};
 std::mutex g_side_mu;
-std::unordered_map<int, std::vector<cudaStream_t>> g_side_idle;
+std::unordered_map<int, SideStreams> g_side;
 }  // namespace
+
+void count_context(int device, int64_t change) {
+  std::vector<cudaStream_t> unused;
+  {
+    std::lock_guard<std::mutex> lock(g_side_mu);
+    SideStreams& d = g_side[device];
+    d.contexts += change;
+    if (d.contexts == 0) unused.swap(d.idle);
+  }
+  for (cudaStream_t t : unused) cudaStreamDestroy(t);
+}
 
 cudaStream_t borrow_stream(int device) {
   {
     std::lock_guard<std::mutex> lock(g_side_mu);
-    auto& idle = g_side_idle[device];
+    auto& idle = g_side[device].idle;
     if (!idle.empty()) {
       const cudaStream_t t = idle.back();
       idle.pop_back();
@@ -4680,7 +4700,7 @@ cudaStream_t borrow_stream(int device) {
 
 void return_stream(int device, cudaStream_t t) {
   std::lock_guard<std::mutex> lock(g_side_mu);
-  g_side_idle[device].push_back(t);
+  g_side[device].idle.push_back(t);
 }
 
 namespace {

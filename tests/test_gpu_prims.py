@@ -355,3 +355,39 @@ def test_device_lines_at_any_address(gb, m, skew):
             assert np.array_equal(g.get_mis(), orc.get_mis())
             assert np.array_equal(g.cluster_ids(), orc.cluster_ids())
             assert np.array_equal(g.degrees(), orc.degrees())
+
+
+def test_overlapped_repairs_of_several_contexts(gb):
+    """Batches of several sub-batches on eight contexts from eight threads at once, each batch larger than the last
+    (buffers grow while other contexts hold the same side streams), contexts closing while others go on.  Every
+    graph's membership, ids and limit equal its own oracle's."""
+    from concurrent.futures import ThreadPoolExecutor
+    import oracle as O
+
+    def work(k):
+        # (vertices, degree, lines, limit): short rows, long rows, fronts on a side stream, host-driven rounds
+        n, degree, sizes, limit = ((3000, 6, (200, 600, 1200), 150000), (None, 8, (300, 700, 1100), 400000),
+                                   (70000, 4, (3000, 6000, 9000), 4000000),
+                                   (70000, 2, (20000, 60000, 90000), 120000000))[k % 4]
+        nindex, nlist = W.rmat_graph(11, degree, k)[1] if n is None else W.er_graph(n, degree, k)
+        n = nindex.size - 1
+        mis = O.greedy_mis(nindex, nlist)
+        orc = O.Oracle.from_csr(nindex, nlist)
+        stream = W.ToggleStream(n, nindex, nlist, k)
+        subs = 0
+        with gb.Graph.from_csr(nindex, nlist) as g:
+            for x in (g, orc):
+                x.max_csr = limit
+                x.set_mis(mis)
+            for m in sizes:
+                u, v, ins = stream.next_batch(m, with_flags=True)
+                g.apply_batch(u, v, ins)
+                orc.apply_batch(u, v, ins)
+                subs = max(subs, g.stats()["sub_batches"])
+                assert np.array_equal(g.get_mis(), orc.get_mis()), (k, m)
+                assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), (k, m)
+                assert g.max_csr == orc.max_csr, (k, m)
+        return subs
+
+    with ThreadPoolExecutor(8) as pool:
+        assert min(pool.map(work, range(16))) > 1

@@ -47,7 +47,7 @@ print("ok")
 """
 
 
-@pytest.mark.parametrize("kind", ["lines", "edges"])
+@pytest.mark.parametrize("kind", ["lines", "edges", "overlap"])
 def test_new_contexts_after_a_device_reset(gpu_lib, kind):
     r = subprocess.run([sys.executable, "-c", CHILD, ROOT, kind], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.split() == ["ok"], r.stderr[-2000:]
