@@ -164,11 +164,25 @@ extern const char* const kStageNames[kStCount];
 // use cudaMalloc / cudaFree.
 extern thread_local cudaStream_t g_alloc_stream;
 
+// One allocation that several buffers share; freed with the last of them.
+struct Slab {
+  void* p = nullptr;
+  cudaStream_t s = nullptr;
+  int refs = 0;
+  void drop() {
+    if (--refs > 0) return;
+    if (s) cudaFreeAsync(p, s);
+    else cudaFree(p);
+    delete this;
+  }
+};
+
 template <typename T>
 struct DBuf {
   T* p = nullptr;
   int64_t cap = 0;
   cudaStream_t s = nullptr;   // stream p was allocated on (stream-ordered), or null
+  Slab* slab = nullptr;       // p lies in it, or null
   void reserve(int64_t count) {
     if (count <= cap) return;
     release();
@@ -192,12 +206,57 @@ struct DBuf {
   }
   void release() {
     if (p) {
-      if (s) cudaFreeAsync(p, s);
+      if (slab) slab->drop();
+      else if (s) cudaFreeAsync(p, s);
       else cudaFree(p);
     }
     p = nullptr;
     cap = 0;
     s = nullptr;
+    slab = nullptr;
+  }
+};
+
+// Buffers that grow together, in one allocation: add() notes the ones that are
+// too small (their contents go), commit() makes them.  An allocation costs 1 to
+// 45 us by how many freed blocks of other contexts the memory pool looks
+// through, and a context's first batch needs some seventy buffers.  Buffers
+// that one event grows or frees belong in one group, and none that trades places
+// with a buffer that is kept longer: a slab lives as long as its last part.
+struct Group {
+  struct Ask {
+    void** p;
+    int64_t* cap;
+    Slab** slab;
+    int64_t count;
+    size_t bytes;
+  };
+  std::vector<Ask> asks;
+  template <typename T>
+  void add(DBuf<T>& b, int64_t count) {
+    if (count <= b.cap) return;
+    b.release();
+    count = count < 16 ? 16 : count;
+    asks.push_back({reinterpret_cast<void**>(&b.p), &b.cap, &b.slab, count,
+                    (sizeof(T) * (size_t)count + 255) & ~(size_t)255});
+  }
+  void commit() {
+    if (asks.empty()) return;
+    size_t total = 0;
+    for (const Ask& a : asks) total += a.bytes;
+    void* p = nullptr;
+    note_alloc();
+    if (g_alloc_stream) MF_CUDA(cudaMallocAsync(&p, total, g_alloc_stream));
+    else MF_CUDA(cudaMalloc(&p, total));
+    Slab* slab = new Slab{p, g_alloc_stream, (int)asks.size()};
+    char* at = static_cast<char*>(p);
+    for (const Ask& a : asks) {
+      *a.p = at;
+      *a.cap = a.count;
+      *a.slab = slab;
+      at += a.bytes;
+    }
+    asks.clear();
   }
 };
 
@@ -929,8 +988,9 @@ constexpr int kWorkWords = kCntBad + 8;
 constexpr int64_t kPlanHost = 160;
 constexpr int64_t kPlanWords = 8 + 3 * kPlanHost;
 // The buffers of the calls below, so that none of them allocates: between the
-// first and swap_overlay the graph is half changed and nothing may fail.
-void reserve_overlay(mf_ctx* c, int64_t m);
+// first and swap_overlay the graph is half changed and nothing may fail.  Those
+// of the batch's size are added to `sized`.
+void reserve_overlay(mf_ctx* c, int64_t m, Group& sized);
 // lines -> c->bu/bv/bins, endpoint slots by vertex, previous occurrences, and
 // the pairs' state changes (nothing changes when a line is invalid)
 void apply_overlay(mf_ctx* c, const BatchIn& in, int64_t m);

@@ -836,18 +836,18 @@ void flag_updates(mf_ctx* c, int64_t m) {
   MF_CUDA(cudaGetLastError());
 }
 
-void reserve_overlay(mf_ctx* c, int64_t m) {
+void reserve_overlay(mf_ctx* c, int64_t m, Group& sized) {
   cudaStream_t s = c->stream;
   const int64_t n = c->n, a = c->a_total, slots = 2 * m;
-  c->bu.reserve(m);
-  c->bv.reserve(m);
-  c->bins.reserve(m);
-  c->app_line.reserve(m);
-  c->keys.reserve(slots);
-  c->vals.reserve(slots);
-  c->slot_keys.reserve(slots);
-  c->slot_vals.reserve(slots);
-  c->prev.reserve(slots);
+  sized.add(c->bu, m);   // these three not again where the lines were copied to them
+  sized.add(c->bv, m);
+  sized.add(c->bins, m);
+  sized.add(c->app_line, m);
+  sized.add(c->keys, slots);
+  sized.add(c->vals, slots);
+  sized.add(c->slot_keys, slots);
+  sized.add(c->slot_vals, slots);
+  sized.add(c->prev, slots);
   // grown with every mark cleared: the rebuild clears the ones it used
   if (c->akill.grow(std::max<int64_t>(a, 1)))
     MF_CUDA(cudaMemsetAsync(c->akill.p, 0, (size_t)c->akill.cap, s));

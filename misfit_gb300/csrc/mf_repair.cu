@@ -3866,23 +3866,37 @@ void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>
 // every graph were tens of MB a context, whatever its size.)
 int64_t max_cands(const mf_ctx* c) { return std::min<int64_t>(kMaxRows, std::max<int32_t>(c->n, 1)); }
 
-void front_reserve(mf_ctx* c, int64_t m) {
+// `sized` and `kept` are made here: the groups of the buffers of the batch's and
+// of the graph's size.  (A front's hop-1 list trades places with the context's,
+// which outlives the other scratch, so it stands alone.)
+void front_reserve(mf_ctx* c, int64_t m, Group& sized, Group& kept) {
   cudaStream_t s = c->stream;
   const int64_t words = ((int64_t)c->n + 31) / 32;
   const int64_t max_ns = 2 * std::min<int64_t>(m, kMaxBatchEdges);
-  auto zeroed = [&](auto& buf, int64_t count) {
-    const bool grown = buf.cap < count;
-    buf.reserve(count);
-    if (grown) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
-  };
-  for (auto& f : c->front) {
-    zeroed(f.bits, std::max<int64_t>(2 * words, 1));
-    zeroed(f.uacc, std::max<int64_t>(max_ns, 1));
-    zeroed(f.cnt, 3);
-    f.hlist.reserve(std::max<int32_t>(c->n, 1));
-    f.cands.reserve(max_cands(c));
-    f.lb_offs.reserve(2 * max_ns + 2);
+  bool grown[2][3];
+  for (int k = 0; k < 2; ++k) {
+    Front& f = c->front[k];
+    const int64_t want[3] = {std::max<int64_t>(2 * words, 1), std::max<int64_t>(max_ns, 1), 3};
+    grown[k][0] = f.bits.cap < want[0];
+    grown[k][1] = f.uacc.cap < want[1];
+    grown[k][2] = f.cnt.cap < want[2];
+    kept.add(f.bits, want[0]);
+    sized.add(f.uacc, want[1]);
+    kept.add(f.cnt, want[2]);
+    kept.add(f.cands, max_cands(c));
+    sized.add(f.lb_offs, 2 * max_ns + 2);
   }
+  auto zero = [&](auto& buf, bool on) {
+    if (on) MF_CUDA(cudaMemsetAsync(buf.p, 0, sizeof(*buf.p) * (size_t)buf.cap, s));
+  };
+  sized.commit();
+  for (int k = 0; k < 2; ++k) zero(c->front[k].uacc, grown[k][1]);
+  kept.commit();
+  for (int k = 0; k < 2; ++k) {
+    zero(c->front[k].bits, grown[k][0]);
+    zero(c->front[k].cnt, grown[k][2]);
+  }
+  for (auto& f : c->front) f.hlist.reserve(std::max<int32_t>(c->n, 1));
 }
 
 // Front of a sub-batch with `ns` seeds: hop-1 and seed bitmaps, the hop-1
@@ -4213,12 +4227,14 @@ void exact_sizes(mf_ctx* c, int64_t ns, uint32_t ep, bool bound_only) {
 // the device.
 FirstQueues first_queues(mf_ctx* c, int64_t upper, unsigned long long* qcnt) {
   const int64_t cap = std::max<int64_t>(upper, 1);
-  c->fpos.reserve(cap);
-  c->un_idx.reserve(cap);
-  c->un_v.reserve(cap);
-  c->un_cnt.reserve(cap);
-  c->rq_idx.reserve(cap);
-  c->rq_v.reserve(cap);
+  Group q;
+  q.add(c->fpos, cap);
+  q.add(c->un_idx, cap);
+  q.add(c->un_v, cap);
+  q.add(c->un_cnt, cap);
+  q.add(c->rq_idx, cap);
+  q.add(c->rq_v, cap);
+  q.commit();
   return FirstQueues{c->un_idx.p, c->un_v.p, qcnt, ChunkQueue{c->rq_idx.p, c->rq_v.p, c->un_cnt.p, qcnt + 1},
                      std::max<int64_t>(c->tune.first_bound, kProbe)};
 }
@@ -4269,8 +4285,10 @@ void cluster_read(mf_ctx* c, const GraphView& g, const int32_t* seeds, int64_t n
   const int64_t past = ncand > nct ? nh : 0;
   const int64_t rows = ns + nct + past;
   unsigned long long* ucnt = reinterpret_cast<unsigned long long*>(c->counters.p);
-  c->live_i.reserve(std::max<int64_t>(rows, 1));
-  c->live_v.reserve(std::max<int64_t>(rows, 1));
+  Group listed;
+  listed.add(c->live_i, std::max<int64_t>(rows, 1));
+  listed.add(c->live_v, std::max<int64_t>(rows, 1));
+  listed.commit();
   c->cidbits.reserve(((int64_t)n + 31) / 32 + 1);
   const unsigned row_blocks = grid_for(rows);
   MF_K(launch_pdl(k_row_skip, row_blocks + warps_grid(((int64_t)n + kCidBitsPerWarp - 1) / kCidBitsPerWarp), kTB, 0, s,
@@ -4316,22 +4334,24 @@ bool host_rounds_forced() {
 
 // The repair's buffers for up to nproc edges.
 void repair_reserve(mf_ctx* c, int64_t nproc) {
-  c->rp_w0.reserve(nproc);
-  c->rp_w1.reserve(nproc);
-  c->rp_n0.reserve(nproc);
-  c->rp_n1.reserve(nproc);
-  c->rp_keys.reserve(2 * nproc);
-  c->rp_vals.reserve(2 * nproc);
-  c->rp_keys2.reserve(2 * nproc);
-  c->rp_vals2.reserve(2 * nproc);
-  c->rp_u8.reserve(2 * nproc);
-  c->rp_pos.reserve(2 * nproc + 1);
-  c->big_pos.reserve(nproc);
-  c->big_r.reserve(nproc);
-  c->big_off.reserve(nproc);
-  c->big_nr.reserve(nproc);
-  c->big_chunks.reserve(nproc + 1);
-  c->big_best.reserve(nproc);
+  Group edges;
+  edges.add(c->rp_w0, nproc);
+  edges.add(c->rp_w1, nproc);
+  edges.add(c->rp_n0, nproc);
+  edges.add(c->rp_n1, nproc);
+  edges.add(c->rp_keys, 2 * nproc);
+  edges.add(c->rp_vals, 2 * nproc);
+  edges.add(c->rp_keys2, 2 * nproc);
+  edges.add(c->rp_vals2, 2 * nproc);
+  edges.add(c->rp_u8, 2 * nproc);
+  edges.add(c->rp_pos, 2 * nproc + 1);
+  edges.add(c->big_pos, nproc);
+  edges.add(c->big_r, nproc);
+  edges.add(c->big_off, nproc);
+  edges.add(c->big_nr, nproc);
+  edges.add(c->big_chunks, nproc + 1);
+  edges.add(c->big_best, nproc);
+  edges.commit();
   c->big_pre.reserve(std::max<int64_t>(4096, std::min<int64_t>((int64_t)1 << 22, 4 * (int64_t)c->n)));
   if (c->big_grid == 0) {
     int sms = 0;
@@ -4745,27 +4765,26 @@ void clear_leftovers(mf_ctx* c) {
 }
 
 // Buffers of the sub-batch plan and of one sub-batch's rows, at their largest.
-void reserve_plan(mf_ctx* c, int64_t m) {
+void reserve_plan(mf_ctx* c, int64_t m, Group& sized, Group& kept) {
   const int64_t edges = std::min<int64_t>(m, kMaxBatchEdges), n1 = std::max<int32_t>(c->n, 1);
-  c->n2cache.reserve(n1);
-  c->n2stamp.reserve(n1);
-  c->n2bound.reserve(n1);
-  c->n2bstamp.reserve(n1);
-  c->i64a.reserve(2 * edges + c->n + 2);
-  c->i64b.reserve(2 * edges + c->n + 2);
-  c->u8a.reserve(2 * edges + c->n + 2);
-  c->seeds.reserve(2 * edges);
-  c->cands.reserve(max_cands(c));
-  c->rowcid.reserve(max_cands(c) + 2 * edges);
-  c->creates.reserve(max_cands(c) + 2 * edges);
-  c->rowlens.reserve(max_cands(c) + 2 * edges + 1);
-  c->plan_cuts.reserve(std::max<int64_t>(m, 1));
-  c->plan_ests.reserve(std::max<int64_t>(m, 1));
-  c->plan_send.reserve(std::max<int64_t>(m, 1));
-  c->plan_flags.reserve(2 * m);
-  c->plan_pos.reserve(2 * m + 1);
-  c->seeds_all.reserve(2 * m);
-  if (m > kSmallBatch) c->plan_edges.reserve(4 * m);
+  kept.add(c->n2cache, n1);
+  kept.add(c->n2stamp, n1);
+  kept.add(c->n2bound, n1);
+  kept.add(c->n2bstamp, n1);
+  sized.add(c->i64a, 2 * edges + c->n + 2);
+  sized.add(c->i64b, 2 * edges + c->n + 2);
+  sized.add(c->seeds, 2 * edges);
+  kept.add(c->cands, max_cands(c));
+  sized.add(c->rowcid, max_cands(c) + 2 * edges);
+  sized.add(c->creates, max_cands(c) + 2 * edges);
+  sized.add(c->rowlens, max_cands(c) + 2 * edges + 1);
+  sized.add(c->plan_cuts, std::max<int64_t>(m, 1));
+  sized.add(c->plan_ests, std::max<int64_t>(m, 1));
+  sized.add(c->plan_send, std::max<int64_t>(m, 1));
+  sized.add(c->plan_flags, 2 * m);
+  sized.add(c->plan_pos, 2 * m + 1);
+  sized.add(c->seeds_all, 2 * m);
+  if (m > kSmallBatch) sized.add(c->plan_edges, 4 * m);
 }
 
 }  // namespace
@@ -4795,9 +4814,10 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
   if (c->mid_batch) clear_leftovers(c);   // of a failed batch, where it could not do so itself
   // every buffer that is needed before the batch's links are in the graph: up
   // to here a batch that runs out of memory has changed nothing
-  reserve_overlay(c, m);
-  reserve_plan(c, m);
-  front_reserve(c, m);
+  Group sized, kept;
+  reserve_overlay(c, m, sized);
+  reserve_plan(c, m, sized, kept);
+  front_reserve(c, m, sized, kept);
   std::optional<StageScope> sc;
   if (c->profile & 4) MF_CUDA(cudaMemsetAsync(cnt + 56, 0, sizeof(int64_t) * 2, s));
 
@@ -5073,8 +5093,10 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     // counters, zeroed by k_seed_rows: [33] live rows, [34] need seeds, [36]
     // the pull's long rows; [48, 49], [53, 54] the queues of the two first-hit
     // searches, [55] the assignment's count
-    c->need.reserve(std::max<int64_t>(ns, 1));
-    c->needv.reserve(std::max<int64_t>(ns, 1));
+    Group needs;
+    needs.add(c->need, std::max<int64_t>(ns, 1));
+    needs.add(c->needv, std::max<int64_t>(ns, 1));
+    needs.commit();
     if (short_rows) {
       MF_K(launch_pdl(k_first_short, grid_for(rows * kGroup), kTB, 0, s, g, seeds, ns, c->cands.p, hc, c->cid.p,
                       v2i, c->rowcid.p, c->creates.p, c->need.p, c->needv.p, ucnt + 34));
