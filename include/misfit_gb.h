@@ -389,7 +389,10 @@ typedef struct mf_batched_opts {
   int block;                  /* threads per persistent CTA: 64..1024, a multiple of 32 (default 512) */
   int ctas_per_sm;            /* persistent CTAs per SM (default 2) */
   int64_t max_cta_updates;    /* batches of at most this many lines may take the kernel (default 8192) */
-  int32_t max_cta_vertices;   /* ... on graphs of at most this many vertices (default 2^20) */
+  int32_t max_cta_vertices;   /* ... on graphs of at most this many vertices (default 2^20).  Up to these
+                                 defaults the library still moves the batches that the multi-launch
+                                 path ends sooner; with a limit above its default all batches within
+                                 the limits take the kernel */
   int use_graph;              /* 1: capture the step as a CUDA graph (default), 0: plain launches */
   int path_threads;           /* host threads driving the batches above the kernel's limits, each
                                  graph on its own stream (1..64, default 8) */

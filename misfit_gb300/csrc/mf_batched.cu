@@ -142,12 +142,16 @@ void need(bool cond, int status, const char* msg) {
   if (!cond) MF_FAIL(status, msg);
 }
 
+// The library's limits.
+constexpr int64_t kCtaUpdates = 8192;
+constexpr int32_t kCtaVertices = 1 << 20;
+
 mf_batched_opts default_opts() {
   mf_batched_opts o;
   o.block = 512;
   o.ctas_per_sm = 2;
-  o.max_cta_updates = 8192;
-  o.max_cta_vertices = 1 << 20;
+  o.max_cta_updates = kCtaUpdates;
+  o.max_cta_vertices = kCtaVertices;
   o.use_graph = 1;
   o.path_threads = 8;
   o.pool_idle_first = 1;
@@ -213,6 +217,8 @@ int run_path_items(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
 // So the longest items move to the path as long as an item's own time in the
 // kernel exceeds what the path then has to do.  Small graphs stay while their
 // item is short: steps of many of them are what the kernel is for.
+// A caller that raises a limit above the library's wants the kernel to take
+// the batches up to it: then the limits alone decide.
 constexpr double kCtaStays = 3.25;          // ms
 constexpr int32_t kCtaStaysVertices = 4096;
 constexpr double kPathOverlap = 3.0;
@@ -304,7 +310,8 @@ void apply_batches(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
       path_items.push_back(i);
     }
   }
-  route_items(ctxs, m, kitems, path_items);
+  if (o.max_cta_updates <= kCtaUpdates && o.max_cta_vertices <= kCtaVertices)
+    route_items(ctxs, m, kitems, path_items);
   std::sort(kitems.begin(), kitems.end(), [](const KernelItem& a, const KernelItem& b) { return a.cost > b.cost; });
   stats.kernel_items = (int64_t)kitems.size();
   stats.path_items = (int64_t)path_items.size();

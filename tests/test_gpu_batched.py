@@ -146,3 +146,13 @@ def test_batched_rejects_bad_batch_before_running():
     finally:
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("seed,opts,small_limit", [
+    (5, {}, None), (6, {"use_graph": 0, "block": 256, "ctas_per_sm": 1}, None),
+    (7, {"block": 1024, "ctas_per_sm": 1}, None), (8, {}, 4000), (9, {"path_threads": 1}, 4000)])
+def test_batched_limits_above_the_defaults_decide_alone(seed, opts, small_limit):
+    """With a raised limit every batch within it is the kernel's, whatever its size: the engine itself is compared,
+    up to 12,000 lines and 12,000 vertices."""
+    kinds = _run(seed, 2, native.batched_opts(max_cta_updates=16384, **opts), small_limit)
+    assert kinds == {"kernel_items": 28, "path_items": 0}
