@@ -221,25 +221,29 @@ int run_path_items(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
 // the batches up to it: then the limits alone decide.
 constexpr double kCtaStays = 3.25;          // ms
 constexpr int32_t kCtaStaysVertices = 4096;
-constexpr double kPathOverlap = 3.0;
+constexpr double kPathOverlap = 3.0;        // of eight threads; one thread overlaps nothing
 
 double cta_ms(const mf_ctx* c, int64_t m) {
   const double row = 1.0 + (c->n > 0 ? (double)(c->nnz + c->a_total) / c->n : 0.0);
   return 0.1 + 4e-6 * (double)c->n + std::max(0.010 * std::sqrt((double)m) * row, 3.6e-4 * (double)m * row);
 }
 
-double path_ms(const mf_ctx* c, int64_t m) { return (0.11 + 2.3e-5 * (double)m + 1e-7 * (double)c->n) / kPathOverlap; }
+double path_ms(const mf_ctx* c, int64_t m, double overlap) {
+  return (0.11 + 2.3e-5 * (double)m + 1e-7 * (double)c->n) / overlap;
+}
 
-void route_items(mf_ctx* const* ctxs, const int64_t* m, std::vector<mf::KernelItem>& kernel, std::vector<int64_t>& path) {
+void route_items(mf_ctx* const* ctxs, const int64_t* m, int threads, std::vector<mf::KernelItem>& kernel,
+                 std::vector<int64_t>& path) {
   using mf::KernelItem;
+  const double overlap = std::min(kPathOverlap, (double)threads);
   double path_total = 0.0;
-  for (int64_t i : path) path_total += path_ms(ctxs[i], m[i]);
+  for (int64_t i : path) path_total += path_ms(ctxs[i], m[i], overlap);
   std::vector<std::pair<double, int64_t>> by_time;   // (one-CTA time, batch)
   for (const KernelItem& k : kernel) by_time.emplace_back(cta_ms(ctxs[k.idx], m[k.idx]), k.idx);
   std::sort(by_time.rbegin(), by_time.rend());
   std::vector<int64_t> moved;
   for (const auto& t : by_time) {
-    const double after = path_total + path_ms(ctxs[t.second], m[t.second]);
+    const double after = path_total + path_ms(ctxs[t.second], m[t.second], overlap);
     if (t.first <= after) break;
     if (t.first <= kCtaStays && ctxs[t.second]->n <= kCtaStaysVertices) continue;
     path_total = after;
@@ -311,7 +315,7 @@ void apply_batches(mf_ctx* const* ctxs, const int32_t* const* u, const int32_t* 
     }
   }
   if (o.max_cta_updates <= kCtaUpdates && o.max_cta_vertices <= kCtaVertices)
-    route_items(ctxs, m, kitems, path_items);
+    route_items(ctxs, m, o.path_threads, kitems, path_items);
   std::sort(kitems.begin(), kitems.end(), [](const KernelItem& a, const KernelItem& b) { return a.cost > b.cost; });
   stats.kernel_items = (int64_t)kitems.size();
   stats.path_items = (int64_t)path_items.size();
