@@ -129,6 +129,19 @@ struct LinesOut {
 // Chunks of the pinned block the file is read through.
 constexpr int64_t kReadChunk = 256 << 10;
 
+// The text and its line starts (nine bytes for each of the file) stay with the
+// context for files up to this size; larger ones give them back.
+constexpr int64_t kTextKept = 4 << 20;
+
+struct TextScratch {
+  mf_ctx* c;
+  ~TextScratch() {
+    if (c->txt.cap <= kTextKept && c->txt_begin.cap <= kTextKept) return;
+    c->txt.release();
+    c->txt_begin.release();
+  }
+};
+
 struct Fd {
   int fd;
   ~Fd() {
@@ -151,6 +164,7 @@ int64_t parse_batch_file_device(mf_ctx* c, const char* path) {
   const int64_t size = S_ISREG(sb.st_mode) && sb.st_size > 0 ? (int64_t)sb.st_size : 0;
   if (size == 0) return 0;
   const int64_t words = (size + 15) / 16;
+  const TextScratch text{c};
   c->txt.reserve(16 * words);
   c->txt_begin.reserve(size);
   if (!c->h_read) {

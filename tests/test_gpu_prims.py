@@ -391,3 +391,25 @@ def test_overlapped_repairs_of_several_contexts(gb):
 
     with ThreadPoolExecutor(8) as pool:
         assert min(pool.map(work, range(16))) > 1
+
+
+@pytest.mark.parametrize("mb", [2, 12])
+def test_parsing_gives_its_text_back(gb, tmp_path, mb):
+    """After a batch file the context holds its lines, nine bytes each, and for files up to 4 MB the text and line
+    starts; not nine bytes for each byte of a large file."""
+    import ctypes
+    lines = mb * 100000
+    rng = np.random.default_rng(mb)
+    u, v = rng.integers(1000000, 2000000, (2, lines))
+    path = str(tmp_path / "1.mtx")
+    with open(path, "w") as f:
+        f.write("".join("%07d %07d padded\n" % p for p in zip(u, v)))
+    rt = ctypes.CDLL({l.split()[-1] for l in open("/proc/self/maps") if "libcudart" in l}.pop())
+    with gb.Graph.from_csr(*W.er_graph(1000, 4, 1)) as g:
+        pool, used = ctypes.c_void_p(), [ctypes.c_uint64(), ctypes.c_uint64()]
+        assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used[0])) == 0   # cudaMemPoolAttrUsedMemCurrent
+        assert g.parse_batch_file(path)[0].size == 0    # ids past the graph: every line is read, none kept
+        assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used[1])) == 0
+    held = used[1].value - used[0].value
+    assert held <= 9 * lines + (1 << 20) + (9 * 23 * lines if mb <= 4 else 0)
