@@ -3862,7 +3862,7 @@ void row_offsets_into(mf_ctx* c, const int32_t* list, int64_t cnt, DBuf<int64_t>
 // Buffers of both fronts at their largest sizes for a batch of m updates, so
 // that no front allocates while another stream may use its memory.  Bitmaps,
 // sums and counters start at zero, and every front leaves them so.
-// Candidates are distinct vertices, so a small graph needs few rows.  (10^6 for
+// Candidates are distinct vertices, so a small graph needs few rows.  (2^21 for
 // every graph were tens of MB a context, whatever its size.)
 int64_t max_cands(const mf_ctx* c) { return std::min<int64_t>(kMaxRows, std::max<int32_t>(c->n, 1)); }
 

@@ -413,3 +413,45 @@ def test_parsing_gives_its_text_back(gb, tmp_path, mb):
         assert rt.cudaMemPoolGetAttribute(pool, 7, ctypes.byref(used[1])) == 0
     held = used[1].value - used[0].value
     assert held <= 9 * lines + (1 << 20) + (9 * 23 * lines if mb <= 4 else 0)
+
+
+@pytest.fixture(scope="module", params=[0, 300])
+def crowded(request):
+    """A graph and two batches of one sub-batch each whose seeds leave fewer rows than there are candidates (a
+    sub-batch has 2^21 rows), all rows short or one of them long; and what the oracle gives."""
+    import oracle as O
+    n, m = 3000000, 1040000
+    rng = np.random.default_rng(1)
+    a, b = rng.integers(0, n, (2, int(1.2 * n)))
+    a[:request.param] = 7
+    ok = a != b
+    nindex, nlist = W.csr_from_pairs(n, a[ok], b[ok])
+    orc = O.Oracle.from_csr(nindex, nlist)
+    mis = O.greedy_mis(nindex, nlist)
+    orc.max_csr = 1 << 40
+    orc.set_mis(mis)
+    batches, want = [], []
+    for _ in range(2):
+        u = rng.integers(0, n, m).astype(np.int32)
+        v = ((u + rng.integers(1, n, m)) % n).astype(np.int32)
+        batches.append((u, v, (rng.random(m) < 0.9).astype(np.uint8)))
+        orc.apply_batch(*batches[-1])
+        want.append((orc.get_mis(), orc.cluster_ids()))
+    return nindex, nlist, mis, batches, want
+
+
+@pytest.mark.parametrize("push", [1, 2])
+def test_more_candidates_than_rows(gb, crowded, push):
+    """Hop-1 vertices past the last candidate row have no row: the hop-2 part reads theirs again (short rows) or
+    searches them for their ids alone, and their tag bits outlive the sub-batch."""
+    nindex, nlist, mis, batches, want = crowded
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        g.max_csr = 1 << 40
+        g.set_mis(mis)
+        g.set_tuning(cand_push=push)
+        for (u, v, ins), (members, ids) in zip(batches, want):
+            g.apply_batch(u, v, ins)
+            st = g.stats()
+            assert st["sub_batches"] == 1 and st["seeds"] + st["candidates"] == 1 << 21   # every row is taken
+            assert np.array_equal(g.get_mis(), members)
+            assert np.array_equal(g.cluster_ids(), ids)
