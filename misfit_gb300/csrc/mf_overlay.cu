@@ -277,6 +277,25 @@ struct PairState {
   int32_t live[2], dead[2];
 };
 
+// Live and dead copies of y in the base positions [k, e) of an unsorted row: read
+// whole, a hub's of 10^4 entries by one thread, so eight loads are in flight (one
+// at a time a batch on unsorted R-MAT scale 17 took 4.7 ms; so 3.8).
+__device__ __noinline__ int2 unsorted_copies(const int32_t* nlist, const uint32_t* live, int64_t k, int64_t e, int32_t y) {
+  constexpr int kStep = 8;
+  int2 c = make_int2(0, 0);
+  for (; k < e; k += kStep) {
+    int32_t z[kStep];
+#pragma unroll
+    for (int j = 0; j < kStep; ++j) z[j] = k + j < e ? __ldg(nlist + k + j) : -1;
+#pragma unroll
+    for (int j = 0; j < kStep; ++j)
+      if (z[j] == y) {
+        if (live_at(live, k + j)) ++c.x; else ++c.y;
+      }
+  }
+  return c;
+}
+
 __device__ __forceinline__ PairState pair_state(const GraphView& g, bool sorted, int32_t a, int32_t b) {
   PairState r;
   const int32_t x[2] = {a, b}, y[2] = {b, a};
@@ -310,12 +329,13 @@ __device__ __forceinline__ PairState pair_state(const GraphView& g, bool sorted,
   for (int q = 0; q < 2; ++q) {
     r.first[q] = lo[q];
     r.end[q] = e[q];
-    for (int64_t k = lo[q]; k < e[q]; ++k) {
-      const int32_t z = __ldg(g.nlist + k);
-      if (z == y[q]) {
+    if (!sorted) {
+      const int2 c = unsorted_copies(g.nlist, g.live, lo[q], e[q], y[q]);
+      r.live[q] = c.x;
+      r.dead[q] = c.y;
+    } else {
+      for (int64_t k = lo[q]; k < e[q] && __ldg(g.nlist + k) == y[q]; ++k) {
         if (live_at(g.live, k)) ++r.live[q]; else ++r.dead[q];
-      } else if (sorted) {
-        break;
       }
     }
     for (int64_t k = ab[q]; k < ae[q]; ++k)
@@ -325,6 +345,58 @@ __device__ __forceinline__ PairState pair_state(const GraphView& g, bool sorted,
       }
   }
   return r;
+}
+
+// What a pair's updates have done so far.
+struct PairWalk {
+  int st;
+  bool appended, old_killed;
+  uint32_t last_seq;
+};
+
+__device__ __forceinline__ void pair_update(PairWalk& w, bool insert, bool base_xy, uint32_t line) {
+  const bool adj = w.st == kStA || (w.st == kStN && base_xy);
+  if (insert && !adj) {
+    if (w.st == kStR) w.st = kStN;
+    else { w.st = kStA; w.appended = true; w.last_seq = line; }
+  } else if (!insert && adj) {
+    if (w.st == kStA) {
+      w.st = kStN;
+      if (w.appended) w.appended = false; else w.old_killed = true;
+    } else {
+      w.st = kStR;
+    }
+  }
+}
+
+// The pair's further updates, from position j of its run on, four read at a
+// time: thousands of them are one thread's work (100,000 of one pair took
+// 25.3 ms one at a time; so 20.1).  Seldom reached, so it stays out of line.
+__device__ __noinline__ PairWalk pair_updates(PairWalk w, const uint64_t* keys, const uint32_t* vals, int64_t j,
+                                              int64_t m, int gbits, uint64_t key, const int32_t* u, const uint8_t* ins,
+                                              int32_t a, bool in_base_ab, bool in_base_ba) {
+  constexpr int kAhead = 4;
+  for (; j < m; j += kAhead) {
+    uint64_t k[kAhead];
+    uint32_t i[kAhead];
+    int32_t x[kAhead];
+    bool insert[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) k[q] = j + q < m ? keys[j + q] : ~key;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) i[q] = k[q] == key ? vals[j + q] : 0;
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      x[q] = k[q] == key ? u[i[q]] : 0;
+      insert[q] = k[q] == key && ins[i[q]] != 0;
+    }
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) {
+      if (k[q] == key) pair_update(w, insert[q], x[q] == a ? in_base_ab : in_base_ba, i[q]);
+      else if (j + q >= m || !same_run(k[q], key, gbits)) return w;
+    }
+  }
+  return w;
 }
 
 // One thread per unordered pair.  Besides the base tombstones it records what
@@ -363,31 +435,13 @@ __global__ void __launch_bounds__(kTB) k_apply_pairs(GraphView g, uint32_t* live
     const PairState ps = pair_state(g, sorted, a, b);
     const bool in_base_ab = ps.live[0] + ps.dead[0] > 0, in_base_ba = ps.live[1] + ps.dead[1] > 0;
     const int st0 = (ps.pos[0] >= 0 || ps.pos[1] >= 0) ? kStA : ((ps.dead[0] + ps.dead[1]) > 0 ? kStR : kStN);
-    int st = st0;
-    bool appended = false, old_killed = false;
-    uint32_t last_seq = 0;
-    for (int64_t j = j0; j < m; ++j) {
-      const uint64_t k = keys[j];
-      if (k != key) {
-        if (!same_run(k, key, gbits)) break;
-        continue;
-      }
-      const uint32_t i = vals[j];
-      const int32_t x = u[i];
-      const bool base_xy = (x == a) ? in_base_ab : in_base_ba;
-      const bool adj = st == kStA || (st == kStN && base_xy);
-      if (ins[i] && !adj) {
-        if (st == kStR) st = kStN;
-        else { st = kStA; appended = true; last_seq = i; }
-      } else if (!ins[i] && adj) {
-        if (st == kStA) {
-          st = kStN;
-          if (appended) appended = false; else old_killed = true;
-        } else {
-          st = kStR;
-        }
-      }
-    }
+    PairWalk w{st0, false, false, 0};
+    pair_update(w, ins[vals[j0]] != 0, u[vals[j0]] == a ? in_base_ab : in_base_ba, vals[j0]);
+    if (j0 + 1 < m && same_run(keys[j0 + 1], key, gbits))
+      w = pair_updates(w, keys, vals, j0 + 1, m, gbits, key, u, ins, a, in_base_ab, in_base_ba);
+    const int st = w.st;
+    const bool appended = w.appended, old_killed = w.old_killed;
+    const uint32_t last_seq = w.last_seq;
     int da = 0, db = 0;   // degree = base - tombstones + added (DeltaOverlay::degree)
     if ((st0 == kStR) != (st == kStR)) {
       const bool on = st0 == kStR;  // untombstone -> set live again

@@ -455,3 +455,46 @@ def test_more_candidates_than_rows(gb, crowded, push):
             assert st["sub_batches"] == 1 and st["seeds"] + st["candidates"] == 1 << 21   # every row is taken
             assert np.array_equal(g.get_mis(), members)
             assert np.array_equal(g.cluster_ids(), ids)
+
+
+@pytest.mark.parametrize("m", [40, 5000])
+@pytest.mark.parametrize("shuffled", [False, True])
+def test_pairs_of_many_updates(gb, m, shuffled):
+    """One to eleven updates of a pair in a batch (the first apart, then four at a time), both directions and every
+    flag, on rows with repeated entries, sorted or not; and one pair for the whole batch."""
+    import oracle as O
+    n = 900
+    rng = np.random.default_rng(m)
+    a, b = rng.integers(0, n, (2, 4000))
+    a[:200], b[:200] = 5, rng.integers(6, 60, 200)        # a hub whose row repeats its entries
+    ok = a != b
+    x, y = np.concatenate([a[ok], b[ok]]), np.concatenate([b[ok], a[ok]])
+    order = np.lexsort((rng.random(x.size) if shuffled else y, x))
+    nlist = y[order].astype(np.int32)
+    nindex = np.concatenate([[0], np.cumsum(np.bincount(x, minlength=n))]).astype(np.int64)
+    mis = O.greedy_mis(nindex, nlist)
+    orc = O.Oracle.from_csr(nindex, nlist)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        for z in (g, orc):
+            z.set_mis(mis)
+        for batch in range(4):
+            if batch == 2:
+                u, v = np.full(m, 5), np.full(m, 7)
+            else:
+                pairs = np.concatenate([np.full((m, 1), 5), rng.integers(6, 60, (m, 1))], 1)
+                far = rng.random(m) < 0.5
+                pairs[far] = rng.integers(0, n, (far.sum(), 2))
+                pairs = np.repeat(pairs, rng.integers(1, 12, m), axis=0)
+                pairs = pairs[pairs[:, 0] != pairs[:, 1]][:m]
+                u, v = pairs[rng.permutation(len(pairs))].T
+            flip = rng.random(u.size) < 0.5
+            u, v = np.where(flip, v, u).astype(np.int32), np.where(flip, u, v).astype(np.int32)
+            ins = rng.integers(0, 2, u.size).astype(np.uint8)
+            g.apply_batch(u, v, ins)
+            orc.apply_batch(u, v, ins)
+            assert np.array_equal(g.degrees(), orc.degrees()), batch
+            for z in range(0, n, 7):
+                assert np.array_equal(g.row(z), orc.row(z)), (batch, z)
+            assert np.array_equal(g.row(5), orc.row(5)), batch
+            assert np.array_equal(g.get_mis(), orc.get_mis()), batch
+            assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), batch
