@@ -877,8 +877,8 @@ def main():
 
     # ---- roofline of the two largest kernels, each timed by CUDA events
     # around its launches on the library's stream inside the timed region:
-    # the pull of the clustering write (k_pull_tails), 28 B per vertex + 4 B
-    # per row entry read, and k_lb_push_hop (the hop-2 reach of the sub-batches
+    # the pull of the clustering write (k_pull_tails), 32 B per vertex, and
+    # k_lb_push_hop (the hop-2 reach of the sub-batches
     # that push instead), 12 B per pushed element (4 B row entry read + 4 B
     # state read + 4 B cid write).  The one with more device time is the line's
     # "roofline"; a push that never ran is left out.
@@ -926,8 +926,8 @@ def main():
                 "algorithmic_bytes_per_launch": bytes_p / max(calls_p, 1), "avg_launch_ms": ms_p / max(calls_p, 1),
                 "launches": int(calls_p),
                 "timed": "per sub-batch: k_pull_tails and k_pull_cand_long (the pull step)",
-                "bytes_note": "28 B per vertex (row bounds, tombstone count, tag, id) + 4 B per row entry read "
-                              "(device counter)",
+                "bytes_note": "32 B per vertex (8 B added-entry offset, 16 B row tail, 4 B tombstone count, 4 B tag or "
+                              "new id); rows read past their tails and ids written are not counted",
                 "traffic_note": "DRAM bytes per launch of k_pull_tails from an ncu capture of this workload" if PULL_DRAM_BYTES_PER_LAUNCH else "not captured"}
         push_hop = roof
         if ms_p > ms:

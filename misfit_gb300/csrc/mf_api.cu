@@ -296,9 +296,10 @@ void run_batch(mf_ctx* c, const mf::BatchIn& in, int64_t m) {
     const unsigned long long* x = w + 2 * mf::kStCount;
     // 4 B row entry + 8 B state read and cid write per pushed element (x[3]:
     // the candidate rows of the sub-batches that pushed); x[2] the row
-    // entries read by the sub-batches that pulled
+    // entries looked at by the sub-batches that pulled (with row tails most
+    // of them lie in the tails, which are counted per vertex)
     c->stage_bytes[mf::kStPush] += 12.0 * (double)(x[0] + x[3]);
-    c->stage_bytes[mf::kStPull] += 4.0 * (double)x[2];
+    if (c->tails.cap == 0) c->stage_bytes[mf::kStPull] += 4.0 * (double)x[2];
     c->stage_bytes[mf::kStPushHop] += 12.0 * (double)x[1];
     if (debug) {
       std::fprintf(stderr,

@@ -5106,8 +5106,9 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
     } else {
       cluster_read(c, g, seeds, ns, nh, h[3], nct, v2i, sc);
     }
-    // Pull or push.  The pull costs ~28 B per vertex plus 4 B per row entry
-    // it reads (as many per vertex as in the last batch that pulled); the
+    // Pull or push.  The pull by the bounds costs ~28 B per vertex plus 4 B per
+    // row entry it looks at (as many per vertex as in the last batch that
+    // pulled; by row tails 32 B and those past the tail, about the same); the
     // push at most 12 B per entry of the candidate rows plus the 8 B per
     // vertex of its finalising pass.  With cand_push 0 the push is taken
     // when that bound is under half the pull's estimate (sparse candidate
@@ -5118,9 +5119,12 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       const double pull_b = (28.0 + 4.0 * c->pull_visit_ratio) * (double)n;
       if (2.0 * push_b < pull_b) use_pull = false;
     }
-    // Row tails where the rows are too many for L2 to hold what the pull reads
-    // (made once per base; on smaller graphs the rows' ends come from L2: at
-    // 10^6 vertices of degree 20 the pull took 60 us without and 70 us with them).
+    // Row tails (made once per base) save the rows' ends in DRAM, one sector
+    // each; where the row array fits in L2 the ends come from there and the tails
+    // only add reads.  Measured: 80 MB of rows (10^6 vertices of degree 20) 60 us
+    // without, 70 us with them; 134 MB (R-MAT scale 20) 1.36x faster batches with
+    // them, 0.5 GB (scale 22) 168 against 71 us.  The line is drawn at the vertices,
+    // which set what the tails cost; degrees far from 16 to 32 were not measured.
     const bool tails = use_pull && n >= kTailsMin;
     if (tails && c->tails.cap < 4 * (int64_t)n) {
       c->tails.reserve(4 * (int64_t)n);
@@ -5158,9 +5162,12 @@ void process_batch(mf_ctx* c, const BatchIn& in, int64_t m) {
       else MF_K(launch_pdl(k_pull_cand, grid_for(n), kTB, 0, s, pa));
       if (c->max_row > c->tune.pull_long)
         MF_K(launch_pdl(k_pull_cand_long, lb_grid(c, k_pull_cand_long), kTB, 0, s, pa));
-      // per vertex: row bounds (8 B of nindex, 8 B of aoff), tombstone count,
-      // tag and id (4 B each); the row entries read are counted on the device
-      if (c->profile) c->stage_bytes[kStPull] += 28.0 * (double)n;
+      // Per vertex, by the bounds: 8 B of nindex, 8 B of aoff, tombstone count,
+      // tag or new id, id (4 B each), and the row entries read, counted on the
+      // device.  By row tails: 8 B of aoff, 16 B of tail, tombstone count, tag or
+      // new id; not counted are the rows read past their tails and the ids
+      // written, so this is a lower bound.
+      if (c->profile) c->stage_bytes[kStPull] += (tails ? 32.0 : 28.0) * (double)n;
     } else {
       if (short_rows) {
         sc.emplace(c, kStPushHop);

@@ -498,3 +498,20 @@ def test_pairs_of_many_updates(gb, m, shuffled):
             assert np.array_equal(g.row(5), orc.row(5)), batch
             assert np.array_equal(g.get_mis(), orc.get_mis()), batch
             assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), batch
+
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20])
+def test_pull_bytes_of_the_profile(gb, n):
+    """By row tails 32 B a vertex and nothing twice; by the bounds 28 B and four for each row entry looked at."""
+    nindex, nlist = W.er_graph(n, 5, 7)
+    with gb.Graph.from_csr(nindex, nlist) as g:
+        g.set_tuning(cand_push=2)
+        g.set_mis(g.greedy_mis())
+        g.profile(1)
+        g.apply_batch(*W.ToggleStream(n, nindex, nlist, 3).next_batch(2000, with_flags=True))
+        _, calls, nbytes = g.profile_read()["pull"]
+    assert calls > 0
+    if n >= 1 << 20:
+        assert nbytes == 32.0 * n * calls
+    else:
+        assert 28.0 * n * calls < nbytes < (28.0 * n + 4.0 * nlist.size) * calls
