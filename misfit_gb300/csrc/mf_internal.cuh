@@ -306,45 +306,6 @@ __device__ __forceinline__ bool thread_row_until(const GraphView& g, int32_t x, 
   return false;
 }
 
-// Warp-cooperative: first element y of row(x) (in order) with pred(y),
-// returned in *hit; false when none.  All lanes must call it.
-template <class P>
-__device__ __forceinline__ bool warp_row_first(const GraphView& g, int32_t x, P pred, int32_t* hit) {
-  const int lane = threadIdx.x & 31;
-  const int64_t b = g.nindex[x], e = g.nindex[x + 1];
-  const bool filt = g.dead[x] != 0;
-  for (int64_t k0 = b; k0 < e; k0 += 32) {
-    const int64_t k = k0 + lane;
-    int32_t y = -1;
-    bool ok = false;
-    if (k < e) {
-      y = __ldg(g.nlist + k);
-      ok = (!filt || live_at(g.live, k)) && pred(y);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (m) {
-      *hit = __shfl_sync(0xffffffffu, y, __ffs(m) - 1);
-      return true;
-    }
-  }
-  const int64_t ab = g.aoff[x], ae = g.aoff[x + 1];
-  for (int64_t k0 = ab; k0 < ae; k0 += 32) {
-    const int64_t k = k0 + lane;
-    int32_t y = -1;
-    bool ok = false;
-    if (k < ae) {
-      y = g.aadj[k];
-      ok = pred(y);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (m) {
-      *hit = __shfl_sync(0xffffffffu, y, __ffs(m) - 1);
-      return true;
-    }
-  }
-  return false;
-}
-
 // Warp-cooperative for-each over row(x) (no order guarantee between lanes).
 template <class F>
 __device__ __forceinline__ void warp_row_each(const GraphView& g, int32_t x, F f) {
@@ -708,8 +669,6 @@ struct mf_ctx {
   mf::DBuf<uint32_t> vals;
   mf::DBuf<int32_t> prev;       // previous edge index per endpoint slot
   mf::DBuf<int64_t> i64a, i64b; // scans
-  mf::DBuf<int32_t> i32a, i32b, i32c;
-  mf::DBuf<uint8_t> u8a;
   // overlay rebuild
   mf::DBuf<int32_t> adelta;     // change of each vertex's added count; zero between batches
   mf::DBuf<uint8_t> akill;      // added entries that go; zero between batches
@@ -860,7 +819,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->plan_cuts); f(c->plan_ests); f(c->plan_send); f(c->plan_pos); f(c->atail); f(c->txt_begin); f(c->txt);
   f(c->n2cache); f(c->n2bound); f(c->un_cnt); f(c->counters); f(c->lb_offs);
   f(c->nlist); f(c->dead); f(c->rcnt); f(c->deg); f(c->aadj); f(c->aown); f(c->aadj_alt); f(c->aown_alt);
-  f(c->cid); f(c->v2i); f(c->v2i_b); f(c->seeds_b); f(c->f1); f(c->bu); f(c->bv); f(c->prev); f(c->i32a); f(c->i32b); f(c->i32c);
+  f(c->cid); f(c->v2i); f(c->v2i_b); f(c->seeds_b); f(c->f1); f(c->bu); f(c->bv); f(c->prev);
   f(c->adelta); f(c->seeds); f(c->cands); f(c->hlist); f(c->touched); f(c->rowcid);
   f(c->rp_w0); f(c->rp_w1); f(c->rp_n0); f(c->rp_n1); f(c->big_r); f(c->heavy_slot); f(c->heavy_list);
   f(c->pull_long); f(c->tails); f(c->plan_edges); f(c->seeds_all); f(c->rq_idx); f(c->rq_v);
@@ -869,7 +828,7 @@ void for_each_buffer(mf_ctx* c, F&& f) {
   f(c->live); f(c->bval); f(c->wval); f(c->vals); f(c->vals_b); f(c->slot_vals); f(c->rp_vals); f(c->rp_vals2);
   f(c->bitmaps); f(c->heavy_bits); f(c->dense_bits); f(c->pbits); f(c->n2stamp);
   f(c->n2bstamp); f(c->cidbits);
-  f(c->mis); f(c->bins); f(c->u8a); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
+  f(c->mis); f(c->bins); f(c->akill); f(c->app_line); f(c->creates); f(c->rp_u8); f(c->plan_flags);
   f(c->xst); f(c->xleave); f(c->cta_vert); f(c->cta_ws);
   f(c->keys); f(c->slot_keys); f(c->rp_keys); f(c->rp_keys2);
   f(c->big_best); f(c->fpos); f(c->work);
