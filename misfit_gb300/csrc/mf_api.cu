@@ -1,5 +1,6 @@
 // mf_api.cu -- extern "C" entry points of libmisfit_gb and the host-side file
 // formats (.egr, MIS file, batch folder).
+#include <cuda.h>
 #include <fcntl.h>
 #include <sys/stat.h>
 #include <unistd.h>
@@ -344,6 +345,38 @@ mf::BatchIn copied_input(mf_ctx* c, const int32_t* u, const int32_t* v, const ui
     MF_CUDA(cudaMemcpyAsync(c->bins.p, ins, (size_t)m, kind, s));
   }
   return {c->bu.p, c->bv.p, c->bins.p};
+}
+
+// Whether a kernel on the context's GPU may read `bytes` bytes at p in place:
+// memory of that GPU, all of it within one allocation, on a word boundary.
+// Anything else goes through a copy, which takes every address that CUDA
+// knows and reports the others.
+bool reads_in_place(const mf_ctx* c, const void* p, size_t bytes, size_t word) {
+  using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found{};
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &fn, 12000, cudaEnableDefault, &found) !=
+            cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      fn = nullptr;
+    }
+    return reinterpret_cast<Query>(fn);
+  }();
+  if (query == nullptr || reinterpret_cast<uintptr_t>(p) % word != 0) return false;
+  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  unsigned type = 0, managed = 0;
+  int device = -1;
+  unsigned long long start = 0;
+  size_t size = 0;
+  void* got[] = {&type, &device, &managed, &start, &size};
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  if (query(5, what, got, at) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_DEVICE && managed == 0 && device == c->device && at >= start &&
+         at - start <= size && bytes <= size - (at - start);
 }
 
 // Host lines of a batch where the device can read them: a small batch in the
@@ -796,9 +829,12 @@ int mf_apply_batch_device(mf_ctx* c, const int32_t* d_u, const int32_t* d_v, con
     need(c && m >= 0 && (m == 0 || (d_u && d_v && d_ins)), MF_EINVAL, "bad arguments");
     need(!c->pending, MF_EINVAL, "asynchronous batches are pending; collect them (mf_collect / mf_sync) first");
     bind(c);
-    // copied, so that any address that a copy can read will do: kernels would
-    // need 4-byte alignment and memory of this GPU
-    run_batch(c, copied_input(c, d_u, d_v, d_ins, m, cudaMemcpyDeviceToDevice), m);
+    const size_t words = sizeof(int32_t) * (size_t)m;
+    if (reads_in_place(c, d_u, words, sizeof(int32_t)) && reads_in_place(c, d_v, words, sizeof(int32_t)) &&
+        reads_in_place(c, d_ins, (size_t)m, 1))
+      run_batch(c, mf::BatchIn{d_u, d_v, d_ins}, m);
+    else
+      run_batch(c, copied_input(c, d_u, d_v, d_ins, m, cudaMemcpyDeviceToDevice), m);
   });
 }
 

@@ -183,10 +183,10 @@ __global__ void k_prev(const uint64_t* keys, const uint32_t* vals, int64_t cnt, 
 
 // A small batch's input in one launch: block 0 stages and checks the lines and
 // groups the pairs, block 1 sorts the endpoint slots and finds the previous
-// occurrences.  Both read the lines where they were staged (pinned host
-// memory, or the context's arrays).  Latency of one block's sort bounds it; as separate
-// launches (three copies, a check, key kernels, three sorts, k_prev) the same
-// work took 16 launches and two round trips to the host.
+// occurrences.  Both read the lines where they are (pinned host memory, the
+// caller's device arrays, or the context's).  Latency of one block's sort bounds
+// it; as separate launches (three copies, a check, key kernels, three sorts,
+// k_prev) the same work took 16 launches and two round trips to the host.
 template <int Items>
 __global__ void __launch_bounds__(1024) k_small_input(BatchIn in, int m, int32_t n, int nbits, int gbits, int32_t* u,
                                                       int32_t* v, uint8_t* ins, uint8_t* app_line, uint64_t* pair_keys,
