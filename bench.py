@@ -51,9 +51,10 @@ UNIT = "updates/s"
 # printed with MISFIT_GB_DEBUG=2).  ncu flushes the caches before each
 # launch, so this is a cold-L2 figure; 12 bytes per element are algorithmic.
 PUSH_HOP_DRAM_BYTES_PER_ELEMENT = 13.95
-# DRAM bytes (read + write) per launch of k_pull_tails on this workload, by ncu
-# (None: not captured).
-PULL_DRAM_BYTES_PER_LAUNCH = None
+# DRAM bytes (read + write) per vertex of k_pull_tails, measured by ncu on the
+# same generator's R-MAT scale 20 (three launches of the timed batch: 48,225,365
+# read and 73,387 written over 1,048,576 vertices; cold L2).
+PULL_DRAM_BYTES_PER_VERTEX = 46.06
 
 
 def parse_args():
@@ -922,13 +923,14 @@ def main():
     if ms_p > 0:
         ach_p = bytes_p / (ms_p / 1e3) / 1e9
         pull = {"bound": "hbm", "achieved": ach_p, "peak": peak, "unit": "GB/s", "frac": ach_p / peak,
-                "traffic": PULL_DRAM_BYTES_PER_LAUNCH, "kernel": "k_pull_tails", "peak_kind": peak_kind,
+                "traffic": PULL_DRAM_BYTES_PER_VERTEX * n, "kernel": "k_pull_tails", "peak_kind": peak_kind,
                 "algorithmic_bytes_per_launch": bytes_p / max(calls_p, 1), "avg_launch_ms": ms_p / max(calls_p, 1),
                 "launches": int(calls_p),
                 "timed": "per sub-batch: k_pull_tails and k_pull_cand_long (the pull step)",
                 "bytes_note": "32 B per vertex (8 B added-entry offset, 16 B row tail, 4 B tombstone count, 4 B tag or "
                               "new id); rows read past their tails and ids written are not counted",
-                "traffic_note": "DRAM bytes per launch of k_pull_tails from an ncu capture of this workload" if PULL_DRAM_BYTES_PER_LAUNCH else "not captured"}
+                "traffic_note": "DRAM bytes per vertex of k_pull_tails from an ncu capture at R-MAT scale 20 (cold "
+                                "L2), times this workload's vertices"}
         push_hop = roof
         if ms_p > ms:
             roof = dict(pull, batch=push_hop.pop("batch"), batch_frac=push_hop.pop("batch_frac"))
