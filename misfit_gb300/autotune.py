@@ -3,7 +3,9 @@
 The batched step's knobs (mf_batched_opts): the persistent kernel's block
 size, its CTAs per SM, the two limits that decide which batches it carries
 (lines per batch, vertices per graph) -- everything above them takes the
-multi-launch path concurrently -- and the host threads of that path.  Which setting is fastest depends on the
+multi-launch path concurrently, and up to the library's own limits so do the
+batches that this path ends sooner -- and the host threads of that path.
+Which setting is fastest depends on the
 GPU and on the mix of graph and batch sizes, so the tuner measures: it runs
 the caller's step once per candidate setting, each time on fresh contexts
 from the same initial state, and keeps the fastest.  Every candidate must

@@ -279,7 +279,7 @@ struct PairState {
 
 // Live and dead copies of y in the base positions [k, e) of an unsorted row: read
 // whole, a hub's of 10^4 entries by one thread, so eight loads are in flight (one
-// at a time a batch on unsorted R-MAT scale 17 took 4.7 ms; so 3.8).
+// at a time a batch on unsorted R-MAT scale 17 took 4.7 ms; so 3.7).
 __device__ __noinline__ int2 unsorted_copies(const int32_t* nlist, const uint32_t* live, int64_t k, int64_t e, int32_t y) {
   constexpr int kStep = 8;
   int2 c = make_int2(0, 0);
@@ -371,7 +371,7 @@ __device__ __forceinline__ void pair_update(PairWalk& w, bool insert, bool base_
 
 // The pair's further updates, from position j of its run on, four read at a
 // time: thousands of them are one thread's work (100,000 of one pair took
-// 25.3 ms one at a time; so 20.1).  Seldom reached, so it stays out of line.
+// 25.3 ms one at a time; so 18.6).  Seldom reached, so it stays out of line.
 __device__ __noinline__ PairWalk pair_updates(PairWalk w, const uint64_t* keys, const uint32_t* vals, int64_t j,
                                               int64_t m, int gbits, uint64_t key, const int32_t* u, const uint8_t* ins,
                                               int32_t a, bool in_base_ab, bool in_base_ba) {
