@@ -111,3 +111,64 @@ def test_first_batch_allocates_in_groups(gpu_lib, kind):
         before = native.allocations()
         g.apply_batch(*W.ToggleStream(nindex.size - 1, nindex, nlist, 6).next_batch(m, with_flags=True))
         assert native.allocations() - before <= 40
+
+
+@pytest.mark.parametrize("kind", ["short", "long", "many", "wide"])
+def test_refused_allocations_of_a_later_larger_batch(gpu_lib, monkeypatch, kind):
+    """The same for the second batch of a context, three times the first: its buffers grow, and what must be zero or
+    mapped nowhere between batches stands in some of them."""
+    nindex, nlist, m, max_csr, push = _case(kind)
+    n = nindex.size - 1
+    mis0 = O.greedy_mis(nindex, nlist)
+    stream = W.ToggleStream(n, nindex, nlist, 7)
+    small = stream.next_batch(m // 3, with_flags=True)
+    large = stream.next_batch(m, with_flags=True)
+    u, v = stream.next_batch(m // 2)
+
+    def start(x):
+        if max_csr:
+            x.max_csr = max_csr
+        x.set_mis(mis0)
+        x.apply_batch(*small)
+
+    monkeypatch.delenv("MISFIT_GB_FAIL_ALLOC", raising=False)
+    with native.Graph.from_csr(nindex, nlist) as g:
+        opened = native.allocations()
+        start(g)
+        k = native.allocations() - opened - 4   # the first batch's, some of which do not count for the refusal
+    refused = 0
+    while True:
+        k += 1
+        monkeypatch.setenv("MISFIT_GB_FAIL_ALLOC", str(k))
+        with native.Graph.from_csr(nindex, nlist) as g:
+            try:
+                start(g)
+            except native.MisfitError:
+                continue   # still the first batch's
+            degrees = g.degrees()
+            try:
+                g.apply_batch(*large)
+                break
+            except native.MisfitError as e:
+                assert e.status == ENOMEM, k
+            refused += 1
+            mis = g.get_mis()
+            assert mis.max() <= 1, k
+            orc = O.Oracle.from_csr(nindex, nlist)
+            start(orc)
+            if not np.array_equal(g.degrees(), degrees):
+                orc.apply_overlay(*large)
+            else:
+                assert np.array_equal(mis, orc.get_mis()) and np.array_equal(g.cluster_ids(), orc.cluster_ids()), k
+            assert np.array_equal(g.degrees(), orc.degrees()), k
+            orc.set_mis(mis)
+            orc.max_csr = g.max_csr
+            g.set_mis(mis)
+            for batch in range(2):
+                ins = orc.flag_updates(u, v)
+                g.apply_batch(u, v, ins)
+                orc.apply_batch(u, v, ins)
+                assert np.array_equal(g.get_mis(), orc.get_mis()), (k, batch)
+                assert np.array_equal(g.cluster_ids(), orc.cluster_ids()), (k, batch)
+                assert np.array_equal(g.degrees(), orc.degrees()), (k, batch)
+    assert refused > 3
